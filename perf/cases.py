@@ -12,6 +12,7 @@ to 2^30 elements) with smaller, odd and ragged ones beside them.
     run(state)          one pass, its outputs
     work(case)          bytes and flops that a pass cannot do without
     tolerance(case)     how far another correct implementation at this precision may be off
+    exact(case, seed)   the outputs of a pass in 64 bits, from plain torch
 """
 
 from __future__ import annotations
@@ -143,7 +144,8 @@ class Block(torch.nn.Module):
 # ---- cases -----------------------------------------------------------------------------------
 
 
-def prepare(case, seed):
+def _inputs(case, seed):
+    """Tensors and weights, made from the seed alone."""
     g = torch.Generator(device="cuda").manual_seed(int(seed))
     dtype = DTYPES[case["dtype"]]
     kind = case["kind"]
@@ -160,16 +162,13 @@ def prepare(case, seed):
         state.update(x=normal(rows, width), b=normal(width, std=0.02), gamma=normal(width, std=0.02, mean=1.0),
                      beta=normal(width, std=0.02), mean=normal(width, std=0.1), var=normal(width, std=0.1).abs() + 1)
     elif kind == "chain":
-        state.update(x=normal(case["rows"], case["width"]), b=normal(case["width"], std=0.02),
-                     fn=torch.compile(chain, backend=compile_graph, dynamic=False))
+        state.update(x=normal(case["rows"], case["width"]), b=normal(case["width"], std=0.02))
     elif kind == "sweep":
-        state.update(a=uniform(case["n"]), b=uniform(case["n"]), to=torch.bfloat16 if dtype == torch.float32 else torch.float32,
-                     fn=torch.compile(six_op_chain, backend=compile_graph, dynamic=False))
+        state.update(a=uniform(case["n"]), b=uniform(case["n"]), to=torch.bfloat16 if dtype == torch.float32 else torch.float32)
     elif kind in ("rows", "view"):
         extent = case["width"] if kind == "rows" else case["rows"]
         state.update(x=normal(case["rows"], case["width"]), gamma=normal(extent, std=0.02, mean=1.0), beta=normal(extent, std=0.02))
     elif kind == "gemm":
-        ops.register_custom_ops()
         m, k, n = case["m"], case["k"], case["n"]
         # a Linear's weight is [n, k]; unit-variance results put the GELU where it bends
         state.update(x=normal(m, k), w=normal(n, k, std=k ** -0.5), bias=normal(n, std=0.02))
@@ -187,8 +186,18 @@ def prepare(case, seed):
             p.copy_(normal(*p.shape, std=0.02, to=torch.float32))
         for norm in (block.ln1, block.ln2):
             norm.weight.add_(1.0)
-        block = block.to(dtype)
-        state.update(x=normal(case["batch"], case["tokens"], d), fn=torch.compile(block, backend=compile_graph, dynamic=False))
+        state.update(x=normal(case["batch"], case["tokens"], d), block=block.to(dtype))
+    return state
+
+
+def prepare(case, seed):
+    state = _inputs(case, seed)
+    kind = state["kind"]
+    if kind == "gemm":
+        ops.register_custom_ops()
+    elif kind in ("chain", "sweep", "block"):
+        function = {"chain": chain, "sweep": six_op_chain}.get(kind) or state["block"]
+        state["fn"] = torch.compile(function, backend=compile_graph, dynamic=False)
     return state
 
 
@@ -272,3 +281,46 @@ def tolerance(case):
         return {"rel": 1e-5, "max": 1e-5} if case["kind"] == "sweep" else {"rel": 2e-6, "max": 1e-5}
     scale = 1.0 if case["dtype"] == "bf16" else 0.125
     return {"rel": 1e-2 * scale, "max": 0.1 * scale}
+
+
+def _six_exact(x, gamma, beta):
+    # argmax picks among equal values by its own rule: its result is whole and is compared as such
+    return {"sum": x.sum(-1), "mean": x.mean(-1), "amax": x.amax(-1), "argmax": None, "softmax": torch.softmax(x, -1),
+            "layer_norm": F.layer_norm(x, [x.shape[-1]], gamma, beta, EPS)}
+
+
+def exact(case, seed):
+    state = _inputs(case, seed)
+    kind = state["kind"]
+    s = {name: value.double() for name, value in state.items() if isinstance(value, torch.Tensor)}
+    with torch.no_grad():
+        if kind == "eager":
+            y = F.gelu(s["x"] + s["b"], approximate="tanh")
+            out = {"y": y, "scaled": y * 0.5, "packed": y.t().contiguous()}
+            out["batch_norm"] = F.batch_norm(y, s["mean"], s["var"], s["gamma"], s["beta"], False, 0.0, EPS)
+            out.update(_six_exact(y, s["gamma"], s["beta"]))
+            return out
+        if kind == "chain":
+            return chain(s["x"], s["b"])
+        if kind == "sweep":
+            return {"chain": six_op_chain(s["a"], s["b"], torch.float64), "sum": s["a"].sum(), "amax": s["a"].amax()}
+        if kind == "rows":
+            return _six_exact(s["x"], s["gamma"], s["beta"])
+        if kind == "view":
+            view = s["x"].t()
+            return dict(_six_exact(view, s["gamma"], s["beta"]), packed=view.contiguous())
+        if kind == "gemm":
+            y = F.linear(s["x"], s["w"], s["bias"])
+            act = case["act"]
+            return y if act == "none" else F.gelu(y, approximate="tanh" if act == "tanh" else "none")
+        if kind == "attention":
+            outs = []
+            for q, k, v in zip(s["q"], s["k"], s["v"]):     # one sequence after another: the scores of all are large
+                scores = (q @ k.transpose(-1, -2)) / case["head"] ** 0.5
+                if case["causal"]:
+                    n = scores.shape[-1]
+                    scores = scores.masked_fill(~torch.ones(n, n, dtype=torch.bool, device=q.device).tril(), float("-inf"))
+                outs.append(torch.softmax(scores, -1) @ v)
+            return torch.stack(outs)
+        block = state["block"].double()
+        return torch.cat([block(part) for part in s["x"].split(4)])
