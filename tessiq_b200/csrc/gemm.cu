@@ -2,19 +2,30 @@
 //
 //   C[b] = act(op(A[b]) @ op(B[b]) + bias)      bf16 or f16 operands, f32 accumulation, one rounding
 //
-// One persistent CTA per SM walks 128 x 256 output tiles. Inside a CTA, ten warps have three jobs:
+// Two kernels share the work by shape (choose_tiling): CTA pairs over 256 x 256, 256 x 192 or 256 x 128 tiles
+// (below), and single CTAs over 128 x 128 tiles, several of which may share a tile's K range. In both,
+// persistent CTAs walk the tiles and ten warps of a CTA have three jobs:
 //
-//   warp 0, one lane   producer: TMA loads (cp.async.bulk.tensor, 128-byte swizzle) of a
-//                      128 x 64 slice of A and a 256 x 64 slice of B into a 3-stage ring in
-//                      shared memory, each stage announced on an mbarrier by its byte count;
-//   warp 1, one lane   issuer: for every stage four tcgen05.mma (128 x 256 x 16) accumulating in
+//   warp 0, one lane   producer: TMA loads (cp.async.bulk.tensor, 128-byte swizzle) of a 64-wide slice
+//                      of A and of B into a ring of stages in shared memory, each stage announced on an
+//                      mbarrier by its byte count;
+//   warp 1, one lane   issuer: for every stage four tcgen05.mma (16 elements of K each) accumulating in
 //                      tensor memory; tcgen05.commit hands the stage back to the producer and, after
 //                      the last slice of a tile, hands the accumulator to the epilogue;
 //   warps 2..9         epilogue: tcgen05.ld of the f32 accumulator (each warp 32 lanes of tensor
-//                      memory by half of the columns), + bias, activation in f32, one rounding, a
+//                      memory by every other 64 columns), + bias, activation in f32, one rounding, a
 //                      regrouping through shared memory, whole-line 128-bit stores.
 //
-// Tensor memory holds two 128 x 256 f32 accumulators (all 512 columns), so the epilogue of tile i
+// The lanes that issue are chosen by elect.sync: with `lane == 0` in its place a k-block cost at least 560
+// cycles whatever the tile's width (8192 x 4096 x 4096, 128 columns a pair: 269 us against 182; 192: 209 / 174),
+// which a 256-wide tile hides and a narrow one does not.
+//
+// A product with few rows is a stream of B. 64 x 4096 x 4096 took 35.2 us as 16 tiles of 256 columns on 16 SMs
+// and takes 14.2 as 32 tiles of 128 columns with four CTAs of a cluster on each, which add their partial
+// sums through distributed shared memory (its bytes: 5.4 us; the launch, the first loads and the
+// two cluster barriers are the rest: 768 x 768 with one row takes 6.3).
+//
+// Tensor memory holds two f32 accumulators, so the epilogue of tile i
 // runs under the MMAs of tile i+1. Either operand may be K-major (row-major A, nn.Linear weight
 // [n,k]) or MN-major (A stored [k,m]; B stored [k,n], the `A @ B` form): transposed operands are
 // consumed in place through the shared-memory descriptor's major bit, never copied
@@ -40,9 +51,9 @@ namespace tq {
 namespace {
 
 constexpr int kTileM = 128;
-constexpr int kTileN = 256;
+constexpr int kTileN = 128;   // of the single-CTA kernel; the pair kernel's width is a template parameter
 constexpr int kTileK = 64;    // 64 two-byte elements = one 128-byte swizzle row
-constexpr int kStages = 3;
+constexpr int kStages = 6;
 constexpr int kMmaK = 16;
 constexpr int kThreads = 320;           // producer warp, issuer warp, eight epilogue warps
 constexpr int kEpilogueThreads = 256;
@@ -50,10 +61,11 @@ constexpr int kEpilogueWarps = kEpilogueThreads / 32;
 constexpr int kStoreColumns = 64;       // columns an epilogue warp regroups at a time
 constexpr uint32_t kStoreBytes = 32 * kStoreColumns * 2;   // 4 KiB of staging per epilogue warp
 constexpr uint32_t kBytesA = kTileM * kTileK * 2;   // 16 KiB
-constexpr uint32_t kBytesB = kTileN * kTileK * 2;   // 32 KiB
+constexpr uint32_t kBytesB = kTileN * kTileK * 2;   // 16 KiB
 constexpr uint32_t kStageBytes = kBytesA + kBytesB;
 constexpr uint32_t kChunkBytes = 64 * kTileK * 2;   // one 64-wide MN chunk of an MN-major operand: 8 KiB
-constexpr uint32_t kTmemColumns = 512;
+constexpr uint32_t kTmemColumns = 2 * kTileN;       // two accumulators
+constexpr int kMaxSplit = 8;                        // CTAs of a cluster that share one tile's K range
 
 constexpr size_t kSmemBytes = 1024 /*alignment slack*/ + static_cast<size_t>(kStages) * kStageBytes +
                               2 * kTileN * sizeof(float) /*bias*/ + 256 /*barriers, tmem slot*/ + kEpilogueWarps * kStoreBytes;
@@ -63,6 +75,8 @@ enum WaitCode { kWaitEmpty = 101, kWaitFull = 102, kWaitTmemEmpty = 103, kWaitTm
 struct GemmParams {
   int m, n, k, batch;
   int tiles_m, tiles_n;
+  int split;                       // CTAs of a cluster that share a tile's K range (single-CTA kernel)
+  int a_rows;                      // rows of A a stage loads (single-CTA kernel): fewer than a tile has where m is smaller
   long long num_tiles;
   const void* bias;
   const void* residual;            // added after the activation, or null
@@ -75,19 +89,9 @@ struct GemmParams {
 
 // Instruction descriptor of tcgen05.mma kind::f16: f32 accumulator, A/B format (0 f16, 1 bf16),
 // major bits (0 K-major, 1 MN-major), N >> 3 at bit 17, M >> 4 at bit 24.
-__host__ __device__ constexpr uint32_t instruction_descriptor(bool bf16, bool a_mn_major, bool b_mn_major) {
+__host__ __device__ constexpr uint32_t instruction_descriptor(bool bf16, bool a_mn_major, bool b_mn_major, int m, int n) {
   return (1u << 4) | ((bf16 ? 1u : 0u) << 7) | ((bf16 ? 1u : 0u) << 10) | ((a_mn_major ? 1u : 0u) << 15) |
-         ((b_mn_major ? 1u : 0u) << 16) | (static_cast<uint32_t>(kTileN >> 3) << 17) |
-         (static_cast<uint32_t>(kTileM >> 4) << 24);
-}
-
-__device__ __forceinline__ float activate(float v, int activation) {
-  if (activation == TQ_ACT_GELU_TANH) {
-    // 0.5 v (1 + tanh(k (v + 0.044715 v^3))) = v / (1 + exp(-2k (v + 0.044715 v^3)))
-    return v * rcp_ftz(1.0f + exp2_ftz(-2.302208198144325f * (v + 0.044715f * v * v * v)));
-  }
-  if (activation == TQ_ACT_GELU_ERF) return 0.5f * v * (1.0f + erff(v * 0.70710678118654752440f));
-  return v;
+         ((b_mn_major ? 1u : 0u) << 16) | (static_cast<uint32_t>(n >> 3) << 17) | (static_cast<uint32_t>(m >> 4) << 24);
 }
 
 // A barrier of the eight epilogue warps (named barrier 1) that also returns whether `ok` held on every
@@ -105,7 +109,7 @@ __device__ __forceinline__ bool epilogue_all(bool ok) {
   return all != 0;
 }
 
-// The same on two elements at once with the .f32x2 forms of add, mul and fma, and with the
+// The activation of two elements at once with the .f32x2 forms of add, mul and fma, and with the
 // activation a compile-time constant: the epilogue of a short-K product (12 k-blocks at K = 768) is
 // what the CTA waits for, and it is bound by the instructions its eight warps issue.
 template <int ACTIVATION>
@@ -166,6 +170,25 @@ __device__ __forceinline__ uint4 finish_unit(const uint32_t (&r0)[32], const uin
   return *reinterpret_cast<const uint4*>(&out);
 }
 
+// Calls `finish` with the activation and the presence of a residual as compile-time constants.
+template <typename F>
+__device__ __forceinline__ void with_activation(int activation, bool residual, F finish) {
+  auto go = [&](auto activation_tag) {
+    if (residual) {
+      finish(activation_tag, std::true_type{});
+    } else {
+      finish(activation_tag, std::false_type{});
+    }
+  };
+  if (activation == TQ_ACT_GELU_TANH) {
+    go(std::integral_constant<int, TQ_ACT_GELU_TANH>{});
+  } else if (activation == TQ_ACT_GELU_ERF) {
+    go(std::integral_constant<int, TQ_ACT_GELU_ERF>{});
+  } else {
+    go(std::integral_constant<int, TQ_ACT_NONE>{});
+  }
+}
+
 // Tiles in groups of 16 rows of tiles, so that the CTAs running at one time share A and B slices
 // in L2.
 __device__ __forceinline__ void tile_coordinates(long long tile, const GemmParams& p, int& batch, int& tile_m, int& tile_n) {
@@ -181,22 +204,32 @@ __device__ __forceinline__ void tile_coordinates(long long tile, const GemmParam
   tile_n = (t % group_span) / rows;
 }
 
-// One epilogue warp's share of a 128 x 256 accumulator: the 32 rows of its tensor-memory lanes by
-// the 128 columns of its half. Per 64 columns: tcgen05.ld (lane i holds row i), + bias, activation,
-// one rounding, then the 32 x 64 block goes through 4 KiB of this warp's shared memory (16-byte
-// units XOR-swizzled by row, conflict-free both ways) so that each store instruction writes four
-// whole 128-byte lines of C instead of 32 scattered 16-byte pieces. A residual tile (added after
-// the activation, before the one rounding) takes the same road the other way: whole lines from
-// global memory into the staging block, then each thread picks up its own row.
-template <typename T>
+// An element of an epilogue warp's staging block (rows of 64 elements, 16-byte units XOR-swizzled by row).
+__device__ __forceinline__ uint16_t staged_element(uint32_t staging, int row, int column) {
+  uint16_t value;
+  asm volatile("ld.shared.u16 %0, [%1];" : "=h"(value) : "r"(staging + row * 128 + (((column >> 3) ^ (row & 7)) << 4) + (column & 7) * 2) : "memory");
+  return value;
+}
+
+// One epilogue warp's share of a 128 x TILE_N accumulator: the 32 rows of its tensor-memory lanes by
+// every other block of 64 columns, beginning with block `half` (of 192 columns one half gets two blocks
+// and the other one; the caller swaps the halves from tile to tile). Per block: tcgen05.ld (lane i holds
+// row i), + bias, activation, one rounding, then the 32 x 64 block goes through 4 KiB of this warp's
+// shared memory (16-byte units XOR-swizzled by row, conflict-free both ways) so that each store
+// instruction writes four whole 128-byte lines of C instead of 32 scattered 16-byte pieces. A residual
+// tile (added after the activation, before the one rounding) takes the same road the other way: whole
+// lines from global memory into the staging block, then each thread picks up its own row. Where C's rows
+// are not made of aligned 16-byte pieces (an odd n) the staged block is written an element a lane, half a row
+// per instruction, in place of one element of each of 32 rows. (Four-byte pieces from each row's first
+// aligned address were slower: 8192 x 9973 x 768 276 us against 231.)
+template <typename T, int TILE_N>
 __device__ __forceinline__ void epilogue_rows(uint32_t tmem_accumulator, int quarter, int half, int lane, const float* bias_tile,
                                               T* c_tile, long long ldc, const T* residual_tile, long long ldr, int rows_left,
                                               int columns_left, int activation, unsigned char* staging, bool vector_ok) {
-  const int row = quarter * 32 + lane;
   const uint32_t staging_address = smem_address(staging);
 #pragma unroll 1
-  for (int step = 0; step < (kTileN / 2) / kStoreColumns; ++step) {
-    const int column0 = half * (kTileN / 2) + step * kStoreColumns;
+  for (int block = half; block < TILE_N / kStoreColumns; block += 2) {
+    const int column0 = block * kStoreColumns;
     uint4 residual_words[8];
     if (residual_tile != nullptr && vector_ok) {      // issued before the tensor-memory load so the two latencies overlap
       const int unit = lane & 7;
@@ -213,8 +246,8 @@ __device__ __forceinline__ void epilogue_rows(uint32_t tmem_accumulator, int qua
     tmem_load_32(tmem_accumulator + column0 + (static_cast<uint32_t>(quarter * 32) << 16), r0);
     tmem_load_32(tmem_accumulator + column0 + 32 + (static_cast<uint32_t>(quarter * 32) << 16), r1);
     tmem_load_wait();
-    if (vector_ok) {
-      if (residual_tile != nullptr) {
+    if (residual_tile != nullptr) {
+      if (vector_ok) {
         const int unit = lane & 7;
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
@@ -223,73 +256,183 @@ __device__ __forceinline__ void epilogue_rows(uint32_t tmem_accumulator, int qua
                        "r"(residual_words[i].x), "r"(residual_words[i].y), "r"(residual_words[i].z), "r"(residual_words[i].w)
                        : "memory");
         }
-        __syncwarp();
-      }
-      auto finish = [&](auto activation_tag, auto residual_tag) {
-        constexpr int kActivation = decltype(activation_tag)::value;
-        constexpr bool kResidual = decltype(residual_tag)::value;
-#pragma unroll
-        for (int unit = 0; unit < 8; ++unit) {
-          uint4 word = make_uint4(0, 0, 0, 0);
-          if constexpr (kResidual) {
-            asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
-                         : "=r"(word.x), "=r"(word.y), "=r"(word.z), "=r"(word.w)
-                         : "r"(staging_address + lane * 128 + ((unit ^ (lane & 7)) << 4))
-                         : "memory");
-          }
-          word = finish_unit<T, kActivation, kResidual>(r0, r1, bias_tile + column0, unit, word);
-          asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(staging_address + lane * 128 + ((unit ^ (lane & 7)) << 4)),
-                       "r"(word.x), "r"(word.y), "r"(word.z), "r"(word.w)
-                       : "memory");
-        }
-      };
-      auto finish_with = [&](auto activation_tag) {
-        if (residual_tile != nullptr) {
-          finish(activation_tag, std::true_type{});
-        } else {
-          finish(activation_tag, std::false_type{});
-        }
-      };
-      if (activation == TQ_ACT_GELU_TANH) {
-        finish_with(std::integral_constant<int, TQ_ACT_GELU_TANH>{});
-      } else if (activation == TQ_ACT_GELU_ERF) {
-        finish_with(std::integral_constant<int, TQ_ACT_GELU_ERF>{});
       } else {
-        finish_with(std::integral_constant<int, TQ_ACT_NONE>{});
+        const int rows = min(32, rows_left - quarter * 32);
+#pragma unroll 4
+        for (int r = 0; r < rows; ++r) {
+          const T* residual_row = residual_tile + static_cast<long long>(quarter * 32 + r) * ldr + column0;
+          for (int j = lane; j < kStoreColumns && column0 + j < columns_left; j += 32) {
+            *reinterpret_cast<T*>(staging + r * 128 + (((j >> 3) ^ (r & 7)) << 4) + (j & 7) * 2) = residual_row[j];
+          }
+        }
       }
       __syncwarp();
+    }
+    // (the eight units are worked out side by side and stored afterwards: a store between them would order
+    // each unit's bias reads behind the one before, and the chain of a unit is what a warp waits for)
+    auto finish = [&](auto activation_tag, auto residual_tag) {
+      constexpr int kActivation = decltype(activation_tag)::value;
+      constexpr bool kResidual = decltype(residual_tag)::value;
+      uint4 words[8];
+#pragma unroll
+      for (int unit = 0; unit < 8; ++unit) {
+        words[unit] = make_uint4(0, 0, 0, 0);
+        if constexpr (kResidual) {
+          asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
+                       : "=r"(words[unit].x), "=r"(words[unit].y), "=r"(words[unit].z), "=r"(words[unit].w)
+                       : "r"(staging_address + lane * 128 + ((unit ^ (lane & 7)) << 4))
+                       : "memory");
+        }
+      }
+#pragma unroll
+      for (int unit = 0; unit < 8; ++unit) words[unit] = finish_unit<T, kActivation, kResidual>(r0, r1, bias_tile + column0, unit, words[unit]);
+#pragma unroll
+      for (int unit = 0; unit < 8; ++unit) {
+        asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(staging_address + lane * 128 + ((unit ^ (lane & 7)) << 4)),
+                     "r"(words[unit].x), "r"(words[unit].y), "r"(words[unit].z), "r"(words[unit].w)
+                     : "memory");
+      }
+    };
+    with_activation(activation, residual_tile != nullptr, finish);
+    __syncwarp();
+    if (vector_ok) {
       const int unit = lane & 7;
       if (column0 + unit * 8 < columns_left) {
+        uint4 words[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
           const int r = i * 4 + (lane >> 3);
-          uint4 word;
           asm volatile("ld.shared.v4.b32 {%0, %1, %2, %3}, [%4];"
-                       : "=r"(word.x), "=r"(word.y), "=r"(word.z), "=r"(word.w)
+                       : "=r"(words[i].x), "=r"(words[i].y), "=r"(words[i].z), "=r"(words[i].w)
                        : "r"(staging_address + r * 128 + ((unit ^ (r & 7)) << 4))
                        : "memory");
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int r = i * 4 + (lane >> 3);
           if (quarter * 32 + r < rows_left) {
-            *reinterpret_cast<uint4*>(c_tile + static_cast<long long>(quarter * 32 + r) * ldc + column0 + unit * 8) = word;
+            *reinterpret_cast<uint4*>(c_tile + static_cast<long long>(quarter * 32 + r) * ldc + column0 + unit * 8) = words[i];
           }
         }
       }
-      __syncwarp();
-    } else if (row < rows_left) {
-      T* c_row = c_tile + static_cast<long long>(row) * ldc + column0;
-      const T* residual_row = residual_tile == nullptr ? nullptr : residual_tile + static_cast<long long>(row) * ldr + column0;
+    } else {
+      const int rows = min(32, rows_left - quarter * 32), columns = columns_left - column0;
+#pragma unroll 1
+      for (int r0 = 0; r0 < rows; r0 += 8) {
+        uint16_t low[8], high[8];      // all eight rows are read before the first is written: the compiler must not order one by one
 #pragma unroll
-      for (int j = 0; j < 64; ++j) {
-        if (column0 + j < columns_left) {
-          float value = activate(__uint_as_float(j < 32 ? r0[j] : r1[j - 32]) + bias_tile[column0 + j], activation);
-          if (residual_row != nullptr) value += to_compute(residual_row[j]);
-          c_row[j] = from_compute<T, float>(value);
+        for (int i = 0; i < 8; ++i) {
+          low[i] = staged_element(staging_address, r0 + i, lane);
+          high[i] = staged_element(staging_address, r0 + i, lane + 32);
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          uint16_t* c_row = reinterpret_cast<uint16_t*>(c_tile + static_cast<long long>(quarter * 32 + r0 + i) * ldc + column0);
+          if (r0 + i < rows && lane < columns) c_row[lane] = low[i];
+          if (r0 + i < rows && lane + 32 < columns) c_row[lane + 32] = high[i];
         }
       }
     }
+    __syncwarp();
   }
 }
 
-template <typename T, bool A_MN, bool B_MN>
+// The end of a tile whose K range was shared by the CTAs of a cluster: every CTA sends each other one its
+// share of the columns as f32 partial sums, through distributed shared memory into the (now idle) stage
+// ring, 16-byte units in the order [sender][column / 4][row] so that a warp's store is one 512-byte run.
+__device__ __forceinline__ void push_partials(uint32_t tmem_accumulator, int quarter, int half, int lane, uint32_t ring, uint32_t rank, int split,
+                                              int rows_left) {
+  const int row = quarter * 32 + lane;
+  const int owned_units = kTileN / 4 / split;             // a power of two: kTileN, split are
+#pragma unroll
+  for (int step = 0; step < 2; ++step) {
+    const int column0 = half * 64 + step * 32;
+    uint32_t r[32];
+    tmem_load_32(tmem_accumulator + column0 + (static_cast<uint32_t>(quarter * 32) << 16), r);
+    tmem_load_wait();
+    if (row < rows_left) {
+#pragma unroll
+      for (int u = 0; u < 8; ++u) {
+        const int unit = column0 / 4 + u;
+        const uint32_t owner = unit / owned_units;
+        const uint32_t local = ring + ((rank * owned_units + unit % owned_units) * kTileM + row) * 16;
+        asm volatile("st.shared::cluster.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(peer_address(local, owner)), "r"(r[4 * u]), "r"(r[4 * u + 1]),
+                     "r"(r[4 * u + 2]), "r"(r[4 * u + 3])
+                     : "memory");
+      }
+    }
+    __syncwarp();
+  }
+}
+
+// Then each CTA adds the partial sums of its own columns in the order of the senders, sixteen columns of
+// a row per thread, and finishes them.
+template <typename T>
+__device__ __forceinline__ void finish_split(uint32_t ring, uint32_t rank, int split, int epilogue_thread, const float* bias_tile, T* c_tile, long long ldc,
+                                             const T* residual_tile, long long ldr, int rows_left, int columns_left, int activation, bool vector_ok) {
+  const int owned = kTileN / split;                       // 16, 32 or 64 columns
+  for (int item = epilogue_thread; item < kTileM * (owned / 16); item += kEpilogueThreads) {
+    const int row = item % kTileM, local0 = (item / kTileM) * 16;
+    const int column0 = static_cast<int>(rank) * owned + local0;
+    if (row >= rows_left || column0 >= columns_left) continue;
+    float2 sum[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) sum[j] = make_float2(0.f, 0.f);
+    for (int sender = 0; sender < split; ++sender) {
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        float4 part;
+        asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                     : "=f"(part.x), "=f"(part.y), "=f"(part.z), "=f"(part.w)
+                     : "r"(ring + ((sender * (owned / 4) + local0 / 4 + u) * kTileM + row) * 16)
+                     : "memory");
+        sum[2 * u] = __fadd2_rn(sum[2 * u], make_float2(part.x, part.y));
+        sum[2 * u + 1] = __fadd2_rn(sum[2 * u + 1], make_float2(part.z, part.w));
+      }
+    }
+    uint32_t r[32];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) r[j] = __float_as_uint(j % 2 ? sum[j / 2].y : sum[j / 2].x);
+    T* c = c_tile + static_cast<long long>(row) * ldc + column0;
+    const T* residual = residual_tile == nullptr ? nullptr : residual_tile + static_cast<long long>(row) * ldr + column0;
+    auto finish = [&](auto activation_tag, auto residual_tag) {
+      constexpr int kActivation = decltype(activation_tag)::value;
+      constexpr bool kResidual = decltype(residual_tag)::value;
+#pragma unroll
+      for (int unit = 0; unit < 2; ++unit) {
+        if (column0 + unit * 8 >= columns_left) break;
+        uint4 word = make_uint4(0, 0, 0, 0);
+        Vec<T, 8>& elements = reinterpret_cast<Vec<T, 8>&>(word);
+        if (vector_ok) {
+          if constexpr (kResidual) word = __ldg(reinterpret_cast<const uint4*>(residual + unit * 8));
+          *reinterpret_cast<uint4*>(c + unit * 8) = finish_unit<T, kActivation, kResidual>(r, r, bias_tile + column0, unit, word);
+        } else {
+          const int count = min(8, columns_left - column0 - unit * 8);
+          if constexpr (kResidual) {
+#pragma unroll
+            for (int j = 0; j < 8; ++j) {
+              if (j < count) elements.v[j] = residual[unit * 8 + j];
+            }
+          }
+          word = finish_unit<T, kActivation, kResidual>(r, r, bias_tile + column0, unit, word);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            if (j < count) c[unit * 8 + j] = elements.v[j];
+          }
+        }
+      }
+    };
+    with_activation(activation, residual != nullptr, finish);
+  }
+}
+
+// Whether C (and the residual) can be written (read) in aligned units of eight columns.
+__device__ __forceinline__ bool whole_units(const GemmParams& p) {
+  return (p.ldc % 8 == 0) && ((reinterpret_cast<uintptr_t>(p.c) & 15) == 0) && (p.stride_c % 8 == 0) && (p.n % 8 == 0) &&
+         (p.residual == nullptr || ((p.ldr % 8 == 0) && ((reinterpret_cast<uintptr_t>(p.residual) & 15) == 0) && (p.stride_r % 8 == 0)));
+}
+
+template <typename T, bool A_MN, bool B_MN, bool SPLIT>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_bias_act_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const GemmParams p) {
   extern __shared__ unsigned char raw_smem[];
@@ -308,7 +451,41 @@ gemm_bias_act_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
-  if (threadIdx.x == 0) {
+  // With SPLIT a cluster of p.split CTAs has one tile, each CTA an even share of its k-blocks; otherwise the
+  // CTAs walk the tiles and take them whole.
+  const uint32_t rank = SPLIT ? cluster_rank() : 0;
+  const long long first_tile = SPLIT ? blockIdx.x / p.split : blockIdx.x;
+  const long long tile_step = SPLIT ? p.num_tiles : gridDim.x;
+  const int all_blocks = (p.k + kTileK - 1) / kTileK;
+  const int first_block = SPLIT ? static_cast<int>(static_cast<long long>(all_blocks) * rank / p.split) : 0;
+  const int k_blocks = (SPLIT ? static_cast<int>(static_cast<long long>(all_blocks) * (rank + 1) / p.split) : all_blocks) - first_block;
+
+  // One stage of the ring: the k-block's slices of A and B.
+  auto load_stage = [&](int s, int kb, int batch, int tile_m, int tile_n) {
+    barrier_expect_tx(full_bar(s), kBytesB + p.a_rows * (kTileK * 2));
+    const uint32_t smem_a = base + s * kStageBytes;
+    const uint32_t smem_b = smem_a + kBytesA;
+    const int k0 = (first_block + kb) * kTileK;
+    if constexpr (A_MN) {
+#pragma unroll
+      for (int i = 0; i < kTileM / 64; ++i) tma_load_3d(smem_a + i * kChunkBytes, &map_a, full_bar(s), tile_m * kTileM + i * 64, k0, batch);
+    } else {
+      tma_load_3d(smem_a, &map_a, full_bar(s), k0, tile_m * kTileM, batch);
+    }
+    if constexpr (B_MN) {
+#pragma unroll
+      for (int i = 0; i < kTileN / 64; ++i) tma_load_3d(smem_b + i * kChunkBytes, &map_b, full_bar(s), tile_n * kTileN + i * 64, k0, batch);
+    } else {
+      tma_load_3d(smem_b, &map_b, full_bar(s), k0, tile_n * kTileN, batch);
+    }
+  };
+
+  // The producer lane sets the barriers up and fills the ring for the first time before the CTA meets, so
+  // that the loads' latency runs under the tensor-memory allocation and the barrier.
+  const int early = min(k_blocks, kStages);
+  if (warp == 0 && elect_one()) {
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&map_a) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&map_b) : "memory");
     if (blockIdx.x == 0) p.status.begin();   // this launch's abort word starts clear
     for (int s = 0; s < kStages; ++s) {
       barrier_init(full_bar(s), 1);
@@ -319,6 +496,9 @@ gemm_bias_act_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
       barrier_init(tmem_empty_bar(a), kEpilogueThreads / 32);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    int batch, tile_m, tile_n;
+    tile_coordinates(first_tile, p, batch, tile_m, tile_n);
+    for (int kb = 0; kb < early; ++kb) load_stage(kb, kb, batch, tile_m, tile_n);
   }
   if (warp == 1) tmem_alloc(tmem_slot, kTmemColumns);
   tcgen05_fence_before();
@@ -326,43 +506,26 @@ gemm_bias_act_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
   tcgen05_fence_after();
   const uint32_t tmem_base = *tmem_slot_pointer;
 
-  const int k_blocks = (p.k + kTileK - 1) / kTileK;
-
   if (warp == 0) {
-    // ---- producer --------------------------------------------------------------------------
-    if (lane == 0) {
-      uint32_t iteration = 0;
+    // ---- producer: what did not fit the first filling ------------------------------------------
+    if (elect_one()) {
+      uint32_t iteration = early;
       bool alive = true;
-      for (long long tile = blockIdx.x; alive && tile < p.num_tiles; tile += gridDim.x) {
+      for (long long tile = first_tile; alive && tile < p.num_tiles; tile += tile_step) {
         int batch, tile_m, tile_n;
         tile_coordinates(tile, p, batch, tile_m, tile_n);
-        for (int kb = 0; kb < k_blocks; ++kb, ++iteration) {
+        for (int kb = tile == first_tile ? early : 0; kb < k_blocks; ++kb, ++iteration) {
           const int s = iteration % kStages;
           const uint32_t phase = (iteration / kStages) & 1;
           if (!barrier_wait(empty_bar(s), phase ^ 1, p.status, kWaitEmpty)) { alive = false; break; }
-          barrier_expect_tx(full_bar(s), kStageBytes);
-          const uint32_t smem_a = base + s * kStageBytes;
-          const uint32_t smem_b = smem_a + kBytesA;
-          const int k0 = kb * kTileK;
-          if constexpr (A_MN) {
-#pragma unroll
-            for (int i = 0; i < kTileM / 64; ++i) tma_load_3d(smem_a + i * kChunkBytes, &map_a, full_bar(s), tile_m * kTileM + i * 64, k0, batch);
-          } else {
-            tma_load_3d(smem_a, &map_a, full_bar(s), k0, tile_m * kTileM, batch);
-          }
-          if constexpr (B_MN) {
-#pragma unroll
-            for (int i = 0; i < kTileN / 64; ++i) tma_load_3d(smem_b + i * kChunkBytes, &map_b, full_bar(s), tile_n * kTileN + i * 64, k0, batch);
-          } else {
-            tma_load_3d(smem_b, &map_b, full_bar(s), k0, tile_n * kTileN, batch);
-          }
+          load_stage(s, kb, batch, tile_m, tile_n);
         }
       }
     }
   } else if (warp == 1) {
     // ---- MMA issuer ------------------------------------------------------------------------
-    if (lane == 0) {
-      constexpr uint32_t idesc = instruction_descriptor(std::is_same_v<T, __nv_bfloat16>, A_MN, B_MN);
+    if (elect_one()) {
+      constexpr uint32_t idesc = instruction_descriptor(std::is_same_v<T, __nv_bfloat16>, A_MN, B_MN, kTileM, kTileN);
       // K-major: 8-row groups are 1024 B apart; a step of 16 along K is 32 B inside the swizzle row.
       // MN-major: 64-wide chunks are kChunkBytes apart, groups of 8 K-rows 1024 B; 16 K-rows = 2048 B.
       constexpr uint32_t lead_a = A_MN ? kChunkBytes : 0, lead_b = B_MN ? kChunkBytes : 0;
@@ -374,7 +537,7 @@ gemm_bias_act_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
       uint32_t s = 0, phase = 0;
       uint32_t local_tile = 0;
       bool alive = true;
-      for (long long tile = blockIdx.x; alive && tile < p.num_tiles; tile += gridDim.x, ++local_tile) {
+      for (long long tile = first_tile; alive && tile < p.num_tiles; tile += tile_step, ++local_tile) {
         const uint32_t acc = local_tile & 1;
         const uint32_t acc_phase = (local_tile >> 1) & 1;
         if (!barrier_wait(tmem_empty_bar(acc), acc_phase ^ 1, p.status, kWaitTmemEmpty)) break;
@@ -396,15 +559,14 @@ gemm_bias_act_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
       }
     }
   } else {
-    // ---- epilogue: warps 2..9; warp w owns tensor-memory lanes 32 (w % 4) .. +31 and the
-    // columns of half (w - 2) / 4 ---------------------------------------------------------------
+    // ---- epilogue: warps 2..9; warp w owns tensor-memory lanes 32 (w % 4) .. +31 and every other
+    // block of 64 columns from block (w - 2) / 4 on ----------------------------------------------
     const int epilogue_thread = threadIdx.x - 64;
     const int quarter = warp & 3, half = (warp - 2) >> 2;
     unsigned char* staging = aligned + kStages * kStageBytes + 2 * kTileN * sizeof(float) + 256 + (warp - 2) * kStoreBytes;
-    const bool vector_ok = (p.ldc % 8 == 0) && ((reinterpret_cast<uintptr_t>(p.c) & 15) == 0) && (p.stride_c % 8 == 0) && (p.n % 8 == 0) &&
-                           (p.residual == nullptr || ((p.ldr % 8 == 0) && ((reinterpret_cast<uintptr_t>(p.residual) & 15) == 0) && (p.stride_r % 8 == 0)));
+    const bool vector_ok = whole_units(p);
     uint32_t local_tile = 0;
-    for (long long tile = blockIdx.x; tile < p.num_tiles; tile += gridDim.x, ++local_tile) {
+    for (long long tile = first_tile; tile < p.num_tiles; tile += tile_step, ++local_tile) {
       int batch, tile_m, tile_n;
       tile_coordinates(tile, p, batch, tile_m, tile_n);
       const uint32_t acc = local_tile & 1;
@@ -420,16 +582,40 @@ gemm_bias_act_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
       // barrier, which also carries the AND of their waits, and all leave together or none does.
       const bool arrived = barrier_wait(tmem_full_bar(acc), acc_phase, p.status, kWaitTmemFull);
       tcgen05_fence_after();
-      if (!epilogue_all(arrived)) break;   // also: bias_tile is complete
-
+      const bool complete = epilogue_all(arrived);     // also: bias_tile is complete
+      if constexpr (!SPLIT) {
+        if (!complete) break;
+      }
       T* c_tile = static_cast<T*>(p.c) + static_cast<long long>(batch) * p.stride_c + static_cast<long long>(tile_m) * kTileM * p.ldc + n0;
       const T* residual_tile = p.residual == nullptr ? nullptr : static_cast<const T*>(p.residual) + static_cast<long long>(batch) * p.stride_r +
                                                                   static_cast<long long>(tile_m) * kTileM * p.ldr + n0;
-      epilogue_rows<T>(tmem_base + acc * kTileN, quarter, half, lane, bias_tile, c_tile, p.ldc, residual_tile, p.ldr, p.m - tile_m * kTileM,
-                       p.n - n0, p.activation, staging, vector_ok);
-      tcgen05_fence_before();
+      const int rows_left = p.m - tile_m * kTileM, columns_left = p.n - n0;
+      if constexpr (SPLIT) {
+        // Every thread of the cluster passes both barriers (the other two warps below), also after a wait
+        // that gave up. After the first all rings are idle: each CTA's MMAs have completed, so they have
+        // read what its loads brought. After the second the partial sums are where they belong.
+        __syncwarp();
+        cluster_sync_all();
+        if (complete) push_partials(tmem_base, quarter, half, lane, base, rank, p.split, rows_left);
+        cluster_sync_all();
+        if (complete) {
+          finish_split<T>(base, rank, p.split, epilogue_thread, bias_tile, c_tile, p.ldc, residual_tile, p.ldr, rows_left, columns_left, p.activation,
+                          vector_ok);
+        }
+      } else {
+        epilogue_rows<T, kTileN>(tmem_base + acc * kTileN, quarter, half, lane, bias_tile, c_tile, p.ldc, residual_tile, p.ldr, rows_left, columns_left,
+                                 p.activation, staging, vector_ok);
+        tcgen05_fence_before();
+        __syncwarp();
+        if (lane == 0) barrier_arrive(tmem_empty_bar(acc));   // this warp has read its part of the accumulator
+      }
+    }
+  }
+  if constexpr (SPLIT) {
+    if (warp < 2) {
       __syncwarp();
-      if (lane == 0) barrier_arrive(tmem_empty_bar(acc));   // this warp has read its part of the accumulator
+      cluster_sync_all();
+      cluster_sync_all();
     }
   }
 
@@ -452,34 +638,40 @@ gemm_bias_act_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
 // bytes of both CTAs' TMA loads (the loads name the leader's barrier; they are plain loads, no
 // multicast); tcgen05.commit reports to the barriers of both CTAs.
 
-constexpr int kPairStages = 5;
+//
+// The tile's width is 256 columns, or 192 or 128 where that leaves fewer SMs idle in the last wave (see
+// choose_tiling): a narrower tile reads A again for every tile of its row and brings fewer products per byte.
+
 constexpr int kPairTileM = 256;
-constexpr uint32_t kPairBytesB = (kTileN / 2) * kTileK * 2;     // 16 KiB: this CTA's half of B
-constexpr uint32_t kPairStageBytes = kBytesA + kPairBytesB;      // 32 KiB per CTA per stage
-constexpr size_t kPairSmemBytes = 1024 + static_cast<size_t>(kPairStages) * kPairStageBytes + 2 * kTileN * sizeof(float) + 256 +
-                                  kEpilogueWarps * kStoreBytes;
 
-__host__ __device__ constexpr uint32_t pair_instruction_descriptor(bool bf16, bool a_mn_major, bool b_mn_major) {
-  return (1u << 4) | ((bf16 ? 1u : 0u) << 7) | ((bf16 ? 1u : 0u) << 10) | ((a_mn_major ? 1u : 0u) << 15) |
-         ((b_mn_major ? 1u : 0u) << 16) | (static_cast<uint32_t>(kTileN >> 3) << 17) |
-         (static_cast<uint32_t>(kPairTileM >> 4) << 24);
-}
+template <int TILE_N>
+struct PairShape {
+  static constexpr uint32_t kBytesB = (TILE_N / 2) * kTileK * 2;     // this CTA's half of B: 16, 12 or 8 KiB
+  static constexpr uint32_t kStageBytes = kBytesA + kBytesB;          // per CTA
+  static constexpr int kStages = TILE_N == 256 ? 5 : TILE_N == 192 ? 6 : 7;
+  static constexpr uint32_t kTmemColumns = TILE_N == 128 ? 256 : 512; // an allocation is a power of two
+  static constexpr size_t kSmemBytes = 1024 + static_cast<size_t>(kStages) * kStageBytes + 2 * TILE_N * sizeof(float) + 256 + kEpilogueWarps * kStoreBytes;
+};
 
-template <typename T, bool A_MN, bool B_MN>
+template <typename T, int TILE_N, bool A_MN, bool B_MN>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_bias_act_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const GemmParams p) {
+  using Shape = PairShape<TILE_N>;
+  constexpr int kPairStages = Shape::kStages;
+  constexpr uint32_t kPairStageBytes = Shape::kStageBytes;
+  static_assert(!B_MN || (TILE_N / 2) % 64 == 0, "an MN-major B comes in chunks of 64 columns per CTA");
   extern __shared__ unsigned char raw_smem[];
   const uint32_t base = (smem_address(raw_smem) + 1023u) & ~1023u;
   unsigned char* aligned = raw_smem + (base - smem_address(raw_smem));
   float* bias_smem = reinterpret_cast<float*>(aligned + kPairStages * kPairStageBytes);
-  const uint32_t barriers = base + kPairStages * kPairStageBytes + 2 * kTileN * sizeof(float);
+  const uint32_t barriers = base + kPairStages * kPairStageBytes + 2 * TILE_N * sizeof(float);
   auto full_bar = [&](int s) { return barriers + 8u * s; };                       // used in the leader only
   auto empty_bar = [&](int s) { return barriers + 8u * (kPairStages + s); };       // one per CTA
   auto tmem_full_bar = [&](int a) { return barriers + 8u * (2 * kPairStages + a); };      // one per CTA
   auto tmem_empty_bar = [&](int a) { return barriers + 8u * (2 * kPairStages + 2 + a); }; // used in the leader only
   const uint32_t tmem_slot = barriers + 8u * (2 * kPairStages + 4);
   volatile uint32_t* tmem_slot_pointer =
-      reinterpret_cast<volatile uint32_t*>(aligned + kPairStages * kPairStageBytes + 2 * kTileN * sizeof(float) + 8 * (2 * kPairStages + 4));
+      reinterpret_cast<volatile uint32_t*>(aligned + kPairStages * kPairStageBytes + 2 * TILE_N * sizeof(float) + 8 * (2 * kPairStages + 4));
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = cluster_rank();           // 0: leader, 1: peer
@@ -487,6 +679,8 @@ gemm_bias_act_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
   const long long pairs = gridDim.x >> 1;
 
   if (threadIdx.x == 0) {
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&map_a) : "memory");
+    asm volatile("prefetch.tensormap [%0];" ::"l"(&map_b) : "memory");
     if (blockIdx.x == 0) p.status.begin();   // this launch's abort word starts clear
     for (int s = 0; s < kPairStages; ++s) {
       barrier_init(full_bar(s), 2);                // one arrive.expect_tx from each CTA's producer
@@ -498,7 +692,7 @@ gemm_bias_act_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
-  if (warp == 1) tmem_alloc_pair(tmem_slot, kTmemColumns);
+  if (warp == 1) tmem_alloc_pair(tmem_slot, Shape::kTmemColumns);
   tcgen05_fence_before();
   __syncthreads();
   cluster_sync_all();                              // the peer's barriers exist before anything signals them
@@ -509,14 +703,14 @@ gemm_bias_act_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
 
   if (warp == 0) {
     // ---- producer (one lane in each CTA) -----------------------------------------------------
-    if (lane == 0) {
+    if (elect_one()) {
       uint32_t iteration = 0;
       bool alive = true;
       for (long long tile = pair; alive && tile < p.num_tiles; tile += pairs) {
         int batch, tile_m, tile_n;
         tile_coordinates(tile, p, batch, tile_m, tile_n);
         const int m0 = tile_m * kPairTileM + static_cast<int>(rank) * kTileM;
-        const int n0 = tile_n * kTileN + static_cast<int>(rank) * (kTileN / 2);
+        const int n0 = tile_n * TILE_N + static_cast<int>(rank) * (TILE_N / 2);
         for (int kb = 0; kb < k_blocks; ++kb, ++iteration) {
           const int s = iteration % kPairStages;
           const uint32_t phase = (iteration / kPairStages) & 1;
@@ -534,7 +728,7 @@ gemm_bias_act_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
           }
           if constexpr (B_MN) {
 #pragma unroll
-            for (int i = 0; i < kTileN / 2 / 64; ++i) tma_load_3d_pair(smem_b + i * kChunkBytes, &map_b, leader_full, n0 + i * 64, k0, batch);
+            for (int i = 0; i < TILE_N / 2 / 64; ++i) tma_load_3d_pair(smem_b + i * kChunkBytes, &map_b, leader_full, n0 + i * 64, k0, batch);
           } else {
             tma_load_3d_pair(smem_b, &map_b, leader_full, k0, n0, batch);
           }
@@ -543,8 +737,8 @@ gemm_bias_act_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
     }
   } else if (warp == 1) {
     // ---- MMA issuer: one lane of the leader CTA, for both ------------------------------------
-    if (lane == 0 && rank == 0) {
-      constexpr uint32_t idesc = pair_instruction_descriptor(std::is_same_v<T, __nv_bfloat16>, A_MN, B_MN);
+    if (rank == 0 && elect_one()) {
+      constexpr uint32_t idesc = instruction_descriptor(std::is_same_v<T, __nv_bfloat16>, A_MN, B_MN, kPairTileM, TILE_N);
       constexpr uint32_t lead_a = A_MN ? kChunkBytes : 0, lead_b = B_MN ? kChunkBytes : 0;
       constexpr uint32_t step_a = A_MN ? 2048 : 32, step_b = B_MN ? 2048 : 32;
       uint32_t local_tile = 0;
@@ -563,7 +757,7 @@ gemm_bias_act_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
         const uint32_t acc_phase = (local_tile >> 1) & 1;
         if (!barrier_wait(tmem_empty_bar(acc), acc_phase ^ 1, p.status, kWaitTmemEmpty)) break;
         tcgen05_fence_after();
-        const uint32_t tmem_d = tmem_base + acc * kTileN;
+        const uint32_t tmem_d = tmem_base + acc * TILE_N;
         uint32_t accumulate = 0;
         for (int kb = 0; kb < k_blocks; ++kb) {
           if (!barrier_wait(full_bar(s), phase, p.status, kWaitFull)) { alive = false; break; }
@@ -583,18 +777,17 @@ gemm_bias_act_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
     // ---- epilogue: this CTA's 128 rows of the pair's tile, eight warps -------------------------
     const int epilogue_thread = threadIdx.x - 64;
     const int quarter = warp & 3, half = (warp - 2) >> 2;
-    unsigned char* staging = aligned + kPairStages * kPairStageBytes + 2 * kTileN * sizeof(float) + 256 + (warp - 2) * kStoreBytes;
-    const bool vector_ok = (p.ldc % 8 == 0) && ((reinterpret_cast<uintptr_t>(p.c) & 15) == 0) && (p.stride_c % 8 == 0) && (p.n % 8 == 0) &&
-                           (p.residual == nullptr || ((p.ldr % 8 == 0) && ((reinterpret_cast<uintptr_t>(p.residual) & 15) == 0) && (p.stride_r % 8 == 0)));
+    unsigned char* staging = aligned + kPairStages * kPairStageBytes + 2 * TILE_N * sizeof(float) + 256 + (warp - 2) * kStoreBytes;
+    const bool vector_ok = whole_units(p);
     uint32_t local_tile = 0;
     for (long long tile = pair; tile < p.num_tiles; tile += pairs, ++local_tile) {
       int batch, tile_m, tile_n;
       tile_coordinates(tile, p, batch, tile_m, tile_n);
       const uint32_t acc = local_tile & 1;
       const uint32_t acc_phase = (local_tile >> 1) & 1;
-      const int n0 = tile_n * kTileN;
-      float* bias_tile = bias_smem + acc * kTileN;
-      for (int j = epilogue_thread; j < kTileN; j += kEpilogueThreads) {
+      const int n0 = tile_n * TILE_N;
+      float* bias_tile = bias_smem + acc * TILE_N;
+      for (int j = epilogue_thread; j < TILE_N; j += kEpilogueThreads) {
         float value = 0.f;
         if (p.bias != nullptr && n0 + j < p.n) value = to_compute(static_cast<const T*>(p.bias)[n0 + j]);
         bias_tile[j] = value;
@@ -609,7 +802,7 @@ gemm_bias_act_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
       T* c_tile = static_cast<T*>(p.c) + static_cast<long long>(batch) * p.stride_c + static_cast<long long>(row0) * p.ldc + n0;
       const T* residual_tile = p.residual == nullptr ? nullptr : static_cast<const T*>(p.residual) + static_cast<long long>(batch) * p.stride_r +
                                                                   static_cast<long long>(row0) * p.ldr + n0;
-      epilogue_rows<T>(tmem_base + acc * kTileN, quarter, half, lane, bias_tile, c_tile, p.ldc, residual_tile, p.ldr, p.m - row0, p.n - n0,
+      epilogue_rows<T, TILE_N>(tmem_base + acc * TILE_N, quarter, half ^ static_cast<int>(acc), lane, bias_tile, c_tile, p.ldc, residual_tile, p.ldr, p.m - row0, p.n - n0,
                        p.activation, staging, vector_ok);
       tcgen05_fence_before();
       __syncwarp();
@@ -624,7 +817,7 @@ gemm_bias_act_pair_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
   cluster_sync_all();
   if (warp == 1) {
     tcgen05_fence_after();
-    tmem_dealloc_pair(tmem_base, kTmemColumns);
+    tmem_dealloc_pair(tmem_base, Shape::kTmemColumns);
   }
 }
 
@@ -650,53 +843,97 @@ tq_status make_map(CUtensorMap* map, tq_dtype dtype, const void* pointer, long l
   return TQ_OK;
 }
 
-template <typename T>
-tq_status launch_pair(bool a_mn, bool b_mn, const CUtensorMap& map_a, const CUtensorMap& map_b, const GemmParams& p, int32_t device, cudaStream_t stream) {
-  auto go = [&](auto kernel) -> tq_status {
-    static std::mutex mutex;
-    {
-      std::lock_guard<std::mutex> lock(mutex);
-      TQ_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kPairSmemBytes)));
+// How a product is cut up: CTA pairs over 256 x tile_n tiles, or single CTAs over 128 x 128 tiles with
+// `split` CTAs of a cluster sharing a tile's K range.
+struct Tiling {
+  bool pair;
+  int tile_n;
+  int split;
+};
+
+// The tiling with the least expected time, in microseconds, from a sweep over m = 1 ... 8192 and seven (k, n)
+// from 768 x 768 to 4096 x 16384 (B200, bf16, + bias + GELU): what a k-block of 64 costs a tile, what a tile
+// costs at least (its epilogue, where K is too short to cover it), and what a launch costs beside its waves.
+// A narrow tile does fewer products per byte it brings from L2 (a 128 x 128 k-block costs 0.23 where half of a
+// 256 x 256 one costs 0.18 per CTA), so it pays only where it saves a wave: 8192 x 3072 x 768 takes 2 waves of
+// 96 wide tiles (45.9 measured) or 2 of 128 tiles of 192 columns (41.0); 8192 x 4096 x 4096 161.8 and 174.0.
+// Sharing a tile's K range pays until the GPU is full: 64 x 4096 x 4096 24.6 alone, 21.2 by 2, 19.3 by 4.
+Tiling choose_tiling(long long m, long long n, long long k, long long batch, bool b_mn, int sms) {
+  const long long blocks = (k + kTileK - 1) / kTileK;
+  Tiling best = {};
+  double least = 0;
+  auto consider = [&](Tiling t, long long tile_m, long long workers, double launch, double block, double tile) {
+    const long long work = ((m + tile_m - 1) / tile_m) * ((n + t.tile_n - 1) / t.tile_n) * batch * t.split;
+    const long long waves = (work + workers - 1) / workers, share = (blocks + t.split - 1) / t.split;
+    const double cost = launch + waves * (share * block > tile || waves == 1 ? share * block : tile);
+    // (clusters of four and eight do not fill the GPU: 36 clusters of four, 18 of eight already took two waves)
+    const bool fits = work <= (t.split > 2 ? sms - sms / 8 : sms) && blocks >= 2 * t.split;
+    if ((t.split == 1 || fits) && (best.split == 0 || cost < least)) {
+      best = t;
+      least = cost;
     }
-    long long pairs = sm_count(device) / 2;
-    if (p.num_tiles < pairs) pairs = p.num_tiles;
-    cudaLaunchConfig_t config = {};
-    config.gridDim = dim3(static_cast<unsigned>(pairs * 2));
-    config.blockDim = dim3(kThreads);
-    config.dynamicSmemBytes = kPairSmemBytes;
-    config.stream = stream;
-    cudaLaunchAttribute attribute[1];
-    attribute[0].id = cudaLaunchAttributeClusterDimension;
-    attribute[0].val.clusterDim.x = 2;
-    attribute[0].val.clusterDim.y = 1;
-    attribute[0].val.clusterDim.z = 1;
-    config.attrs = attribute;
-    config.numAttrs = 1;
-    TQ_CUDA(cudaLaunchKernelEx(&config, kernel, map_a, map_b, p));
-    return check_launch("gemm_bias_act_pair_kernel");
   };
-  if (!a_mn && !b_mn) return go(gemm_bias_act_pair_kernel<T, false, false>);
-  if (!a_mn && b_mn) return go(gemm_bias_act_pair_kernel<T, false, true>);
-  if (a_mn && !b_mn) return go(gemm_bias_act_pair_kernel<T, true, false>);
-  return go(gemm_bias_act_pair_kernel<T, true, true>);
+  for (int split = 1; split <= kMaxSplit; split *= 2) consider({false, kTileN, split}, kTileM, sms, split > 1 ? 8.5 : 7.5, 0.235, 3.9);
+  if (m > kTileM) {
+    consider({true, 256, 1}, kPairTileM, sms / 2, 9.0, 0.36, 6.2);
+    if (!b_mn) consider({true, 192, 1}, kPairTileM, sms / 2, 8.5, 0.28, 5.6);
+    consider({true, 128, 1}, kPairTileM, sms / 2, 8.0, 0.205, 3.5);
+  }
+  return best;
+}
+
+// One launch of `kernel` with clusters of `cluster` CTAs.
+template <typename Kernel>
+tq_status launch_kernel(Kernel kernel, const char* name, long long ctas, int cluster, size_t smem, const CUtensorMap& map_a, const CUtensorMap& map_b,
+                        const GemmParams& p, cudaStream_t stream) {
+  TQ_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+  cudaLaunchConfig_t config = {};
+  config.gridDim = dim3(static_cast<unsigned>(ctas));
+  config.blockDim = dim3(kThreads);
+  config.dynamicSmemBytes = smem;
+  config.stream = stream;
+  cudaLaunchAttribute attribute[1];
+  attribute[0].id = cudaLaunchAttributeClusterDimension;
+  attribute[0].val.clusterDim.x = cluster;
+  attribute[0].val.clusterDim.y = 1;
+  attribute[0].val.clusterDim.z = 1;
+  config.attrs = attribute;
+  config.numAttrs = cluster > 1 ? 1 : 0;
+  TQ_CUDA(cudaLaunchKernelEx(&config, kernel, map_a, map_b, p));
+  return check_launch(name);
+}
+
+template <typename T, bool A_MN, bool B_MN>
+tq_status launch_tiling(const Tiling& tiling, const CUtensorMap& map_a, const CUtensorMap& map_b, const GemmParams& p, int32_t device, cudaStream_t stream) {
+  const long long sms = sm_count(device);
+  if (!tiling.pair) {
+    if (tiling.split > 1) {
+      return launch_kernel(gemm_bias_act_kernel<T, A_MN, B_MN, true>, "gemm_bias_act_kernel", p.num_tiles * tiling.split, tiling.split, kSmemBytes, map_a,
+                           map_b, p, stream);
+    }
+    return launch_kernel(gemm_bias_act_kernel<T, A_MN, B_MN, false>, "gemm_bias_act_kernel", p.num_tiles < sms ? p.num_tiles : sms, 1, kSmemBytes, map_a,
+                         map_b, p, stream);
+  }
+  const long long pairs = p.num_tiles < sms / 2 ? p.num_tiles : sms / 2;
+  auto go = [&](auto tile_n) {
+    constexpr int kWidth = decltype(tile_n)::value;
+    return launch_kernel(gemm_bias_act_pair_kernel<T, kWidth, A_MN, B_MN>, "gemm_bias_act_pair_kernel", pairs * 2, 2, PairShape<kWidth>::kSmemBytes, map_a,
+                         map_b, p, stream);
+  };
+  if constexpr (!B_MN) {
+    if (tiling.tile_n == 192) return go(std::integral_constant<int, 192>{});
+  }
+  if (tiling.tile_n == 128) return go(std::integral_constant<int, 128>{});
+  return go(std::integral_constant<int, 256>{});
 }
 
 template <typename T>
-tq_status launch(bool a_mn, bool b_mn, const CUtensorMap& map_a, const CUtensorMap& map_b, const GemmParams& p, int32_t device, cudaStream_t stream) {
-  auto go = [&](auto kernel) -> tq_status {
-    static std::mutex mutex;
-    {
-      std::lock_guard<std::mutex> lock(mutex);
-      TQ_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmemBytes)));
-    }
-    long long ctas = p.num_tiles < sm_count(device) ? p.num_tiles : sm_count(device);
-    kernel<<<static_cast<unsigned>(ctas), kThreads, kSmemBytes, stream>>>(map_a, map_b, p);
-    return check_launch("gemm_bias_act_kernel");
-  };
-  if (!a_mn && !b_mn) return go(gemm_bias_act_kernel<T, false, false>);
-  if (!a_mn && b_mn) return go(gemm_bias_act_kernel<T, false, true>);
-  if (a_mn && !b_mn) return go(gemm_bias_act_kernel<T, true, false>);
-  return go(gemm_bias_act_kernel<T, true, true>);
+tq_status launch(bool a_mn, bool b_mn, const Tiling& tiling, const CUtensorMap& map_a, const CUtensorMap& map_b, const GemmParams& p, int32_t device,
+                 cudaStream_t stream) {
+  if (!a_mn && !b_mn) return launch_tiling<T, false, false>(tiling, map_a, map_b, p, device, stream);
+  if (!a_mn && b_mn) return launch_tiling<T, false, true>(tiling, map_a, map_b, p, device, stream);
+  if (a_mn && !b_mn) return launch_tiling<T, true, false>(tiling, map_a, map_b, p, device, stream);
+  return launch_tiling<T, true, true>(tiling, map_a, map_b, p, device, stream);
 }
 
 }  // namespace
@@ -745,13 +982,13 @@ extern "C" tq_status tq_gemm_bias_act_residual_launch(tq_dtype dtype, tq_activat
   const tq::WaitStatus status = tq::wait_status_for(device);
   TQ_REQUIRE(status.abort != nullptr, TQ_RESOURCE_EXHAUSTED, "no device memory for the status word");
 
-  // Large problems run on CTA pairs (256 x 256 tiles, half the shared-memory operand traffic per
-  // SM); problems with at most one row of 128 x 256 tiles keep the single-CTA kernel.
-  const bool pair = m > tq::kTileM;
+  const tq::Tiling tiling = tq::choose_tiling(m, n, k, batch, trans_b == 0, tq::sm_count(device));
   CUtensorMap map_a, map_b;
   const long long batch_a = stride_a > 0 ? batch : 1, batch_b = stride_b > 0 ? batch : 1;
-  const int b_rows = pair ? tq::kTileN / 2 : tq::kTileN;
-  if (tq_status s = tq::make_map(&map_a, dtype, a, a_inner, a_outer, lda, batch_a, stride_a, 64, trans_a ? 64 : tq::kTileM)) return s;
+  // (rows of the tile that A does not have are not brought; what lies there gives rows of C nobody stores)
+  const int a_rows = tiling.pair || trans_a || m > tq::kTileM ? tq::kTileM : static_cast<int>((m + 7) / 8 * 8);
+  const int b_rows = tiling.pair ? tiling.tile_n / 2 : tiling.tile_n;
+  if (tq_status s = tq::make_map(&map_a, dtype, a, a_inner, a_outer, lda, batch_a, stride_a, 64, trans_a ? 64 : a_rows)) return s;
   if (tq_status s = tq::make_map(&map_b, dtype, b, b_inner, b_outer, ldb, batch_b, stride_b, 64, trans_b ? b_rows : 64)) return s;
   TQ_REQUIRE(batch == 1 || (stride_a > 0 && stride_b > 0), TQ_UNSUPPORTED,
              "a batch that shares one operand (stride 0) has no kernel; fold the batch into m instead");
@@ -761,9 +998,11 @@ extern "C" tq_status tq_gemm_bias_act_residual_launch(tq_dtype dtype, tq_activat
   p.n = static_cast<int>(n);
   p.k = static_cast<int>(k);
   p.batch = static_cast<int>(batch);
-  const int tile_m = pair ? tq::kPairTileM : tq::kTileM;
+  const int tile_m = tiling.pair ? tq::kPairTileM : tq::kTileM;
   p.tiles_m = static_cast<int>((m + tile_m - 1) / tile_m);
-  p.tiles_n = static_cast<int>((n + tq::kTileN - 1) / tq::kTileN);
+  p.tiles_n = static_cast<int>((n + tiling.tile_n - 1) / tiling.tile_n);
+  p.split = tiling.split;
+  p.a_rows = a_rows;
   p.num_tiles = static_cast<long long>(p.tiles_m) * p.tiles_n * batch;
   p.bias = bias;
   p.residual = residual;
@@ -775,10 +1014,6 @@ extern "C" tq_status tq_gemm_bias_act_residual_launch(tq_dtype dtype, tq_activat
   p.activation = activation;
   p.status = status;
   cudaStream_t cuda_stream = static_cast<cudaStream_t>(stream);
-  if (pair) {
-    if (dtype == TQ_BF16) return tq::launch_pair<__nv_bfloat16>(trans_a != 0, trans_b == 0, map_a, map_b, p, device, cuda_stream);
-    return tq::launch_pair<__half>(trans_a != 0, trans_b == 0, map_a, map_b, p, device, cuda_stream);
-  }
-  if (dtype == TQ_BF16) return tq::launch<__nv_bfloat16>(trans_a != 0, trans_b == 0, map_a, map_b, p, device, cuda_stream);
-  return tq::launch<__half>(trans_a != 0, trans_b == 0, map_a, map_b, p, device, cuda_stream);
+  if (dtype == TQ_BF16) return tq::launch<__nv_bfloat16>(trans_a != 0, trans_b == 0, tiling, map_a, map_b, p, device, cuda_stream);
+  return tq::launch<__half>(trans_a != 0, trans_b == 0, tiling, map_a, map_b, p, device, cuda_stream);
 }

@@ -102,6 +102,31 @@ def test_residual_rides_in_the_epilogue(tq, m, n, k, act):
     assert poll() == 0
 
 
+@pytest.mark.parametrize("m, n, k, dtype", [
+    (100, 200, 320, torch.bfloat16),      # single CTAs, K whole
+    (1000, 768, 768, torch.bfloat16),     # ... K shared by two CTAs of a cluster
+    (128, 1001, 512, torch.float16),      # ... by four, rows of C that are not whole 16-byte units
+    (1, 136, 1040, torch.bfloat16),       # ... by eight, uneven shares, one row of A loaded in a box of eight
+    (20000, 130, 72, torch.bfloat16),     # CTA pairs, 256 x 128 tiles
+    (2500, 1000, 136, torch.float16),     # ... 256 x 192: the epilogue's halves take turns at the third block
+    (4224, 777, 768, torch.bfloat16),     # ... 256 x 256, odd rows of C
+])
+@pytest.mark.parametrize("transposed", [False, True], ids=["linear", "matmul"])
+def test_every_tiling(tq, m, n, k, dtype, transposed):
+    if transposed:
+        n = (n + 7) // 8 * 8              # B stored [k, n]: its rows have to start on 16-byte boundaries
+    g = torch.Generator().manual_seed(m + n + k)
+    a = (torch.randn(m, k, generator=g) * 0.5).to(dtype)
+    w = (torch.randn(n, k, generator=g) * (1.0 / np.sqrt(k))).to(dtype)
+    bias = (torch.randn(n, generator=g) * 0.5).to(dtype)
+    r = torch.randn(m, n, generator=g).to(dtype)
+    b = w.t().contiguous().cuda() if transposed else w.cuda().t()
+    exact = truth(a, w.t(), bias, "gelu_erf")
+    check(tq.gemm(a.cuda(), b, bias.cuda(), "gelu"), exact, dtype, k)
+    check(tq.gemm(a.cuda(), b, bias.cuda(), "gelu", r.cuda()), exact + r.double(), dtype, k)
+    assert poll() == 0
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("act", ["gelu", "gelu_tanh"])
 def test_gelu_epilogues_over_the_whole_range(tq, dtype, act):
