@@ -229,7 +229,7 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
   if (warp >= 8) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kOtherRegisters));
   if (warp == 8) {
     // ---- producer: the tiles of step 1 onwards (step 0's went out before the CTA met) ------------
-    if (lane == 0) {
+    if (elect_one()) {
       for (int j = 1; j < total_steps; ++j) {
         const int s = j % kRing;
         const uint32_t phase = (j / kRing) & 1;
@@ -249,7 +249,7 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
     // 12 of them plus two commits: one thread for both groups was the kernel's bottleneck. Each
     // group's issuer follows its own group only, so neither group waits for the other.
     const int g = warp - 9;
-    if (lane == 0 && steps[g] > 0) {
+    if (steps[g] > 0 && elect_one()) {
       constexpr uint32_t idesc_s = attn_instruction_descriptor<T>(kKeys, false);
       constexpr uint32_t idesc_o = attn_instruction_descriptor<T>(kHeadDim, true);
       // Descriptors as (low, high) words: one constant high word, low words stepped by adds.
@@ -568,6 +568,13 @@ bool legal_strides(const void* pointer, const int64_t* strides, long long head_d
 }
 
 }  // namespace
+
+// decode.cu
+tq_status attention_decode(tq_dtype dtype, const void* q, const void* k, const void* v, void* out, long long batch, long long heads,
+                           long long q_tokens, long long k_tokens, long long head_dim, const int64_t* q_strides, const int64_t* k_strides,
+                           const int64_t* v_strides, const int64_t* out_strides, float scale_log2, bool causal, int32_t device, cudaStream_t stream);
+constexpr int kDecodeQueries = 4;
+
 }  // namespace tq
 
 extern "C" tq_status tq_attention_launch(tq_dtype dtype, const void* q, const void* k, const void* v, void* out, int64_t batch,
@@ -609,6 +616,12 @@ extern "C" tq_status tq_attention_launch(tq_dtype dtype, const void* q, const vo
              "misaligned result or negative result stride");
   tq::DeviceScope device_scope(device);
   if (tq_status s = device_scope.status()) return s;
+  // A few query rows leave nothing for the tensor cores to reuse: K and V are streamed instead. (The result's
+  // batch * heads * split CTAs stay below 2^28.)
+  if (q_tokens <= tq::kDecodeQueries) {
+    return tq::attention_decode(dtype, q, k, v, out, batch, heads, q_tokens, k_tokens, head_dim, q_strides, k_strides, v_strides, out_strides,
+                                static_cast<float>(scale * 1.4426950408889634), causal != 0, device, static_cast<cudaStream_t>(stream));
+  }
   const tq::WaitStatus status = tq::wait_status_for(device);
   TQ_REQUIRE(status.abort != nullptr, TQ_RESOURCE_EXHAUSTED, "no device memory for the status word");
 

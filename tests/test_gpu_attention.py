@@ -102,6 +102,21 @@ def test_attention_with_other_head_widths(tq, width, causal):
     assert poll() == 0
 
 
+@pytest.mark.parametrize("queries, keys", [(1, 1), (1, 31), (1, 1000), (2, 129), (3, 700), (4, 2), (4, 515), (5, 515)])
+@pytest.mark.parametrize("width, dtype", [(64, torch.bfloat16), (128, torch.float16), (32, torch.bfloat16), (40, torch.float16), (8, torch.bfloat16)])
+@pytest.mark.parametrize("causal", [True, False], ids=["causal", "full"])
+def test_few_queries_against_a_cache(tq, queries, keys, width, dtype, causal):
+    """One to four query rows stream the keys (5 is the first size the tensor-core kernel takes); 515 and 1000
+    keys are shared by a cluster. Keys and values are views of a longer cache."""
+    q = draw((2, queries, 3, width), dtype, 31).transpose(1, 2)
+    cache = draw((2, 2, 3, keys + 9, width), dtype, 32)
+    k, v = cache[0][:, :, 4:keys + 4], cache[1][:, :, 4:keys + 4]
+    cache = cache.cuda()
+    got = tq.attention(q.cuda(), cache[0][:, :, 4:keys + 4], cache[1][:, :, 4:keys + 4], width ** -0.5, causal)
+    check(got, q, k, v, width ** -0.5, causal, oracle_atol=2e-2)
+    assert poll() == 0
+
+
 def test_attention_golden(tq, golden):
     q, k, v = (torch.from_numpy(golden[n].copy()).view(torch.bfloat16) for n in ("attn_q", "attn_k", "attn_v"))
     for causal, name in ((True, "attn_causal_bf16"), (False, "attn_full_bf16")):
