@@ -38,7 +38,7 @@ from torch.utils._python_dispatch import _disable_current_modes
 
 from . import ops
 from .executor import GraphedRecipe, NativeRecipe, Recipe, Step, note_torch_work
-from .kernel import DTYPE_NAMES, FusedKernel, classify_read
+from .kernel import DTYPE_NAMES, FusedKernel, broadcast_shape, classify_read
 from ._lib import Declined
 
 aten = torch.ops.aten
@@ -689,7 +689,7 @@ def _fused_step(node: fx.Node, kernel: FusedKernel, inputs: list[fx.Node]) -> St
     def run(env):
         tensors = [env[i.name] for i in inputs]
         tensors = [t if (s or t.is_contiguous()) else ops.contiguous(t) for t, s in zip(tensors, strided)]
-        shape = torch.broadcast_shapes(*[t.shape for t in tensors])   # from the operands, so one recipe serves every size
+        shape = broadcast_shape(*[t.shape for t in tensors])   # from the operands, so one recipe serves every size
         out = torch.empty(shape, dtype=dtype, device=tensors[0].device)
         kernel.launch(tensors, out, stream=None)
         return out
@@ -721,13 +721,16 @@ def _kernel_step(node: fx.Node) -> Step | None:
     reads = [a.name for a in node.all_input_nodes]
 
     def step(kind, fn):
-        def run(env, fn=fn):
-            return fn(*fx.node.map_arg(args, lambda n: env[n.name]), **fx.node.map_arg(kwargs, lambda n: env[n.name]))
+        bind = _binder(args, kwargs)
+
+        def run(env):
+            positional, named = bind(env)
+            return fn(*positional, **named)
 
         return Step(kind, node.name, run, reads)
 
     if target in VIEWS:
-        return step("view", target)
+        return step("view", target if kwargs else _VIEW_METHODS.get(target, target))
     value = node.meta.get("val")
     first = args[0].meta.get("val") if args and _is_tensor_node(args[0]) else None
     if first is not None and first.dtype not in DTYPE_NAMES:
@@ -762,6 +765,26 @@ def _kernel_step(node: fx.Node) -> Step | None:
             return step("gemm", _or_torch(ops.addmm, target))
     del value
     return None
+
+
+# The tensor methods behind the commonest view operators: the same views at half the cost of a call through
+# the operator registry, of which a decoder block makes thirty.
+_VIEW_METHODS = {aten.view.default: torch.Tensor.view, aten.reshape.default: torch.Tensor.reshape, aten.permute.default: torch.Tensor.permute,
+                 aten.transpose.int: torch.Tensor.transpose, aten.t.default: torch.Tensor.t, aten.unsqueeze.default: torch.Tensor.unsqueeze}
+
+
+def _binder(args, kwargs) -> Callable:
+    """A function from the values by name to a node's (args, kwargs). Where every node among them is an
+    argument of its own that is one lookup each; anything deeper is walked."""
+    def holds_node(value) -> bool:
+        found: list = []
+        fx.node.map_arg(value, lambda n: found.append(n) or n)
+        return bool(found)
+
+    if holds_node(kwargs) or any(holds_node(a) and not isinstance(a, fx.Node) for a in args):
+        return lambda env: (fx.node.map_arg(args, lambda n: env[n.name]), fx.node.map_arg(kwargs, lambda n: env[n.name]))
+    slots = [(a.name, None) if isinstance(a, fx.Node) else (None, a) for a in args]
+    return lambda env: ([value if name is None else env[name] for name, value in slots], kwargs)
 
 
 def _or_torch(kernel_fn: Callable, target) -> Callable:

@@ -15,6 +15,7 @@ from __future__ import annotations
 
 import ctypes
 import math
+from functools import lru_cache
 from typing import Sequence
 
 import torch
@@ -53,11 +54,12 @@ def dtype_code(dtype: torch.dtype) -> int:
 def _device_of(tensors: Sequence[torch.Tensor]) -> int:
     device = None
     for t in tensors:
+        index = t.get_device()
         if not t.is_cuda:
             raise ValueError(f"tessiq_b200 kernels take CUDA tensors, not a tensor on {t.device}")
         if device is None:
-            device = t.device.index
-        elif t.device.index != device:
+            device = index
+        elif index != device:
             raise ValueError("the tensors of one launch must be on one device")
     return 0 if device is None else device
 
@@ -65,12 +67,45 @@ def _device_of(tensors: Sequence[torch.Tensor]) -> int:
 def _stream(stream: int | None, device: int) -> int:
     """`None` means torch's current stream on `device`; an integer is a raw cudaStream_t."""
     if stream is None:
-        return torch.cuda.current_stream(device).cuda_stream
+        return torch._C._cuda_getCurrentRawStream(device)
     return int(stream)
 
 
-def _pointer(t: torch.Tensor | None) -> ctypes.c_void_p:
-    return ctypes.c_void_p(0 if t is None else t.data_ptr())
+def _pointer(t: torch.Tensor | None) -> int:
+    return 0 if t is None else t.data_ptr()
+
+
+# What a launch derives from its operands' types, shapes and strides alone is worked out once per such
+# signature: the checks, extents and argument arrays of a launch of a few microseconds cost tens of them in
+# Python. A plan holds numbers only, never an address or a tensor; its table is emptied when it is full.
+_PLANS = 256
+
+
+def _signature(*tensors: torch.Tensor | None) -> tuple:
+    return tuple([None if t is None else (t.dtype, t.shape, t.stride()) for t in tensors])
+
+
+def _keep(plans: dict, key: tuple, plan):
+    if len(plans) >= _PLANS:
+        plans.clear()
+    plans[key] = plan
+    return plan
+
+
+def broadcast_shape(*shapes: Sequence[int]) -> tuple[int, ...]:
+    """torch.broadcast_shapes for plain sizes (which takes ten microseconds over three operands)."""
+    result = tuple(shapes[0])
+    for shape in shapes[1:]:
+        if tuple(shape) == result:
+            continue
+        rank = max(len(shape), len(result))
+        merged = []
+        for x, y in zip((1,) * (rank - len(result)) + result, (1,) * (rank - len(shape)) + tuple(shape)):
+            if x != y and x != 1 and y != 1:
+                return tuple(torch.broadcast_shapes(*[tuple(each) for each in shapes]))     # raises, with torch's message
+            merged.append(y if x == 1 else x)
+        result = tuple(merged)
+    return result
 
 
 class Kernel:
@@ -192,6 +227,9 @@ class FusedKernel(Kernel):
         handle = ctypes.c_void_p()
         check(lib.tq_fused_create(program.encode(), ctypes.byref(handle)))
         self._handle = handle
+        self._pointers = ctypes.c_void_p * max(len(names), 1)
+        self._doubles = ctypes.c_double * max(len(self.scalars), 1)
+        self._plans: dict = {}
 
     def __del__(self):
         handle = getattr(self, "_handle", None)
@@ -216,13 +254,29 @@ class FusedKernel(Kernel):
         if len(scalars) != len(self.scalars):
             raise ValueError(f"fused kernel '{self.output}' takes {len(self.scalars)} scalars, not {len(scalars)}")
         device = _device_of([*inputs, out])
+        elements, divisors, layouts = self.plan(inputs, out)
+        if elements:
+            self.start(inputs, out.data_ptr(), elements, divisors, layouts, scalars, device, _stream(stream, device))
+
+    def start(self, inputs, out_pointer, elements, divisors, layouts, scalars, device, stream) -> None:
+        """The launch itself, for operands that `plan` has seen."""
+        check(lib.tq_fused_launch(self._handle, self._pointers(*[t.data_ptr() for t in inputs]), out_pointer, elements, divisors, layouts,
+                                  self._doubles(*[float(s) for s in scalars]), device, stream))
+
+    def plan(self, inputs, out):
+        """(elements, divisors, layouts) of a launch over operands of these types, shapes and strides."""
+        key = _signature(out, *inputs)
+        found = self._plans.get(key)
+        return found if found is not None else _keep(self._plans, key, self._plan(inputs, out))
+
+    def _plan(self, inputs, out):
         if not out.is_contiguous():
             raise ValueError("the output of a fused kernel must be packed")
         if DTYPE_NAMES.get(out.dtype) != self.out_dtype:
             raise ValueError(f"fused kernel '{self.output}' writes {self.out_dtype}, the output tensor is {out.dtype}")
         elements = out.numel()
         if elements == 0:
-            return
+            return 0, None, None
         out_shape = list(out.shape)
         divisors, layouts = [], []
         for name, t, read, dtype in zip(self.inputs, inputs, self.reads, self.input_dtypes):
@@ -248,12 +302,9 @@ class FusedKernel(Kernel):
                 if t.numel() == 0 or elements % t.numel():
                     raise ValueError(f"operand '{name}' with {t.numel()} elements does not repeat evenly over {elements}")
                 divisors.append(elements // t.numel())
-        pointers = (ctypes.c_void_p * max(len(inputs), 1))(*[t.data_ptr() for t in inputs])
         divisor_array = (ctypes.c_int64 * max(len(divisors), 1))(*divisors)
         layout_array = (_lib.tq_layout * max(len(layouts), 1))(*layouts)
-        scalar_array = (ctypes.c_double * max(len(scalars), 1))(*[float(s) for s in scalars])
-        check(lib.tq_fused_launch(self._handle, pointers, _pointer(out), elements, divisor_array, layout_array,
-                                  scalar_array, device, ctypes.c_void_p(_stream(stream, device))))
+        return elements, divisor_array, layout_array
 
 
 def reduction_extents(shape: Sequence[int], first_axis: int, last_axis: int) -> tuple[int, int, int]:
@@ -365,16 +416,22 @@ class ReductionKernel(Kernel):
         launch_reduce(self.op, x, out, outer, reduce, inner, device, _stream(stream, device))
 
 
+@lru_cache(maxsize=1024)
+def reduce_workspace_bytes(code: int, dtype: int, outer: int, reduce: int, inner: int, device: int) -> int:
+    nbytes = ctypes.c_size_t()
+    check(lib.tq_reduce_workspace_bytes(code, dtype, outer, reduce, inner, device, ctypes.byref(nbytes)))
+    return nbytes.value
+
+
 def launch_reduce(op: str, x: torch.Tensor, out: torch.Tensor, outer: int, reduce: int, inner: int,
                   device: int, stream: int) -> None:
     code, dtype = REDUCE_OPS[op], dtype_code(x.dtype)
-    nbytes = ctypes.c_size_t()
-    check(lib.tq_reduce_workspace_bytes(code, dtype, outer, reduce, inner, device, ctypes.byref(nbytes)))
-    scratch = workspace(device, stream, nbytes.value)
-    check(lib.tq_reduce_launch(code, dtype, _pointer(x), _pointer(out), outer, reduce, inner, _pointer(scratch),
-                               0 if scratch is None else scratch.numel(), device, ctypes.c_void_p(stream)))
+    scratch = workspace(device, stream, reduce_workspace_bytes(code, dtype, outer, reduce, inner, device))
+    check(lib.tq_reduce_launch(code, dtype, x.data_ptr(), out.data_ptr(), outer, reduce, inner, _pointer(scratch),
+                               0 if scratch is None else scratch.numel(), device, stream))
 
 
+@lru_cache(maxsize=1024)
 def transposed_passes(kind: str, dtype: torch.dtype, batch: int, rows: int, cols: int, device: int = 0) -> int:
     """Passes over HBM tq_*_transposed_launch makes for this shape: 2 (a cluster keeps a slab of
     columns in shared memory) or 3 (statistics, then a transposing normalise)."""
@@ -407,21 +464,26 @@ def prefers_transposed(kind: str, dtype: torch.dtype, batch: int = 0, rows: int 
     return batch * rows * cols * dtype.itemsize >= (64 << 20) and rows % 64 == 0 and (cols * dtype.itemsize) % 512 == 0
 
 
+@lru_cache(maxsize=1024)
+def transposed_workspace_bytes(layer_norm: bool, dtype: int, batch: int, rows: int, cols: int, device: int) -> int:
+    nbytes = ctypes.c_size_t()
+    check(lib.tq_transposed_workspace_bytes(1 if layer_norm else 0, dtype, batch, rows, cols, device, ctypes.byref(nbytes)))
+    return nbytes.value
+
+
 def launch_transposed(kind: str, base: torch.Tensor, weight, bias, out: torch.Tensor, batch: int, rows: int, cols: int,
                       eps: float, device: int, stream: int) -> None:
     """softmax ("softmax") or LayerNorm ("layer_norm") over `rows` of the packed base[batch, rows, cols],
     written transposed into the packed out[batch, cols, rows] (tq_*_transposed_launch)."""
     layer_norm = kind == "layer_norm"
-    nbytes = ctypes.c_size_t()
-    check(lib.tq_transposed_workspace_bytes(1 if layer_norm else 0, dtype_code(base.dtype), batch, rows, cols, device, ctypes.byref(nbytes)))
-    scratch = workspace(device, stream, nbytes.value)
+    scratch = workspace(device, stream, transposed_workspace_bytes(layer_norm, dtype_code(base.dtype), batch, rows, cols, device))
     if layer_norm:
         check(lib.tq_layer_norm_transposed_launch(dtype_code(base.dtype), _pointer(base), _pointer(weight), _pointer(bias), _pointer(out),
                                                   batch, rows, cols, float(eps), _pointer(scratch), 0 if scratch is None else scratch.numel(),
-                                                  device, ctypes.c_void_p(stream)))
+                                                  device, stream))
     else:
         check(lib.tq_softmax_transposed_launch(dtype_code(base.dtype), _pointer(base), _pointer(out), batch, rows, cols, _pointer(scratch),
-                                               0 if scratch is None else scratch.numel(), device, ctypes.c_void_p(stream)))
+                                               0 if scratch is None else scratch.numel(), device, stream))
 
 
 class PackKernel(Kernel):
@@ -433,22 +495,25 @@ class PackKernel(Kernel):
 
     def __init__(self, input: str = "x", output: str = "out"):
         super().__init__([input], output)
+        self._plans: dict = {}
 
     def output_shape(self, inputs):
         self._check_count(inputs)
         return list(inputs[0].shape)
 
+    def _plan(self, x, out):
+        if not out.is_contiguous() or list(out.shape) != list(x.shape) or out.dtype != x.dtype:
+            raise ValueError("the pack kernel writes a packed tensor of the view's shape and type")
+        rank = x.dim()
+        return x.element_size(), rank, (ctypes.c_int64 * max(rank, 1))(*x.shape), (ctypes.c_int64 * max(rank, 1))(*x.stride())
+
     def launch(self, inputs, out, stream=0):
         self._check_count(inputs)
         (x,) = inputs
         device = _device_of([x, out])
-        if not out.is_contiguous() or list(out.shape) != list(x.shape) or out.dtype != x.dtype:
-            raise ValueError("the pack kernel writes a packed tensor of the view's shape and type")
-        rank = x.dim()
-        sizes = (ctypes.c_int64 * max(rank, 1))(*x.shape)
-        strides = (ctypes.c_int64 * max(rank, 1))(*x.stride())
-        check(lib.tq_pack_launch(x.element_size(), rank, sizes, strides, _pointer(x), _pointer(out), device,
-                                 ctypes.c_void_p(_stream(stream, device))))
+        key = _signature(x, out)
+        plan = self._plans.get(key) or _keep(self._plans, key, self._plan(x, out))
+        check(lib.tq_pack_launch(*plan, x.data_ptr(), out.data_ptr(), device, _stream(stream, device)))
 
 
 class SoftmaxKernel(Kernel):
@@ -475,7 +540,7 @@ class SoftmaxKernel(Kernel):
         outer = math.prod(x.shape[:along])
         inner = math.prod(x.shape[along + 1 :])
         check(lib.tq_softmax_launch(dtype_code(x.dtype), dtype_code(out.dtype), _pointer(x), _pointer(out), outer,
-                                    extent, inner, device, ctypes.c_void_p(_stream(stream, device))))
+                                    extent, inner, device, _stream(stream, device)))
 
 
 class LayerNormKernel(Kernel):
@@ -512,7 +577,7 @@ class LayerNormKernel(Kernel):
                 stat_dtype = t.dtype
         check(lib.tq_layer_norm_launch(dtype_code(x.dtype), _pointer(x), _pointer(weight), _pointer(bias), _pointer(out),
                                        _pointer(mean), _pointer(rstd), dtype_code(stat_dtype), rows, width,
-                                       float(self.eps), device, ctypes.c_void_p(_stream(stream, device))))
+                                       float(self.eps), device, _stream(stream, device)))
 
 
 class GemmKernel(Kernel):
@@ -528,6 +593,7 @@ class GemmKernel(Kernel):
         super().__init__(names, output)
         self.activation = {"none": _lib.ACT_NONE, "gelu": _lib.ACT_GELU_ERF, "gelu_erf": _lib.ACT_GELU_ERF,
                            "gelu_tanh": _lib.ACT_GELU_TANH}[activation]
+        self._plans: dict = {}
         self.has_bias = has_bias
         self.has_residual = has_residual      # launch takes [a, b, (bias), (residual)]: act(a @ b + bias) + residual
 
@@ -552,6 +618,14 @@ class GemmKernel(Kernel):
         bias = inputs[2] if self.has_bias else None
         residual = inputs[-1] if self.has_residual else None
         device = _device_of([t for t in (a, b, bias, residual, out) if t is not None])
+        key = _signature(a, b, bias, residual, out)
+        plan = self._plans.get(key) or _keep(self._plans, key, self._plan(inputs, a, b, bias, residual, out))
+        dtype, lda, trans_a, ldb, trans_b, m, n, k, batch, stride_a, stride_b = plan
+        check(lib.tq_gemm_bias_act_residual_launch(dtype, self.activation, a.data_ptr(), lda, trans_a, b.data_ptr(), ldb, trans_b,
+                                                   _pointer(bias), _pointer(residual), n, m * n, out.data_ptr(), n, m, n, k,
+                                                   batch, stride_a, stride_b, m * n, device, _stream(stream, device)))
+
+    def _plan(self, inputs, a, b, bias, residual, out):
         if a.dim() != b.dim() or a.dim() not in (2, 3):
             raise _lib.Declined("the GEMM kernel takes two matrices or two batches of matrices")
         if a.dtype != b.dtype or out.dtype != a.dtype:
@@ -573,9 +647,7 @@ class GemmKernel(Kernel):
         trans_b, ldb = self._operand(b)
         stride_a = a.stride(0) if a.dim() == 3 else 0
         stride_b = b.stride(0) if b.dim() == 3 else 0
-        check(lib.tq_gemm_bias_act_residual_launch(dtype_code(a.dtype), self.activation, _pointer(a), lda, trans_a, _pointer(b),
-                                                   ldb, trans_b, _pointer(bias), _pointer(residual), n, m * n, _pointer(out), n, m, n, k,
-                                                   batch, stride_a, stride_b, m * n, device, ctypes.c_void_p(_stream(stream, device))))
+        return dtype_code(a.dtype), lda, trans_a, ldb, trans_b, m, n, k, batch, stride_a, stride_b
 
 
 class AttentionKernel(Kernel):
@@ -593,6 +665,7 @@ class AttentionKernel(Kernel):
     def __init__(self, scale: float, causal: bool, inputs=None, output: str = "out"):
         super().__init__(list(inputs) if inputs is not None else ["q", "k", "v"], output)
         self.scale, self.causal = float(scale), bool(causal)
+        self._plans: dict = {}
 
     def output_shape(self, inputs):
         return list(inputs[0].shape)
@@ -609,6 +682,12 @@ class AttentionKernel(Kernel):
         self._check_count(inputs)
         q, k, v = inputs
         device = _device_of([q, k, v, out])
+        key = _signature(q, k, v, out)
+        dtype, extents = self._plans.get(key) or _keep(self._plans, key, self._plan(q, k, v, out))
+        check(lib.tq_attention_launch(dtype, q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), *extents, self.scale, int(self.causal), device,
+                                      _stream(stream, device)))
+
+    def _plan(self, q, k, v, out):
         if not (q.dtype == k.dtype == v.dtype == out.dtype):
             raise _lib.Declined("attention operands and result must share one element type")
         strides = [self._strides(t) for t in (q, k, v, out)]
@@ -617,6 +696,4 @@ class AttentionKernel(Kernel):
             raise ValueError(f"attention shapes do not agree: q {tuple(q.shape)}, k {tuple(k.shape)}, v {tuple(v.shape)}")
         if tuple(out.shape) != tuple(q.shape):
             raise ValueError("the attention result has the shape of q")
-        check(lib.tq_attention_launch(dtype_code(q.dtype), _pointer(q), _pointer(k), _pointer(v), _pointer(out), batch, heads,
-                                      q_tokens, k.shape[2], head_dim, *strides, self.scale, int(self.causal), device,
-                                      ctypes.c_void_p(_stream(stream, device))))
+        return dtype_code(q.dtype), (batch, heads, q_tokens, k.shape[2], head_dim, *strides)

@@ -18,8 +18,9 @@ from typing import Sequence
 import torch
 
 from . import _lib
-from .kernel import (DTYPE_NAMES, AttentionKernel, FusedKernel, GemmKernel, LayerNormKernel, PackKernel, SoftmaxKernel, _device_of,
-                     _pointer, _stream, check_status, classify_read, dtype_code, launch_reduce, launch_transposed, prefers_transposed)
+from .kernel import (DTYPE_NAMES, REDUCE_OPS, AttentionKernel, FusedKernel, GemmKernel, LayerNormKernel, PackKernel, SoftmaxKernel, _device_of,
+                     _keep, _pointer, _stream, broadcast_shape, check_status, classify_read, dtype_code, launch_reduce, launch_transposed,
+                     prefers_transposed, reduce_workspace_bytes, workspace)
 from ._lib import Declined, check, lib
 
 import ctypes
@@ -37,6 +38,12 @@ def _kernel(program: str) -> FusedKernel:
     return FusedKernel(program)
 
 
+_pack = PackKernel()
+_softmax_kernel, _layer_norm_kernel = lru_cache(maxsize=64)(SoftmaxKernel), lru_cache(maxsize=64)(LayerNormKernel)
+_gemm_kernel, _attention_kernel = lru_cache(maxsize=64)(GemmKernel), lru_cache(maxsize=64)(AttentionKernel)
+_PLAIN = (torch.Tensor, torch.nn.Parameter)     # a subclass, or a tracer's stand-in, goes the long way every time
+
+
 def fused(program: str, inputs: Sequence[torch.Tensor], out: torch.Tensor, scalars: Sequence[float] = ()) -> torch.Tensor:
     """Runs a fusion-group program (include/tessiq_b200.h) over `inputs` into `out`."""
     _kernel(program).launch(list(inputs), out, stream=None, scalars=scalars)
@@ -48,13 +55,13 @@ def contiguous(x: torch.Tensor) -> torch.Tensor:
     if x.is_contiguous():
         return x
     out = torch.empty(x.shape, dtype=x.dtype, device=x.device)
-    PackKernel().launch([x], out, stream=None)
+    _pack.launch([x], out, stream=None)
     return out
 
 
 def clone(x: torch.Tensor) -> torch.Tensor:
     out = torch.empty(x.shape, dtype=x.dtype, device=x.device)
-    PackKernel().launch([x], out, stream=None)
+    _pack.launch([x], out, stream=None)
     return out
 
 
@@ -124,12 +131,30 @@ def elementwise(op: str, *operands, math_mode: str = "fast", out: torch.Tensor |
     operands must share an element type (mixed types are promoted by torch on its host path in the
     reference, which here is a decline); Python numbers become kernel scalars. `out` writes into an
     existing tensor (an operand itself for the in-place form) under the reference's conditions."""
+    if out is None:
+        key = [op, math_mode]
+        for o in operands:
+            if type(o) in _PLAIN:
+                key += (o.dtype, o.shape, o.stride(), o.get_device())
+            elif isinstance(o, torch.Tensor):
+                key = None
+                break
+            else:
+                key.append(type(o))
+        key = None if key is None else tuple(key)
+        plan = _elementwise_plans.get(key)
+        if plan is not None:
+            kernel, size, stride, dtype, where, device, start = plan
+            result = torch.empty_strided(size, stride, dtype=dtype, device=where)
+            kernel.start([o for o in operands if isinstance(o, torch.Tensor)], result.data_ptr(), *start,
+                         [o for o in operands if not isinstance(o, torch.Tensor)], device, _stream(None, device))
+            return result
     tensors = [o for o in operands if isinstance(o, torch.Tensor)]
     if not tensors:
         raise ValueError(f"{op} needs at least one tensor operand")
     if op not in UNARY and op not in BINARY and op != "where":
         raise Declined(f"no elementwise kernel named '{op}'")
-    _device_of(tensors)
+    device = _device_of(tensors)
     out_shape = list(torch.broadcast_shapes(*[tuple(t.shape) for t in tensors]))
     value_dtypes = {t.dtype for t in (tensors[1:] if op == "where" else tensors)}
     if len(value_dtypes) != 1:
@@ -161,8 +186,14 @@ def elementwise(op: str, *operands, math_mode: str = "fast", out: torch.Tensor |
         names.append(name)
     lines.append(f"r = {op} {' '.join(names)}")
     lines.append(f"out r {DTYPE_NAMES[out_dtype]}")
-    fused("\n".join(lines), inputs, packed, scalars)
+    kernel = _kernel("\n".join(lines))
+    kernel.launch(inputs, packed, stream=None, scalars=scalars)
+    if out is None and key is not None:
+        _keep(_elementwise_plans, key, (kernel, result.shape, result.stride(), result.dtype, result.device, device, kernel.plan(inputs, packed)))
     return result
+
+
+_elementwise_plans: dict = {}
 
 
 def elementwise_(op: str, target: torch.Tensor, *others, math_mode: str = "fast") -> torch.Tensor:
@@ -182,6 +213,19 @@ def cast(x: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
 
 def _reduce(op: str, x: torch.Tensor, dim, keepdim: bool) -> torch.Tensor:
     device = _device_of([x])
+    key = None
+    axes = tuple(dim) if isinstance(dim, (list, tuple)) else (dim,)
+    if type(x) in _PLAIN and all(type(d) is int or d is None for d in axes):
+        key = (op, x.dtype, x.shape, x.stride(), device, axes, dim is None, bool(keepdim))
+        plan = _reduce_plans.get(key)
+        if plan is not None:
+            code, dtype, extents, out_dtype, shape, nbytes = plan
+            out = torch.empty(shape, dtype=out_dtype, device=x.device)
+            stream = _stream(None, device)
+            scratch = workspace(device, stream, nbytes)
+            check(lib.tq_reduce_launch(code, dtype, x.data_ptr(), out.data_ptr(), *extents, _pointer(scratch),
+                                       0 if scratch is None else scratch.numel(), device, stream))
+            return out
     rank = x.dim()
     if rank == 0:
         raise Declined("a reduction of a tensor without axes has no kernel")  # reduction.cpp:110-113
@@ -203,7 +247,13 @@ def _reduce(op: str, x: torch.Tensor, dim, keepdim: bool) -> torch.Tensor:
         extents = (math.prod(kept_shape), math.prod(x.shape[d] for d in dims), 1)
     out = torch.empty(kept_shape, dtype=out_dtype, device=x.device)
     launch_reduce(op, base, out, *extents, device, _stream(None, device))
+    if key is not None and base.data_ptr() == x.data_ptr():      # read where it lies: the extents say all there is to say
+        code, dtype = REDUCE_OPS[op], dtype_code(x.dtype)
+        _keep(_reduce_plans, key, (code, dtype, extents, out_dtype, final_shape, reduce_workspace_bytes(code, dtype, *extents, device)))
     return out.reshape(final_shape)
+
+
+_reduce_plans: dict = {}
 
 
 def _extents_in_place(x: torch.Tensor, dims: list[int], kept: list[int]):
@@ -289,7 +339,7 @@ def softmax(x: torch.Tensor, dim: int = -1, half_to_float: bool = False) -> torc
     x = contiguous(x)
     out = torch.empty(x.shape, dtype=out_dtype, device=x.device)
     if x.numel():
-        SoftmaxKernel(dim, half_to_float).launch([x], out, stream=None)
+        _softmax_kernel(dim, half_to_float).launch([x], out, stream=None)
     return out
 
 
@@ -308,7 +358,7 @@ def native_layer_norm(x, normalized_shape, weight, bias, eps):
     mean = torch.empty(stat_shape, dtype=x.dtype, device=x.device)
     rstd = torch.empty(stat_shape, dtype=x.dtype, device=x.device)
     if x.numel():
-        LayerNormKernel(k, eps).launch([x, weight, bias], out, stream=None, mean=mean, rstd=rstd)
+        _layer_norm_kernel(k, float(eps)).launch([x, weight, bias], out, stream=None, mean=mean, rstd=rstd)
     return out, mean, rstd
 
 
@@ -327,7 +377,7 @@ def layer_norm(x, normalized_shape, weight=None, bias=None, eps=1e-5):
     x = contiguous(x)
     out = torch.empty_like(x)
     if x.numel():
-        LayerNormKernel(len(list(normalized_shape)), eps).launch(
+        _layer_norm_kernel(len(list(normalized_shape)), float(eps)).launch(
             [x, None if weight is None else contiguous(weight), None if bias is None else contiguous(bias)], out, stream=None)
     return out
 
@@ -342,7 +392,7 @@ def rms_norm(x, weight, eps):
     rows = x.numel() // max(width, 1)
     if x.numel():
         check(lib.tq_rms_norm_launch(dtype_code(x.dtype), _pointer(x), _pointer(None if weight is None else contiguous(weight)),
-                                     _pointer(out), rows, width, float(eps), device, ctypes.c_void_p(_stream(None, device))))
+                                     _pointer(out), rows, width, float(eps), device, _stream(None, device)))
     return out
 
 
@@ -367,7 +417,7 @@ def batch_norm_eval(x, weight, bias, running_mean, running_var, eps):
                                         _pointer(None if bias is None else contiguous(bias)),
                                         _pointer(contiguous(running_mean)), _pointer(contiguous(running_var)),
                                         _pointer(out), n, c, inner, float(eps), device,
-                                        ctypes.c_void_p(_stream(None, device))))
+                                        _stream(None, device)))
     return out
 
 
@@ -383,7 +433,7 @@ def _realigned(t):
     if t is None or t.data_ptr() % 16 == 0 or t.numel() == 0:
         return t
     fresh = torch.empty(t.shape, dtype=t.dtype, device=t.device)
-    PackKernel().launch([t], fresh, stream=None)
+    _pack.launch([t], fresh, stream=None)
     return fresh
 
 
@@ -391,7 +441,7 @@ def _gemm(a, b, bias, activation, residual=None):
     out = torch.empty([*a.shape[:-1], b.shape[-1]], dtype=a.dtype, device=a.device)
     if out.numel() == 0:
         return out
-    kernel = GemmKernel(activation, has_bias=bias is not None, has_residual=residual is not None)
+    kernel = _gemm_kernel(activation, has_bias=bias is not None, has_residual=residual is not None)
     try:
         kernel.launch([t for t in (a, b, bias, residual) if t is not None], out, stream=None)
     except Declined:
@@ -452,7 +502,7 @@ def attention(q, k, v, scale=None, causal=False, token_major=True):
     else:
         out = torch.empty([batch, heads, tokens, width], dtype=q.dtype, device=q.device)
     if out.numel():
-        AttentionKernel(scale, causal).launch([q, k, v], out, stream=None)
+        _attention_kernel(float(scale), bool(causal)).launch([q, k, v], out, stream=None)
     return out
 
 

@@ -504,3 +504,31 @@ def test_devices_option_is_checked_when_the_graph_is_compiled():
         B.compile_graph(gm, [torch.zeros(2)], options={"shard": [0]})
     with pytest.raises(ValueError, match="unknown"):
         B.compile_graph(gm, [torch.zeros(2)], options={"device_list": [0]})
+
+
+def test_broadcast_shape_is_torchs():
+    from tessiq_b200.kernel import broadcast_shape
+
+    shapes = [(), (1,), (5,), (4, 1), (4, 5), (1, 5), (3, 1, 1), (3, 4, 5), (0,), (1, 0)]
+    for a in shapes:
+        for b in shapes:
+            for c in ((), (4, 5)):
+                try:
+                    expected = tuple(torch.broadcast_shapes(a, b, c))
+                except RuntimeError:
+                    with pytest.raises(RuntimeError):
+                        broadcast_shape(a, b, c)
+                else:
+                    assert broadcast_shape(a, torch.Size(b), list(c)) == expected
+
+
+def test_a_steps_arguments_are_bound_as_the_graph_holds_them():
+    from tessiq_b200.backend import _binder
+
+    graph = torch.fx.Graph()
+    x, y = graph.placeholder("x"), graph.placeholder("y")
+    env = {"x": 1, "y": 2}
+    for args, kwargs in [((x, [3, 4], None), {}), ((x, y, 0.5), {"dim": 1}), (([x, y], 0), {}), ((x, [y, 4]), {}), ((x,), {"other": y}), ((), {})]:
+        bound, named = _binder(args, kwargs)(env)
+        expected, expected_named = torch.fx.node.map_arg(args, lambda n: env[n.name]), torch.fx.node.map_arg(kwargs, lambda n: env[n.name])
+        assert list(bound) == list(expected) and dict(named) == dict(expected_named)

@@ -308,3 +308,41 @@ def _sharded_compile_worker():
 @pytest.mark.skipif(torch.cuda.device_count() < 2, reason="needs two GPUs")
 def test_compiled_block_runs_sharded_over_two_gpus_of_one_process():
     _sharded_compile_worker()
+
+
+def test_a_kept_plan_serves_its_own_signature_only():
+    """The second call over a signature takes the kept plan: it must agree with the first, and with calls
+    that differ in one respect only (stride, type, broadcasting, a scalar's kind, an axis, another stream)."""
+    from tessiq_b200 import ops as tq
+
+    base = torch.randn(48, 64, device="cuda")
+    views = [base, base.t().contiguous().t(), base[:, ::2], base[:1].expand(48, 64), base[:40], base.t(), base.bfloat16()]
+    row = torch.randn(64, device="cuda")
+    for _ in range(3):
+        for v in views:
+            for _ in range(2):
+                if v.shape[-1] == 64:
+                    other = row.to(v.dtype)
+                    got = tq.elementwise("add", v, other)
+                    assert torch.equal(got, v + other) and got.stride() == (v + other).stride()
+                for scalar in (2, 2.0, 0.25):
+                    assert torch.equal(tq.elementwise("mul", v, scalar), v * scalar)
+                for keepdim in (False, True):
+                    for dim in (0, 1, -1, (0, 1), None):
+                        got = tq.amax(v, dim, keepdim)
+                        expected = v.amax(() if dim is None else dim, keepdim)
+                        assert got.shape == expected.shape and torch.equal(got, expected)
+                assert torch.equal(tq.contiguous(v), v)
+        with pytest.raises((TypeError, ValueError)):
+            tq.sum(base, 1.0)
+        with pytest.raises(ValueError):
+            tq.elementwise("add", base.cpu(), row.cpu())
+        with pytest.raises((TypeError, ValueError)):
+            tq.elementwise("add", base, row.half())
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        big = torch.randn(1 << 20, device="cuda")
+        total = tq.sum(big)
+    side.synchronize()
+    assert abs(total.item() - big.double().sum().item()) < 1e-5 * big.abs().sum().item()
