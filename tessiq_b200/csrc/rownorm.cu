@@ -7,9 +7,11 @@
 //                    shared memory -> distributed shared memory: every CTA writes its block value
 //                    into each peer's slot array, one cluster barrier, every CTA folds the slots
 //                    in rank order, so all CTAs hold the same bits.
+//   ragged rows      rows that do not start on 16-byte boundaries (an odd width): the same, but the
+//                    vectors are those of memory, with up to seven elements before the first and after
+//                    the last of them apart; persistent teams keep weight and bias shifted to match.
 //   loop-per-row     any width or alignment: one CTA streams the row three times (two for
-//                    RMSNorm). The fallback for rows that are unaligned or beyond what a cluster
-//                    can hold.
+//                    RMSNorm). The fallback for f64 and for rows beyond what a cluster can hold.
 //   softmax-columns  softmax over an axis that is not the last one: one thread per column, an
 //                    online max/sum pass and a write pass, coalesced along the kept axis.
 //
@@ -315,6 +317,206 @@ __global__ void __launch_bounds__(THREADS) row_cluster_kernel(RowArgs args, int 
                                   rank == 0 && threadIdx.x == 0, fold_row);
 }
 
+// exp(d) for d <= 0 as the kernels of a type take it: rows of f32 that no vector fits used expf before they
+// had a kernel of their own, and 2^(d log2 e) rounds the product, which f32 results would show.
+template <typename T> __device__ __forceinline__ float ragged_exp(float d) {
+  if constexpr (sizeof(T) == 4) {
+    return expf(d);
+  } else {
+    return exp2_approx(d * 1.4426950408889634f);
+  }
+}
+
+// VEC elements of `values` (an array of `count`, 16-byte aligned) from element `at` on: two aligned loads
+// shifted together, so that a thread's share of a weight row costs two load instructions and not VEC. At the
+// end of the array, where the second load would leave it, element by element.
+template <typename T, int VEC>
+__device__ __forceinline__ Vec<T, VEC> load_shifted(const T* values, int at, int count) {
+  const int aligned = at / VEC * VEC, shift = at - aligned;
+  Vec<T, VEC> out;
+  if (shift == 0 || aligned + 2 * VEC <= count) {
+    const uint4 low = __ldg(reinterpret_cast<const uint4*>(values + aligned));
+    uint4 high = low;
+    if (shift != 0) high = __ldg(reinterpret_cast<const uint4*>(values + aligned) + 1);
+    uint32_t word[8] = {low.x, low.y, low.z, low.w, high.x, high.y, high.z, high.w};
+    const int bytes = shift * static_cast<int>(sizeof(T));
+    const bool by_two = (bytes & 8) != 0, by_one = (bytes & 4) != 0;
+#pragma unroll
+    for (int i = 0; i < 6; ++i) word[i] = by_two ? word[i + 2] : word[i];
+#pragma unroll
+    for (int i = 0; i < 5; ++i) word[i] = by_one ? word[i + 1] : word[i];
+    uint32_t result[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) result[i] = (bytes & 2) != 0 ? __funnelshift_r(word[i], word[i + 1], 16) : word[i];
+    out = *reinterpret_cast<Vec<T, VEC>*>(result);
+  } else {
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) out.v[e] = values[at + e];
+  }
+  return out;
+}
+
+// Rows of any width and alignment, held in registers. A row's whole 16-byte vectors (of memory, not of the
+// row) are spread over the team as in the kernels above; the fewer than VEC elements before the first and
+// after the last are one element each of the team's first 2 * VEC threads, so nothing outside the row is
+// read. Weight and bias belong to elements, so a thread's share of them starts `head` elements into the row:
+// shifted together once, and kept (in registers, or in the thread's own slots of shared memory where there
+// are more than two vectors: with four in registers only 16 warps fit an SM) for as long as the team's rows have the same head. Teams step through the rows
+// by a multiple of VEC rows, which keeps the head the same whatever the width.
+//
+// Bound: HBM. The loop kernel read every row three times, an element per load: 20000 x 1003 bf16 softmax
+// took 61.0 us, LayerNorm 61.8, where the bytes take 12.4; these take 17.6 and 25 (rows of 1000: 15.3 and 18.5).
+template <typename T, typename OutT, int VEC, int K, int OP, int THREADS>
+__global__ void __launch_bounds__(THREADS == 32 ? kBlock : THREADS, (K <= 4 ? 1024 : 768) / (THREADS == 32 ? kBlock : THREADS))
+row_ragged_kernel(RowArgs args, int cluster) {
+  constexpr int kTeams = THREADS == 32 ? kWarps : 1, kThreads = THREADS * kTeams;
+  constexpr bool kInRegisters = K <= 2, kScaled = OP != kSoftmax;
+  __shared__ float warp_scratch[THREADS / 32];
+  __shared__ float slots[4][kMaxCluster];
+  extern __shared__ uint4 kept_words[];
+  Vec<T, VEC>* kept = reinterpret_cast<Vec<T, VEC>*>(kept_words) + threadIdx.x;     // [2 * K][kThreads]
+
+  const int member = THREADS == 32 ? threadIdx.x & 31 : threadIdx.x;
+  const long long team = THREADS == 32 ? static_cast<long long>(blockIdx.x) * kTeams + (threadIdx.x >> 5) : blockIdx.x / cluster;
+  const long long teams = THREADS == 32 ? static_cast<long long>(gridDim.x) * kTeams : gridDim.x / cluster;
+  const int rank = THREADS == 32 ? 0 : static_cast<int>(blockIdx.x % cluster);
+  const int first = rank * K * THREADS + member;
+  const int width = static_cast<int>(args.width);
+  const T* weight = static_cast<const T*>(args.weight);
+  const T* bias = static_cast<const T*>(args.bias);
+
+  Vec<T, VEC> w[kInRegisters ? K : 1], b[kInRegisters ? K : 1];
+  T w_edge{}, b_edge{};
+  int kept_head = -1, parity = 0;
+  for (long long row = team; row < args.rows; row += teams, parity ^= 1) {
+    const T* in_row = static_cast<const T*>(args.in) + row * args.width;
+    OutT* out_row = static_cast<OutT*>(args.out) + row * args.width;
+    const int head = min(width, static_cast<int>((VEC - reinterpret_cast<uintptr_t>(in_row) / sizeof(T) % VEC) % VEC));
+    const int vectors = (width - head) / VEC, tail = width - head - vectors * VEC;
+    int edge = -1;
+    if (rank == 0 && member < head) edge = member;
+    if (rank == 0 && member >= VEC && member - VEC < tail) edge = head + vectors * VEC + member - VEC;
+
+    Vec<T, VEC> x[K];
+    T x_edge{};
+#pragma unroll
+    for (int j = 0; j < K; ++j) {
+      if (first + j * THREADS < vectors) x[j] = load_stream<T, VEC>(in_row + head + (first + j * THREADS) * VEC);
+    }
+    if (edge >= 0) x_edge = in_row[edge];
+    if constexpr (kScaled) {
+      if (head != kept_head) {
+        kept_head = head;
+        if (edge >= 0 && weight) w_edge = weight[edge];
+        if (edge >= 0 && bias) b_edge = bias[edge];
+#pragma unroll
+        for (int j = 0; j < K; ++j) {
+          if (first + j * THREADS < vectors) {
+            const int at = head + (first + j * THREADS) * VEC;
+            Vec<T, VEC> scale, shift;
+            if (weight) scale = load_shifted<T, VEC>(weight, at, width);
+            if (bias) shift = load_shifted<T, VEC>(bias, at, width);
+            if constexpr (kInRegisters) {
+              w[j] = scale;
+              b[j] = shift;
+            } else {
+              kept[(2 * j) * kThreads] = scale;
+              kept[(2 * j + 1) * kThreads] = shift;
+            }
+          }
+        }
+      }
+    }
+
+    auto fold_row = [&](float value, bool is_max, int stage) {
+      if constexpr (THREADS == 32) {
+        return is_max ? warp_fold<float, true>(value) : warp_fold<float, false>(value);
+      } else {
+        // (two sets of slots in turn: a CTA may write the next row's while a peer still reads this one's)
+        float* slot = slots[2 * stage + parity];
+        return is_max ? cluster_fold<float, true, THREADS / 32>(value, warp_scratch, slot, cluster)
+                      : cluster_fold<float, false, THREADS / 32>(value, warp_scratch, slot, cluster);
+      }
+    };
+    const float edge_value = to_compute(x_edge);
+    // f(element value, vector, element) for every element of the vectors this thread holds
+    auto each = [&](auto f) {
+#pragma unroll
+      for (int j = 0; j < K; ++j) {
+        if (first + j * THREADS < vectors) {
+#pragma unroll
+          for (int e = 0; e < VEC; ++e) f(widen(x[j], e), j, e);
+        }
+      }
+    };
+    // result(vector, element) rounded and stored
+    auto write = [&](auto result) {
+#pragma unroll
+      for (int j = 0; j < K; ++j) {
+        if (first + j * THREADS < vectors) {
+          Vec<OutT, VEC> y;
+          if constexpr (sizeof(OutT) == 2) {
+#pragma unroll
+            for (int e = 0; e < VEC; e += 2) {
+              const float low = result(j, e), high = result(j, e + 1);
+              store_pair(&y.v[e], make_float2(low, high));
+            }
+          } else {
+#pragma unroll
+            for (int e = 0; e < VEC; ++e) y.v[e] = from_compute<OutT, float>(result(j, e));
+          }
+          store_stream<OutT, VEC>(out_row + head + (first + j * THREADS) * VEC, y);
+        }
+      }
+    };
+
+    if constexpr (OP == kSoftmax) {
+      float local = edge >= 0 ? edge_value : -std::numeric_limits<float>::infinity();
+      each([&](float v, int, int) { local = nan_max(local, v); });
+      const float row_max = fold_row(local, true, 0);
+      const float edge_exp = edge >= 0 ? ragged_exp<T>(edge_value - row_max) : 0.f;
+      float sum = edge_exp;
+      each([&](float v, int j, int e) {
+        const float value = ragged_exp<T>(v - row_max);
+        sum += value;
+        if constexpr (sizeof(T) == 4) x[j].v[e] = value;
+      });
+      const float inverse = 1.f / fold_row(sum, false, 1);
+      write([&](int j, int e) { return (sizeof(T) == 4 ? widen(x[j], e) : ragged_exp<T>(widen(x[j], e) - row_max)) * inverse; });
+      if (edge >= 0) out_row[edge] = from_compute<OutT, float>(edge_exp * inverse);
+    } else {
+      float mean = 0.f;
+      if constexpr (OP == kLayerNorm) {
+        float sum = edge >= 0 ? edge_value : 0.f;
+        each([&](float v, int, int) { sum += v; });
+        mean = fold_row(sum, false, 0) / static_cast<float>(width);
+      }
+      float squares = edge >= 0 ? (edge_value - mean) * (edge_value - mean) : 0.f;
+      each([&](float v, int, int) { squares += (v - mean) * (v - mean); });
+      const float variance = fold_row(squares, false, 1) / static_cast<float>(width);
+      const float rstd = 1.f / sqrtf(variance + static_cast<float>(args.eps));
+      if (first == 0) {
+        if constexpr (OP == kLayerNorm) store_stat<T>(args.mean, row, mean, args.stat_is_f32);
+        store_stat<T>(args.rstd, row, rstd, args.stat_is_f32);
+      }
+      auto finish = [&](float v, float scale, float shift) {
+        float value = (v - mean) * rstd;
+        if (weight) value *= scale;
+        if (bias) value += shift;
+        return value;
+      };
+      Vec<T, VEC> scale, shift;
+      write([&](int j, int e) {
+        if constexpr (kInRegisters) return finish(widen(x[j], e), widen(w[j], e), widen(b[j], e));
+        if (e == 0 && weight) scale = kept[(2 * j) * kThreads];
+        if (e == 0 && bias) shift = kept[(2 * j + 1) * kThreads];
+        return finish(widen(x[j], e), widen(scale, e), widen(shift, e));
+      });
+      if (edge >= 0) out_row[edge] = from_compute<OutT, float>(finish(edge_value, to_compute(w_edge), to_compute(b_edge)));
+    }
+  }
+}
+
 // Any width, any alignment: one CTA per row, scalar loads, the row re-read for each statistic.
 template <typename T, typename OutT, int OP>
 __global__ void __launch_bounds__(kBlock) row_loop_kernel(RowArgs args) {
@@ -475,6 +677,61 @@ tq_status run_vector(const RowArgs& args, cudaStream_t stream, bool* handled) {
   return launch_rows(row_cluster_kernel<T, OutT, VEC, 8, OP>, blocks, cluster, stream, args, "row_cluster_kernel");
 }
 
+template <typename T, typename OutT, int VEC, int K, int OP, int THREADS>
+tq_status launch_ragged(const RowArgs& args, int cluster, cudaStream_t stream) {
+  constexpr int kTeams = THREADS == 32 ? kWarps : 1, kThreads = THREADS * kTeams;
+  constexpr size_t kSmem = OP != kSoftmax && K > 2 ? 2 * K * kThreads * sizeof(Vec<T, VEC>) : 0;
+  auto kernel = row_ragged_kernel<T, OutT, VEC, K, OP, THREADS>;
+  if (kSmem > 48 * 1024) TQ_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmem)));
+  int device = 0, resident = 0;
+  TQ_CUDA(cudaGetDevice(&device));
+  TQ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&resident, kernel, kThreads, kSmem));
+  // As many teams as run at once (or as there are rows), a multiple of VEC of them.
+  const long long wanted = (args.rows + kTeams - 1) / kTeams, room = static_cast<long long>(sm_count(device)) * (resident > 0 ? resident : 1) / cluster;
+  long long groups = wanted < room ? wanted : room;
+  groups = (groups + VEC - 1) / VEC * VEC;
+  cudaLaunchConfig_t config = {};
+  config.gridDim = dim3(static_cast<unsigned>(groups * cluster));
+  config.blockDim = dim3(kThreads);
+  config.dynamicSmemBytes = kSmem;
+  config.stream = stream;
+  cudaLaunchAttribute attribute[1];
+  attribute[0].id = cudaLaunchAttributeClusterDimension;
+  attribute[0].val.clusterDim.x = cluster;
+  attribute[0].val.clusterDim.y = 1;
+  attribute[0].val.clusterDim.z = 1;
+  config.attrs = attribute;
+  config.numAttrs = cluster > 1 ? 1 : 0;
+  TQ_CUDA(cudaLaunchKernelEx(&config, kernel, args, cluster));
+  return check_launch("row_ragged_kernel");
+}
+
+// Rows that are not made of aligned vectors, when the result's vectors fall where the input's do and weight
+// and bias are aligned themselves.
+template <typename T, typename OutT, int VEC, int OP>
+tq_status run_ragged(const RowArgs& args, cudaStream_t stream, bool* handled) {
+  *handled = true;
+  const long long vectors = args.width / VEC;
+  const bool scales = (args.weight == nullptr || aligned_to(args.weight, 16)) && (args.bias == nullptr || aligned_to(args.bias, 16));
+  const bool in_step = scales && reinterpret_cast<uintptr_t>(args.in) / sizeof(T) % VEC == reinterpret_cast<uintptr_t>(args.out) / sizeof(OutT) % VEC;
+  // Four vectors a thread up to 1024 of them: 20000 x 2003 bf16 LayerNorm / softmax 40 / 34 us with 64 threads
+  // against 60 / 44 with 32 that hold eight, 5000 x 8003 40 / 37 with 256 against 44 / 39; but 80000 x 1003 88 / 79
+  // with 64 that hold two against 80 / 63 with 32 that hold four.
+  if (in_step) {
+    if (vectors <= 32) return launch_ragged<T, OutT, VEC, 1, OP, 32>(args, 1, stream);
+    if (vectors <= 64) return launch_ragged<T, OutT, VEC, 2, OP, 32>(args, 1, stream);
+    if (vectors <= 128) return launch_ragged<T, OutT, VEC, 4, OP, 32>(args, 1, stream);
+    if (vectors <= 256) return launch_ragged<T, OutT, VEC, 4, OP, 64>(args, 1, stream);
+    if (vectors <= 512) return launch_ragged<T, OutT, VEC, 4, OP, 128>(args, 1, stream);
+    if (vectors <= 1024) return launch_ragged<T, OutT, VEC, 4, OP, 256>(args, 1, stream);
+    for (int cluster = 1; cluster <= kMaxCluster; cluster *= 2) {
+      if (vectors <= static_cast<long long>(kBlock) * kMaxVectors * cluster) return launch_ragged<T, OutT, VEC, 8, OP, kBlock>(args, cluster, stream);
+    }
+  }
+  *handled = false;
+  return TQ_OK;
+}
+
 template <typename T, typename OutT, int OP>
 tq_status run_rows(const RowArgs& args, cudaStream_t stream) {
   if constexpr (!std::is_same_v<T, double>) {
@@ -487,6 +744,10 @@ tq_status run_rows(const RowArgs& args, cudaStream_t stream) {
     if (vectorisable) {
       bool handled = false;
       if (tq_status s = run_vector<T, OutT, kVec, OP>(args, stream, &handled)) return s;
+      if (handled) return TQ_OK;
+    } else {
+      bool handled = false;
+      if (tq_status s = run_ragged<T, OutT, kVec, OP>(args, stream, &handled)) return s;
       if (handled) return TQ_OK;
     }
   }
