@@ -397,7 +397,15 @@ reduce_cta_per_slice(const T* __restrict__ in, typename R::Out* __restrict__ out
 // inner > 1. Thread layout: tx = threadIdx.x % lanes_x runs along inner (VEC columns each),
 // ty = threadIdx.x / lanes_x along reduce. grid = (column tiles, split, outer); the cluster, when
 // there is one, runs along grid.y.
-template <typename T, typename R, int VEC, bool RING>
+//
+// RAGGED (with the ring and 32 lanes): rows that do not start on a vector's boundary, because inner is odd or
+// the tensor starts in between. A warp takes every eighth row, and eight rows of any width are a whole number
+// of 16-byte units, so all rows of a warp have their vectors at the same place: `before` columns to the
+// left of the tile's first. A tile is 31 vectors wide and the 32 lanes cover it wherever that is; what they
+// read beside it are elements of its neighbours, gathered and never used. Only a vector that would begin before
+// the tensor (its first row) or end behind it (its last) is read column by column. Rows of odd length used
+// to be read an element, or four bytes, a lane: 40256 x 709 bf16 44.6 us a reduction where the bytes take 8.8.
+template <typename T, typename R, int VEC, bool RING, bool RAGGED = false>
 __global__ void __launch_bounds__(kBlock, sizeof(typename R::Acc) > 8 ? 4 : 5)
 reduce_columns(const T* __restrict__ in, typename R::Out* __restrict__ out, long long reduce,
                long long inner, int lanes_x, int split, int cluster, int mean,
@@ -413,13 +421,21 @@ reduce_columns(const T* __restrict__ in, typename R::Out* __restrict__ out, long
   const int lanes_y = kBlock / lanes_x;
   const long long slice = blockIdx.z;
   const int part = blockIdx.y;
-  const long long column = (static_cast<long long>(blockIdx.x) * lanes_x + tx) * VEC;
-  const bool in_range = column < inner;
+  const int tile_columns = RAGGED ? (lanes_x - 1) * VEC : lanes_x * VEC;
+  const long long first_column = static_cast<long long>(blockIdx.x) * tile_columns;
 
   long long chunk = (reduce + split - 1) / split;
   const long long begin = static_cast<long long>(part) * chunk;
   long long end = begin + chunk;
   if (end > reduce) end = reduce;
+
+  int before = 0;
+  if constexpr (RAGGED) {
+    const T* row_start = in + (slice * reduce + begin + ty) * inner + first_column;
+    before = static_cast<int>(reinterpret_cast<uintptr_t>(row_start) / sizeof(T) % VEC);
+  }
+  const long long column = first_column + tx * VEC - before;       // of this thread's vectors
+  const bool in_range = column < inner;
 
   typename R::template Local<1> local[VEC];
 #pragma unroll
@@ -442,8 +458,28 @@ reduce_columns(const T* __restrict__ in, typename R::Out* __restrict__ out, long
       Vec<T, VEC>* ring = reinterpret_cast<Vec<T, VEC>*>(cluster_scratch + lanes_x * VEC) + threadIdx.x;     // slot d at + d * kBlock
       const uint32_t ring_address = static_cast<uint32_t>(__cvta_generic_to_shared(ring));
       constexpr uint32_t kSlotBytes = static_cast<uint32_t>(kBlock) * kBytes;
-      const long long first = begin + ty;
-      const int count = first < end ? static_cast<int>((end - first + lanes_y - 1) / lanes_y) : 0;   // the host keeps this below 2^31
+      long long first = begin + ty;
+      int count = first < end ? static_cast<int>((end - first + lanes_y - 1) / lanes_y) : 0;   // the host keeps this below 2^31
+      // (RAGGED) the row whose vector would leave the tensor: column by column
+      auto by_columns = [&](long long row) {
+#pragma unroll
+        for (int e = 0; e < VEC; ++e) {
+          if (column + e >= 0 && column + e < inner) R::template step<1>(local[e], base[row * inner + e], row);
+        }
+      };
+      bool leaves = false;
+      if constexpr (RAGGED) {
+        const long long at = slice * reduce * inner + column;      // element of the tensor, of the vector in row 0
+        if (count > 0 && at + first * inner < 0) {
+          by_columns(first);
+          first += lanes_y;
+          --count;
+        }
+        if (count > 0 && at + (first + static_cast<long long>(count - 1) * lanes_y) * inner + VEC > static_cast<long long>(gridDim.z) * reduce * inner) {
+          leaves = true;
+          --count;
+        }
+      }
       const T* source = base + first * inner;
       const long long stride = static_cast<long long>(lanes_y) * inner;
       long long ri = first;
@@ -494,6 +530,9 @@ reduce_columns(const T* __restrict__ in, typename R::Out* __restrict__ out, long
 #pragma unroll
         for (int e = 0; e < VEC; ++e) R::template set_count<1>(local[e], count);
       }
+      if constexpr (RAGGED) {
+        if (leaves) by_columns(first + static_cast<long long>(count) * lanes_y);
+      }
     } else {
       for (long long r = begin + ty; r < end; r += static_cast<long long>(lanes_y) * UNROLL) {
         Vec<T, VEC> x[UNROLL];
@@ -523,10 +562,17 @@ reduce_columns(const T* __restrict__ in, typename R::Out* __restrict__ out, long
 #pragma unroll
   for (int e = 0; e < VEC; ++e) acc[e] = R::template to_acc<1>(local[e]);
 #pragma unroll
-  for (int e = 0; e < VEC; ++e) rows_scratch[(ty * lanes_x + tx) * VEC + e] = acc[e];
+  for (int e = 0; e < VEC; ++e) {
+    const int item = tx * VEC + e - before;
+    if (!RAGGED || (item >= 0 && item < tile_columns)) rows_scratch[ty * lanes_x * VEC + item] = acc[e];
+  }
   __syncthreads();
-  const bool holder = ty == 0;
+  const bool holder = ty == 0 && (!RAGGED || tx < lanes_x - 1);
   if (holder) {
+    if constexpr (RAGGED) {
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) acc[e] = rows_scratch[tx * VEC + e];
+    }
     for (int y = 1; y < lanes_y; ++y) {
 #pragma unroll
       for (int e = 0; e < VEC; ++e) {
@@ -543,7 +589,9 @@ reduce_columns(const T* __restrict__ in, typename R::Out* __restrict__ out, long
   const int slice_items = items / cluster;  // a multiple of VEC: cluster <= lanes_x, both powers of 2
   unsigned rank = 0;
   typename R::Out* out_row = out + slice * inner;
-  const long long tile_column = static_cast<long long>(blockIdx.x) * items;
+  const long long tile_column = first_column;
+  // what of the tile's items is a column of this tile
+  const long long live = inner - tile_column < tile_columns ? inner - tile_column : tile_columns;
   const int clusters = split / cluster;
   const long long tile = slice * gridDim.x + blockIdx.x;
   Acc* tile_partials = partials + tile * clusters * items;
@@ -564,7 +612,7 @@ reduce_columns(const T* __restrict__ in, typename R::Out* __restrict__ out, long
       for (int j = 1; j < cluster; ++j) total = R::combine(total, cluster_scratch[j * slice_items + threadIdx.x]);
       const int item = rank * slice_items + threadIdx.x;
       if (clusters == 1) {
-        if (tile_column + item < inner) out_row[tile_column + item] = R::finish(total, reduce, mean != 0);
+        if (item < live) out_row[tile_column + item] = R::finish(total, reduce, mean != 0);
       } else {
         tile_partials[(part / cluster) * items + item] = total;
       }
@@ -572,9 +620,11 @@ reduce_columns(const T* __restrict__ in, typename R::Out* __restrict__ out, long
     if (clusters == 1) return;
   } else {
     if (clusters == 1) {
-      if (holder && in_range) {
+      if (holder) {
 #pragma unroll
-        for (int e = 0; e < VEC; ++e) out_row[column + e] = R::finish(acc[e], reduce, mean != 0);
+        for (int e = 0; e < VEC; ++e) {
+          if (tx * VEC + e < live) out_row[tile_column + tx * VEC + e] = R::finish(acc[e], reduce, mean != 0);
+        }
       }
       return;
     }
@@ -597,7 +647,7 @@ reduce_columns(const T* __restrict__ in, typename R::Out* __restrict__ out, long
   if (!is_last) return;
   __threadfence();
   for (int item = threadIdx.x; item < items; item += kBlock) {
-    if (tile_column + item >= inner) continue;
+    if (item >= live) continue;
     Acc total = R::identity();
     for (int j = 0; j < clusters; j += 4) {
       Acc batch[4];
@@ -849,6 +899,7 @@ struct Plan {
   int lanes_x = 32;   // columns kernel: threads along inner
   int vec = 1;        // columns kernel: elements per thread along inner
   bool ring = false;  // columns kernel: stream through the per-thread cp.async ring
+  bool ragged = false;   // columns kernel: rows that do not start on a vector's boundary
   long long tiles = 0;        // ticketed outputs: slices, or outer * column tiles
   long long column_tiles = 0;
   size_t acc_bytes = 0;
@@ -903,7 +954,7 @@ int floor_pow2(long long v) {
 }
 
 Plan plan(tq_reduce_op op, tq_dtype dtype, long long outer, long long reduce, long long inner,
-          int32_t device, int vec_bytes_limit) {
+          int32_t device, int vec_bytes_limit, bool may_be_ragged = true) {
   Plan p;
   const int size = dtype_size(dtype);
   const int sms = sm_count(device);
@@ -940,6 +991,11 @@ Plan plan(tq_reduce_op op, tq_dtype dtype, long long outer, long long reduce, lo
     if (vec < 1) vec = 1;
     while (vec > 1 && inner % vec != 0) vec /= 2;
     if ((op == TQ_ARGMAX || op == kOpMoments) && vec > 4) vec = 4;  // their per-column state is large; 16-byte loads measured no better (argmax) or worse (moments)
+    // Rows no whole vector fits go to the ragged form, unless they are so short that most of its lanes would
+    // have no column, or the pass is one of statistics (their callers ask for whole vectors).
+    const int whole = (op == TQ_ARGMAX ? 4 : 8) < 16 / size ? (op == TQ_ARGMAX ? 4 : 8) : 16 / size;
+    p.ragged = may_be_ragged && vec < whole && (size == 2 || size == 4) && op < kOpSoftmaxStat && inner >= 12 * whole && reduce < (1ll << 31);
+    if (p.ragged) vec = whole;
     p.vec = vec;
     long long groups = (inner + vec - 1) / vec;
     // A warp reads 32 vectors (512 bytes) of one row; the CTA's 8 warps read 8 consecutive rows.
@@ -947,15 +1003,17 @@ Plan plan(tq_reduce_op op, tq_dtype dtype, long long outer, long long reduce, lo
     // loads, 64 lanes along `inner` and one wave of CTAs; 2-byte types and argmax (whose state
     // costs registers) with the cp.async ring and 32 lanes.
     p.ring = (size <= 2 || op == TQ_ARGMAX || op >= kOpSoftmaxStat) && reduce < (1ll << 31);   // the ring counts a thread's rows in 32 bits
+    if (p.ragged) p.ring = true;
     int lanes = p.ring ? 32 : 64;
-    while (lanes > 1 && lanes / 2 >= groups) lanes /= 2;
+    while (lanes > 1 && lanes / 2 >= groups && !p.ragged) lanes /= 2;
     p.lanes_x = lanes;
-    p.column_tiles = (groups + lanes - 1) / lanes;
+    p.column_tiles = p.ragged ? (inner + (lanes - 1) * vec - 1) / ((lanes - 1) * vec) : (groups + lanes - 1) / lanes;
     const long long base_ctas = p.column_tiles * outer;
     // One or two waves of CTAs (all of a wave resident at once, equal work each).
     const int waves = (p.ring && !(op == TQ_ARGMAX && size <= 2)) ? 2 : 1;
     long long want = (target_ctas * waves + base_ctas - 1) / base_ctas;
-    const long long per_pass = static_cast<long long>(kBlock / lanes) * kUnroll;
+    // (the ragged form: at least twice the ring's depth of rows a thread; 5003 x 1250 bf16 split finer is all folding)
+    const long long per_pass = static_cast<long long>(kBlock / lanes) * (p.ragged ? 2 * kRingDepth : kUnroll);
     long long most = reduce / per_pass;
     if (most < 1) most = 1;
     if (want > most) want = most;
@@ -1053,6 +1111,13 @@ tq_status run(const Plan& p, const void* in, void* out, long long outer, long lo
         return check_launch("reduce_columns");
       };
       constexpr int kColumnVec = kVec > 8 ? 8 : kVec;
+      if (p.ragged) {
+        if constexpr (sizeof(T) == 2 || sizeof(T) == 4) {
+          constexpr int kWhole = std::is_same_v<Acc, Indexed<typename Compute<T>::type>> ? 4 : kColumnVec;
+          return p.vec == kWhole ? go(reduce_columns<T, R, kWhole, true, true>, kWhole)
+                                 : fail(TQ_INTERNAL, "no ragged column kernel for %d elements per thread", p.vec);
+        }
+      }
       if (p.vec == 1) return p.ring ? go(reduce_columns<T, R, 1, true>, 1) : go(reduce_columns<T, R, 1, false>, 1);
       if constexpr (kColumnVec >= 2) {
         if (p.vec == 2) return p.ring ? go(reduce_columns<T, R, 2, true>, 2) : go(reduce_columns<T, R, 2, false>, 2);
@@ -1305,8 +1370,9 @@ tq_status tq_reduce_launch_static(tq_reduce_op op, tq_dtype dtype, const void* i
   TQ_REQUIRE(tq::aligned_to(in, size), TQ_INVALID_ARGUMENT, "input pointer is not aligned to its element type");
   tq::DeviceScope device_scope(device);
   if (tq_status s = device_scope.status()) return s;
-  const tq::Plan p = tq::plan(op, dtype, outer, reduce, inner, device,
-                              inner == 1 ? 16 : tq::column_vec_bytes(in, inner, size));
+  const int limit = inner == 1 ? 16 : tq::column_vec_bytes(in, inner, size);
+  tq::Plan p = tq::plan(op, dtype, outer, reduce, inner, device, limit);
+  if (p.partial_bytes + p.ticket_bytes > tq::kStaticScratchBytes) p = tq::plan(op, dtype, outer, reduce, inner, device, limit, false);
   const size_t need = p.partial_bytes + p.ticket_bytes;
   TQ_REQUIRE(need <= tq::kStaticScratchBytes, TQ_RESOURCE_EXHAUSTED,
              "this reduction needs %zu bytes of scratch; the built-in scratch of tq_reduce_launch_static holds %zu. "

@@ -961,3 +961,96 @@ def test_config_2_full_size_pack_round_trip(tq):
     again = tq.contiguous(packed.t())          # transposing twice is the identity, bit for bit
     assert torch.equal(again, xd)
     assert torch.equal(packed[::517].cpu(), x.t()[::517])
+
+
+def _inside(t, shift):
+    """The same values starting `shift` elements into an allocation."""
+    held = torch.empty(t.numel() + 16, dtype=t.dtype, device="cuda")
+    view = held[shift:shift + t.numel()].view(t.shape)
+    view.copy_(t)
+    return view
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("rows, width", [(5, 1), (40, 3), (11, 9), (70, 33), (300, 515), (61, 1003), (4000, 1021), (19, 2051), (13, 4099),
+                                         (9, 8201), (9, 16390), (5, 33001), (3, 131071), (2, 140001)])
+def test_rows_that_start_between_vectors(tq, dtype, rows, width):
+    """Every team size of the ragged row kernel, from rows without a whole vector to rows beyond a cluster's
+    registers; 4000 rows: a team takes several. The third shift puts weight and bias off their boundaries too,
+    which the loop kernel takes."""
+    g = torch.Generator().manual_seed(rows * width)
+    x = (torch.randn(rows, width, generator=g) * 2 + 0.5).to(dtype)
+    w, b = (1 + torch.randn(width, generator=g) * 0.1).to(dtype), (torch.randn(width, generator=g) * 0.1).to(dtype)
+    close = close32 if dtype == torch.float32 else close16
+    for shift, weight_shift in ((0, 0), (1, 0), (3, 1)):
+        xd, wd, bd = _inside(x, shift), _inside(w, weight_shift), _inside(b, weight_shift)
+        close(tq.softmax(xd, -1), tessiq0.softmax(x, -1))
+        y, mean, rstd = tq.native_layer_norm(xd, [width], wd, bd, 1e-5)
+        exact = torch.nn.functional.layer_norm(x.double(), [width], w.double(), b.double(), 1e-5)
+        if width > 1:
+            scale = exact.abs().max().item()
+            # one rounding of the result, and f32 statistics over `width` elements
+            bound = {torch.float32: 0.0, torch.bfloat16: 2.0**-8, torch.float16: 2.0**-11}[dtype]
+            assert ((y.cpu().double() - exact).abs() <= bound * exact.abs() + 2e-6 * scale + 1e-6).all()
+            assert torch.allclose(mean.cpu().double().flatten(), x.double().mean(-1), rtol=2 * bound + 1e-5, atol=1e-5)
+        close(tq.layer_norm(xd, [width], None, None, 1e-5), torch.nn.functional.layer_norm(x.double(), [width], eps=1e-5).to(dtype))
+        if width > 1:
+            exact = x.double() * torch.rsqrt(x.double().square().mean(-1, keepdim=True) + 1e-5) * w.double()
+            close(tq.rms_norm(xd, wd, 1e-5), exact.to(dtype))
+    if dtype != torch.float32:
+        close32(tq.softmax(_inside(x, 1), -1, half_to_float=True), torch.softmax(x.double(), -1).float(), rtol=1e-5, scale=1e-5)
+
+
+def test_ragged_rows_with_special_values(tq):
+    x = torch.randn(6, 1003, generator=torch.Generator().manual_seed(2))
+    x[1, 17] = float("nan")
+    x[2] = float("-inf")
+    x[3, 1002] = float("inf")
+    x[4] = 1e30
+    x[5, :1000] = float("-inf")
+    for t in (x, x.bfloat16()):
+        got = tq.softmax(dev(t), -1).cpu()
+        torch.testing.assert_close(got, tessiq0.softmax(t, -1), rtol=1e-5 if t is x else 1e-2, atol=1e-7, equal_nan=True)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16, torch.int32])
+@pytest.mark.parametrize("shape, dim", [((1003, 205), 0), ((5003, 1250), 0), ((3, 129, 997), 1), ((7, 96), 0), ((700, 249), 0), ((9, 3001), 0),
+                                        ((40000, 131), 0), ((2, 300, 104), 1)])
+def test_columns_of_rows_that_start_between_vectors(tq, dtype, shape, dim):
+    """The ragged columns kernel: tiles of 31 vectors at the tile's edges, a first and a last row whose vectors
+    would leave the tensor, starts between vectors (with them also widths that are whole vectors), more warps
+    than rows, and splits with and without tickets."""
+    g = torch.Generator().manual_seed(shape[-1])
+    x = (torch.randn(*shape, generator=g) * 50).to(dtype)
+    for shift in (0, 1, 2, 5):
+        xd = _inside(x, shift)
+        assert torch.equal(tq.amax(xd, dim).cpu(), x.amax(dim)) and torch.equal(tq.amin(xd, dim).cpu(), x.amin(dim))
+        index = tq.argmax(xd, dim).cpu()
+        # the lowest index of the largest value
+        assert torch.equal(index, (x == x.amax(dim, keepdim=True)).int().argmax(dim))
+        total = tq.sum(xd, dim).cpu()
+        if dtype == torch.int32:
+            assert torch.equal(total, x.long().sum(dim))
+            continue
+        bound = {torch.float32: 0.0, torch.bfloat16: 2.0**-8, torch.float16: 2.0**-11}[dtype]
+        exact, budget = x.double().sum(dim), 1e-6 * x.double().abs().sum(dim)      # f32 sums in a tree, one rounding of the result
+        finite = exact.abs() < 60000 if dtype == torch.float16 else torch.ones_like(exact, dtype=torch.bool)
+        assert ((total.double() - exact).abs() <= bound * exact.abs() + budget)[finite].all()
+        mean = tq.mean(xd, dim).cpu().double()
+        assert ((mean - exact / x.shape[dim]).abs() <= bound * (exact / x.shape[dim]).abs() + budget / x.shape[dim] + 1e-7).all()
+    special = x.clone() if dtype != torch.int32 else None
+    if special is not None:
+        special.view(-1)[-3] = float("nan")
+        special.view(-1)[1] = float("inf")
+        got, expected = tq.amax(_inside(special, 1), dim).cpu(), special.amax(dim)
+        torch.testing.assert_close(got, expected, rtol=0, atol=0, equal_nan=True)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.uint8, torch.float64])
+@pytest.mark.parametrize("rows, cols", [(1, 70), (63, 65), (64, 129), (709, 403), (2, 3)])
+def test_transposes_that_fill_no_whole_tile(tq, dtype, rows, cols):
+    if dtype == torch.uint8:
+        x = torch.randint(0, 2, (3, rows, cols)).bool()
+    else:
+        x = torch.randn(3, rows, cols).to(dtype)
+    assert torch.equal(tq.contiguous(_inside(x, 1).transpose(1, 2)).cpu(), x.transpose(1, 2))
