@@ -2,39 +2,44 @@
 //
 //   out[b,h,i,:] = sum_j softmax_j(scale * q[b,h,i,:] . k[b,h,j,:]) v[b,h,j,:]     (j <= i when causal)
 //
-// bf16 or f16 operands with 64-element heads, f32 scores and sums, one rounding of the result. The
-// score matrix never leaves the SM: one CTA owns 256 query rows of one head (two tiles of 128) and
-// walks the keys 128 at a time with a row reference point and row sum (the online form of softmax).
+// bf16 or f16 operands, heads of up to 128 elements, f32 scores and sums, one rounding of the result. The
+// score matrix never leaves the SM: one CTA owns 128 query rows of one head and walks the keys 64 at a time
+// with a row reference point and row sum (the online form of softmax).
 //
-//   warps 0..3 / 4..7   one softmax group per query tile, one thread per query row: tcgen05.ld of
-//                       the row's 128 f32 scores (held in registers for both the maximum and the
-//                       exponentials), ex2, row sum; the probabilities go back into tensor memory
-//                       with tcgen05.st as packed bf16/f16 pairs — the A operand of the second
-//                       product. The result accumulates in tensor memory across the steps and is
-//                       read once, at the end.
-//   warp 8, one lane    producer: TMA loads (128-byte swizzle) of the two query tiles once, then one
-//                       128 x 64 key tile and one value tile per step into two 4-stage rings; the
-//                       first loads leave before the CTA's set-up barrier.
-//   warps 9 and 10,     issuers, one per group: S = Q K^T (128 x 128 x 64, both operands K-major in
-//   one lane each       shared memory) and O = P V (128 x 64 x 128, P from tensor memory, V consumed
-//                       MN-major exactly as it lies in memory). A tcgen05.mma costs its issuing
-//                       thread about a hundred cycles and a step needs twelve, so one thread for
-//                       both groups was the bottleneck; with one each, no group waits for the other.
+//   warps 0..3          softmax, one thread per query row: tcgen05.ld of the row's 64 f32 scores (held in
+//                       registers for both the maximum and the exponentials), ex2, row sum; the
+//                       probabilities go back into tensor memory with tcgen05.st as packed bf16/f16 pairs —
+//                       the A operand of the second product. The result accumulates in tensor memory
+//                       across the steps and is read once, at the end.
+//   warp 4, one lane    producer: TMA loads (128-byte swizzle) of the query tile once, then one key tile and
+//                       one value tile per step into two rings; the first filling leaves before the CTA's
+//                       set-up barrier.
+//   warp 5, one lane    issuer: S = Q K^T (128 x 64 x head, both operands K-major in shared memory) and
+//                       O = P V (128 x head x 64, P from tensor memory, V consumed MN-major exactly as it
+//                       lies in memory). The scores of step j + 1 are computed while the softmax warps work
+//                       on step j, which hand the columns back as soon as they have them in registers.
 //
 // softmax is exp(s - m) / sum exp(s - m) for ANY m, so a row keeps the maximum of its first key tile
 // as its reference point and moves it only when a later tile rises more than 2^8 above it — then,
-// and only then, the row's sum and its 64 accumulators in tensor memory are rescaled (a warp-wide
+// and only then, the row's sum and its accumulators in tensor memory are rescaled (a warp-wide
 // slow path, rare on real data). Without that, nothing is read back per step: the second product
 // accumulates O += P V in place. Probabilities are at most 2^8, well inside bf16 and f16.
 //
-// Each group has 256 columns of tensor memory: the scores (0..127), the probabilities as packed
-// pairs (128..191) and the result (192..255). A group takes its scores into registers at the start
-// of a step and hands the columns back at once, so the scores of step j + 1 are computed while the
-// group is still working on step j. The softmax groups run with 224
-// registers per thread, the other four warps with 56 (setmaxnreg). Q, K, V and
-// the result are addressed through (batch, head, token) strides, so the three slices of a fused QKV
-// projection are read in place and the result is written directly in [batch, token, head, 64] order:
-// none of the four packing copies around `bmm -> where -> softmax -> bmm` remains.
+// What bounds it: a step of one CTA is a chain (scores seen, tcgen05.ld, maximum, ex2, tcgen05.st, signal) of about
+// 1 500 cycles of which the special-function unit works 512, so an SM needs several chains. Three CTAs of one
+// softmax warp per scheduler each (two for heads above 64) keep the unit busy 65 % of the time, and one CTA's
+// start and end run under the others' steps. One CTA an SM with two groups of 128 rows and 128-key steps, as it
+// was, spent 5 000 cycles on every start: 64 x 12 heads, 1024 tokens of 64 causal 256 -> 225 us, no mask 377 -> 320,
+// 4 x 12 x 4096 no mask 332 -> 312; 64 x 6 heads of 128, whose second group had idled, 235 -> 175.
+// Measured beside it: two CTAs with two groups each and the probabilities over the scores (four chains, each
+// with both products inside it) 216 / 307 / 312 / 205; one exponential in four, or in sixteen, as a polynomial of
+// degree 5 on the FMA pipes 328 and 322 instead of 312; scalar instead of two-element FMA and add 311 - 318; the
+// row sum after the signal 333; skipping the rows past the diagonal of a whole warp: no change.
+//
+// The softmax warps run with 120 registers per thread (200 for wide heads), the other four with 40 (56)
+// (setmaxnreg). Q, K, V and the result are addressed through (batch, head, token) strides, so the three slices
+// of a fused QKV projection are read in place and the result is written directly in [batch, token, head, head_dim]
+// order: none of the four packing copies around `bmm -> where -> softmax -> bmm` remains.
 //
 // Every wait is bounded; a wait that gives up sets the device status word (tq_status_poll) and the
 // CTA leaves through the normal teardown, freeing its tensor memory. No load uses multicast.
@@ -55,38 +60,37 @@ namespace tq {
 namespace {
 
 constexpr int kHeadDim = 64;
-constexpr int kRows = 128;            // query rows per softmax group
-constexpr int kGroups = 2;            // query tiles per CTA
-constexpr int kKeys = 128;            // keys per step
-constexpr int kRing = 4;              // stages of the key ring and of the value ring
-constexpr int kAttnThreads = 384;     // 8 softmax warps; producer and issuer in a third group of four warps
-// setmaxnreg moves registers inside the CTA's own allocation (384 threads x 168 at launch): what the
-// third group of four warps gives up is exactly what the eight softmax warps take. An increase
-// beyond what was released would wait for ever.
-constexpr int kLaunchRegisters = 168, kSoftmaxRegisters = 224, kOtherRegisters = 56;
-static_assert(256 * (kSoftmaxRegisters - kLaunchRegisters) <= 128 * (kLaunchRegisters - kOtherRegisters),
-              "the softmax warps would wait for registers nobody releases");
-static_assert(kLaunchRegisters == (65536 / kAttnThreads) / 8 * 8, "ptxas gives a CTA of this size this many registers per thread");
-constexpr uint32_t kSubTileBytes = kRows * kHeadDim * 2;     // 16 KiB: 128 rows of 64 elements, one TMA box, one swizzled operand tile
-// Shared memory for heads of D elements (D = 64, or 128 = two sub-tiles side by side per tile): the
-// query tiles (two groups of 64-wide heads, or the one group of 128-wide heads: 32 KiB either way),
-// the key ring, the value ring, the barriers. Heads of 128 get three stages per ring: four would not fit.
+constexpr int kRows = 128;            // query rows per CTA
+constexpr int kKeys = 64;             // keys per step
+constexpr int kAttnThreads = 256;     // four softmax warps; producer and issuer in a second group of four
+constexpr uint32_t kQueryBytes = kRows * kHeadDim * 2;       // 16 KiB: 128 rows of 64 elements, one TMA box, one swizzled operand tile
+constexpr uint32_t kSubTileBytes = kKeys * kHeadDim * 2;     // 8 KiB: the same of 64 keys or values
+// Heads of up to 64 elements run three CTAs an SM, heads of up to 128 (two 64-wide sub-tiles side by side in
+// every tile) two. Shared memory: the query tile, the key ring, the value ring, the barriers. Tensor memory,
+// f32 columns: scores (64), packed probabilities (32), result (64 or 128). An allocation is a power of two, so
+// the narrow form takes two (scores and result, probabilities: 160 columns, and three CTAs have 480 of the 512)
+// and the wide one a single one of 256.
 template <int D>
 struct AttnLayout {
   static constexpr int kSubTiles = D / kHeadDim;
+  static constexpr int kCtasPerSm = D == kHeadDim ? 3 : 2;
+  static constexpr int kRing = D == kHeadDim ? 3 : 2;          // stages of the key ring and of the value ring
   static constexpr uint32_t kTileBytes = kSubTiles * kSubTileBytes;
-  static constexpr int kActiveGroups = D == kHeadDim ? kGroups : 1;
-  static constexpr int kRingStages = D == kHeadDim ? kRing : 3;
-  static constexpr uint32_t kOffsetQ = 0;
-  static constexpr uint32_t kOffsetK = kOffsetQ + kActiveGroups * kTileBytes;
-  static constexpr uint32_t kOffsetV = kOffsetK + kRingStages * kTileBytes;
-  static constexpr uint32_t kOffsetBarriers = kOffsetV + kRingStages * kTileBytes;
+  static constexpr uint32_t kOffsetK = kSubTiles * kQueryBytes;
+  static constexpr uint32_t kOffsetV = kOffsetK + kRing * kTileBytes;
+  static constexpr uint32_t kOffsetBarriers = kOffsetV + kRing * kTileBytes;
   static constexpr size_t kSmemBytes = 1024 + kOffsetBarriers + 256;
+  static constexpr uint32_t kTmemColumns = D == kHeadDim ? 128 : 256;      // scores from column 0 on
+  static constexpr uint32_t kColumnO = D == kHeadDim ? 64 : 128;
+  // setmaxnreg moves registers inside the CTA's own allocation: what the second group of four warps gives up is
+  // at least what the softmax warps take. An increase beyond what was released would wait for ever.
+  static constexpr int kLaunchRegisters = (65536 / kCtasPerSm / kAttnThreads) / 8 * 8;
+  static constexpr int kSoftmaxRegisters = D == kHeadDim ? 120 : 200, kOtherRegisters = D == kHeadDim ? 40 : 56;
+  static_assert(128 * (kSoftmaxRegisters - kLaunchRegisters) <= 128 * (kLaunchRegisters - kOtherRegisters),
+                "the softmax warps would wait for registers nobody releases");
 };
-static_assert(AttnLayout<128>::kSmemBytes <= 227 * 1024, "the wide-head staging has to fit one CTA's shared memory");
-constexpr uint32_t kAttnTmemColumns = 512;   // two groups x 256 columns
-constexpr uint32_t kGroupColumns = 256;      // of a group: scores 0..127, probabilities (packed pairs) 128..191, result 192..255 (192..319 for the one group of 128-wide heads)
-constexpr uint32_t kColumnP = 128, kColumnO = 192;
+static_assert(AttnLayout<64>::kSmemBytes <= 74 * 1024 && AttnLayout<128>::kSmemBytes <= 112 * 1024, "the staging has to fit as often as there are CTAs an SM");
+constexpr uint32_t kTmemColumnsP = 32;
 constexpr float kSlack = 8.f;                // a row's reference point moves when a tile's maximum is more than 2^kSlack above it
 
 enum AttnWait { kWaitQ = 201, kWaitKeyEmpty = 202, kWaitValueEmpty = 203, kWaitKeyFull = 204, kWaitValueFull = 205,
@@ -136,13 +140,13 @@ __device__ __forceinline__ uint32_t pack_pair(float low, float high) {
 }
 
 template <typename T, int D>
-__global__ void __launch_bounds__(kAttnThreads, 1)
+__global__ void __launch_bounds__(kAttnThreads, AttnLayout<D>::kCtasPerSm)
 attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                  const __grid_constant__ CUtensorMap map_v, const AttnParams p) {
   using L = AttnLayout<D>;
-  constexpr int kRing = L::kRingStages;                 // (hides the namespace's value: heads of 128 have three stages)
-  constexpr uint32_t kTileBytes = L::kTileBytes, kOffsetQ = L::kOffsetQ, kOffsetK = L::kOffsetK, kOffsetV = L::kOffsetV;
-  constexpr uint32_t kOffsetBarriers = L::kOffsetBarriers;
+  constexpr int kRing = L::kRing;
+  constexpr uint32_t kTileBytes = L::kTileBytes, kOffsetK = L::kOffsetK, kOffsetV = L::kOffsetV;
+  constexpr uint32_t kOffsetBarriers = L::kOffsetBarriers, kColumnO = L::kColumnO;
   constexpr int kSubTiles = L::kSubTiles;
   extern __shared__ unsigned char raw_smem[];
   const uint32_t base = (smem_address(raw_smem) + 1023u) & ~1023u;
@@ -154,11 +158,11 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
   auto k_empty = [&](int s) { return barriers + 8u * (1 + kRing + s); };
   auto v_full = [&](int s) { return barriers + 8u * (1 + 2 * kRing + s); };
   auto v_empty = [&](int s) { return barriers + 8u * (1 + 3 * kRing + s); };
-  auto s_full = [&](int g) { return barriers + 8u * (1 + 4 * kRing + g); };                   // the scores of a step are in tensor memory
-  auto s_free = [&](int g) { return barriers + 8u * (1 + 4 * kRing + kGroups + g); };          // ... and in the group's registers
-  auto p_full = [&](int g) { return barriers + 8u * (1 + 4 * kRing + 2 * kGroups + g); };      // the probabilities of a step are in tensor memory
-  auto pv_done = [&](int g) { return barriers + 8u * (1 + 4 * kRing + 3 * kGroups + g); };     // ... and the second product has consumed them
-  constexpr int kBarrierCount = 1 + 4 * kRing + 4 * kGroups;
+  const uint32_t s_full = barriers + 8u * (1 + 4 * kRing);      // the scores of a step are in tensor memory
+  const uint32_t s_free = s_full + 8;                           // ... and in the softmax warps' registers
+  const uint32_t p_full = s_full + 16;                          // the probabilities of a step are in tensor memory
+  const uint32_t pv_done = s_full + 24;                         // ... and the second product has consumed them
+  constexpr int kBarrierCount = 1 + 4 * kRing + 4;
   const uint32_t tmem_slot = barriers + 8u * kBarrierCount;
   volatile uint32_t* tmem_slot_pointer = reinterpret_cast<volatile uint32_t*>(aligned + kOffsetBarriers + 8 * kBarrierCount);
 
@@ -168,95 +172,80 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
   const int q_block = p.q_blocks - 1 - static_cast<int>(blockIdx.x % p.q_blocks);
   const int head_index = static_cast<int>(blockIdx.x / p.q_blocks);
   const int head = head_index % p.heads, batch = head_index / p.heads;
-  const int q0 = q_block * L::kActiveGroups * kRows;
+  const int q0 = q_block * kRows;
   const int key_tiles = (p.k_tokens + kKeys - 1) / kKeys;
-  // steps of group g: none when its rows lie beyond the queries; under a causal mask only the key
-  // tiles that hold a key <= its last row
-  int steps[kGroups];
-#pragma unroll
-  for (int g = 0; g < kGroups; ++g) {
-    const int first = q0 + g * kRows;
-    steps[g] = (g >= L::kActiveGroups || first >= p.q_tokens)
-                   ? 0 : (p.causal ? min(key_tiles, (min(first + kRows, p.q_tokens) - 1) / kKeys + 1) : key_tiles);
-  }
-  const int total_steps = max(steps[0], steps[1]);
+  // under a causal mask only the key tiles that hold a key <= the CTA's last row; at least one step
+  const int steps = p.causal ? min(key_tiles, (min(q0 + kRows, p.q_tokens) - 1) / kKeys + 1) : key_tiles;
 
-  // The producer lane sets the barriers up and sends the first loads (both query tiles, the first
-  // key and value tiles) on their way before the CTA meets: their latency runs under the
-  // tensor-memory allocation and the barrier.
-  const bool producer = threadIdx.x == 8 * 32;
-  if (producer) {
+  auto load_tile = [&](const CUtensorMap* map, uint32_t ring, uint32_t full, int j) {
+    barrier_expect_tx(full, kTileBytes);
+    for (int h = 0; h < kSubTiles; ++h)
+      tma_load_4d(base + ring + (j % kRing) * kTileBytes + h * kSubTileBytes, map, full, h * kHeadDim, j * kKeys, head, batch);
+  };
+
+  // The producer lane sets the barriers up and fills the rings for the first time before the CTA meets: the
+  // loads' latency runs under the tensor-memory allocation and the barrier.
+  const int early = min(steps, kRing);
+  if (warp == 4 && elect_one()) {
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_q) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_k) : "memory");
     asm volatile("prefetch.tensormap [%0];" ::"l"(&map_v) : "memory");
-    if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) p.status.begin();   // this launch's abort word starts clear
+    if (blockIdx.x == 0) p.status.begin();   // this launch's abort word starts clear
     barrier_init(q_full, 1);
     for (int s = 0; s < kRing; ++s) {
       barrier_init(k_full(s), 1);
-      barrier_init(k_empty(s), kGroups);      // each group hands a tile back once its product has read it
+      barrier_init(k_empty(s), 1);
       barrier_init(v_full(s), 1);
-      barrier_init(v_empty(s), kGroups);
+      barrier_init(v_empty(s), 1);
     }
-    for (int g = 0; g < kGroups; ++g) {
-      barrier_init(s_full(g), 1);
-      barrier_init(pv_done(g), 1);
-      barrier_init(p_full(g), kRows / 32);          // one arrival per warp of the group
-      barrier_init(s_free(g), kRows / 32);
-    }
+    barrier_init(s_full, 1);
+    barrier_init(pv_done, 1);
+    barrier_init(p_full, kRows / 32);          // one arrival per softmax warp
+    barrier_init(s_free, kRows / 32);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    if (total_steps > 0) {
-      int valid = 0;
-      for (int g = 0; g < kGroups; ++g) valid += steps[g] > 0 ? 1 : 0;
-      barrier_expect_tx(q_full, valid * kTileBytes);
-      for (int g = 0; g < kGroups; ++g) {
-        if (steps[g] > 0) {
-          for (int h = 0; h < kSubTiles; ++h)
-            tma_load_4d(base + kOffsetQ + g * kTileBytes + h * kSubTileBytes, &map_q, q_full, h * kHeadDim, q0 + g * kRows, head, batch);
-        }
-      }
-      barrier_expect_tx(k_full(0), kTileBytes);
-      for (int h = 0; h < kSubTiles; ++h) tma_load_4d(base + kOffsetK + h * kSubTileBytes, &map_k, k_full(0), h * kHeadDim, 0, head, batch);
-      barrier_expect_tx(v_full(0), kTileBytes);
-      for (int h = 0; h < kSubTiles; ++h) tma_load_4d(base + kOffsetV + h * kSubTileBytes, &map_v, v_full(0), h * kHeadDim, 0, head, batch);
+    barrier_expect_tx(q_full, kSubTiles * kQueryBytes);
+    for (int h = 0; h < kSubTiles; ++h) tma_load_4d(base + h * kQueryBytes, &map_q, q_full, h * kHeadDim, q0, head, batch);
+    for (int j = 0; j < early; ++j) {
+      load_tile(&map_k, kOffsetK, k_full(j), j);
+      load_tile(&map_v, kOffsetV, v_full(j), j);
     }
   }
-  if (warp == 9) tmem_alloc(tmem_slot, kAttnTmemColumns);
+  if (warp == 5) {
+    if constexpr (D == kHeadDim) {
+      tmem_alloc_more(tmem_slot, L::kTmemColumns);
+      tmem_alloc(tmem_slot + 4, kTmemColumnsP);
+    } else {
+      tmem_alloc(tmem_slot, L::kTmemColumns);
+    }
+  }
   tcgen05_fence_before();
   __syncthreads();
   tcgen05_fence_after();
-  const uint32_t tmem_base = *tmem_slot_pointer;
+  const uint32_t tmem_base = tmem_slot_pointer[0];
+  const uint32_t tmem_p = D == kHeadDim ? tmem_slot_pointer[1] : tmem_base + 64;
 
-  if (warp >= 8) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kOtherRegisters));
-  if (warp == 8) {
-    // ---- producer: the tiles of step 1 onwards (step 0's went out before the CTA met) ------------
+  if (warp >= 4) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(L::kOtherRegisters));
+  if (warp == 4) {
+    // ---- producer: what did not fit the first filling --------------------------------------------
     if (elect_one()) {
-      for (int j = 1; j < total_steps; ++j) {
+      for (int j = early; j < steps; ++j) {
         const int s = j % kRing;
         const uint32_t phase = (j / kRing) & 1;
         if (!barrier_wait(k_empty(s), phase ^ 1, p.status, kWaitKeyEmpty)) break;
-        barrier_expect_tx(k_full(s), kTileBytes);
-        for (int h = 0; h < kSubTiles; ++h)
-          tma_load_4d(base + kOffsetK + s * kTileBytes + h * kSubTileBytes, &map_k, k_full(s), h * kHeadDim, j * kKeys, head, batch);
+        load_tile(&map_k, kOffsetK, k_full(s), j);
         if (!barrier_wait(v_empty(s), phase ^ 1, p.status, kWaitValueEmpty)) break;
-        barrier_expect_tx(v_full(s), kTileBytes);
-        for (int h = 0; h < kSubTiles; ++h)
-          tma_load_4d(base + kOffsetV + s * kTileBytes + h * kSubTileBytes, &map_v, v_full(s), h * kHeadDim, j * kKeys, head, batch);
+        load_tile(&map_v, kOffsetV, v_full(s), j);
       }
     }
-  } else if (warp == 9 || warp == 10) {
-    // ---- issuers: warp 9 for group 0, warp 10 for group 1 -------------------------------------
-    // A tcgen05.mma costs its issuing thread on the order of a hundred cycles here, and a step is
-    // 12 of them plus two commits: one thread for both groups was the kernel's bottleneck. Each
-    // group's issuer follows its own group only, so neither group waits for the other.
-    const int g = warp - 9;
-    if (steps[g] > 0 && elect_one()) {
+  } else if (warp == 5) {
+    // ---- issuer ----------------------------------------------------------------------------------
+    if (elect_one()) {
       constexpr uint32_t idesc_s = attn_instruction_descriptor<T>(kKeys, false);
       constexpr uint32_t idesc_o = attn_instruction_descriptor<T>(kHeadDim, true);
       // Descriptors as (low, high) words: one constant high word, low words stepped by adds.
       constexpr uint32_t kHighWord = kDescriptorHigh;
-      const uint32_t low_q = descriptor_low(base + kOffsetQ + g * kTileBytes, 0), low_k = descriptor_low(base + kOffsetK, 0);
+      const uint32_t low_q = descriptor_low(base, 0), low_k = descriptor_low(base + kOffsetK, 0);
       const uint32_t low_v = descriptor_low(base + kOffsetV, kSubTileBytes);
-      const uint32_t columns = tmem_base + static_cast<uint32_t>(g) * kGroupColumns;
       // S(i) = Q K_i^T: both operands K-major, 16 elements of K = 32 B in the swizzle row
       auto scores = [&](int i) {
         const uint32_t k = low_k + (i % kRing) * (kTileBytes >> 4);
@@ -265,10 +254,10 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
         for (int h = 0; h < kSubTiles; ++h) {
 #pragma unroll
           for (int kk = 0; kk < kHeadDim / 16; ++kk)
-            mma_f16_split(columns, low_q + h * (kSubTileBytes >> 4) + kk * 2, kHighWord, k + h * (kSubTileBytes >> 4) + kk * 2, kHighWord, idesc_s,
+            mma_f16_split(tmem_base, low_q + h * (kQueryBytes >> 4) + kk * 2, kHighWord, k + h * (kSubTileBytes >> 4) + kk * 2, kHighWord, idesc_s,
                           (h != 0 || kk != 0) ? 1u : 0u);
         }
-        mma_commit(s_full(g));
+        mma_commit(s_full);
       };
       // O += P_i V_i (O = for the first step): P from tensor memory (16 keys = 8 columns), V MN-major
       // from shared memory (16 keys = 2048 B)
@@ -279,87 +268,72 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
         for (int h = 0; h < kSubTiles; ++h) {
 #pragma unroll
           for (int kk = 0; kk < kKeys / 16; ++kk)
-            mma_f16_tmem_a(columns + kColumnO + h * kHeadDim, columns + kColumnP + kk * 8, v + h * (kSubTileBytes >> 4) + kk * (2048 >> 4), kHighWord,
-                           idesc_o, (i != 0 || kk != 0) ? 1u : 0u);
+            mma_f16_tmem_a(tmem_base + kColumnO + h * kHeadDim, tmem_p + kk * 8, v + h * (kSubTileBytes >> 4) + kk * (2048 >> 4), kHighWord, idesc_o,
+                           (i != 0 || kk != 0) ? 1u : 0u);
         }
-        mma_commit(pv_done(g));
+        mma_commit(pv_done);
       };
-      bool alive = barrier_wait(q_full, 0, p.status, kWaitQ) && barrier_wait(k_full(0), 0, p.status, kWaitKeyFull);
-      if (alive) {
+      if (barrier_wait(q_full, 0, p.status, kWaitQ) && barrier_wait(k_full(0), 0, p.status, kWaitKeyFull)) {
         tcgen05_fence_after();
         scores(0);
-      }
-      for (int i = 0; alive && i < steps[g]; ++i) {
-        // the scores of step i + 1, once the group holds those of step i in registers
-        if (i + 1 < steps[g]) {
-          if (!barrier_wait(k_full((i + 1) % kRing), ((i + 1) / kRing) & 1, p.status, kWaitKeyFull)) break;
-          if (!barrier_wait(s_free(g), i & 1, p.status, kWaitBufferFree)) break;
+        for (int i = 0; i < steps; ++i) {
+          // the scores of step i + 1, once the softmax warps hold those of step i in registers
+          if (i + 1 < steps) {
+            if (!barrier_wait(k_full((i + 1) % kRing), ((i + 1) / kRing) & 1, p.status, kWaitKeyFull)) break;
+            if (!barrier_wait(s_free, i & 1, p.status, kWaitBufferFree)) break;
+            tcgen05_fence_after();
+            scores(i + 1);
+          }
+          // the second product of step i, once its probabilities are in tensor memory
+          if (!barrier_wait(v_full(i % kRing), (i / kRing) & 1, p.status, kWaitValueFull)) break;
+          if (!barrier_wait(p_full, i & 1, p.status, kWaitProbabilities)) break;
           tcgen05_fence_after();
-          scores(i + 1);
+          partial(i);
         }
-        // the second product of step i, once the group's probabilities are in tensor memory
-        if (!barrier_wait(v_full(i % kRing), (i / kRing) & 1, p.status, kWaitValueFull)) break;
-        if (!barrier_wait(p_full(g), i & 1, p.status, kWaitProbabilities)) break;
-        tcgen05_fence_after();
-        partial(i);
       }
     }
-  } else if (warp < 8) {
-    // ---- softmax groups: warp w of a group owns tensor-memory lanes 32 (w % 4) .. +31 ---------
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kSoftmaxRegisters));
-    const int g = warp >> 2, quarter = warp & 3;
-    const int row = quarter * 32 + lane;
-    const int query = q0 + g * kRows + row;
-    const uint32_t lane_base = static_cast<uint32_t>(quarter * 32) << 16;
-    const uint32_t tmem_group = tmem_base + static_cast<uint32_t>(g) * kGroupColumns + lane_base;
-    const int my_steps = steps[g];
+  } else if (warp < 4) {
+    // ---- softmax: warp w owns tensor-memory lanes 32 w .. +31, one thread per query row ------------
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(L::kSoftmaxRegisters));
+    const int query = q0 + static_cast<int>(threadIdx.x);
+    const uint32_t lanes = static_cast<uint32_t>(warp * 32) << 16;
+    const uint32_t tmem_s = tmem_base + lanes, tmem_o = tmem_base + kColumnO + lanes, tmem_mine = tmem_p + lanes;
     float reference = -INFINITY, row_sum = 0.f;     // -inf: the row has seen no finite score yet
     bool alive = true;
     const int last_allowed = p.causal ? min(query, p.k_tokens - 1) : p.k_tokens - 1;   // the last key this row may see
+    const int open_until = p.causal ? min(q0, p.k_tokens - 1) : p.k_tokens - 1;         // ... and the last that every row of the CTA may
 
-    // one row of scores: 128 columns, one wait
-    auto load_row = [&](uint32_t address, uint32_t (&r)[kKeys], bool edge, int limit) {
-#pragma unroll
-      for (int c = 0; c < kKeys / 32; ++c) tmem_load_32(address + c * 32, *reinterpret_cast<uint32_t(*)[32]>(&r[c * 32]));
+    // the second product of step j has finished: its probabilities and its value tile are spent
+    auto wait_product = [&](int j) {
+      if (!barrier_wait(pv_done, j & 1, p.status, kWaitPartial)) return false;
+      tcgen05_fence_after();
+      if (threadIdx.x == 0) barrier_arrive(v_empty(j % kRing));
+      return true;
+    };
+
+    for (int j = 0; j < steps; ++j) {
+      if (!barrier_wait(s_full, j & 1, p.status, kWaitScores)) { alive = false; break; }
+      tcgen05_fence_after();
+      if (threadIdx.x == 0) barrier_arrive(k_empty(j % kRing));      // the first product has read key tile j
+      // this step's scores: one row per thread, held in registers for both the maximum and the
+      // exponentials; the columns go back to the issuer at once
+      uint32_t r[kKeys];
+      tmem_load_32(tmem_s, *reinterpret_cast<uint32_t(*)[32]>(&r[0]));
+      tmem_load_32(tmem_s + 32, *reinterpret_cast<uint32_t(*)[32]>(&r[32]));
       tmem_load_wait();
-      if (edge) {
+      tcgen05_fence_before();
+      __syncwarp();
+      if (lane == 0) barrier_arrive(s_free);
+      const int key0 = j * kKeys;
+      if (key0 + kKeys - 1 > open_until) {            // uniform in the CTA
+        const int limit = last_allowed - key0;        // columns > limit are masked for this row
 #pragma unroll
         for (int i = 0; i < kKeys; ++i) {
           if (i > limit) r[i] = 0xff800000u;   // -inf
         }
       }
-    };
-    // the second product of step j has finished: its probabilities and its value tile are spent
-    auto wait_product = [&](int j) {
-      if (!barrier_wait(pv_done(g), j & 1, p.status, kWaitPartial)) return false;
-      tcgen05_fence_after();
-      if (threadIdx.x == g * kRows) {
-        barrier_arrive(v_empty(j % kRing));
-        if (j >= steps[1 - g]) barrier_arrive(v_empty(j % kRing));     // for the other group too, if it has no step j
-      }
-      return true;
-    };
 
-    for (int j = 0; j < my_steps; ++j) {
-      if (!barrier_wait(s_full(g), j & 1, p.status, kWaitScores)) { alive = false; break; }
-      tcgen05_fence_after();
-      if (threadIdx.x == g * kRows) {      // the first product has read key tile j: hand it back (for the other group too, if it has no step j)
-        barrier_arrive(k_empty(j % kRing));
-        if (j >= steps[1 - g]) barrier_arrive(k_empty(j % kRing));
-      }
-      // this step's scores: one row per thread, held in registers for both the maximum and the
-      // exponentials; the columns go back to the issuer at once
-      const int key0 = j * kKeys;
-      const int limit = last_allowed - key0;                       // columns > limit are masked for this row
-      const bool edge = key0 + kKeys - 1 > (p.causal ? min(q0 + g * kRows, p.k_tokens - 1) : p.k_tokens - 1);   // uniform in the group
-      uint32_t r[kKeys];
-      load_row(tmem_group, r, edge, limit);
-      tcgen05_fence_before();
-      __syncwarp();
-      if (lane == 0) barrier_arrive(s_free(g));
-
-      // (three-input maximum, and below two-element FMA and add: the step is bound by the number of
-      // instructions its eight softmax warps issue, so every element costs half an instruction for
+      // (three-input maximum, and below two-element FMA and add: every element costs half an instruction for
       // the maximum, half for the scaling, one ex2, half for the sum and half for the rounding)
       float m0 = -INFINITY, m1 = -INFINITY, m2 = -INFINITY, m3 = -INFINITY;
 #pragma unroll
@@ -382,145 +356,81 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
       const bool rescale = j != 0 && __any_sync(0xffffffffu, moves);
       const float shift = reference == -INFINITY ? 0.f : -reference * p.scale_log2;       // all scores -inf so far: every probability is 0
 
-      // probabilities and their sum; the probabilities go back into tensor memory as the A operand of
-      // the second product (16-bit pairs)
-      float2 sum0 = make_float2(0.f, 0.f), sum1 = sum0, sum2 = sum0, sum3 = sum0;
+      // probabilities and their sum; the probabilities go into tensor memory as the A operand of the second
+      // product (16-bit pairs)
+      float2 sum0 = make_float2(0.f, 0.f), sum1 = sum0;
       uint32_t packed[kKeys / 2];
       const float2 scale2 = make_float2(p.scale_log2, p.scale_log2), shift2 = make_float2(shift, shift);
 #pragma unroll
-      for (int chunk = 0; chunk < kKeys / 8; ++chunk) {
-        const float2 t0 = __ffma2_rn(make_float2(__uint_as_float(r[chunk * 8 + 0]), __uint_as_float(r[chunk * 8 + 1])), scale2, shift2);
-        const float2 t1 = __ffma2_rn(make_float2(__uint_as_float(r[chunk * 8 + 2]), __uint_as_float(r[chunk * 8 + 3])), scale2, shift2);
-        const float2 t2 = __ffma2_rn(make_float2(__uint_as_float(r[chunk * 8 + 4]), __uint_as_float(r[chunk * 8 + 5])), scale2, shift2);
-        const float2 t3 = __ffma2_rn(make_float2(__uint_as_float(r[chunk * 8 + 6]), __uint_as_float(r[chunk * 8 + 7])), scale2, shift2);
+      for (int chunk = 0; chunk < kKeys / 4; ++chunk) {
+        const float2 t0 = __ffma2_rn(make_float2(__uint_as_float(r[chunk * 4 + 0]), __uint_as_float(r[chunk * 4 + 1])), scale2, shift2);
+        const float2 t1 = __ffma2_rn(make_float2(__uint_as_float(r[chunk * 4 + 2]), __uint_as_float(r[chunk * 4 + 3])), scale2, shift2);
         const float2 e0 = make_float2(exp2_ftz(t0.x), exp2_ftz(t0.y));
         const float2 e1 = make_float2(exp2_ftz(t1.x), exp2_ftz(t1.y));
-        const float2 e2 = make_float2(exp2_ftz(t2.x), exp2_ftz(t2.y));
-        const float2 e3 = make_float2(exp2_ftz(t3.x), exp2_ftz(t3.y));
         sum0 = __fadd2_rn(sum0, e0);
         sum1 = __fadd2_rn(sum1, e1);
-        sum2 = __fadd2_rn(sum2, e2);
-        sum3 = __fadd2_rn(sum3, e3);
-        packed[chunk * 4 + 0] = pack_pair<T>(e0.x, e0.y);
-        packed[chunk * 4 + 1] = pack_pair<T>(e1.x, e1.y);
-        packed[chunk * 4 + 2] = pack_pair<T>(e2.x, e2.y);
-        packed[chunk * 4 + 3] = pack_pair<T>(e3.x, e3.y);
+        packed[chunk * 2 + 0] = pack_pair<T>(e0.x, e0.y);
+        packed[chunk * 2 + 1] = pack_pair<T>(e1.x, e1.y);
       }
-      const float2 sum01 = __fadd2_rn(sum0, sum1), sum23 = __fadd2_rn(sum2, sum3);
-      const float tile_sum = (sum01.x + sum01.y) + (sum23.x + sum23.y);
-      row_sum = row_sum * factor + tile_sum;
+      const float2 sum01 = __fadd2_rn(sum0, sum1);
+      row_sum = row_sum * factor + (sum01.x + sum01.y);
 
-      // The previous step's product still reads the probability columns and adds into the result:
-      // wait for it (it had this step's loads and exponentials to finish), then write.
+      // The previous step's product still reads the probability columns and adds into the result: wait for it
+      // (it had this step's loads and exponentials to finish), then write.
       if (j > 0) {
         if (!wait_product(j - 1)) { alive = false; break; }
         if (rescale) {       // rare: some row of this warp moved its reference point
-          if constexpr (D == kHeadDim) {
-            uint32_t o0[32], o1[32];
-            tmem_load_32(tmem_group + kColumnO, o0);
-            tmem_load_32(tmem_group + kColumnO + 32, o1);
+#pragma unroll 1
+          for (int c = 0; c < D / 16; ++c) {      // sixteen result columns at a time: the probabilities are still in registers
+            uint32_t o[16];
+            tmem_load_16(tmem_o + c * 16, o);
             tmem_load_wait();
 #pragma unroll
-            for (int i = 0; i < 32; ++i) {
-              o0[i] = __float_as_uint(__uint_as_float(o0[i]) * factor);
-              o1[i] = __float_as_uint(__uint_as_float(o1[i]) * factor);
-            }
-            tmem_store_32(tmem_group + kColumnO, o0);
-            tmem_store_32(tmem_group + kColumnO + 32, o1);
-          } else {             // 128 result columns, 32 at a time: the probabilities are still in registers
-#pragma unroll 1
-            for (int c = 0; c < D / 32; ++c) {
-              uint32_t o[32];
-              tmem_load_32(tmem_group + kColumnO + c * 32, o);
-              tmem_load_wait();
-#pragma unroll
-              for (int i = 0; i < 32; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * factor);
-              tmem_store_32(tmem_group + kColumnO + c * 32, o);
-            }
+            for (int i = 0; i < 16; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * factor);
+            tmem_store_16(tmem_o + c * 16, o);
           }
         }
       }
-      tmem_store_32(tmem_group + kColumnP, *reinterpret_cast<const uint32_t(*)[32]>(&packed[0]));
-      tmem_store_32(tmem_group + kColumnP + 32, *reinterpret_cast<const uint32_t(*)[32]>(&packed[32]));
+      tmem_store_32(tmem_mine, packed);
       tmem_store_wait();
       tcgen05_fence_before();
       __syncwarp();
-      if (lane == 0) barrier_arrive(p_full(g));
+      if (lane == 0) barrier_arrive(p_full);
     }
 
-    if constexpr (D != kHeadDim) {
-      // the one group of wide heads: the result row leaves tensor memory 32 columns at a time
-      if (alive && my_steps > 0 && wait_product(my_steps - 1)) {
-        // (the tensor-memory loads are warp-wide: every lane takes part, rows beyond the queries only skip the stores)
-        const bool stores = query < p.q_tokens;
-        const float inverse = 1.0f / row_sum;
-        T* out_row = static_cast<T*>(p.out) + batch * p.out_batch + head * p.out_head + static_cast<long long>(query) * p.out_token;
-        const bool vector_ok = (reinterpret_cast<uintptr_t>(out_row) & 15) == 0;
-        const int width = p.head_dim;
+    if (alive && wait_product(steps - 1)) {
+      // the result row leaves tensor memory 32 columns at a time (the loads are warp-wide: every lane takes
+      // part, rows beyond the queries only skip the stores)
+      const bool stores = query < p.q_tokens;
+      const float inverse = 1.0f / row_sum;
+      T* out_row = static_cast<T*>(p.out) + batch * p.out_batch + head * p.out_head + static_cast<long long>(query) * p.out_token;
+      const bool vector_ok = (reinterpret_cast<uintptr_t>(out_row) & 15) == 0;
+      const int width = p.head_dim;       // a multiple of 8: whole 16-byte vectors
 #pragma unroll 1
-        for (int c = 0; c < D / 32; ++c) {
-          if (c * 32 >= width) break;
-          uint32_t o[32];
-          tmem_load_32(tmem_group + kColumnO + c * 32, o);
-          tmem_load_wait();
-          if (!stores) continue;
-          if (vector_ok) {
-#pragma unroll
-            for (int v = 0; v < 4; ++v) {
-              if (c * 32 + v * 8 < width) {
-                uint4 word;
-                word.x = pack_pair<T>(__uint_as_float(o[v * 8 + 0]) * inverse, __uint_as_float(o[v * 8 + 1]) * inverse);
-                word.y = pack_pair<T>(__uint_as_float(o[v * 8 + 2]) * inverse, __uint_as_float(o[v * 8 + 3]) * inverse);
-                word.z = pack_pair<T>(__uint_as_float(o[v * 8 + 4]) * inverse, __uint_as_float(o[v * 8 + 5]) * inverse);
-                word.w = pack_pair<T>(__uint_as_float(o[v * 8 + 6]) * inverse, __uint_as_float(o[v * 8 + 7]) * inverse);
-                *reinterpret_cast<uint4*>(out_row + c * 32 + v * 8) = word;
-              }
-            }
-          } else {
-#pragma unroll
-            for (int i = 0; i < 32; ++i) {
-              if (c * 32 + i < width) out_row[c * 32 + i] = from_compute<T, float>(__uint_as_float(o[i]) * inverse);
-            }
-          }
-        }
-      }
-    } else
-    if (alive && my_steps > 0 && wait_product(my_steps - 1)) {
-      uint32_t o0[32], o1[32];
-      tmem_load_32(tmem_group + kColumnO, o0);
-      tmem_load_32(tmem_group + kColumnO + 32, o1);
-      tmem_load_wait();
-      if (query < p.q_tokens) {
-        const float inverse = 1.0f / row_sum;
-        T* out_row = static_cast<T*>(p.out) + batch * p.out_batch + head * p.out_head + static_cast<long long>(query) * p.out_token;
-        const bool vector_ok = (reinterpret_cast<uintptr_t>(out_row) & 15) == 0;
-        const int width = p.head_dim;       // a multiple of 8: whole 16-byte vectors
-        if (vector_ok) {
+      for (int c = 0; c < D / 32; ++c) {
+        if (c * 32 >= width) break;
+        uint32_t o[32];
+        tmem_load_32(tmem_o + c * 32, o);
+        tmem_load_wait();
+        if (stores && vector_ok) {
 #pragma unroll
           for (int v = 0; v < 4; ++v) {
-            uint4 word;
-            if (v * 8 < width) {
-              word.x = pack_pair<T>(__uint_as_float(o0[v * 8 + 0]) * inverse, __uint_as_float(o0[v * 8 + 1]) * inverse);
-              word.y = pack_pair<T>(__uint_as_float(o0[v * 8 + 2]) * inverse, __uint_as_float(o0[v * 8 + 3]) * inverse);
-              word.z = pack_pair<T>(__uint_as_float(o0[v * 8 + 4]) * inverse, __uint_as_float(o0[v * 8 + 5]) * inverse);
-              word.w = pack_pair<T>(__uint_as_float(o0[v * 8 + 6]) * inverse, __uint_as_float(o0[v * 8 + 7]) * inverse);
-              *reinterpret_cast<uint4*>(out_row + v * 8) = word;
-            }
-            if (32 + v * 8 < width) {
-              word.x = pack_pair<T>(__uint_as_float(o1[v * 8 + 0]) * inverse, __uint_as_float(o1[v * 8 + 1]) * inverse);
-              word.y = pack_pair<T>(__uint_as_float(o1[v * 8 + 2]) * inverse, __uint_as_float(o1[v * 8 + 3]) * inverse);
-              word.z = pack_pair<T>(__uint_as_float(o1[v * 8 + 4]) * inverse, __uint_as_float(o1[v * 8 + 5]) * inverse);
-              word.w = pack_pair<T>(__uint_as_float(o1[v * 8 + 6]) * inverse, __uint_as_float(o1[v * 8 + 7]) * inverse);
-              *reinterpret_cast<uint4*>(out_row + 32 + v * 8) = word;
+            if (c * 32 + v * 8 < width) {
+              uint4 word;
+              word.x = pack_pair<T>(__uint_as_float(o[v * 8 + 0]) * inverse, __uint_as_float(o[v * 8 + 1]) * inverse);
+              word.y = pack_pair<T>(__uint_as_float(o[v * 8 + 2]) * inverse, __uint_as_float(o[v * 8 + 3]) * inverse);
+              word.z = pack_pair<T>(__uint_as_float(o[v * 8 + 4]) * inverse, __uint_as_float(o[v * 8 + 5]) * inverse);
+              word.w = pack_pair<T>(__uint_as_float(o[v * 8 + 6]) * inverse, __uint_as_float(o[v * 8 + 7]) * inverse);
+              *reinterpret_cast<uint4*>(out_row + c * 32 + v * 8) = word;
             }
           }
-        } else {
+        } else if (stores) {
 #pragma unroll
           for (int i = 0; i < 32; ++i) {
-            if (i < width) out_row[i] = from_compute<T, float>(__uint_as_float(o0[i]) * inverse);
-            if (32 + i < width) out_row[32 + i] = from_compute<T, float>(__uint_as_float(o1[i]) * inverse);
+            if (c * 32 + i < width) out_row[c * 32 + i] = from_compute<T, float>(__uint_as_float(o[i]) * inverse);
           }
         }
+        __syncwarp();
       }
     }
   }
@@ -528,9 +438,10 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
   // ---- teardown: every thread arrives here, also after a wait that gave up -------------------
   tcgen05_fence_before();
   __syncthreads();
-  if (warp == 9) {
+  if (warp == 5) {
     tcgen05_fence_after();
-    tmem_dealloc(tmem_base, kAttnTmemColumns);
+    if constexpr (D == kHeadDim) tmem_dealloc(tmem_p, kTmemColumnsP);
+    tmem_dealloc(tmem_base, L::kTmemColumns);
   }
 }
 
@@ -539,7 +450,7 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
 // 0, and so do the columns beyond a head narrower than 64: zeros add nothing to q . k and give
 // result columns nobody stores, so a narrow head runs through the same 64-wide tiles.
 tq_status attention_map(CUtensorMap* map, tq_dtype dtype, const void* pointer, long long head_dim, long long tokens, long long heads,
-                        long long batch, const int64_t* strides) {
+                        long long batch, const int64_t* strides, int rows) {
   EncodeTiled encode = encode_tiled();
   TQ_REQUIRE(encode != nullptr, TQ_EXTERNAL, "the CUDA driver does not provide cuTensorMapEncodeTiled");
   const cuuint64_t dims[4] = {static_cast<cuuint64_t>(head_dim), static_cast<cuuint64_t>(tokens), static_cast<cuuint64_t>(heads),
@@ -550,7 +461,7 @@ tq_status attention_map(CUtensorMap* map, tq_dtype dtype, const void* pointer, l
   const long long batch_stride = batch > 1 ? strides[0] : head_dim;
   const cuuint64_t byte_strides[3] = {static_cast<cuuint64_t>(token_stride) * 2, static_cast<cuuint64_t>(head_stride) * 2,
                                       static_cast<cuuint64_t>(batch_stride) * 2};
-  const cuuint32_t box[4] = {static_cast<cuuint32_t>(kHeadDim), static_cast<cuuint32_t>(kRows), 1, 1};
+  const cuuint32_t box[4] = {static_cast<cuuint32_t>(kHeadDim), static_cast<cuuint32_t>(rows), 1, 1};
   const cuuint32_t element_strides[4] = {1, 1, 1, 1};
   const CUresult result = encode(map, dtype == TQ_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 4,
                                  const_cast<void*>(pointer), dims, byte_strides, box, element_strides, CU_TENSOR_MAP_INTERLEAVE_NONE,
@@ -626,9 +537,9 @@ extern "C" tq_status tq_attention_launch(tq_dtype dtype, const void* q, const vo
   TQ_REQUIRE(status.abort != nullptr, TQ_RESOURCE_EXHAUSTED, "no device memory for the status word");
 
   CUtensorMap map_q, map_k, map_v;
-  if (tq_status s = tq::attention_map(&map_q, dtype, q, head_dim, q_tokens, heads, batch, q_strides)) return s;
-  if (tq_status s = tq::attention_map(&map_k, dtype, k, head_dim, k_tokens, heads, batch, k_strides)) return s;
-  if (tq_status s = tq::attention_map(&map_v, dtype, v, head_dim, k_tokens, heads, batch, v_strides)) return s;
+  if (tq_status s = tq::attention_map(&map_q, dtype, q, head_dim, q_tokens, heads, batch, q_strides, tq::kRows)) return s;
+  if (tq_status s = tq::attention_map(&map_k, dtype, k, head_dim, k_tokens, heads, batch, k_strides, tq::kKeys)) return s;
+  if (tq_status s = tq::attention_map(&map_v, dtype, v, head_dim, k_tokens, heads, batch, v_strides, tq::kKeys)) return s;
 
   tq::AttnParams p = {};
   p.batch = static_cast<int>(batch);
@@ -636,9 +547,8 @@ extern "C" tq_status tq_attention_launch(tq_dtype dtype, const void* q, const vo
   p.q_tokens = static_cast<int>(q_tokens);
   p.k_tokens = static_cast<int>(k_tokens);
   p.head_dim = static_cast<int>(head_dim);
-  const bool wide = head_dim > tq::kHeadDim;             // two sub-tiles side by side, one group of 128 rows per CTA
-  const long long cta_rows = (wide ? 1 : tq::kGroups) * tq::kRows;
-  p.q_blocks = static_cast<int>((q_tokens + cta_rows - 1) / cta_rows);
+  const bool wide = head_dim > tq::kHeadDim;             // two sub-tiles side by side
+  p.q_blocks = static_cast<int>((q_tokens + tq::kRows - 1) / tq::kRows);
   p.causal = causal != 0;
   p.scale_log2 = static_cast<float>(scale * 1.4426950408889634);
   p.out = out;
