@@ -256,10 +256,11 @@ __device__ __forceinline__ A load_partial(const A* pointer) {
   }
 }
 
-template <typename R>
+// Over each aligned set of LANES lanes of the warp.
+template <typename R, int LANES = 32>
 __device__ __forceinline__ typename R::Acc warp_reduce(typename R::Acc a) {
 #pragma unroll
-  for (int offset = 16; offset > 0; offset >>= 1) a = R::combine(a, R::shuffle(a, offset));
+  for (int offset = LANES / 2; offset > 0; offset >>= 1) a = R::combine(a, R::shuffle(a, offset));
   return a;
 }
 
@@ -317,18 +318,21 @@ __device__ __forceinline__ void fold_span(const T* __restrict__ row, long long b
 // ---------------------------------------------------------------------------------------------
 // Kernels
 
-// One warp per slice. grid.x * kWarps >= outer.
-template <typename T, typename R, int VEC>
+// LANES lanes per slice: a warp, or eight lanes for slices of at most 512 bytes, of which a warp then has four
+// under way where one left it with 256 bytes and half its lanes idle. (Eight is also as many lanes as a slice can have
+// elements before its first vector.) grid.x * kWarps * (32 / LANES) >= outer.
+template <typename T, typename R, int VEC, int LANES>
 __global__ void __launch_bounds__(kBlock)
 reduce_warp_per_slice(const T* __restrict__ in, typename R::Out* __restrict__ out, long long outer,
                       long long reduce, int mean) {
-  const int lane = threadIdx.x & 31;
-  const long long slice = static_cast<long long>(blockIdx.x) * kWarps + (threadIdx.x >> 5);
-  if (slice >= outer) return;
+  static_assert(LANES >= VEC, "a slice's head and tail are one element per lane");
+  const int lane = threadIdx.x % LANES;
+  const long long slice = static_cast<long long>(blockIdx.x) * (kBlock / LANES) + threadIdx.x / LANES;
   typename R::template Local<VEC> local = R::template local_identity<VEC>();
-  fold_span<T, R, VEC>(in + slice * reduce, 0, reduce, lane, 32, local);
-  typename R::Acc acc = warp_reduce<R>(R::template to_acc<VEC>(local));
-  if (lane == 0) out[slice] = R::finish(acc, reduce, mean != 0);
+  if (slice < outer) fold_span<T, R, VEC>(in + slice * reduce, 0, reduce, lane, LANES, local);
+  __syncwarp();
+  typename R::Acc acc = warp_reduce<R, LANES>(R::template to_acc<VEC>(local));
+  if (lane == 0 && slice < outer) out[slice] = R::finish(acc, reduce, mean != 0);
 }
 
 // `split` CTAs per slice, `cluster` of them in one thread-block cluster (cluster divides split).
@@ -1075,10 +1079,15 @@ tq_status run(const Plan& p, const void* in, void* out, long long outer, long lo
   constexpr int kVec = 16 / sizeof(T);
   switch (p.shape) {
     case Shape::kWarpPerSlice: {
-      const long long blocks = (outer + kWarps - 1) / kWarps;
+      const bool narrow = reduce * static_cast<long long>(sizeof(T)) <= 512;
+      const int slices = narrow ? kBlock / 8 : kWarps;
+      const long long blocks = (outer + slices - 1) / slices;
       TQ_REQUIRE(blocks <= 0x7fffffffLL, TQ_UNSUPPORTED, "%lld slices are more than a grid holds", outer);
-      reduce_warp_per_slice<T, R, kVec><<<static_cast<unsigned>(blocks), kBlock, 0, stream>>>(
-          input, output, outer, reduce, mean ? 1 : 0);
+      if (narrow) {
+        reduce_warp_per_slice<T, R, kVec, 8><<<static_cast<unsigned>(blocks), kBlock, 0, stream>>>(input, output, outer, reduce, mean ? 1 : 0);
+      } else {
+        reduce_warp_per_slice<T, R, kVec, 32><<<static_cast<unsigned>(blocks), kBlock, 0, stream>>>(input, output, outer, reduce, mean ? 1 : 0);
+      }
       return check_launch("reduce_warp_per_slice");
     }
     case Shape::kCtaPerSlice: {

@@ -1054,3 +1054,23 @@ def test_transposes_that_fill_no_whole_tile(tq, dtype, rows, cols):
     else:
         x = torch.randn(3, rows, cols).to(dtype)
     assert torch.equal(tq.contiguous(_inside(x, 1).transpose(1, 2)).cpu(), x.transpose(1, 2))
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64, torch.bfloat16, torch.float16, torch.int32, torch.int64])
+@pytest.mark.parametrize("rows, width", [(1, 1), (3, 7), (33, 15), (1000, 31), (257, 64), (70, 65), (999, 128), (31, 129), (64, 256), (65, 257)])
+def test_reductions_of_short_rows(tq, dtype, rows, width):
+    """Eight lanes a row up to 512 bytes, a warp beyond: row counts that leave sets of lanes without a row, and
+    rows that start between vectors."""
+    x = (torch.randn(rows, width, generator=torch.Generator().manual_seed(rows + width)) * 50).to(dtype)
+    for shift in (0, 1, 3):
+        xd = _inside(x, shift)
+        assert torch.equal(tq.amax(xd, -1).cpu(), x.amax(-1)) and torch.equal(tq.amin(xd, -1).cpu(), x.amin(-1))
+        assert torch.equal(tq.argmax(xd, -1).cpu(), (x == x.amax(-1, keepdim=True)).int().argmax(-1))
+        total = tq.sum(xd, -1).cpu()
+        if dtype in (torch.int32, torch.int64):
+            assert torch.equal(total, x.long().sum(-1))
+            continue
+        bound = {torch.bfloat16: 2.0**-8, torch.float16: 2.0**-11}.get(dtype, 0.0)
+        exact, budget = x.double().sum(-1), 1e-6 * x.double().abs().sum(-1)       # f32 sums in a tree, one rounding of the result
+        assert ((total.double() - exact).abs() <= bound * exact.abs() + budget).all()
+        assert ((tq.mean(xd, -1).cpu().double() - exact / width).abs() <= bound * (exact / width).abs() + budget / width).all()
