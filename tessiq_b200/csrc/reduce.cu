@@ -318,9 +318,10 @@ __device__ __forceinline__ void fold_span(const T* __restrict__ row, long long b
 // ---------------------------------------------------------------------------------------------
 // Kernels
 
-// LANES lanes per slice: a warp, or eight lanes for slices of at most 512 bytes, of which a warp then has four
-// under way where one left it with 256 bytes and half its lanes idle. (Eight is also as many lanes as a slice can have
-// elements before its first vector.) grid.x * kWarps * (32 / LANES) >= outer.
+// LANES lanes per slice: a warp, or eight or sixteen lanes for short slices, of which a warp then has four or two
+// under way where one of 256 bytes left it with half its lanes idle: 10^6 x 64 f32 sum 187 us with 32 lanes, 53 with
+// eight (bytes: 40). (Eight is also as many lanes as a slice can have elements before its first vector.)
+// grid.x * kBlock / LANES >= outer.
 template <typename T, typename R, int VEC, int LANES>
 __global__ void __launch_bounds__(kBlock)
 reduce_warp_per_slice(const T* __restrict__ in, typename R::Out* __restrict__ out, long long outer,
@@ -960,6 +961,7 @@ int floor_pow2(long long v) {
 Plan plan(tq_reduce_op op, tq_dtype dtype, long long outer, long long reduce, long long inner,
           int32_t device, int vec_bytes_limit, bool may_be_ragged = true) {
   Plan p;
+  p.device = device;
   const int size = dtype_size(dtype);
   const int sms = sm_count(device);
   const long long target_ctas = static_cast<long long>(sms) * 4;
@@ -1079,11 +1081,22 @@ tq_status run(const Plan& p, const void* in, void* out, long long outer, long lo
   constexpr int kVec = 16 / sizeof(T);
   switch (p.shape) {
     case Shape::kWarpPerSlice: {
-      const bool narrow = reduce * static_cast<long long>(sizeof(T)) <= 512;
-      const int slices = narrow ? kBlock / 8 : kWarps;
+      // Short slices share a warp. Measured (300000 slices, us with 32 / 16 / 8 lanes): 500 bf16 sum 98.7 / 61.3 / 53.6, argmax
+      // 154.8 / 90.4 / 66.9; 250 f32 sum 78.0 / 51.9 / 50.2; 500 f32 sum 89.6 / 94.3 / 101, argmax 116 / 95 / 102; 80000 of 1000
+      // bf16 sum 28.0 / 28.5 / 31.7, argmax 44.6 / 34.7 / 35.2. Of few slices eight lanes make too few warps: 1000 of 250 f32
+      // 3.1 / 3.2 / 4.0.
+      const long long slice_bytes = reduce * static_cast<long long>(sizeof(T));
+      constexpr bool kBusy = sizeof(T) == 2 || std::is_same_v<R, ArgmaxReducer<T>>;
+      const bool many = outer >= 64ll * sm_count(p.device);
+      const int lanes = slice_bytes <= 512 || (slice_bytes <= 1024 && sizeof(T) == 2 && many) ? 8
+                        : slice_bytes <= 1024 || (slice_bytes <= 2048 && kBusy)               ? 16
+                                                                                             : 32;
+      const int slices = kBlock / lanes;
       const long long blocks = (outer + slices - 1) / slices;
       TQ_REQUIRE(blocks <= 0x7fffffffLL, TQ_UNSUPPORTED, "%lld slices are more than a grid holds", outer);
-      if (narrow) {
+      if (lanes == 16) {
+        reduce_warp_per_slice<T, R, kVec, 16><<<static_cast<unsigned>(blocks), kBlock, 0, stream>>>(input, output, outer, reduce, mean ? 1 : 0);
+      } else if (lanes == 8) {
         reduce_warp_per_slice<T, R, kVec, 8><<<static_cast<unsigned>(blocks), kBlock, 0, stream>>>(input, output, outer, reduce, mean ? 1 : 0);
       } else {
         reduce_warp_per_slice<T, R, kVec, 32><<<static_cast<unsigned>(blocks), kBlock, 0, stream>>>(input, output, outer, reduce, mean ? 1 : 0);

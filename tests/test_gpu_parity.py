@@ -1057,10 +1057,11 @@ def test_transposes_that_fill_no_whole_tile(tq, dtype, rows, cols):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float64, torch.bfloat16, torch.float16, torch.int32, torch.int64])
-@pytest.mark.parametrize("rows, width", [(1, 1), (3, 7), (33, 15), (1000, 31), (257, 64), (70, 65), (999, 128), (31, 129), (64, 256), (65, 257)])
+@pytest.mark.parametrize("rows, width", [(1, 1), (3, 7), (33, 15), (1000, 31), (257, 64), (70, 65), (999, 128), (31, 129), (64, 256), (65, 257),
+                                         (9480, 300), (40, 300), (40, 1001), (13, 1025)])
 def test_reductions_of_short_rows(tq, dtype, rows, width):
-    """Eight lanes a row up to 512 bytes, a warp beyond: row counts that leave sets of lanes without a row, and
-    rows that start between vectors."""
+    """Eight or sixteen lanes a row, or a warp, by bytes, type and number of rows (9480: enough for eight lanes over more than
+    512 bytes): row counts that leave sets of lanes without a row, and rows that start between vectors."""
     x = (torch.randn(rows, width, generator=torch.Generator().manual_seed(rows + width)) * 50).to(dtype)
     for shift in (0, 1, 3):
         xd = _inside(x, shift)
