@@ -105,9 +105,10 @@ template <typename C, bool kMax> __device__ __forceinline__ C fold(C a, C b) {
   return a + b;
 }
 
-template <typename C, bool kMax> __device__ __forceinline__ C warp_fold(C v) {
+// Over each aligned set of LANES lanes of the warp.
+template <typename C, bool kMax, int LANES = 32> __device__ __forceinline__ C warp_fold(C v) {
 #pragma unroll
-  for (int offset = 16; offset > 0; offset >>= 1) {
+  for (int offset = LANES / 2; offset > 0; offset >>= 1) {
     v = fold<C, kMax>(v, __shfl_xor_sync(0xffffffffu, v, offset));
   }
   return v;
@@ -273,23 +274,24 @@ __device__ __forceinline__ void finish_row(Vec<T, VEC> (&x)[K], int first, int s
   }
 }
 
-// One warp per row; 8 rows per CTA.
-template <typename T, typename OutT, int VEC, int K, int OP>
+// LANES lanes per row: a warp, or eight lanes for rows of at most 32 vectors, of which a warp then has four.
+template <typename T, typename OutT, int VEC, int K, int OP, int LANES = 32>
 __global__ void __launch_bounds__(kBlock) row_warp_kernel(RowArgs args) {
-  const int lane = threadIdx.x & 31;
-  const long long row = static_cast<long long>(blockIdx.x) * kWarps + (threadIdx.x >> 5);
-  if (row >= args.rows) return;
-  const int vectors = static_cast<int>(args.width / VEC);
+  const int lane = threadIdx.x % LANES;
+  const long long row = static_cast<long long>(blockIdx.x) * (kBlock / LANES) + threadIdx.x / LANES;
+  if (LANES == 32 && row >= args.rows) return;
+  // (lanes without a row stay for the shuffles: they have no vectors)
+  const int vectors = row < args.rows ? static_cast<int>(args.width / VEC) : 0;
   const T* in_row = static_cast<const T*>(args.in) + row * args.width;
   Vec<T, VEC> x[K];
 #pragma unroll
   for (int j = 0; j < K; ++j) {
-    if (lane + j * 32 < vectors) x[j] = load_stream<T, VEC>(in_row + static_cast<long long>(lane + j * 32) * VEC);
+    if (lane + j * LANES < vectors) x[j] = load_stream<T, VEC>(in_row + static_cast<long long>(lane + j * LANES) * VEC);
   }
   auto fold_row = [](float value, bool is_max, int) {
-    return is_max ? warp_fold<float, true>(value) : warp_fold<float, false>(value);
+    return is_max ? warp_fold<float, true, LANES>(value) : warp_fold<float, false, LANES>(value);
   };
-  finish_row<T, OutT, VEC, K, OP>(x, lane, 32, vectors, args, row, lane == 0, fold_row);
+  finish_row<T, OutT, VEC, K, OP>(x, lane, LANES, vectors, args, row, lane == 0 && row < args.rows, fold_row);
 }
 
 // A cluster of `cluster` CTAs per row. blockIdx.x = row * cluster + rank.
@@ -635,7 +637,18 @@ tq_status run_vector(const RowArgs& args, cudaStream_t stream, bool* handled) {
     const long long blocks = (args.rows + kWarps - 1) / kWarps;
     TQ_REQUIRE(blocks <= 0x7fffffffLL, TQ_UNSUPPORTED, "%lld rows are more than a grid holds", args.rows);
     const unsigned grid = static_cast<unsigned>(blocks);
-    if (vectors <= 32) {
+    // Short rows of a large tensor: a warp per row left half its lanes idle and 128 to 512 bytes under way. 10^6 x 64 f32
+    // softmax / LayerNorm 149 / 194 us with 32 lanes, 78 / 78 with eight (bytes: 79); bf16 194 / 245 and 52 / 64 (40); 10^6 x
+    // 128 f32 182 / 214 and 154 / 155. Of few rows eight lanes make too few warps: 8192 x 128 f32 LayerNorm 3.9 and 4.4.
+    const unsigned short_grid = static_cast<unsigned>((args.rows + kBlock / 8 - 1) / (kBlock / 8));
+    const bool many = args.rows >= (vectors <= 16 ? 8192 : 16384);
+    if (vectors <= 8 && many) {
+      row_warp_kernel<T, OutT, VEC, 1, OP, 8><<<short_grid, kBlock, 0, stream>>>(args);
+    } else if (vectors <= 16 && many) {
+      row_warp_kernel<T, OutT, VEC, 2, OP, 8><<<short_grid, kBlock, 0, stream>>>(args);
+    } else if (vectors <= 32 && many) {
+      row_warp_kernel<T, OutT, VEC, 4, OP, 8><<<short_grid, kBlock, 0, stream>>>(args);
+    } else if (vectors <= 32) {
       row_warp_kernel<T, OutT, VEC, 1, OP><<<grid, kBlock, 0, stream>>>(args);
     } else if (vectors <= 64) {
       row_warp_kernel<T, OutT, VEC, 2, OP><<<grid, kBlock, 0, stream>>>(args);

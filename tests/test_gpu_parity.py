@@ -1075,3 +1075,23 @@ def test_reductions_of_short_rows(tq, dtype, rows, width):
         exact, budget = x.double().sum(-1), 1e-6 * x.double().abs().sum(-1)       # f32 sums in a tree, one rounding of the result
         assert ((total.double() - exact).abs() <= bound * exact.abs() + budget).all()
         assert ((tq.mean(xd, -1).cpu().double() - exact / width).abs() <= bound * (exact / width).abs() + budget / width).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("rows", [8191, 8193, 16385])
+@pytest.mark.parametrize("vectors", [1, 7, 8, 9, 16, 17, 32, 33])
+def test_short_rows_of_whole_vectors(tq, dtype, rows, vectors):
+    """From 8192 rows on eight lanes share a row of up to 16 vectors, from 16384 on of up to 32; 8193 and 16385 leave sets
+    of lanes without one."""
+    width = vectors * (16 // dtype.itemsize)
+    g = torch.Generator().manual_seed(width)
+    x = (torch.randn(rows, width, generator=g) * 2 + 0.5).to(dtype)
+    w, b = (1 + torch.randn(width, generator=g) * 0.1).to(dtype), (torch.randn(width, generator=g) * 0.1).to(dtype)
+    close = close32 if dtype == torch.float32 else close16
+    close(tq.softmax(dev(x), -1), tessiq0.softmax(x, -1))
+    y, mean, rstd = tq.native_layer_norm(dev(x), [width], dev(w), dev(b), 1e-5)
+    exact = torch.nn.functional.layer_norm(x.double(), [width], w.double(), b.double(), 1e-5)
+    close(y, exact.to(dtype))
+    close(mean.flatten(), x.double().mean(-1).to(dtype))
+    exact = x.double() * torch.rsqrt(x.double().square().mean(-1, keepdim=True) + 1e-5) * w.double()
+    close(tq.rms_norm(dev(x), dev(w), 1e-5), exact.to(dtype))
