@@ -267,6 +267,12 @@ __device__ __forceinline__ void store_stream(T* pointer, const Vec<T, N>& value)
   }
 }
 
+// Shared memory of another CTA may be written only once that CTA has begun to run, which being scheduled together
+// does not say. Every thread of the cluster calls cluster_start() once, early, and cluster_started() before
+// the first such write: the barrier's latency then passes under the loads in between.
+__device__ __forceinline__ void cluster_start() { asm volatile("barrier.cluster.arrive.relaxed;" ::: "memory"); }
+__device__ __forceinline__ void cluster_started() { asm volatile("barrier.cluster.wait;" ::: "memory"); }
+
 __device__ __forceinline__ float warp_sum(float v) {
 #pragma unroll
   for (int offset = 16; offset > 0; offset >>= 1) v += __shfl_xor_sync(0xffffffffu, v, offset);

@@ -129,7 +129,8 @@ __device__ __forceinline__ C block_fold(C v, C* warp_scratch) {
 }
 
 // Every thread of every CTA of the cluster gets the cluster-wide result. `slots` is an array of
-// kMaxCluster values in this CTA's shared memory that no other statistic uses.
+// kMaxCluster values in this CTA's shared memory that no other statistic uses. (The peers' slots are written
+// before any barrier of this function, so its caller has passed cluster_started().)
 template <typename C, bool kMax, int WARPS = kWarps>
 __device__ __forceinline__ C cluster_fold(C v, C* warp_scratch, C* slots, int cluster) {
   v = block_fold<C, kMax, WARPS>(v, warp_scratch);
@@ -304,6 +305,7 @@ __global__ void __launch_bounds__(THREADS) row_cluster_kernel(RowArgs args, int 
   const int vectors = static_cast<int>(args.width / VEC);
   const T* in_row = static_cast<const T*>(args.in) + row * args.width;
   const int first = rank * K * THREADS + threadIdx.x;
+  if (cluster > 1) cluster_start();
   Vec<T, VEC> x[K];
 #pragma unroll
   for (int j = 0; j < K; ++j) {
@@ -311,6 +313,7 @@ __global__ void __launch_bounds__(THREADS) row_cluster_kernel(RowArgs args, int 
       x[j] = load_stream<T, VEC>(in_row + static_cast<long long>(first + j * THREADS) * VEC);
     }
   }
+  if (cluster > 1) cluster_started();
   auto fold_row = [&](float value, bool is_max, int stage) {
     return is_max ? cluster_fold<float, true, THREADS / 32>(value, warp_scratch, slots[stage], cluster)
                   : cluster_fold<float, false, THREADS / 32>(value, warp_scratch, slots[stage], cluster);
@@ -390,6 +393,8 @@ row_ragged_kernel(RowArgs args, int cluster) {
   Vec<T, VEC> w[kInRegisters ? K : 1], b[kInRegisters ? K : 1];
   T w_edge{}, b_edge{};
   int kept_head = -1, parity = 0;
+  // (a cluster without a row takes part in no barrier)
+  if (THREADS > 32 && cluster > 1 && team < args.rows) cluster_start();
   for (long long row = team; row < args.rows; row += teams, parity ^= 1) {
     const T* in_row = static_cast<const T*>(args.in) + row * args.width;
     OutT* out_row = static_cast<OutT*>(args.out) + row * args.width;
@@ -430,6 +435,7 @@ row_ragged_kernel(RowArgs args, int cluster) {
       }
     }
 
+    if (THREADS > 32 && cluster > 1 && row == team) cluster_started();
     auto fold_row = [&](float value, bool is_max, int stage) {
       if constexpr (THREADS == 32) {
         return is_max ? warp_fold<float, true>(value) : warp_fold<float, false>(value);
