@@ -357,6 +357,7 @@ reduce_cta_per_slice(const T* __restrict__ in, typename R::Out* __restrict__ out
   long long end = begin + chunk;
   if (end > reduce) end = reduce;
 
+  if (cluster > 1) cluster_start();
   typename R::template Local<VEC> local = R::template local_identity<VEC>();
   fold_span<T, R, VEC>(in + slice * reduce, begin, end, threadIdx.x, kBlock, local);
   Acc acc = block_reduce<R>(R::template to_acc<VEC>(local), warp_scratch);
@@ -364,6 +365,7 @@ reduce_cta_per_slice(const T* __restrict__ in, typename R::Out* __restrict__ out
   if (cluster > 1) {
     cg::cluster_group group = cg::this_cluster();
     const unsigned rank = group.block_rank();
+    cluster_started();
     if (threadIdx.x == 0) {
       Acc* leader = group.map_shared_rank(cluster_scratch, 0);
       leader[rank] = acc;
@@ -421,6 +423,7 @@ reduce_columns(const T* __restrict__ in, typename R::Out* __restrict__ out, long
   Acc* cluster_scratch = rows_scratch + kBlock * VEC;                    // [lanes_x * VEC]
   __shared__ bool is_last;
 
+  if (cluster > 1) cluster_start();
   const int tx = threadIdx.x % lanes_x;
   const int ty = threadIdx.x / lanes_x;
   const int lanes_y = kBlock / lanes_x;
@@ -604,6 +607,7 @@ reduce_columns(const T* __restrict__ in, typename R::Out* __restrict__ out, long
   if (cluster > 1) {
     cg::cluster_group group = cg::this_cluster();
     rank = group.block_rank();
+    cluster_started();
     if (holder) {
       const int item = tx * VEC;
       Acc* owner = group.map_shared_rank(cluster_scratch, item / slice_items);

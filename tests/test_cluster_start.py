@@ -50,7 +50,7 @@ def unguarded(text):
         exposed = grown
 
 
-@pytest.mark.parametrize("source", ["rownorm.cu", "slabnorm.cu", "decode.cu", "gemm.cu"])
+@pytest.mark.parametrize("source", ["rownorm.cu", "reduce.cu", "slabnorm.cu", "decode.cu", "gemm.cu"])
 def test_no_peer_is_touched_before_it_runs(source):
     text = (CSRC / source).read_text()
     assert any(TOUCH.search(body) for _, _, body in functions(text)), "the file no longer uses a peer's shared memory"
