@@ -322,10 +322,11 @@ __global__ void __launch_bounds__(THREADS) row_cluster_kernel(RowArgs args, int 
                                   rank == 0 && threadIdx.x == 0, fold_row);
 }
 
-// exp(d) for d <= 0 as the kernels of a type take it: rows of f32 that no vector fits used expf before they
-// had a kernel of their own, and 2^(d log2 e) rounds the product, which f32 results would show.
-template <typename T> __device__ __forceinline__ float ragged_exp(float d) {
-  if constexpr (sizeof(T) == 4) {
+// exp(d) for d <= 0 as exact as results of type OutT can show. 2^(d log2 e) rounds its product, which puts a
+// probability e^-80 of the largest off by up to 4e-6 of itself: nothing in 16 bits, but f32 results (of f32 rows, or of
+// 16-bit rows with half_to_float) take expf.
+template <typename OutT> __device__ __forceinline__ float ragged_exp(float d) {
+  if constexpr (sizeof(OutT) == 4) {
     return expf(d);
   } else {
     return exp2_approx(d * 1.4426950408889634f);
@@ -482,15 +483,15 @@ row_ragged_kernel(RowArgs args, int cluster) {
       float local = edge >= 0 ? edge_value : -std::numeric_limits<float>::infinity();
       each([&](float v, int, int) { local = nan_max(local, v); });
       const float row_max = fold_row(local, true, 0);
-      const float edge_exp = edge >= 0 ? ragged_exp<T>(edge_value - row_max) : 0.f;
+      const float edge_exp = edge >= 0 ? ragged_exp<OutT>(edge_value - row_max) : 0.f;
       float sum = edge_exp;
       each([&](float v, int j, int e) {
-        const float value = ragged_exp<T>(v - row_max);
+        const float value = ragged_exp<OutT>(v - row_max);
         sum += value;
         if constexpr (sizeof(T) == 4) x[j].v[e] = value;
       });
       const float inverse = 1.f / fold_row(sum, false, 1);
-      write([&](int j, int e) { return (sizeof(T) == 4 ? widen(x[j], e) : ragged_exp<T>(widen(x[j], e) - row_max)) * inverse; });
+      write([&](int j, int e) { return (sizeof(T) == 4 ? widen(x[j], e) : ragged_exp<OutT>(widen(x[j], e) - row_max)) * inverse; });
       if (edge >= 0) out_row[edge] = from_compute<OutT, float>(edge_exp * inverse);
     } else {
       float mean = 0.f;

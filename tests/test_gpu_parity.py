@@ -1001,6 +1001,20 @@ def test_rows_that_start_between_vectors(tq, dtype, rows, width):
         close32(tq.softmax(_inside(x, 1), -1, half_to_float=True), torch.softmax(x.double(), -1).float(), rtol=1e-5, scale=1e-5)
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("width", [65, 1003, 8201])
+def test_small_probabilities_of_ragged_rows_in_f32(tq, dtype, width):
+    """A row of f32 results keeps a small probability to a few units in the last place, whatever the input's type:
+    against the row's largest (the sum is a factor of the whole row) p = e^(x - max) within expf's 2 ulp and a
+    rounding each of p and of the largest: 4 * 2^-23."""
+    x = -torch.rand(7, width, generator=torch.Generator().manual_seed(width)) * 80.0
+    x[:, 3] = 0.0
+    x = x.to(dtype)
+    got = tq.softmax(_inside(x, 1), -1, half_to_float=dtype != torch.float32).cpu().double()
+    error = (got / got[:, 3:4] / torch.exp(x.double()) - 1).abs().max().item()
+    assert error <= 4 * 2.0**-23, f"{error:.2e}"
+
+
 def test_ragged_rows_with_special_values(tq):
     x = torch.randn(6, 1003, generator=torch.Generator().manual_seed(2))
     x[1, 17] = float("nan")
