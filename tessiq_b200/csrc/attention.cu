@@ -19,7 +19,7 @@
 //                       lies in memory). The scores of step j + 1 are computed while the softmax warps work
 //                       on step j, which hand the columns back as soon as they have them in registers.
 //
-// softmax is exp(s - m) / sum exp(s - m) for ANY m, so a row keeps the maximum of its first key tile
+// softmax is exp(s - m) / sum exp(s - m) for ANY m, so a row keeps the maximum of its first two key tiles
 // as its reference point and moves it only when a later tile rises more than 2^8 above it — then,
 // and only then, the row's sum and its accumulators in tensor memory are rescaled (a warp-wide
 // slow path, rare on real data). Without that, nothing is read back per step: the second product
@@ -205,10 +205,8 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     barrier_expect_tx(q_full, kSubTiles * kQueryBytes);
     for (int h = 0; h < kSubTiles; ++h) tma_load_4d(base + h * kQueryBytes, &map_q, q_full, h * kHeadDim, q0, head, batch);
-    for (int j = 0; j < early; ++j) {
-      load_tile(&map_k, kOffsetK, k_full(j), j);
-      load_tile(&map_v, kOffsetV, v_full(j), j);
-    }
+    for (int j = 0; j < early; ++j) load_tile(&map_k, kOffsetK, k_full(j), j);
+    for (int j = 0; j < early; ++j) load_tile(&map_v, kOffsetV, v_full(j), j);
   }
   if (warp == 5) {
     if constexpr (D == kHeadDim) {
@@ -247,17 +245,16 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
       const uint32_t low_q = descriptor_low(base, 0), low_k = descriptor_low(base + kOffsetK, 0);
       const uint32_t low_v = descriptor_low(base + kOffsetV, kSubTileBytes);
       // S(i) = Q K_i^T: both operands K-major, 16 elements of K = 32 B in the swizzle row
-      auto scores = [&](int i) {
+      auto scores = [&](int i, uint32_t into) {
         const uint32_t k = low_k + (i % kRing) * (kTileBytes >> 4);
         // (a 128-wide head is two 64-wide sub-tiles side by side: the same steps in the second one)
 #pragma unroll
         for (int h = 0; h < kSubTiles; ++h) {
 #pragma unroll
           for (int kk = 0; kk < kHeadDim / 16; ++kk)
-            mma_f16_split(tmem_base, low_q + h * (kQueryBytes >> 4) + kk * 2, kHighWord, k + h * (kSubTileBytes >> 4) + kk * 2, kHighWord, idesc_s,
+            mma_f16_split(into, low_q + h * (kQueryBytes >> 4) + kk * 2, kHighWord, k + h * (kSubTileBytes >> 4) + kk * 2, kHighWord, idesc_s,
                           (h != 0 || kk != 0) ? 1u : 0u);
         }
-        mma_commit(s_full);
       };
       // O += P_i V_i (O = for the first step): P from tensor memory (16 keys = 8 columns), V MN-major
       // from shared memory (16 keys = 2048 B)
@@ -273,16 +270,22 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
         }
         mma_commit(pv_done);
       };
-      if (barrier_wait(q_full, 0, p.status, kWaitQ) && barrier_wait(k_full(0), 0, p.status, kWaitKeyFull)) {
+      if (barrier_wait(q_full, 0, p.status, kWaitQ) && barrier_wait(k_full(0), 0, p.status, kWaitKeyFull) &&
+          (steps == 1 || barrier_wait(k_full(1), 0, p.status, kWaitKeyFull))) {
         tcgen05_fence_after();
-        scores(0);
+        // (the second tile's scores too, for the reference point: into result columns, which nothing uses before the first
+        // product of probabilities and values)
+        scores(0, tmem_base);
+        if (steps > 1) scores(1, tmem_base + kColumnO);
+        mma_commit(s_full);
         for (int i = 0; i < steps; ++i) {
           // the scores of step i + 1, once the softmax warps hold those of step i in registers
           if (i + 1 < steps) {
             if (!barrier_wait(k_full((i + 1) % kRing), ((i + 1) / kRing) & 1, p.status, kWaitKeyFull)) break;
             if (!barrier_wait(s_free, i & 1, p.status, kWaitBufferFree)) break;
             tcgen05_fence_after();
-            scores(i + 1);
+            scores(i + 1, tmem_base);
+            mma_commit(s_full);
           }
           // the second product of step i, once its probabilities are in tensor memory
           if (!barrier_wait(v_full(i % kRing), (i / kRing) & 1, p.status, kWaitValueFull)) break;
@@ -311,20 +314,14 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
       return true;
     };
 
-    for (int j = 0; j < steps; ++j) {
-      if (!barrier_wait(s_full, j & 1, p.status, kWaitScores)) { alive = false; break; }
-      tcgen05_fence_after();
-      if (threadIdx.x == 0) barrier_arrive(k_empty(j % kRing));      // the first product has read key tile j
-      // this step's scores: one row per thread, held in registers for both the maximum and the
-      // exponentials; the columns go back to the issuer at once
-      uint32_t r[kKeys];
-      tmem_load_32(tmem_s, *reinterpret_cast<uint32_t(*)[32]>(&r[0]));
-      tmem_load_32(tmem_s + 32, *reinterpret_cast<uint32_t(*)[32]>(&r[32]));
+    // One tile's scores: a row per thread, held in registers for both the maximum and the exponentials.
+    uint32_t r[kKeys];
+    auto load_scores = [&](uint32_t from) {
+      tmem_load_32(from, *reinterpret_cast<uint32_t(*)[32]>(&r[0]));
+      tmem_load_32(from + 32, *reinterpret_cast<uint32_t(*)[32]>(&r[32]));
       tmem_load_wait();
-      tcgen05_fence_before();
-      __syncwarp();
-      if (lane == 0) barrier_arrive(s_free);
-      const int key0 = j * kKeys;
+    };
+    auto mask = [&](int key0) {
       if (key0 + kKeys - 1 > open_until) {            // uniform in the CTA
         const int limit = last_allowed - key0;        // columns > limit are masked for this row
 #pragma unroll
@@ -332,9 +329,10 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
           if (i > limit) r[i] = 0xff800000u;   // -inf
         }
       }
-
-      // (three-input maximum, and below two-element FMA and add: every element costs half an instruction for
-      // the maximum, half for the scaling, one ex2, half for the sum and half for the rounding)
+    };
+    // (three-input maximum, and below two-element FMA and add: every element costs half an instruction for
+    // the maximum, half for the scaling, one ex2, half for the sum and half for the rounding)
+    auto maximum = [&]() {
       float m0 = -INFINITY, m1 = -INFINITY, m2 = -INFINITY, m3 = -INFINITY;
 #pragma unroll
       for (int i = 0; i < kKeys; i += 8) {
@@ -343,15 +341,38 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
         m2 = max3(m2, __uint_as_float(r[i + 4]), __uint_as_float(r[i + 5]));
         m3 = max3(m3, __uint_as_float(r[i + 6]), __uint_as_float(r[i + 7]));
       }
-      const float tile_max = fmaxf(fmaxf(m0, m1), fmaxf(m2, m3));
-      // The reference point: the first tile's maximum, moved only when a tile rises more than
+      return fmaxf(fmaxf(m0, m1), fmaxf(m2, m3));
+    };
+
+    // The second tile's maximum, for the row's reference point.
+    float second_max = -INFINITY;
+    if (steps > 1) {
+      alive = barrier_wait(s_full, 0, p.status, kWaitScores);
+      if (alive) {
+        tcgen05_fence_after();
+        load_scores(tmem_o);
+        mask(kKeys);
+        second_max = maximum();
+      }
+    }
+    for (int j = 0; alive && j < steps; ++j) {
+      if (!barrier_wait(s_full, j & 1, p.status, kWaitScores)) { alive = false; break; }
+      tcgen05_fence_after();
+      if (threadIdx.x == 0) barrier_arrive(k_empty(j % kRing));      // the first product has read key tile j
+      load_scores(tmem_s);         // the columns go back to the issuer at once
+      tcgen05_fence_before();
+      __syncwarp();
+      if (lane == 0) barrier_arrive(s_free);
+      mask(j * kKeys);
+      const float tile_max = maximum();
+      // The reference point: the first two tiles' maximum, moved only when a tile rises more than
       // 2^kSlack above it (from -inf, any finite maximum does). `factor` rescales what the row has
       // gathered so far; it is 1 for a row that stays.
       float factor = 1.f;
       const bool moves = j == 0 || (tile_max - reference) * p.scale_log2 > kSlack;       // false for NaN
       if (moves) {
         if (j != 0) factor = exp2_ftz((reference - tile_max) * p.scale_log2);             // from -inf: 0, and nothing was gathered
-        reference = tile_max;
+        reference = j == 0 ? fmaxf(tile_max, second_max) : tile_max;
       }
       const bool rescale = j != 0 && __any_sync(0xffffffffu, moves);
       const float shift = reference == -INFINITY ? 0.f : -reference * p.scale_log2;       // all scores -inf so far: every probability is 0
