@@ -442,12 +442,17 @@ tq_status tq_gemm_bias_act_residual_launch(tq_dtype dtype,
  * every key. bf16 or f16; scores, maxima and sums in f32; one rounding of the result.
  *   q is [batch, heads, q_tokens, head_dim], k and v are [batch, heads, k_tokens, head_dim], out is
  *   [batch, heads, q_tokens, head_dim]; each is addressed through three ELEMENT strides
+/* Which kernel the launch below runs for `heads` (batch times heads) of these extents: keys streamed by CUDA cores
+ * (decoding), or the tensor-core kernel with 64 or 128 keys a step, in its form for many queries or for a few. It depends
+ * on the number of SMs of `device`; device -1 stands for a B200 and needs no GPU. */
+enum { TQ_ATTENTION_STREAMED = 0, TQ_ATTENTION_TILES = 1, TQ_ATTENTION_TILES_FEW = 2 };
+tq_status tq_attention_form(int64_t heads, int64_t q_tokens, int64_t k_tokens, int64_t head_dim, int32_t causal, int32_t device,
+                            int32_t* form, int32_t* keys);
  *   {batch, head, token} and its head_dim elements are contiguous — so the slices of a fused QKV
  *   projection are read where they lie and the result can be written in [batch, token, head, dim]
  *   order.
- * head_dim is 8, 16, ... 128: the kernel works on 64-wide tiles, one per head up to 64 elements and two
- * side by side beyond (then one group of 128 query rows per CTA instead of two); the columns a head
- * does not have are filled with zeros by TMA. Declines (TQ_UNSUPPORTED): any other head_dim, a scale that is not positive and finite, q/k/v that
+ * head_dim is 8, 16, ... 128: the tensor-core kernel works on 64-wide tiles, one per head up to 64 elements and two
+ * side by side beyond; the columns a head does not have are filled with zeros by TMA. Declines (TQ_UNSUPPORTED): any other head_dim, a scale that is not positive and finite, q/k/v that
  * are not 16-byte aligned or whose strides are not positive multiples of 8 elements (TMA's rules).
  * Bounded waits report through tq_status_poll like the GEMM's. */
 tq_status tq_attention_launch(tq_dtype dtype,

@@ -3,10 +3,10 @@
 //   out[b,h,i,:] = sum_j softmax_j(scale * q[b,h,i,:] . k[b,h,j,:]) v[b,h,j,:]     (j <= i when causal)
 //
 // bf16 or f16 operands, heads of up to 128 elements, f32 scores and sums, one rounding of the result. The
-// score matrix never leaves the SM: one CTA owns 128 query rows of one head and walks the keys 64 at a time
-// with a row reference point and row sum (the online form of softmax).
+// score matrix never leaves the SM: one CTA owns 128 query rows of one head and walks the keys 64 or 128 at a
+// time (choose_attention_form) with a row reference point and row sum (the online form of softmax).
 //
-//   warps 0..3          softmax, one thread per query row: tcgen05.ld of the row's 64 f32 scores (held in
+//   warps 0..3          softmax, one thread per query row: tcgen05.ld of the row's f32 scores of a step (held in
 //                       registers for both the maximum and the exponentials), ex2, row sum; the
 //                       probabilities go back into tensor memory with tcgen05.st as packed bf16/f16 pairs —
 //                       the A operand of the second product. The result accumulates in tensor memory
@@ -14,29 +14,37 @@
 //   warp 4, one lane    producer: TMA loads (128-byte swizzle) of the query tile once, then one key tile and
 //                       one value tile per step into two rings; the first filling leaves before the CTA's
 //                       set-up barrier.
-//   warp 5, one lane    issuer: S = Q K^T (128 x 64 x head, both operands K-major in shared memory) and
-//                       O = P V (128 x head x 64, P from tensor memory, V consumed MN-major exactly as it
+//   warp 5, one lane    issuer: S = Q K^T (128 x keys x head, both operands K-major in shared memory) and
+//                       O = P V (128 x head x keys, P from tensor memory, V consumed MN-major exactly as it
 //                       lies in memory). The scores of step j + 1 are computed while the softmax warps work
 //                       on step j, which hand the columns back as soon as they have them in registers.
 //
-// softmax is exp(s - m) / sum exp(s - m) for ANY m, so a row keeps the maximum of its first two key tiles
+// softmax is exp(s - m) / sum exp(s - m) for ANY m, so a row keeps the maximum of its first 128 keys
 // as its reference point and moves it only when a later tile rises more than 2^8 above it — then,
 // and only then, the row's sum and its accumulators in tensor memory are rescaled (a warp-wide
 // slow path, rare on real data). Without that, nothing is read back per step: the second product
-// accumulates O += P V in place. Probabilities are at most 2^8, well inside bf16 and f16.
+// accumulates O += P V in place. Probabilities are at most 2^8, well inside bf16 and f16. (With 64 keys a step the second
+// tile's scores are computed ahead for it, into the result's columns: from the first 64 keys alone a row's largest
+// probability was exactly 1 less often, and the error against 64 bits 1 to 3 % larger.)
 //
-// What bounds it: a step of one CTA is a chain (scores seen, tcgen05.ld, maximum, ex2, tcgen05.st, signal) of about
+// A few queries (FEW) leave three of the four softmax warps without a row and the tensor cores idle, so their probabilities
+// are taken as two 16-bit operands, the rounded value and what rounding took off: the result is as exact as the
+// streaming kernel's, whose probabilities are never rounded (error against 64 bits 1.65e-3 in bf16, all of it the result's
+// rounding; 2.3e-3 with one operand).
+//
+// What bounds it: a step of 64 keys of one CTA is a chain (scores seen, tcgen05.ld, maximum, ex2, tcgen05.st, signal) of about
 // 1 500 cycles of which the special-function unit works 512, so an SM needs several chains. Three CTAs of one
 // softmax warp per scheduler each (two for heads above 64) keep the unit busy 65 % of the time, and one CTA's
-// start and end run under the others' steps. One CTA an SM with two groups of 128 rows and 128-key steps, as it
-// was, spent 5 000 cycles on every start: 64 x 12 heads, 1024 tokens of 64 causal 256 -> 225 us, no mask 377 -> 320,
-// 4 x 12 x 4096 no mask 332 -> 312; 64 x 6 heads of 128, whose second group had idled, 235 -> 175.
-// Measured beside it: two CTAs with two groups each and the probabilities over the scores (four chains, each
+// start and end run under the others' steps; two CTAs with 128 keys a step pay a step's hand-overs half as often and reach
+// as much. One CTA an SM with two groups of 128 rows and 128-key steps, as it
+// was once, spent 5 000 cycles on every start: 64 x 12 heads, 1024 tokens of 64 causal 256 us, now 229, no mask 377, now 323,
+// 4 x 12 x 4096 no mask 332, now 296; 64 x 6 heads of 128, whose second group had idled, 235, now 175.
+// Measured beside it (before the reference point took 128 keys, when the first two of those were 225 and 320): two CTAs with two groups each and the probabilities over the scores (four chains, each
 // with both products inside it) 216 / 307 / 312 / 205; one exponential in four, or in sixteen, as a polynomial of
 // degree 5 on the FMA pipes 328 and 322 instead of 312; scalar instead of two-element FMA and add 311 - 318; the
 // row sum after the signal 333; skipping the rows past the diagonal of a whole warp: no change.
 //
-// The softmax warps run with 120 registers per thread (200 for wide heads), the other four with 40 (56)
+// The softmax warps run with 120 registers per thread where three CTAs share an SM, 200 where two do, the other four with 40 and 56
 // (setmaxnreg). Q, K, V and the result are addressed through (batch, head, token) strides, so the three slices
 // of a fused QKV projection are read in place and the result is written directly in [batch, token, head, head_dim]
 // order: none of the four packing copies around `bmm -> where -> softmax -> bmm` remains.
@@ -61,36 +69,40 @@ namespace {
 
 constexpr int kHeadDim = 64;
 constexpr int kRows = 128;            // query rows per CTA
-constexpr int kKeys = 64;             // keys per step
 constexpr int kAttnThreads = 256;     // four softmax warps; producer and issuer in a second group of four
 constexpr uint32_t kQueryBytes = kRows * kHeadDim * 2;       // 16 KiB: 128 rows of 64 elements, one TMA box, one swizzled operand tile
-constexpr uint32_t kSubTileBytes = kKeys * kHeadDim * 2;     // 8 KiB: the same of 64 keys or values
-// Heads of up to 64 elements run three CTAs an SM, heads of up to 128 (two 64-wide sub-tiles side by side in
-// every tile) two. Shared memory: the query tile, the key ring, the value ring, the barriers. Tensor memory,
-// f32 columns: scores (64), packed probabilities (32), result (64 or 128). An allocation is a power of two, so
-// the narrow form takes two (scores and result, probabilities: 160 columns, and three CTAs have 480 of the 512)
-// and the wide one a single one of 256.
-template <int D>
+// D: heads of up to 64 elements, or of up to 128 (two 64-wide sub-tiles side by side in every tile). KEYS: keys per step. FEW:
+// the form for a few queries, whose probabilities take two operands (below). Shared memory: the query tile, the key
+// ring, the value ring, the barriers. Tensor memory, f32 columns: scores (KEYS), packed probabilities (KEYS / 2, twice with FEW),
+// result (D). An allocation is a power of two, so heads of 64 with 64 keys a step take two (scores and result,
+// probabilities: 160 columns, and three CTAs have 480 of the 512) and the other forms a single one.
+template <int D, int KEYS, bool FEW>
 struct AttnLayout {
   static constexpr int kSubTiles = D / kHeadDim;
-  static constexpr int kCtasPerSm = D == kHeadDim ? 3 : 2;
-  static constexpr int kRing = D == kHeadDim ? 3 : 2;          // stages of the key ring and of the value ring
+  static constexpr bool kTwoAllocations = D == kHeadDim && KEYS == 64 && !FEW;
+  static constexpr int kCtasPerSm = kTwoAllocations ? 3 : KEYS == 64 || (D == kHeadDim && !FEW) ? 2 : 1;
+  static constexpr int kRing = D == kHeadDim && KEYS == 64 ? 3 : 2;          // stages of the key ring and of the value ring
+  static constexpr uint32_t kSubTileBytes = KEYS * kHeadDim * 2;            // 8 or 16 KiB: 64 elements of a tile's keys or values
   static constexpr uint32_t kTileBytes = kSubTiles * kSubTileBytes;
   static constexpr uint32_t kOffsetK = kSubTiles * kQueryBytes;
   static constexpr uint32_t kOffsetV = kOffsetK + kRing * kTileBytes;
   static constexpr uint32_t kOffsetBarriers = kOffsetV + kRing * kTileBytes;
   static constexpr size_t kSmemBytes = 1024 + kOffsetBarriers + 256;
-  static constexpr uint32_t kTmemColumns = D == kHeadDim ? 128 : 256;      // scores from column 0 on
-  static constexpr uint32_t kColumnO = D == kHeadDim ? 64 : 128;
+  static constexpr uint32_t kColumnP = KEYS, kColumnO = kTwoAllocations ? 64 : D == kHeadDim && !FEW ? KEYS + KEYS / 2 : 2 * KEYS;
+  static constexpr uint32_t kTmemColumns = kTwoAllocations ? 128 : kColumnO + D <= 256 ? 256 : 512;      // scores from column 0 on
+  static_assert(kTwoAllocations || (kColumnP + (FEW ? KEYS : KEYS / 2) <= kColumnO && kColumnO + D <= kTmemColumns), "the columns overlap");
+  static_assert(kTwoAllocations ? kCtasPerSm * 160 <= 512 : kCtasPerSm * kTmemColumns <= 512, "more CTAs an SM than it has tensor memory for");
+  static_assert(kCtasPerSm * (kSmemBytes + 1024) <= 228 * 1024, "the staging has to fit as often as there are CTAs an SM");
   // setmaxnreg moves registers inside the CTA's own allocation: what the second group of four warps gives up is
-  // at least what the softmax warps take. An increase beyond what was released would wait for ever.
+  // at least what the softmax warps take. An increase beyond what was released would wait for ever. (A CTA that has
+  // its SM to itself has registers enough from the start.)
   static constexpr int kLaunchRegisters = (65536 / kCtasPerSm / kAttnThreads) / 8 * 8;
-  static constexpr int kSoftmaxRegisters = D == kHeadDim ? 120 : 200, kOtherRegisters = D == kHeadDim ? 40 : 56;
-  static_assert(128 * (kSoftmaxRegisters - kLaunchRegisters) <= 128 * (kLaunchRegisters - kOtherRegisters),
+  static constexpr int kSoftmaxRegisters = kCtasPerSm == 3 ? 120 : 200, kOtherRegisters = kCtasPerSm == 3 ? 40 : 56;
+  static constexpr bool kMovesRegisters = kCtasPerSm > 1;
+  static_assert(!kMovesRegisters || 128 * (kSoftmaxRegisters - kLaunchRegisters) <= 128 * (kLaunchRegisters - kOtherRegisters),
                 "the softmax warps would wait for registers nobody releases");
 };
-static_assert(AttnLayout<64>::kSmemBytes <= 74 * 1024 && AttnLayout<128>::kSmemBytes <= 112 * 1024, "the staging has to fit as often as there are CTAs an SM");
-constexpr uint32_t kTmemColumnsP = 32;
+constexpr uint32_t kTmemColumnsP = 32;       // of the second allocation
 constexpr float kSlack = 8.f;                // a row's reference point moves when a tile's maximum is more than 2^kSlack above it
 
 enum AttnWait { kWaitQ = 201, kWaitKeyEmpty = 202, kWaitValueEmpty = 203, kWaitKeyFull = 204, kWaitValueFull = 205,
@@ -98,7 +110,7 @@ enum AttnWait { kWaitQ = 201, kWaitKeyEmpty = 202, kWaitValueEmpty = 203, kWaitK
 
 struct AttnParams {
   int batch, heads, q_tokens, k_tokens;
-  int head_dim;                    // 8, 16, ... 64: narrower heads ride in 64-wide tiles whose other columns TMA fills with zeros
+  int head_dim;                    // 8, 16, ... 128: narrower heads ride in tiles of 64 or 128 whose other columns TMA fills with zeros
   int q_blocks;                    // CTAs per head
   int causal;
   float scale_log2;                // scale * log2(e)
@@ -139,11 +151,25 @@ __device__ __forceinline__ uint32_t pack_pair(float low, float high) {
   }
 }
 
-template <typename T, int D>
-__global__ void __launch_bounds__(kAttnThreads, AttnLayout<D>::kCtasPerSm)
+// What rounding took off a pair of probabilities, rounded itself.
+template <typename T>
+__device__ __forceinline__ uint32_t pack_rest(uint32_t rounded, float2 exact) {
+  if constexpr (std::is_same_v<T, __nv_bfloat16>) {
+    return pack_pair<T>(exact.x - __uint_as_float(rounded << 16), exact.y - __uint_as_float(rounded & 0xffff0000u));
+  } else {
+    const float2 wide = __half22float2(*reinterpret_cast<const __half2*>(&rounded));
+    return pack_pair<T>(exact.x - wide.x, exact.y - wide.y);
+  }
+}
+
+template <typename T, int D, int KEYS, bool FEW>
+__global__ void __launch_bounds__(kAttnThreads, AttnLayout<D, KEYS, FEW>::kCtasPerSm)
 attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                  const __grid_constant__ CUtensorMap map_v, const AttnParams p) {
-  using L = AttnLayout<D>;
+  using L = AttnLayout<D, KEYS, FEW>;
+  constexpr int kKeys = KEYS;
+  constexpr bool kAhead = KEYS < 128;      // the reference point takes the second tile's scores too
+  constexpr uint32_t kSubTileBytes = L::kSubTileBytes;
   constexpr int kRing = L::kRing;
   constexpr uint32_t kTileBytes = L::kTileBytes, kOffsetK = L::kOffsetK, kOffsetV = L::kOffsetV;
   constexpr uint32_t kOffsetBarriers = L::kOffsetBarriers, kColumnO = L::kColumnO;
@@ -209,7 +235,7 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
     for (int j = 0; j < early; ++j) load_tile(&map_v, kOffsetV, v_full(j), j);
   }
   if (warp == 5) {
-    if constexpr (D == kHeadDim) {
+    if constexpr (L::kTwoAllocations) {
       tmem_alloc_more(tmem_slot, L::kTmemColumns);
       tmem_alloc(tmem_slot + 4, kTmemColumnsP);
     } else {
@@ -220,9 +246,9 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
   __syncthreads();
   tcgen05_fence_after();
   const uint32_t tmem_base = tmem_slot_pointer[0];
-  const uint32_t tmem_p = D == kHeadDim ? tmem_slot_pointer[1] : tmem_base + 64;
+  const uint32_t tmem_p = L::kTwoAllocations ? tmem_slot_pointer[1] : tmem_base + L::kColumnP;
 
-  if (warp >= 4) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(L::kOtherRegisters));
+  if (L::kMovesRegisters && warp >= 4) asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(L::kOtherRegisters));
   if (warp == 4) {
     // ---- producer: what did not fit the first filling --------------------------------------------
     if (elect_one()) {
@@ -267,16 +293,22 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
           for (int kk = 0; kk < kKeys / 16; ++kk)
             mma_f16_tmem_a(tmem_base + kColumnO + h * kHeadDim, tmem_p + kk * 8, v + h * (kSubTileBytes >> 4) + kk * (2048 >> 4), kHighWord, idesc_o,
                            (i != 0 || kk != 0) ? 1u : 0u);
+          if constexpr (FEW) {      // ... and what rounding took off the probabilities
+#pragma unroll
+            for (int kk = 0; kk < kKeys / 16; ++kk)
+              mma_f16_tmem_a(tmem_base + kColumnO + h * kHeadDim, tmem_p + kKeys / 2 + kk * 8, v + h * (kSubTileBytes >> 4) + kk * (2048 >> 4), kHighWord,
+                             idesc_o, 1u);
+          }
         }
         mma_commit(pv_done);
       };
       if (barrier_wait(q_full, 0, p.status, kWaitQ) && barrier_wait(k_full(0), 0, p.status, kWaitKeyFull) &&
-          (steps == 1 || barrier_wait(k_full(1), 0, p.status, kWaitKeyFull))) {
+          (!kAhead || steps == 1 || barrier_wait(k_full(1), 0, p.status, kWaitKeyFull))) {
         tcgen05_fence_after();
         // (the second tile's scores too, for the reference point: into result columns, which nothing uses before the first
         // product of probabilities and values)
         scores(0, tmem_base);
-        if (steps > 1) scores(1, tmem_base + kColumnO);
+        if (kAhead && steps > 1) scores(1, tmem_base + kColumnO);
         mma_commit(s_full);
         for (int i = 0; i < steps; ++i) {
           // the scores of step i + 1, once the softmax warps hold those of step i in registers
@@ -297,7 +329,7 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
     }
   } else if (warp < 4) {
     // ---- softmax: warp w owns tensor-memory lanes 32 w .. +31, one thread per query row ------------
-    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(L::kSoftmaxRegisters));
+    if constexpr (L::kMovesRegisters) asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(L::kSoftmaxRegisters));
     const int query = q0 + static_cast<int>(threadIdx.x);
     const uint32_t lanes = static_cast<uint32_t>(warp * 32) << 16;
     const uint32_t tmem_s = tmem_base + lanes, tmem_o = tmem_base + kColumnO + lanes, tmem_mine = tmem_p + lanes;
@@ -305,6 +337,18 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
     bool alive = true;
     const int last_allowed = p.causal ? min(query, p.k_tokens - 1) : p.k_tokens - 1;   // the last key this row may see
     const int open_until = p.causal ? min(q0, p.k_tokens - 1) : p.k_tokens - 1;         // ... and the last that every row of the CTA may
+
+    if (FEW && q0 + warp * 32 >= p.q_tokens) {
+      // A warp without a query takes part in the hand-overs only: its rows of scores and of the result mean nothing.
+      for (int j = 0; alive && j < steps; ++j) {
+        alive = barrier_wait(s_full, j & 1, p.status, kWaitScores);
+        if (alive && lane == 0) barrier_arrive(s_free);
+        if (alive && j > 0) alive = barrier_wait(pv_done, (j - 1) & 1, p.status, kWaitPartial);
+        if (alive && lane == 0) barrier_arrive(p_full);
+        __syncwarp();
+      }
+      alive = false;
+    }
 
     // the second product of step j has finished: its probabilities and its value tile are spent
     auto wait_product = [&](int j) {
@@ -315,13 +359,13 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
     };
 
     // One tile's scores: a row per thread, held in registers for both the maximum and the exponentials.
-    uint32_t r[kKeys];
-    auto load_scores = [&](uint32_t from) {
-      tmem_load_32(from, *reinterpret_cast<uint32_t(*)[32]>(&r[0]));
-      tmem_load_32(from + 32, *reinterpret_cast<uint32_t(*)[32]>(&r[32]));
+    using Scores = uint32_t[kKeys];
+    auto load_scores = [&](Scores& r, uint32_t from) {
+#pragma unroll
+      for (int i = 0; i < kKeys; i += 32) tmem_load_32(from + i, *reinterpret_cast<uint32_t(*)[32]>(&r[i]));
       tmem_load_wait();
     };
-    auto mask = [&](int key0) {
+    auto mask = [&](Scores& r, int key0) {
       if (key0 + kKeys - 1 > open_until) {            // uniform in the CTA
         const int limit = last_allowed - key0;        // columns > limit are masked for this row
 #pragma unroll
@@ -332,7 +376,7 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
     };
     // (three-input maximum, and below two-element FMA and add: every element costs half an instruction for
     // the maximum, half for the scaling, one ex2, half for the sum and half for the rounding)
-    auto maximum = [&]() {
+    auto maximum = [&](const Scores& r) {
       float m0 = -INFINITY, m1 = -INFINITY, m2 = -INFINITY, m3 = -INFINITY;
 #pragma unroll
       for (int i = 0; i < kKeys; i += 8) {
@@ -346,25 +390,27 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
 
     // The second tile's maximum, for the row's reference point.
     float second_max = -INFINITY;
-    if (steps > 1) {
+    if (kAhead && alive && steps > 1) {
       alive = barrier_wait(s_full, 0, p.status, kWaitScores);
       if (alive) {
+        Scores r;
         tcgen05_fence_after();
-        load_scores(tmem_o);
-        mask(kKeys);
-        second_max = maximum();
+        load_scores(r, tmem_o);
+        mask(r, kKeys);
+        second_max = maximum(r);
       }
     }
     for (int j = 0; alive && j < steps; ++j) {
       if (!barrier_wait(s_full, j & 1, p.status, kWaitScores)) { alive = false; break; }
       tcgen05_fence_after();
       if (threadIdx.x == 0) barrier_arrive(k_empty(j % kRing));      // the first product has read key tile j
-      load_scores(tmem_s);         // the columns go back to the issuer at once
+      Scores r;
+      load_scores(r, tmem_s);         // the columns go back to the issuer at once
       tcgen05_fence_before();
       __syncwarp();
       if (lane == 0) barrier_arrive(s_free);
-      mask(j * kKeys);
-      const float tile_max = maximum();
+      mask(r, j * kKeys);
+      const float tile_max = maximum(r);
       // The reference point: the first two tiles' maximum, moved only when a tile rises more than
       // 2^kSlack above it (from -inf, any finite maximum does). `factor` rescales what the row has
       // gathered so far; it is 1 for a row that stays.
@@ -380,7 +426,7 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
       // probabilities and their sum; the probabilities go into tensor memory as the A operand of the second
       // product (16-bit pairs)
       float2 sum0 = make_float2(0.f, 0.f), sum1 = sum0;
-      uint32_t packed[kKeys / 2];
+      uint32_t packed[kKeys / 2], rest[FEW ? kKeys / 2 : 1];
       const float2 scale2 = make_float2(p.scale_log2, p.scale_log2), shift2 = make_float2(shift, shift);
 #pragma unroll
       for (int chunk = 0; chunk < kKeys / 4; ++chunk) {
@@ -392,6 +438,10 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
         sum1 = __fadd2_rn(sum1, e1);
         packed[chunk * 2 + 0] = pack_pair<T>(e0.x, e0.y);
         packed[chunk * 2 + 1] = pack_pair<T>(e1.x, e1.y);
+        if constexpr (FEW) {
+          rest[chunk * 2 + 0] = pack_rest<T>(packed[chunk * 2 + 0], e0);
+          rest[chunk * 2 + 1] = pack_rest<T>(packed[chunk * 2 + 1], e1);
+        }
       }
       const float2 sum01 = __fadd2_rn(sum0, sum1);
       row_sum = row_sum * factor + (sum01.x + sum01.y);
@@ -412,7 +462,11 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
           }
         }
       }
-      tmem_store_32(tmem_mine, packed);
+#pragma unroll
+      for (int i = 0; i < kKeys / 2; i += 32) {
+        tmem_store_32(tmem_mine + i, *reinterpret_cast<uint32_t(*)[32]>(&packed[i]));
+        if constexpr (FEW) tmem_store_32(tmem_mine + kKeys / 2 + i, *reinterpret_cast<uint32_t(*)[32]>(&rest[i]));
+      }
       tmem_store_wait();
       tcgen05_fence_before();
       __syncwarp();
@@ -461,14 +515,14 @@ attention_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constan
   __syncthreads();
   if (warp == 5) {
     tcgen05_fence_after();
-    if constexpr (D == kHeadDim) tmem_dealloc(tmem_p, kTmemColumnsP);
+    if constexpr (L::kTwoAllocations) tmem_dealloc(tmem_p, kTmemColumnsP);
     tmem_dealloc(tmem_base, L::kTmemColumns);
   }
 }
 
 // A four-axis map over one of Q, K, V: `head_dim` contiguous elements, then tokens, heads, batch with
-// the caller's element strides; box = 64 x 128 x 1 x 1, 128-byte swizzle. Rows beyond the tokens read
-// 0, and so do the columns beyond a head narrower than 64: zeros add nothing to q . k and give
+// the caller's element strides; box = 64 x `rows` x 1 x 1 (128 queries, or a step's keys), 128-byte swizzle. Rows beyond the tokens read
+// 0, and so do the columns beyond a head narrower than its tiles: zeros add nothing to q . k and give
 // result columns nobody stores, so a narrow head runs through the same 64-wide tiles.
 tq_status attention_map(CUtensorMap* map, tq_dtype dtype, const void* pointer, long long head_dim, long long tokens, long long heads,
                         long long batch, const int64_t* strides, int rows) {
@@ -507,7 +561,61 @@ tq_status attention_decode(tq_dtype dtype, const void* q, const void* k, const v
                            const int64_t* v_strides, const int64_t* out_strides, float scale_log2, bool causal, int32_t device, cudaStream_t stream);
 constexpr int kDecodeQueries = 4;
 
+struct AttentionForm {
+  bool decode;      // decode.cu
+  int keys;         // keys a step of the tensor-core kernel
+  bool few;         // its form for a few queries
+};
+
+// Kernel times (graphs of launches over rotating operands, B200, bf16, us) behind the rules. `heads` is batch times heads.
+//
+// One to four queries: streaming the keys (decode.cu) costs multiply-adds per query, the tensor cores' few-query form does not, but
+// it walks a head's keys in one CTA. Four queries of 64 x 12 heads over 1000 keys: heads of 64 streamed 73, few 53; heads of 128
+// 143 and 74; two queries of heads of 128 85 and 74, one 75 and 74; but over 100 keys, heads of 64, 14.0 and 17. Where heads do
+// not fill the SMs a head's keys are shared when streamed: four queries of 8 heads of 128 over 4000 keys 36 and 47, of 96 heads
+// 80 and 50. From there to one head an SM clusters of four no longer fit: one query, 144 heads of 96, 4000 keys 57 and 53.
+//
+// More queries: 128 keys a step halve the hand-overs of a chain, but only two CTAs share an SM (one for heads above 64)
+// where 64 keys let three (two). 1 x 8 x 4096 causal 68.9 with 64, 54.4 with 128; 64 x 12 x 1024 causal 228.7 and 228.7; 5 ... 9 waves
+// of 200 to 256 tokens 0 - 4 % better with 64; 64 x 6 x 1024 of 128 174.7 and 225. Without a mask, CTAs that fit
+// three an SM but not two are one wave with 64 (384 CTAs over 4096 keys 90.6 and 92.9). Up to 64 keys half of a 128-key step would be empty
+// (64 x 12 x 64 11.4 and 15.5).
+AttentionForm choose_attention_form(long long heads, long long q_tokens, long long k_tokens, long long head_dim, bool causal, long long sms) {
+  const bool wide = head_dim > kHeadDim;
+  if (q_tokens <= kDecodeQueries) {
+    const long long keys = causal && q_tokens < k_tokens ? q_tokens : k_tokens;       // that any query sees
+    const bool no_fours = heads * 25 > sms * 24;                                    // clusters of four: 142 of them on 148 SMs
+    if (heads > sms) {
+      const long long enough = q_tokens >= 3 ? (wide ? heads / 4 : heads / 2) : heads;
+      if ((wide ? q_tokens >= 2 : q_tokens >= 3) && keys >= enough && keys >= 64) return {false, 64, true};
+    } else if (keys > kHeadDim) {
+      const bool half = heads * 2 > sms;
+      const bool many = q_tokens >= 3 && (wide ? half || keys <= 512 : keys <= 128 || (half && keys <= 300) || no_fours);
+      if (many || (wide && no_fours && keys >= 256)) return {false, 128, true};
+    }
+    return {true, 0, false};
+  }
+  const long long ctas = heads * ((q_tokens + kRows - 1) / kRows);
+  if (k_tokens <= 64) return {false, 64, false};
+  if (wide) return {false, ctas <= sms ? 128 : 64, false};
+  const bool thirds = !causal && ctas > 2 * sms && ctas <= 3 * sms;
+  return {false, ctas <= 2 * sms || (k_tokens >= 512 && !thirds) ? 128 : 64, false};
+}
+
 }  // namespace tq
+
+extern "C" tq_status tq_attention_form(int64_t heads, int64_t q_tokens, int64_t k_tokens, int64_t head_dim, int32_t causal, int32_t device, int32_t* form,
+                                       int32_t* keys) {
+  TQ_REQUIRE(form != nullptr && keys != nullptr, TQ_INVALID_ARGUMENT, "null out-pointer");
+  TQ_REQUIRE(heads > 0 && q_tokens > 0 && k_tokens > 0, TQ_INVALID_ARGUMENT, "extents must be positive, not heads=%lld q_tokens=%lld k_tokens=%lld",
+             (long long)heads, (long long)q_tokens, (long long)k_tokens);
+  TQ_REQUIRE(head_dim >= 8 && head_dim <= 2 * tq::kHeadDim && head_dim % 8 == 0, TQ_UNSUPPORTED,
+             "fused attention has a kernel for heads of 8, 16, ... %d elements, not %lld", 2 * tq::kHeadDim, (long long)head_dim);
+  const tq::AttentionForm chosen = tq::choose_attention_form(heads, q_tokens, k_tokens, head_dim, causal != 0, device < 0 ? 148 : tq::sm_count(device));
+  *form = chosen.decode ? TQ_ATTENTION_STREAMED : chosen.few ? TQ_ATTENTION_TILES_FEW : TQ_ATTENTION_TILES;
+  *keys = chosen.keys;
+  return TQ_OK;
+}
 
 extern "C" tq_status tq_attention_launch(tq_dtype dtype, const void* q, const void* k, const void* v, void* out, int64_t batch,
                                          int64_t heads, int64_t q_tokens, int64_t k_tokens, int64_t head_dim,
@@ -548,9 +656,10 @@ extern "C" tq_status tq_attention_launch(tq_dtype dtype, const void* q, const vo
              "misaligned result or negative result stride");
   tq::DeviceScope device_scope(device);
   if (tq_status s = device_scope.status()) return s;
-  // A few query rows leave nothing for the tensor cores to reuse: K and V are streamed instead. (The result's
-  // batch * heads * split CTAs stay below 2^28.)
-  if (q_tokens <= tq::kDecodeQueries) {
+  const bool wide = head_dim > tq::kHeadDim;             // two sub-tiles side by side
+  const tq::AttentionForm form = tq::choose_attention_form(batch * heads, q_tokens, k_tokens, head_dim, causal != 0, tq::sm_count(device));
+  // (The decoding form's batch * heads * split CTAs stay below 2^28.)
+  if (form.decode) {
     return tq::attention_decode(dtype, q, k, v, out, batch, heads, q_tokens, k_tokens, head_dim, q_strides, k_strides, v_strides, out_strides,
                                 static_cast<float>(scale * 1.4426950408889634), causal != 0, device, static_cast<cudaStream_t>(stream));
   }
@@ -559,8 +668,8 @@ extern "C" tq_status tq_attention_launch(tq_dtype dtype, const void* q, const vo
 
   CUtensorMap map_q, map_k, map_v;
   if (tq_status s = tq::attention_map(&map_q, dtype, q, head_dim, q_tokens, heads, batch, q_strides, tq::kRows)) return s;
-  if (tq_status s = tq::attention_map(&map_k, dtype, k, head_dim, k_tokens, heads, batch, k_strides, tq::kKeys)) return s;
-  if (tq_status s = tq::attention_map(&map_v, dtype, v, head_dim, k_tokens, heads, batch, v_strides, tq::kKeys)) return s;
+  if (tq_status s = tq::attention_map(&map_k, dtype, k, head_dim, k_tokens, heads, batch, k_strides, form.keys)) return s;
+  if (tq_status s = tq::attention_map(&map_v, dtype, v, head_dim, k_tokens, heads, batch, v_strides, form.keys)) return s;
 
   tq::AttnParams p = {};
   p.batch = static_cast<int>(batch);
@@ -568,7 +677,6 @@ extern "C" tq_status tq_attention_launch(tq_dtype dtype, const void* q, const vo
   p.q_tokens = static_cast<int>(q_tokens);
   p.k_tokens = static_cast<int>(k_tokens);
   p.head_dim = static_cast<int>(head_dim);
-  const bool wide = head_dim > tq::kHeadDim;             // two sub-tiles side by side
   p.q_blocks = static_cast<int>((q_tokens + tq::kRows - 1) / tq::kRows);
   p.causal = causal != 0;
   p.scale_log2 = static_cast<float>(scale * 1.4426950408889634);
@@ -580,21 +688,23 @@ extern "C" tq_status tq_attention_launch(tq_dtype dtype, const void* q, const vo
   const long long ctas = static_cast<long long>(p.q_blocks) * heads * batch;
   TQ_REQUIRE(ctas < (1LL << 31), TQ_UNSUPPORTED, "too many query blocks for one launch");
   cudaStream_t cuda_stream = static_cast<cudaStream_t>(stream);
-  auto go = [&](auto kernel, size_t smem) -> tq_status {
-    static std::mutex mutex;
-    {
-      std::lock_guard<std::mutex> lock(mutex);
+  auto go = [&](auto width, auto keys, auto few) -> tq_status {
+    constexpr int kWidth = decltype(width)::value, kKeys = decltype(keys)::value;
+    constexpr bool kFew = decltype(few)::value;
+    constexpr size_t smem = tq::AttnLayout<kWidth, kKeys, kFew>::kSmemBytes;
+    auto start = [&](auto kernel) -> tq_status {
       TQ_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-    }
-    kernel<<<static_cast<unsigned>(ctas), tq::kAttnThreads, smem, cuda_stream>>>(map_q, map_k, map_v, p);
-    return tq::check_launch("attention_kernel");
+      kernel<<<static_cast<unsigned>(ctas), tq::kAttnThreads, smem, cuda_stream>>>(map_q, map_k, map_v, p);
+      return tq::check_launch("attention_kernel");
+    };
+    if (dtype == TQ_BF16) return start(tq::attention_kernel<__nv_bfloat16, kWidth, kKeys, kFew>);
+    return start(tq::attention_kernel<__half, kWidth, kKeys, kFew>);
   };
-  if (wide) {
-    constexpr size_t smem = tq::AttnLayout<2 * tq::kHeadDim>::kSmemBytes;
-    if (dtype == TQ_BF16) return go(tq::attention_kernel<__nv_bfloat16, 2 * tq::kHeadDim>, smem);
-    return go(tq::attention_kernel<__half, 2 * tq::kHeadDim>, smem);
-  }
-  constexpr size_t smem = tq::AttnLayout<tq::kHeadDim>::kSmemBytes;
-  if (dtype == TQ_BF16) return go(tq::attention_kernel<__nv_bfloat16, tq::kHeadDim>, smem);
-  return go(tq::attention_kernel<__half, tq::kHeadDim>, smem);
+  auto with_width = [&](auto keys, auto few) {
+    return wide ? go(std::integral_constant<int, 2 * tq::kHeadDim>{}, keys, few) : go(std::integral_constant<int, tq::kHeadDim>{}, keys, few);
+  };
+  auto with_keys = [&](auto few) {
+    return form.keys == 128 ? with_width(std::integral_constant<int, 128>{}, few) : with_width(std::integral_constant<int, 64>{}, few);
+  };
+  return form.few ? with_keys(std::true_type{}) : with_keys(std::false_type{});
 }

@@ -657,6 +657,13 @@ class AttentionKernel(Kernel):
     is [batch, heads, tokens, 64] in any such layout too — e.g. a transposed view of a
     [batch, tokens, heads * 64] buffer, which is what the projection after it reads. The reference
     runs bmm, mask, softmax, bmm with the scores in memory (csrc/tessiq/codegen/gemm.cpp:100-175,
+def attention_form(heads: int, q_tokens: int, k_tokens: int, head_dim: int, causal: bool, device: int = 0) -> tuple[str, int]:
+    """The kernel an attention launch runs: ("streamed", 0), or ("tiles" | "few", keys a step); device -1: on a B200, without a GPU."""
+    form, keys = ctypes.c_int32(), ctypes.c_int32()
+    check(lib.tq_attention_form(heads, q_tokens, k_tokens, head_dim, int(causal), device, ctypes.byref(form), ctypes.byref(keys)))
+    return ("streamed", "tiles", "few")[form.value], keys.value
+
+
     csrc/custom_ops/softmax/softmax.cu:19-61)."""
 
     kind = "attention"

@@ -106,14 +106,125 @@ def test_attention_with_other_head_widths(tq, width, causal):
 @pytest.mark.parametrize("width, dtype", [(64, torch.bfloat16), (128, torch.float16), (32, torch.bfloat16), (40, torch.float16), (8, torch.bfloat16)])
 @pytest.mark.parametrize("causal", [True, False], ids=["causal", "full"])
 def test_few_queries_against_a_cache(tq, queries, keys, width, dtype, causal):
-    """One to four query rows stream the keys (5 is the first size the tensor-core kernel takes); 515 and 1000
-    keys are shared by a cluster. Keys and values are views of a longer cache."""
+    """One to four query rows of a few heads stream the keys, unless they are so few that tiles are quicker (5 queries are the first
+    that always take tiles); 515 and 1000 keys are shared by a cluster. Keys and values are views of a longer cache."""
     q = draw((2, queries, 3, width), dtype, 31).transpose(1, 2)
     cache = draw((2, 2, 3, keys + 9, width), dtype, 32)
     k, v = cache[0][:, :, 4:keys + 4], cache[1][:, :, 4:keys + 4]
     cache = cache.cuda()
     got = tq.attention(q.cuda(), cache[0][:, :, 4:keys + 4], cache[1][:, :, 4:keys + 4], width ** -0.5, causal)
     check(got, q, k, v, width ** -0.5, causal, oracle_atol=2e-2)
+    assert poll() == 0
+
+
+FORMS = [  # batch, heads, queries, keys, width, causal, kernel, keys a step
+    (2, 3, 64, 64, 64, True, "tiles", 64), (2, 3, 200, 64, 64, False, "tiles", 64), (1, 2, 200, 50, 128, False, "tiles", 64),
+    (1, 2, 200, 65, 64, False, "tiles", 128), (1, 2, 300, 129, 64, True, "tiles", 128), (1, 3, 300, 515, 40, False, "tiles", 128),
+    (1, 2, 128, 1000, 128, False, "tiles", 128), (1, 3, 333, 333, 96, True, "tiles", 128), (1, 2, 700, 700, 64, True, "tiles", 128),
+    (40, 12, 5, 100, 64, False, "tiles", 64), (20, 16, 129, 129, 64, True, "tiles", 64), (50, 6, 200, 200, 64, False, "tiles", 64),
+    (13, 12, 64, 300, 128, False, "tiles", 64), (10, 16, 130, 130, 128, True, "tiles", 64), (7, 24, 20, 65, 72, False, "tiles", 64),
+    (30, 12, 130, 600, 64, False, "tiles", 128), (26, 12, 60, 600, 64, False, "tiles", 64),
+    (25, 6, 4, 64, 128, False, "few", 64), (25, 6, 4, 100, 64, False, "few", 64), (25, 6, 3, 77, 32, False, "few", 64),
+    (50, 6, 3, 400, 64, False, "few", 64), (50, 6, 2, 515, 96, False, "few", 64), (25, 6, 4, 1000, 128, False, "few", 64),
+    (1, 3, 4, 65, 64, False, "few", 128), (1, 3, 3, 100, 40, False, "few", 128), (1, 3, 4, 500, 128, False, "few", 128),
+    (24, 6, 1, 515, 72, False, "few", 128), (25, 3, 3, 1000, 128, False, "few", 128), (8, 18, 4, 900, 64, False, "few", 128),
+    (1, 3, 4, 900, 64, False, "streamed", 0), (50, 6, 1, 300, 128, False, "streamed", 0), (24, 6, 1, 600, 64, False, "streamed", 0),
+    (25, 6, 4, 900, 64, True, "streamed", 0),
+]
+
+
+@pytest.mark.parametrize("shape", FORMS, ids=lambda s: "x".join(map(str, s[:5])) + ("c" if s[5] else "") + s[6] + str(s[7]))
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_every_form(tq, shape, dtype):
+    """Each kernel that a call can take, around its tiles' edges: one step and several, a last step with one key, keys a step
+    that divide nothing, several CTAs an SM."""
+    from tessiq_b200.kernel import attention_form
+
+    batch, heads, queries, keys, width, causal, form, step = shape
+    assert attention_form(batch * heads, queries, keys, width, causal, device=-1) == (form, step)
+    q, k, v = (draw((batch, heads, n, width), dtype, 50 + i) for i, n in enumerate((queries, keys, keys)))
+    got = tq.attention(q.cuda(), k.cuda(), v.cuda(), width ** -0.5, causal)
+    check(got[:2], q[:2], k[:2], v[:2], width ** -0.5, causal, half_oracle=False)
+    exact = torch.from_numpy(restate.attention(*(t[-2:].double().numpy() for t in (q, k, v)), width ** -0.5, causal))
+    error = (got[-2:].cpu().double() - exact).abs()
+    ulp = 2.0**-8 if dtype == torch.bfloat16 else 2.0**-11
+    if form != "tiles":          # probabilities are not rounded: one rounding of the result, and f32 sums
+        assert (error <= 1.001 * ulp * exact.abs() + 2e-5 * exact.abs().max()).all()
+    else:
+        assert (error <= ulp * exact.abs() + ulp * v.abs().max().item()).all()
+    assert poll() == 0
+
+
+@pytest.mark.parametrize("batch, tokens", [(1, 128), (1, 300), (20, 256)], ids=["one step", "128 keys a step", "64 keys a step"])
+def test_the_largest_probability_is_exact(tq, batch, tokens):
+    """A row's reference point is the maximum over its first 128 keys, so where that is the row's maximum, its probability is
+    exactly 1 and loses nothing to 16 bits. Key 100 alone has a score, other than 0, and a value: the result is one
+    probability over the (f32) sum, within its own rounding."""
+    heads = 16
+    g = torch.Generator().manual_seed(60)
+    q = torch.zeros(batch, heads, tokens, 64)
+    q[..., 0] = torch.rand(batch, heads, tokens, generator=g) * 36 + 4
+    k, v = torch.zeros(batch, heads, tokens, 64), torch.zeros(batch, heads, tokens, 64)
+    k[..., 100, 0] = 1.0
+    v[..., 100, :] = 1.0
+    q, k, v = q.bfloat16(), k.bfloat16(), v.bfloat16()
+    got = tq.attention(q.cuda(), k.cuda(), v.cuda(), 0.125, False).cpu().double()[..., 0]
+    top = torch.exp(q[..., 0].double() * 0.125)                      # e^0.5 ... e^5
+    exact = top / (top + tokens - 1)
+    assert ((got - exact).abs() <= 2.0**-8 * exact * 1.002).all()      # half a unit in the last of bf16's eight places
+
+
+def _exact_with_specials(q, k, v, scale):
+    """float64 attention, NaN and infinity as they fall out of the arithmetic."""
+    scores = scale * q.double() @ k.double().transpose(-1, -2)
+    return torch.softmax(scores, dim=-1) @ v.double()
+
+
+@pytest.mark.parametrize("queries", [1, 4])
+@pytest.mark.parametrize("heads, keys", [(96, 300), (2, 900), (2, 7)], ids=["one CTA a head", "eight CTAs a head", "sets without a key"])
+@pytest.mark.parametrize("where", ["first", "middle", "last"])
+def test_decode_with_special_values(tq, queries, heads, keys, where):
+    """What is not finite meets ordinary values three times (lanes, warps, CTAs of a cluster) and must come through each
+    as float64 gives it: a NaN or an infinity in one key or one value, rows of -inf scores, and one
+    score far above all others, in the first, a middle and the last share of the keys (7 keys leave most sets empty)."""
+    from tessiq_b200.kernel import attention_form
+
+    batch, width = (8 if heads == 96 else 2), 64
+    assert attention_form(batch * heads, queries, keys, width, False, device=-1)[0] == "streamed"
+    at = {"first": 0, "middle": keys // 2, "last": keys - 1}[where]
+    q = draw((batch, heads, queries, width), torch.bfloat16, 41).abs() + 0.5       # no zero meets an infinity
+    k = draw((batch, heads, keys, width), torch.bfloat16, 42)
+    v = draw((batch, heads, keys, width), torch.bfloat16, 43)
+    inf, nan = float("inf"), float("nan")
+
+    qd, part = q.cuda(), (slice(1, 2), slice(0, 2))         # the changed head and one beside it are compared
+
+    def run(change):
+        kk, vv = k.clone(), v.clone()
+        change(kk, vv)
+        got = tq.attention(qd, kk.cuda(), vv.cuda(), width ** -0.5, False).cpu().double()[part]
+        exact = _exact_with_specials(q[part], kk[part], vv[part], width ** -0.5)
+        assert torch.equal(torch.isnan(got), torch.isnan(exact)) and torch.equal(torch.isinf(got), torch.isinf(exact))
+        infinite = torch.isinf(exact)
+        assert torch.equal(got[infinite], exact[infinite])
+        finite = torch.isfinite(exact)
+        # a rounding of the result, and of f32 sums over the keys
+        assert ((got - exact).abs() <= 2.0**-8 * exact.abs() + 2e-5)[finite].all()
+        return exact
+
+    def key(kk, value, head=1):
+        kk[1, head, at, 5] = value
+
+    run(lambda kk, vv: key(kk, nan))
+    run(lambda kk, vv: key(kk, inf))                        # one score +inf: inf - inf
+    assert torch.isfinite(run(lambda kk, vv: key(kk, -inf))).all()      # one score -inf: a probability of 0
+    run(lambda kk, vv: vv[1, 1].__setitem__((at, 3), nan))
+    assert torch.isinf(run(lambda kk, vv: vv[1, 1].__setitem__((at, 3), -inf))).any()
+    run(lambda kk, vv: vv[1, 1, at, 3:5].copy_(torch.tensor([inf, nan])))
+    run(lambda kk, vv: kk[1, 1, :, 0].fill_(-inf))          # every score of a head -inf: 0 / 0
+    run(lambda kk, vv: kk[1, 1, : max(1, keys - 3), 0].fill_(-inf))     # ... of all keys but the last three
+    dominated = run(lambda kk, vv: kk[1, 1, at].fill_(4.0))             # scores of about 40 above the others' 1
+    torch.testing.assert_close(dominated[0, 1], v[1, 1, at].double().expand_as(dominated[0, 1]), rtol=0, atol=1e-3)
     assert poll() == 0
 
 
