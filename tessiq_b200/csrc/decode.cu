@@ -2,11 +2,12 @@
 //
 //   out[b,h,i,:] = sum_j softmax_j(scale * q[b,h,i,:] . k[b,h,j,:]) v[b,h,j,:]     (j <= i when causal), i < 4
 //
-// With one to four query rows there is nothing for the tensor cores to reuse: each key and value is read
-// once and takes part in a handful of multiply-adds, so the kernel is a stream of K and V (bound: HBM).
-// The tensor-core kernel pads the queries to 256 rows and walks a head's keys in one CTA per SM: for 64 x 12
-// heads of 64 over 1000 keys it took 77.9 us where the bytes take 30.5; this one takes 41.1 (4.8 TB/s; 64 x 16
-// heads over 3000 keys 129 = 6.1 TB/s; four queries 73).
+// With one or two query rows there is nothing for the tensor cores to reuse: each key and value is read
+// once and takes part in a handful of multiply-adds, so the kernel is a stream of K and V (bound: HBM). Three or
+// four come here only where sharing a head's keys among CTAs is worth more (choose_attention_form).
+// The tensor-core kernel, which pads the queries to a tile and walks a head's keys in one CTA, took 77.9 us for 64 x 12
+// heads of 64 over 1000 keys when its tile was 256 rows, where the bytes take 30.5; this one takes 41.1 (4.8 TB/s; 64 x 16
+// heads over 3000 keys 129 = 6.1 TB/s).
 //
 // A key's row is spread over LANES neighbouring lanes, 16 bytes each, so that a load instruction of a warp
 // covers 32 / LANES whole rows; a lane keeps kUnroll keys and as many values in flight (8 KiB a warp for one
@@ -15,6 +16,8 @@
 // keys (maximum, sum and result in f32, probabilities never rounded), and the sets meet once, at the end:
 // by shuffles in the warp, through shared memory in the CTA, and through distributed shared memory in the
 // cluster of up to eight CTAs that share one head's keys when there are too few heads to fill the GPU.
+#include <mutex>
+
 #include "common.h"
 #include "tcgen05.h"
 
@@ -302,6 +305,44 @@ tq_status launch_width(const DecodeParams& p, long long heads_in_all, cudaStream
   return launch_queries<T, 16>(p, heads_in_all, stream);
 }
 
+// How many clusters of 1, 2, 4 and 8 CTAs run at once (148 SMs: 592, 296, 142 and 71), asked once per device; every form of the
+// kernel is built for four CTAs an SM.
+struct DecodeRoom {
+  long long of[4];
+};
+
+DecodeRoom decode_room(int32_t device) {
+  static std::mutex mutex;
+  static DecodeRoom known[64] = {};
+  const long long sms = sm_count(device);
+  const DecodeRoom assumed = {{4 * sms, 2 * sms, sms * 24 / 25, sms * 12 / 25}};
+  if (device < 0 || device >= 64) return assumed;
+  std::lock_guard<std::mutex> lock(mutex);
+  DecodeRoom& room = known[device];
+  if (room.of[0] == 0) {
+    room = assumed;
+    for (int i = 1; i < 4; ++i) {
+      cudaLaunchConfig_t config = {};
+      config.gridDim = dim3(1u << i);
+      config.blockDim = dim3(kDecodeThreads);
+      cudaLaunchAttribute attribute[1];
+      attribute[0].id = cudaLaunchAttributeClusterDimension;
+      attribute[0].val.clusterDim.x = 1u << i;
+      attribute[0].val.clusterDim.y = 1;
+      attribute[0].val.clusterDim.z = 1;
+      config.attrs = attribute;
+      config.numAttrs = 1;
+      int clusters = 0;
+      if (cudaOccupancyMaxActiveClusters(&clusters, attention_decode_kernel<__nv_bfloat16, 8, 1>, &config) != cudaSuccess || clusters <= 0) {
+        cudaGetLastError();
+        break;
+      }
+      room.of[i] = clusters;
+    }
+  }
+  return room;
+}
+
 }  // namespace
 
 // Called by tq_attention_launch, which has checked the arguments: 1 to kDecodeQueries query rows.
@@ -325,12 +366,14 @@ tq_status attention_decode(tq_dtype dtype, const void* q, const void* k, const v
   p.head_dim = static_cast<int>(head_dim);
   p.causal = causal;
   p.scale_log2 = scale_log2;
-  // Share a head's keys as long as all CTAs run at once (four an SM) and have some keys each: 96 heads of 4000
-  // keys take 46.1, 30.9, 23.6, 29.1 us shared by 1, 2, 4, 8 CTAs, 768 of 1000 keys 44.4, 43.9, 49.9, 64.8, and
-  // 1024 of 3000 keys 129.6, 138.9, 145.1, 161.8.
-  const long long resident = 4LL * sm_count(device), keys = causal && q_tokens < k_tokens ? q_tokens : k_tokens;
+  // Share a head's keys as long as all clusters run at once (four CTAs an SM, less what graphics processing clusters leave over) and have some
+  // keys each: 96 heads of 4000 keys take 46.8, 30.6, 22.3, 26.1 us shared by 1, 2, 4, 8 CTAs, 144 heads, for which
+  // clusters of four are two more than run at once, 48.4, 33.3, 38.7, 37.7, 768 of 1000 keys 44.4, 43.9, 49.9, 64.8, and 1024 of 3000
+  // keys 129.6, 138.9, 145.1, 161.8.
+  const long long keys = causal && q_tokens < k_tokens ? q_tokens : k_tokens;
+  const DecodeRoom room = decode_room(device);
   p.split = 1;
-  while (p.split < kDecodeMaxSplit && batch * heads * p.split * 2 <= resident && keys >= 96LL * p.split) p.split *= 2;
+  for (int i = 1; i < 4 && batch * heads <= room.of[i] && keys >= (96LL << (i - 1)); ++i) p.split = 1 << i;
   if (dtype == TQ_BF16) return launch_width<__nv_bfloat16>(p, batch * heads, stream);
   return launch_width<__half>(p, batch * heads, stream);
 }
