@@ -366,6 +366,11 @@ tq_status tq_batch_norm_eval_launch(tq_dtype dtype,
 typedef int32_t tq_activation;
 enum { TQ_ACT_NONE = 0, TQ_ACT_GELU_ERF = 1, TQ_ACT_GELU_TANH = 2 };
 
+/* How the launches below cut up a product of this shape: tiles of 256 rows by `tile_n` columns on pairs of CTAs (`ctas` 2), or of
+ * 128 rows on single ones (`ctas` 1), `split` of which share a tile's K range. It depends on how many CTAs and
+ * clusters `device` runs at once; device -1 stands for a B200 and needs no GPU. */
+tq_status tq_gemm_tiling(int64_t m, int64_t n, int64_t k, int64_t batch, int32_t trans_b, int32_t device,
+                         int32_t* ctas, int32_t* tile_n, int32_t* split);
 /* C[b] = act(op(A[b]) @ op(B[b]) + bias), row-major, bf16 or f16 operands, f32 accumulation in
  * tensor memory, one rounding to the output type after bias and activation.
  *   op(A) is [m,k]: trans_a == 0 -> A is row-major [m,k] with leading dimension lda (elements);
@@ -437,17 +442,17 @@ tq_status tq_gemm_bias_act_residual_launch(tq_dtype dtype,
 /* (csrc/custom_ops/softmax/softmax.cu:19-61), a second bmm, and the pack kernels around them    */
 /* (csrc/tessiq/codegen/pack.cpp:41-94), with the [batch, heads, T, T] scores in device memory. */
 
-/* out[b,h,i,:] = sum_j softmax_j(scale * q[b,h,i,:] . k[b,h,j,:]) * v[b,h,j,:], over j <= i when
- * causal != 0 (a lower-triangular mask aligned at the first query and the first key), else over
- * every key. bf16 or f16; scores, maxima and sums in f32; one rounding of the result.
- *   q is [batch, heads, q_tokens, head_dim], k and v are [batch, heads, k_tokens, head_dim], out is
- *   [batch, heads, q_tokens, head_dim]; each is addressed through three ELEMENT strides
 /* Which kernel the launch below runs for `heads` (batch times heads) of these extents: keys streamed by CUDA cores
  * (decoding), or the tensor-core kernel with 64 or 128 keys a step, in its form for many queries or for a few. It depends
  * on the number of SMs of `device`; device -1 stands for a B200 and needs no GPU. */
 enum { TQ_ATTENTION_STREAMED = 0, TQ_ATTENTION_TILES = 1, TQ_ATTENTION_TILES_FEW = 2 };
 tq_status tq_attention_form(int64_t heads, int64_t q_tokens, int64_t k_tokens, int64_t head_dim, int32_t causal, int32_t device,
                             int32_t* form, int32_t* keys);
+/* out[b,h,i,:] = sum_j softmax_j(scale * q[b,h,i,:] . k[b,h,j,:]) * v[b,h,j,:], over j <= i when
+ * causal != 0 (a lower-triangular mask aligned at the first query and the first key), else over
+ * every key. bf16 or f16; scores, maxima and sums in f32; one rounding of the result.
+ *   q is [batch, heads, q_tokens, head_dim], k and v are [batch, heads, k_tokens, head_dim], out is
+ *   [batch, heads, q_tokens, head_dim]; each is addressed through three ELEMENT strides
  *   {batch, head, token} and its head_dim elements are contiguous — so the slices of a fused QKV
  *   projection are read where they lie and the result can be written in [batch, token, head, dim]
  *   order.

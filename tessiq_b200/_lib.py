@@ -81,14 +81,15 @@ SIGNATURES = {
                                       c_int32, c_void_p]),
     "tq_batch_norm_eval_launch": (c_int32, [c_int32, c_int32, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p,
                                              c_void_p, c_int64, c_int64, c_int64, c_double, c_int32, c_void_p]),
+    "tq_gemm_tiling": (c_int32, [c_int64, c_int64, c_int64, c_int64, c_int32, c_int32, POINTER(c_int32), POINTER(c_int32), POINTER(c_int32)]),
     "tq_gemm_bias_act_launch": (c_int32, [c_int32, c_int32, c_void_p, c_int64, c_int32, c_void_p, c_int64,
                                            c_int32, c_void_p, c_void_p, c_int64, c_int64, c_int64, c_int64,
                                            c_int64, c_int64, c_int64, c_int64, c_int32, c_void_p]),
     "tq_gemm_bias_act_residual_launch": (c_int32, [c_int32, c_int32, c_void_p, c_int64, c_int32, c_void_p, c_int64, c_int32, c_void_p,
                                                     c_void_p, c_int64, c_int64, c_void_p, c_int64, c_int64, c_int64, c_int64, c_int64,
                                                     c_int64, c_int64, c_int64, c_int32, c_void_p]),
-    "tq_attention_launch": (c_int32, [c_int32, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int64, c_int64, c_int64,
     "tq_attention_form": (c_int32, [c_int64, c_int64, c_int64, c_int64, c_int32, c_int32, POINTER(c_int32), POINTER(c_int32)]),
+    "tq_attention_launch": (c_int32, [c_int32, c_void_p, c_void_p, c_void_p, c_void_p, c_int64, c_int64, c_int64, c_int64, c_int64,
                                        POINTER(c_int64), POINTER(c_int64), POINTER(c_int64), POINTER(c_int64), c_double, c_int32,
                                        c_int32, c_void_p]),
     "tq_recipe_create": (c_int32, [POINTER(c_void_p)]),

@@ -51,9 +51,8 @@ namespace tq {
 namespace {
 
 constexpr int kTileM = 128;
-constexpr int kTileN = 128;   // of the single-CTA kernel; the pair kernel's width is a template parameter
+constexpr int kSplitTileN = 128;   // of tiles whose K range a cluster shares; otherwise widths are template parameters
 constexpr int kTileK = 64;    // 64 two-byte elements = one 128-byte swizzle row
-constexpr int kStages = 6;
 constexpr int kMmaK = 16;
 constexpr int kThreads = 320;           // producer warp, issuer warp, eight epilogue warps
 constexpr int kEpilogueThreads = 256;
@@ -61,14 +60,8 @@ constexpr int kEpilogueWarps = kEpilogueThreads / 32;
 constexpr int kStoreColumns = 64;       // columns an epilogue warp regroups at a time
 constexpr uint32_t kStoreBytes = 32 * kStoreColumns * 2;   // 4 KiB of staging per epilogue warp
 constexpr uint32_t kBytesA = kTileM * kTileK * 2;   // 16 KiB
-constexpr uint32_t kBytesB = kTileN * kTileK * 2;   // 16 KiB
-constexpr uint32_t kStageBytes = kBytesA + kBytesB;
 constexpr uint32_t kChunkBytes = 64 * kTileK * 2;   // one 64-wide MN chunk of an MN-major operand: 8 KiB
-constexpr uint32_t kTmemColumns = 2 * kTileN;       // two accumulators
 constexpr int kMaxSplit = 8;                        // CTAs of a cluster that share one tile's K range
-
-constexpr size_t kSmemBytes = 1024 /*alignment slack*/ + static_cast<size_t>(kStages) * kStageBytes +
-                              2 * kTileN * sizeof(float) /*bias*/ + 256 /*barriers, tmem slot*/ + kEpilogueWarps * kStoreBytes;
 
 enum WaitCode { kWaitEmpty = 101, kWaitFull = 102, kWaitTmemEmpty = 103, kWaitTmemFull = 104 };
 
@@ -227,6 +220,7 @@ __device__ __forceinline__ void epilogue_rows(uint32_t tmem_accumulator, int qua
                                               T* c_tile, long long ldc, const T* residual_tile, long long ldr, int rows_left,
                                               int columns_left, int activation, unsigned char* staging, bool vector_ok) {
   const uint32_t staging_address = smem_address(staging);
+  if (quarter * 32 >= rows_left) return;       // C has none of this warp's rows
 #pragma unroll 1
   for (int block = half; block < TILE_N / kStoreColumns; block += 2) {
     const int column0 = block * kStoreColumns;
@@ -343,7 +337,7 @@ __device__ __forceinline__ void epilogue_rows(uint32_t tmem_accumulator, int qua
 __device__ __forceinline__ void push_partials(uint32_t tmem_accumulator, int quarter, int half, int lane, uint32_t ring, uint32_t rank, int split,
                                               int rows_left) {
   const int row = quarter * 32 + lane;
-  const int owned_units = kTileN / 4 / split;             // a power of two: kTileN, split are
+  const int owned_units = kSplitTileN / 4 / split;             // a power of two: kSplitTileN, split are
 #pragma unroll
   for (int step = 0; step < 2; ++step) {
     const int column0 = half * 64 + step * 32;
@@ -370,7 +364,7 @@ __device__ __forceinline__ void push_partials(uint32_t tmem_accumulator, int qua
 template <typename T>
 __device__ __forceinline__ void finish_split(uint32_t ring, uint32_t rank, int split, int epilogue_thread, const float* bias_tile, T* c_tile, long long ldc,
                                              const T* residual_tile, long long ldr, int rows_left, int columns_left, int activation, bool vector_ok) {
-  const int owned = kTileN / split;                       // 16, 32 or 64 columns
+  const int owned = kSplitTileN / split;                       // 16, 32 or 64 columns
   for (int item = epilogue_thread; item < kTileM * (owned / 16); item += kEpilogueThreads) {
     const int row = item % kTileM, local0 = (item / kTileM) * 16;
     const int column0 = static_cast<int>(rank) * owned + local0;
@@ -432,14 +426,28 @@ __device__ __forceinline__ bool whole_units(const GemmParams& p) {
          (p.residual == nullptr || ((p.ldr % 8 == 0) && ((reinterpret_cast<uintptr_t>(p.residual) & 15) == 0) && (p.stride_r % 8 == 0)));
 }
 
-template <typename T, bool A_MN, bool B_MN, bool SPLIT>
+template <int TILE_N>
+struct SingleShape {
+  static constexpr uint32_t kBytesB = TILE_N * kTileK * 2;            // 16 or 32 KiB
+  static constexpr uint32_t kStageBytes = kBytesA + kBytesB;
+  static constexpr int kStages = TILE_N == 128 ? 6 : 3;
+  static constexpr uint32_t kTmemColumns = 2 * TILE_N;                // two accumulators
+  static constexpr size_t kSmemBytes = 1024 /*alignment slack*/ + static_cast<size_t>(kStages) * kStageBytes + 2 * TILE_N * sizeof(float) /*bias*/ +
+                                       256 /*barriers, tmem slot*/ + kEpilogueWarps * kStoreBytes;
+};
+
+template <typename T, int TILE_N, bool A_MN, bool B_MN, bool SPLIT>
 __global__ void __launch_bounds__(kThreads, 1)
 gemm_bias_act_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const GemmParams p) {
+  using Shape = SingleShape<TILE_N>;
+  constexpr int kStages = Shape::kStages;
+  constexpr uint32_t kBytesB = Shape::kBytesB, kStageBytes = Shape::kStageBytes;
+  static_assert(!SPLIT || TILE_N == kSplitTileN, "the partial sums' way through the ring is laid out for one width");
   extern __shared__ unsigned char raw_smem[];
   const uint32_t base = (smem_address(raw_smem) + 1023u) & ~1023u;   // swizzled tiles need 1024-byte alignment
   unsigned char* aligned = raw_smem + (base - smem_address(raw_smem));
-  float* bias_smem = reinterpret_cast<float*>(aligned + kStages * kStageBytes);        // [2][kTileN]
-  const uint32_t barriers = base + kStages * kStageBytes + 2 * kTileN * sizeof(float);
+  float* bias_smem = reinterpret_cast<float*>(aligned + kStages * kStageBytes);        // [2][TILE_N]
+  const uint32_t barriers = base + kStages * kStageBytes + 2 * TILE_N * sizeof(float);
   // barrier slots, 8 bytes each: full[kStages], empty[kStages], tmem_full[2], tmem_empty[2]
   auto full_bar = [&](int s) { return barriers + 8u * s; };
   auto empty_bar = [&](int s) { return barriers + 8u * (kStages + s); };
@@ -447,7 +455,7 @@ gemm_bias_act_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
   auto tmem_empty_bar = [&](int a) { return barriers + 8u * (2 * kStages + 2 + a); };
   const uint32_t tmem_slot = barriers + 8u * (2 * kStages + 4);
   volatile uint32_t* tmem_slot_pointer =
-      reinterpret_cast<volatile uint32_t*>(aligned + kStages * kStageBytes + 2 * kTileN * sizeof(float) + 8 * (2 * kStages + 4));
+      reinterpret_cast<volatile uint32_t*>(aligned + kStages * kStageBytes + 2 * TILE_N * sizeof(float) + 8 * (2 * kStages + 4));
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
 
@@ -474,9 +482,9 @@ gemm_bias_act_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     }
     if constexpr (B_MN) {
 #pragma unroll
-      for (int i = 0; i < kTileN / 64; ++i) tma_load_3d(smem_b + i * kChunkBytes, &map_b, full_bar(s), tile_n * kTileN + i * 64, k0, batch);
+      for (int i = 0; i < TILE_N / 64; ++i) tma_load_3d(smem_b + i * kChunkBytes, &map_b, full_bar(s), tile_n * TILE_N + i * 64, k0, batch);
     } else {
-      tma_load_3d(smem_b, &map_b, full_bar(s), k0, tile_n * kTileN, batch);
+      tma_load_3d(smem_b, &map_b, full_bar(s), k0, tile_n * TILE_N, batch);
     }
   };
 
@@ -500,7 +508,7 @@ gemm_bias_act_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     tile_coordinates(first_tile, p, batch, tile_m, tile_n);
     for (int kb = 0; kb < early; ++kb) load_stage(kb, kb, batch, tile_m, tile_n);
   }
-  if (warp == 1) tmem_alloc(tmem_slot, kTmemColumns);
+  if (warp == 1) tmem_alloc(tmem_slot, Shape::kTmemColumns);
   tcgen05_fence_before();
   __syncthreads();
   tcgen05_fence_after();
@@ -525,7 +533,7 @@ gemm_bias_act_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
   } else if (warp == 1) {
     // ---- MMA issuer ------------------------------------------------------------------------
     if (elect_one()) {
-      constexpr uint32_t idesc = instruction_descriptor(std::is_same_v<T, __nv_bfloat16>, A_MN, B_MN, kTileM, kTileN);
+      constexpr uint32_t idesc = instruction_descriptor(std::is_same_v<T, __nv_bfloat16>, A_MN, B_MN, kTileM, TILE_N);
       // K-major: 8-row groups are 1024 B apart; a step of 16 along K is 32 B inside the swizzle row.
       // MN-major: 64-wide chunks are kChunkBytes apart, groups of 8 K-rows 1024 B; 16 K-rows = 2048 B.
       constexpr uint32_t lead_a = A_MN ? kChunkBytes : 0, lead_b = B_MN ? kChunkBytes : 0;
@@ -542,7 +550,7 @@ gemm_bias_act_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
         const uint32_t acc_phase = (local_tile >> 1) & 1;
         if (!barrier_wait(tmem_empty_bar(acc), acc_phase ^ 1, p.status, kWaitTmemEmpty)) break;
         tcgen05_fence_after();
-        const uint32_t tmem_d = tmem_base + acc * kTileN;
+        const uint32_t tmem_d = tmem_base + acc * TILE_N;
         uint32_t accumulate = 0;
         for (int kb = 0; kb < k_blocks; ++kb) {
           if (!barrier_wait(full_bar(s), phase, p.status, kWaitFull)) { alive = false; break; }
@@ -563,7 +571,7 @@ gemm_bias_act_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
     // block of 64 columns from block (w - 2) / 4 on ----------------------------------------------
     const int epilogue_thread = threadIdx.x - 64;
     const int quarter = warp & 3, half = (warp - 2) >> 2;
-    unsigned char* staging = aligned + kStages * kStageBytes + 2 * kTileN * sizeof(float) + 256 + (warp - 2) * kStoreBytes;
+    unsigned char* staging = aligned + kStages * kStageBytes + 2 * TILE_N * sizeof(float) + 256 + (warp - 2) * kStoreBytes;
     const bool vector_ok = whole_units(p);
     uint32_t local_tile = 0;
     for (long long tile = first_tile; tile < p.num_tiles; tile += tile_step, ++local_tile) {
@@ -571,9 +579,9 @@ gemm_bias_act_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
       tile_coordinates(tile, p, batch, tile_m, tile_n);
       const uint32_t acc = local_tile & 1;
       const uint32_t acc_phase = (local_tile >> 1) & 1;
-      const int n0 = tile_n * kTileN;
-      float* bias_tile = bias_smem + acc * kTileN;
-      for (int j = epilogue_thread; j < kTileN; j += kEpilogueThreads) {
+      const int n0 = tile_n * TILE_N;
+      float* bias_tile = bias_smem + acc * TILE_N;
+      for (int j = epilogue_thread; j < TILE_N; j += kEpilogueThreads) {
         float value = 0.f;
         if (p.bias != nullptr && n0 + j < p.n) value = to_compute(static_cast<const T*>(p.bias)[n0 + j]);
         bias_tile[j] = value;
@@ -603,7 +611,7 @@ gemm_bias_act_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
                           vector_ok);
         }
       } else {
-        epilogue_rows<T, kTileN>(tmem_base + acc * kTileN, quarter, half, lane, bias_tile, c_tile, p.ldc, residual_tile, p.ldr, rows_left, columns_left,
+        epilogue_rows<T, TILE_N>(tmem_base + acc * TILE_N, quarter, half, lane, bias_tile, c_tile, p.ldc, residual_tile, p.ldr, rows_left, columns_left,
                                  p.activation, staging, vector_ok);
         tcgen05_fence_before();
         __syncwarp();
@@ -624,7 +632,7 @@ gemm_bias_act_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_con
   __syncthreads();
   if (warp == 1) {
     tcgen05_fence_after();
-    tmem_dealloc(tmem_base, kTmemColumns);
+    tmem_dealloc(tmem_base, Shape::kTmemColumns);
   }
 }
 
@@ -851,33 +859,87 @@ struct Tiling {
   int split;
 };
 
-// The tiling with the least expected time, in microseconds, from a sweep over m = 1 ... 8192 and seven (k, n)
-// from 768 x 768 to 4096 x 16384 (B200, bf16, + bias + GELU): what a k-block of 64 costs a tile, what a tile
-// costs at least (its epilogue, where K is too short to cover it), and what a launch costs beside its waves.
-// A narrow tile does fewer products per byte it brings from L2 (a 128 x 128 k-block costs 0.23 where half of a
-// 256 x 256 one costs 0.18 per CTA), so it pays only where it saves a wave: 8192 x 3072 x 768 takes 2 waves of
-// 96 wide tiles (45.9 measured) or 2 of 128 tiles of 192 columns (41.0); 8192 x 4096 x 4096 161.8 and 174.0.
-// Sharing a tile's K range pays until the GPU is full: 64 x 4096 x 4096 24.6 alone, 21.2 by 2, 19.3 by 4.
-Tiling choose_tiling(long long m, long long n, long long k, long long batch, bool b_mn, int sms) {
+// How many clusters of 1, 2, 4 and 8 single CTAs run at once. Clusters of four and eight do not fill the GPU, since
+// one lies within a graphics processing cluster, whose number of SMs differs from unit to unit and from GPU to GPU
+// (33 and 15 on the B200 that the choice below was fitted on, which is what is assumed where there is none to ask).
+struct ClusterRoom {
+  long long of[4];
+};
+
+ClusterRoom assumed_room(long long sms) { return {{sms, sms / 2, sms * 33 / 148, sms * 15 / 148}}; }
+
+// The device that is current, asked once.
+ClusterRoom cluster_room(int32_t device) {
+  static std::mutex mutex;
+  static ClusterRoom known[64] = {};
+  const ClusterRoom assumed = assumed_room(sm_count(device));
+  if (device < 0 || device >= 64) return assumed;
+  std::lock_guard<std::mutex> lock(mutex);
+  ClusterRoom& room = known[device];
+  if (room.of[0] == 0) {
+    room = assumed;
+    auto kernel = gemm_bias_act_kernel<__nv_bfloat16, kSplitTileN, false, false, true>;
+    constexpr size_t kSmem = SingleShape<kSplitTileN>::kSmemBytes;
+    bool ok = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSmem)) == cudaSuccess;
+    for (int i = 1; ok && i < 4; ++i) {
+      cudaLaunchConfig_t config = {};
+      config.gridDim = dim3(1u << i);
+      config.blockDim = dim3(kThreads);
+      config.dynamicSmemBytes = kSmem;
+      cudaLaunchAttribute attribute[1];
+      attribute[0].id = cudaLaunchAttributeClusterDimension;
+      attribute[0].val.clusterDim.x = 1u << i;
+      attribute[0].val.clusterDim.y = 1;
+      attribute[0].val.clusterDim.z = 1;
+      config.attrs = attribute;
+      config.numAttrs = 1;
+      int clusters = 0;
+      ok = cudaOccupancyMaxActiveClusters(&clusters, kernel, &config) == cudaSuccess && clusters > 0;
+      if (ok) room.of[i] = clusters;
+    }
+    if (!ok) cudaGetLastError();
+  }
+  return room;
+}
+
+// The tiling with the least expected time, in microseconds. The constants are fitted to kernel times (graphs of launches over
+// rotating operands, B200, bf16) of every tiling at 346 shapes: m = 1 ... 8192 for sixteen (k, n) from 64 x 512 to 4096 x
+// 16384, and batches of 1 ... 2048 small products. A launch costs `launch`, each wave a k-block of 64 `block` per k-block, and
+// each wave but the last at least `tile` (its epilogue, where K is too short to cover it). Over those shapes the choice
+// takes 0.6 % longer than the best tiling on average; above 5 % only where a few rows could share K among more or fewer CTAs
+// (512 x 1024 x 1024: 9.0 by four against 8.2 by two).
+// A narrow tile does fewer products per byte it brings from L2 (a 128 x 128 k-block costs 0.22 where half of a
+// 256 x 256 one costs 0.16 per CTA), so it pays only where it saves a wave: 8192 x 3072 x 768 (m, n, k) takes 31 as 256 x 256, 37 as
+// 256 x 128; 4096 x 768 x 3072 takes 23.4 as 256 x 256, 21.1 as 256 x 192; 8192 x 768 x 768 14.4 and, as 256 x 128, 13.8.
+// A single CTA's 256-wide tile halves the epilogues of products with few rows and a short K: 768 products of 1 x 1000 x 64
+// take 54.5 where 128-wide tiles take 67.
+// Sharing a tile's K range pays until the GPU is full: 64 x 4096 x 4096 19.3 by one CTA, 14.4 by two, 12.2 by four; but more
+// clusters than there is room for take a second wave: 512 x 512 x 2048 is 16 clusters of eight, of which 15 run at once: 15.8
+// against 8.8 by four.
+Tiling choose_tiling(long long m, long long n, long long k, long long batch, bool b_mn, long long sms, const ClusterRoom& room) {
   const long long blocks = (k + kTileK - 1) / kTileK;
   Tiling best = {};
   double least = 0;
   auto consider = [&](Tiling t, long long tile_m, long long workers, double launch, double block, double tile) {
-    const long long work = ((m + tile_m - 1) / tile_m) * ((n + t.tile_n - 1) / t.tile_n) * batch * t.split;
-    const long long waves = (work + workers - 1) / workers, share = (blocks + t.split - 1) / t.split;
-    const double cost = launch + waves * (share * block > tile || waves == 1 ? share * block : tile);
-    // (clusters of four and eight do not fill the GPU: 36 clusters of four, 18 of eight already took two waves)
-    const bool fits = work <= (t.split > 2 ? sms - sms / 8 : sms) && blocks >= 2 * t.split;
-    if ((t.split == 1 || fits) && (best.split == 0 || cost < least)) {
+    const long long tiles = ((m + tile_m - 1) / tile_m) * ((n + t.tile_n - 1) / t.tile_n) * batch;
+    const double waves = static_cast<double>((tiles + workers - 1) / workers), share = static_cast<double>((blocks + t.split - 1) / t.split);
+    const double cost = launch + share * block + (waves - 1) * (share * block > tile ? share * block : tile);
+    if (best.split == 0 || cost < least) {
       best = t;
       least = cost;
     }
   };
-  for (int split = 1; split <= kMaxSplit; split *= 2) consider({false, kTileN, split}, kTileM, sms, split > 1 ? 8.5 : 7.5, 0.235, 3.9);
+  consider({false, 128, 1}, kTileM, sms, 7.51, 0.223, 2.87);
+  consider({false, 256, 1}, kTileM, sms, 7.77, 0.501, 5.50);
+  double hops = 0;
+  for (int i = 1; (1 << i) <= kMaxSplit; ++i) {
+    hops += 0.567;
+    if (blocks >= (2 << i)) consider({false, kSplitTileN, 1 << i}, kTileM, room.of[i], 8.15 + hops, 0.268, 14.6);
+  }
   if (m > kTileM) {
-    consider({true, 256, 1}, kPairTileM, sms / 2, 9.0, 0.36, 6.2);
-    if (!b_mn) consider({true, 192, 1}, kPairTileM, sms / 2, 8.5, 0.28, 5.6);
-    consider({true, 128, 1}, kPairTileM, sms / 2, 8.0, 0.205, 3.5);
+    consider({true, 256, 1}, kPairTileM, sms / 2, 8.48, 0.323, 4.80);
+    if (!b_mn) consider({true, 192, 1}, kPairTileM, sms / 2, 9.32, 0.270, 8.14);
+    consider({true, 128, 1}, kPairTileM, sms / 2, 7.75, 0.217, 2.77);
   }
   return best;
 }
@@ -907,12 +969,15 @@ template <typename T, bool A_MN, bool B_MN>
 tq_status launch_tiling(const Tiling& tiling, const CUtensorMap& map_a, const CUtensorMap& map_b, const GemmParams& p, int32_t device, cudaStream_t stream) {
   const long long sms = sm_count(device);
   if (!tiling.pair) {
-    if (tiling.split > 1) {
-      return launch_kernel(gemm_bias_act_kernel<T, A_MN, B_MN, true>, "gemm_bias_act_kernel", p.num_tiles * tiling.split, tiling.split, kSmemBytes, map_a,
-                           map_b, p, stream);
-    }
-    return launch_kernel(gemm_bias_act_kernel<T, A_MN, B_MN, false>, "gemm_bias_act_kernel", p.num_tiles < sms ? p.num_tiles : sms, 1, kSmemBytes, map_a,
-                         map_b, p, stream);
+    const long long ctas = tiling.split > 1 ? p.num_tiles * tiling.split : p.num_tiles < sms ? p.num_tiles : sms;
+    auto go = [&](auto tile_n, auto split) {
+      constexpr int kWidth = decltype(tile_n)::value;
+      return launch_kernel(gemm_bias_act_kernel<T, kWidth, A_MN, B_MN, decltype(split)::value>, "gemm_bias_act_kernel", ctas, tiling.split,
+                           SingleShape<kWidth>::kSmemBytes, map_a, map_b, p, stream);
+    };
+    if (tiling.split > 1) return go(std::integral_constant<int, kSplitTileN>{}, std::true_type{});
+    if (tiling.tile_n == 256) return go(std::integral_constant<int, 256>{}, std::false_type{});
+    return go(std::integral_constant<int, 128>{}, std::false_type{});
   }
   const long long pairs = p.num_tiles < sms / 2 ? p.num_tiles : sms / 2;
   auto go = [&](auto tile_n) {
@@ -938,6 +1003,24 @@ tq_status launch(bool a_mn, bool b_mn, const Tiling& tiling, const CUtensorMap& 
 
 }  // namespace
 }  // namespace tq
+
+extern "C" tq_status tq_gemm_tiling(int64_t m, int64_t n, int64_t k, int64_t batch, int32_t trans_b, int32_t device, int32_t* ctas, int32_t* tile_n,
+                                    int32_t* split) {
+  TQ_REQUIRE(ctas != nullptr && tile_n != nullptr && split != nullptr, TQ_INVALID_ARGUMENT, "null out-pointer");
+  TQ_REQUIRE(m > 0 && n > 0 && k > 0 && batch > 0, TQ_INVALID_ARGUMENT, "extents must be positive, not m=%lld n=%lld k=%lld batch=%lld", (long long)m,
+             (long long)n, (long long)k, (long long)batch);
+  tq::ClusterRoom room = tq::assumed_room(148);
+  if (device >= 0) {
+    tq::DeviceScope device_scope(device);
+    if (tq_status s = device_scope.status()) return s;
+    room = tq::cluster_room(device);
+  }
+  const tq::Tiling tiling = tq::choose_tiling(m, n, k, batch, trans_b == 0, room.of[0], room);
+  *ctas = tiling.pair ? 2 : 1;
+  *tile_n = tiling.tile_n;
+  *split = tiling.split;
+  return TQ_OK;
+}
 
 extern "C" tq_status tq_gemm_bias_act_launch(tq_dtype dtype, tq_activation activation, const void* a, int64_t lda,
                                              int32_t trans_a, const void* b, int64_t ldb, int32_t trans_b,
@@ -982,7 +1065,7 @@ extern "C" tq_status tq_gemm_bias_act_residual_launch(tq_dtype dtype, tq_activat
   const tq::WaitStatus status = tq::wait_status_for(device);
   TQ_REQUIRE(status.abort != nullptr, TQ_RESOURCE_EXHAUSTED, "no device memory for the status word");
 
-  const tq::Tiling tiling = tq::choose_tiling(m, n, k, batch, trans_b == 0, tq::sm_count(device));
+  const tq::Tiling tiling = tq::choose_tiling(m, n, k, batch, trans_b == 0, tq::sm_count(device), tq::cluster_room(device));
   CUtensorMap map_a, map_b;
   const long long batch_a = stride_a > 0 ? batch : 1, batch_b = stride_b > 0 ? batch : 1;
   // (rows of the tile that A does not have are not brought; what lies there gives rows of C nobody stores)

@@ -580,6 +580,13 @@ class LayerNormKernel(Kernel):
                                        float(self.eps), device, _stream(stream, device)))
 
 
+def gemm_tiling(m: int, n: int, k: int, batch: int = 1, trans_b: bool = True, device: int = 0) -> tuple[int, int, int]:
+    """(CTAs a tile, tile columns, CTAs that share a tile's K range) of the GEMM launch for this shape; device -1: of a B200, without a GPU."""
+    out = [ctypes.c_int32() for _ in range(3)]
+    check(lib.tq_gemm_tiling(m, n, k, batch, int(trans_b), device, *[ctypes.byref(o) for o in out]))
+    return tuple(o.value for o in out)
+
+
 class GemmKernel(Kernel):
     """C = act(op(A) @ op(B) + bias) on the tensor cores. Operands are described by their strides
     and consumed in place, so `packs_inputs` is False (csrc/tessiq/torch/fused.h:144-200,
@@ -650,13 +657,6 @@ class GemmKernel(Kernel):
         return dtype_code(a.dtype), lda, trans_a, ldb, trans_b, m, n, k, batch, stride_a, stride_b
 
 
-class AttentionKernel(Kernel):
-    """out = softmax(scale * q @ k.T [causal]) @ v in one launch, the scores kept on the SM.
-    `launch` takes [q, k, v], each [batch, heads, tokens, 64] in any layout whose last axis is
-    contiguous (views of a fused QKV projection are read in place, `packs_inputs` is False); `out`
-    is [batch, heads, tokens, 64] in any such layout too — e.g. a transposed view of a
-    [batch, tokens, heads * 64] buffer, which is what the projection after it reads. The reference
-    runs bmm, mask, softmax, bmm with the scores in memory (csrc/tessiq/codegen/gemm.cpp:100-175,
 def attention_form(heads: int, q_tokens: int, k_tokens: int, head_dim: int, causal: bool, device: int = 0) -> tuple[str, int]:
     """The kernel an attention launch runs: ("streamed", 0), or ("tiles" | "few", keys a step); device -1: on a B200, without a GPU."""
     form, keys = ctypes.c_int32(), ctypes.c_int32()
@@ -664,6 +664,13 @@ def attention_form(heads: int, q_tokens: int, k_tokens: int, head_dim: int, caus
     return ("streamed", "tiles", "few")[form.value], keys.value
 
 
+class AttentionKernel(Kernel):
+    """out = softmax(scale * q @ k.T [causal]) @ v in one launch, the scores kept on the SM.
+    `launch` takes [q, k, v], each [batch, heads, tokens, 64] in any layout whose last axis is
+    contiguous (views of a fused QKV projection are read in place, `packs_inputs` is False); `out`
+    is [batch, heads, tokens, 64] in any such layout too — e.g. a transposed view of a
+    [batch, tokens, heads * 64] buffer, which is what the projection after it reads. The reference
+    runs bmm, mask, softmax, bmm with the scores in memory (csrc/tessiq/codegen/gemm.cpp:100-175,
     csrc/custom_ops/softmax/softmax.cu:19-61)."""
 
     kind = "attention"

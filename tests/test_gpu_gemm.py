@@ -102,28 +102,54 @@ def test_residual_rides_in_the_epilogue(tq, m, n, k, act):
     assert poll() == 0
 
 
-@pytest.mark.parametrize("m, n, k, dtype", [
-    (100, 200, 320, torch.bfloat16),      # single CTAs, K whole
-    (1000, 768, 768, torch.bfloat16),     # ... K shared by two CTAs of a cluster
-    (128, 1001, 512, torch.float16),      # ... by four, rows of C that are not whole 16-byte units
-    (1, 136, 1040, torch.bfloat16),       # ... by eight, uneven shares, one row of A loaded in a box of eight
-    (20000, 130, 72, torch.bfloat16),     # CTA pairs, 256 x 128 tiles
-    (2500, 1000, 136, torch.float16),     # ... 256 x 192: the epilogue's halves take turns at the third block
-    (4224, 777, 768, torch.bfloat16),     # ... 256 x 256, odd rows of C
+@pytest.mark.parametrize("m, n, k, dtype, linear, matmul", [      # (CTAs a tile, its columns, CTAs sharing K) with B stored [n, k] and [k, n]
+    (100, 200, 320, torch.bfloat16, (1, 128, 1), (1, 128, 1)),
+    (100, 40001, 64, torch.float16, (1, 128, 1), (1, 128, 1)),        # three tiles a CTA: both accumulators are used again
+    (5000, 385, 64, torch.bfloat16, (1, 256, 1), (1, 256, 1)),
+    (7000, 1999, 64, torch.bfloat16, (1, 256, 1), (1, 256, 1)),       # three tiles a CTA, odd rows of C
+    (5000, 8, 1040, torch.bfloat16, (1, 128, 2), (1, 128, 2)),
+    (1, 136, 1040, torch.bfloat16, (1, 128, 4), (1, 128, 4)),         # uneven shares of K, one row of A loaded in a box of eight
+    (128, 1001, 1600, torch.float16, (1, 128, 8), (1, 128, 8)),       # rows of C that are not whole 16-byte units
+    (5000, 130, 4096, torch.bfloat16, (2, 128, 1), (2, 128, 1)),
+    (5000, 1001, 520, torch.float16, (2, 128, 1), (2, 128, 1)),       # three tiles a pair
+    (5000, 385, 1040, torch.bfloat16, (2, 192, 1), (2, 256, 1)),      # 192 columns: K-major B only
+    (5000, 1999, 1600, torch.bfloat16, (2, 192, 1), (2, 256, 1)),     # three tiles a pair: the halves of the epilogue take turns at the third block
+    (4224, 777, 768, torch.bfloat16, (2, 256, 1), (2, 256, 1)),
+    (5000, 1999, 64, torch.float16, (2, 256, 1), (2, 256, 1)),        # three tiles a pair
 ])
 @pytest.mark.parametrize("transposed", [False, True], ids=["linear", "matmul"])
-def test_every_tiling(tq, m, n, k, dtype, transposed):
+def test_every_tiling(tq, m, n, k, dtype, linear, matmul, transposed):
+    """Each form of the kernel, with one and with several tiles a CTA, and with a residual; the tilings are those of
+    the B200 that stands in for it where none is asked, since a unit's clusters may fit once more or less."""
+    from tessiq_b200.kernel import gemm_tiling
+
     if transposed:
         n = (n + 7) // 8 * 8              # B stored [k, n]: its rows have to start on 16-byte boundaries
+    assert gemm_tiling(m, n, k, trans_b=not transposed, device=-1) == (matmul if transposed else linear)
     g = torch.Generator().manual_seed(m + n + k)
-    a = (torch.randn(m, k, generator=g) * 0.5).to(dtype)
-    w = (torch.randn(n, k, generator=g) * (1.0 / np.sqrt(k))).to(dtype)
-    bias = (torch.randn(n, generator=g) * 0.5).to(dtype)
-    r = torch.randn(m, n, generator=g).to(dtype)
-    b = w.t().contiguous().cuda() if transposed else w.cuda().t()
+    a = (torch.randn(m, k, generator=g) * 0.5).to(dtype).cuda()
+    w = (torch.randn(n, k, generator=g) * (1.0 / np.sqrt(k))).to(dtype).cuda()
+    bias = (torch.randn(n, generator=g) * 0.5).to(dtype).cuda()
+    r = torch.randn(m, n, generator=g).to(dtype).cuda()
+    b = w.t().contiguous() if transposed else w.t()
     exact = truth(a, w.t(), bias, "gelu_erf")
-    check(tq.gemm(a.cuda(), b, bias.cuda(), "gelu"), exact, dtype, k)
-    check(tq.gemm(a.cuda(), b, bias.cuda(), "gelu", r.cuda()), exact + r.double(), dtype, k)
+    check(tq.gemm(a, b, bias, "gelu"), exact.cpu(), dtype, k)
+    check(tq.gemm(a, b, bias, "gelu", r), (exact + r.double()).cpu(), dtype, k)
+    assert poll() == 0
+
+
+@pytest.mark.parametrize("batch, m, n, k, tiling", [
+    (5, 1, 769, 1040, (1, 128, 2)), (2, 40, 200, 768, (1, 128, 4)), (2, 1, 136, 1600, (1, 128, 8)),      # a shared K range in each product
+    (300, 1, 1000, 64, (1, 256, 1)), (5, 130, 1999, 1040, (2, 192, 1)), (5, 7000, 130, 64, (2, 256, 1)), (3, 7000, 8, 1600, (2, 128, 1)),
+])
+def test_tilings_of_batches(tq, batch, m, n, k, tiling):
+    from tessiq_b200.kernel import gemm_tiling
+
+    assert gemm_tiling(m, n, k, batch, device=-1) == tiling
+    g = torch.Generator().manual_seed(m + n + k)
+    a = (torch.randn(batch, m, k, generator=g) * 0.5).bfloat16().cuda()
+    w = (torch.randn(batch, n, k, generator=g) * (1.0 / np.sqrt(k))).bfloat16().cuda()
+    check(tq.bmm(a, w.transpose(1, 2)), truth(a, w.transpose(1, 2), None, None).cpu(), torch.bfloat16, k)
     assert poll() == 0
 
 
