@@ -54,9 +54,23 @@ struct SumReducer {
   template <int VEC> using Local = Acc;
   template <int VEC> __device__ static Acc local_identity() { return identity(); }
   template <int VEC> __device__ static void step(Acc& local, T v, long long) { local += static_cast<Acc>(to_compute(v)); }
+  // (a vector is summed in a tree of its own first: few lanes a slice make a lane's chain of additions long, which sums of
+  // 32 bits show; 16-bit results are rounded far above it)
   template <int VEC> __device__ static void step_vector(Acc& local, const Vec<T, VEC>& x, long long) {
+    if constexpr (sizeof(T) == 2) {
 #pragma unroll
-    for (int e = 0; e < VEC; ++e) local += static_cast<Acc>(to_compute(x.v[e]));
+      for (int e = 0; e < VEC; ++e) local += static_cast<Acc>(to_compute(x.v[e]));
+    } else {
+      Acc part[VEC];
+#pragma unroll
+      for (int e = 0; e < VEC; ++e) part[e] = static_cast<Acc>(to_compute(x.v[e]));
+#pragma unroll
+      for (int width = VEC / 2; width > 0; width /= 2) {
+#pragma unroll
+        for (int e = 0; e < width; ++e) part[e] += part[e + width];
+      }
+      local += part[0];
+    }
   }
   template <int VEC> __device__ static Acc to_acc(Acc local) { return local; }
   __device__ static Out finish(Acc a, long long count, bool mean) {
@@ -445,11 +459,16 @@ reduce_columns(const T* __restrict__ in, typename R::Out* __restrict__ out, long
   const long long column = first_column + tx * VEC - before;       // of this thread's vectors
   const bool in_range = column < inner;
 
-  typename R::template Local<1> local[VEC];
+  // The ragged form gives a thread more rows than the plain one does. f32 sums take every fourth row into a chain of its own,
+  // so that they lose no digits by it.
+  constexpr int kMoreChains = RAGGED && std::is_same_v<R, SumReducer<float>> ? 3 : 0;
+  typename R::template Local<1> local[VEC], more[kMoreChains ? kMoreChains * VEC : 1];
 #pragma unroll
   for (int e = 0; e < VEC; ++e) local[e] = R::template local_identity<1>();
 
   if (in_range) {
+#pragma unroll
+  for (int i = 0; i < kMoreChains * VEC; ++i) more[i] = local[0];
     const T* base = in + slice * reduce * inner + column;
     constexpr int kBytes = static_cast<int>(sizeof(T)) * VEC;
     constexpr int UNROLL = kUnroll;
@@ -525,7 +544,13 @@ reduce_columns(const T* __restrict__ in, typename R::Out* __restrict__ out, long
               ri += lanes_y;
             } else {
 #pragma unroll
-              for (int e = 0; e < VEC; ++e) R::template step<1>(local[e], x.v[e], ri);
+              for (int e = 0; e < VEC; ++e) {
+                if constexpr (kMoreChains > 0) {
+                  R::template step<1>(d % 4 ? more[(d % 4 - 1) * VEC + e] : local[e], x.v[e], ri);
+                } else {
+                  R::template step<1>(local[e], x.v[e], ri);
+                }
+              }
               ri += lanes_y;
             }
             if (i + d + kRingDepth - 1 < count) copy((d + kRingDepth - 1) % kRingDepth);   // into the slot read one row ago
@@ -568,7 +593,10 @@ reduce_columns(const T* __restrict__ in, typename R::Out* __restrict__ out, long
   // Across ty, through shared memory, in a fixed order.
   Acc acc[VEC];
 #pragma unroll
-  for (int e = 0; e < VEC; ++e) acc[e] = R::template to_acc<1>(local[e]);
+  for (int e = 0; e < VEC; ++e) {
+    acc[e] = R::template to_acc<1>(local[e]);
+    if constexpr (kMoreChains > 0) acc[e] = (acc[e] + more[e]) + (more[VEC + e] + more[2 * VEC + e]);
+  }
 #pragma unroll
   for (int e = 0; e < VEC; ++e) {
     const int item = tx * VEC + e - before;

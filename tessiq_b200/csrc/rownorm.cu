@@ -157,12 +157,32 @@ __device__ __forceinline__ void store_stat(void* pointer, long long row, float v
   }
 }
 
+// f(0) + ... + f(VEC - 1): in a tree for rows of f32, whose sums show the order (few lanes a row make a lane's chain of
+// additions long), one after the other for 16-bit rows, whose results are rounded far above it.
+template <bool TREE, int VEC, typename F>
+__device__ __forceinline__ void add_vector(float& sum, F f) {
+  if constexpr (TREE) {
+    float part[VEC];
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) part[e] = f(e);
+#pragma unroll
+    for (int width = VEC / 2; width > 0; width /= 2) {
+#pragma unroll
+      for (int e = 0; e < width; ++e) part[e] += part[e + width];
+    }
+    sum += part[0];
+  } else {
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) sum += f(e);
+  }
+}
+
 // The arithmetic shared by the register-resident kernels. `x` holds this thread's vectors of the
 // row exactly as loaded: half-precision rows stay packed (two elements per register) and are
 // widened on the fly in every pass, so a thread keeps twice the bytes in flight per register.
 // `first` + j * `step` is the index of vector j within the row; vectors at or beyond `vectors` do
 // not exist. fold_row(value, is_max, stage) reduces a float over the whole row.
-template <typename T, typename OutT, int VEC, int K, int OP, typename FoldFn>
+template <typename T, typename OutT, int VEC, int K, int OP, bool TREE = false, typename FoldFn>
 __device__ __forceinline__ void finish_row(Vec<T, VEC> (&x)[K], int first, int step, int vectors,
                                            const RowArgs& args, long long row, bool writes_stats,
                                            FoldFn fold_row) {
@@ -184,12 +204,11 @@ __device__ __forceinline__ void finish_row(Vec<T, VEC> (&x)[K], int first, int s
 #pragma unroll
     for (int j = 0; j < K; ++j) {
       if (first + j * step < vectors) {
-#pragma unroll
-        for (int e = 0; e < VEC; ++e) {
+        add_vector<TREE, VEC>(sum, [&](int e) {
           const float value = exp2_approx((widen(x[j], e) - row_max) * kLog2e);
-          sum += value;
           if constexpr (kKeepsFloats) x[j].v[e] = from_compute<T, float>(value);
-        }
+          return value;
+        });
       }
     }
     const float inverse = 1.f / fold_row(sum, /*is_max=*/false, 1);
@@ -223,8 +242,7 @@ __device__ __forceinline__ void finish_row(Vec<T, VEC> (&x)[K], int first, int s
 #pragma unroll
       for (int j = 0; j < K; ++j) {
         if (first + j * step < vectors) {
-#pragma unroll
-          for (int e = 0; e < VEC; ++e) sum += widen(x[j], e);
+          add_vector<TREE, VEC>(sum, [&](int e) { return widen(x[j], e); });
         }
       }
       mean = fold_row(sum, false, 0) / width;
@@ -233,11 +251,10 @@ __device__ __forceinline__ void finish_row(Vec<T, VEC> (&x)[K], int first, int s
 #pragma unroll
     for (int j = 0; j < K; ++j) {
       if (first + j * step < vectors) {
-#pragma unroll
-        for (int e = 0; e < VEC; ++e) {
+        add_vector<TREE, VEC>(squares, [&](int e) {
           const float centred = widen(x[j], e) - mean;
-          squares += centred * centred;
-        }
+          return centred * centred;
+        });
       }
     }
     const float variance = fold_row(squares, false, 1) / width;
@@ -292,7 +309,7 @@ __global__ void __launch_bounds__(kBlock) row_warp_kernel(RowArgs args) {
   auto fold_row = [](float value, bool is_max, int) {
     return is_max ? warp_fold<float, true, LANES>(value) : warp_fold<float, false, LANES>(value);
   };
-  finish_row<T, OutT, VEC, K, OP>(x, lane, LANES, vectors, args, row, lane == 0 && row < args.rows, fold_row);
+  finish_row<T, OutT, VEC, K, OP, sizeof(T) == 4 && LANES < 32>(x, lane, LANES, vectors, args, row, lane == 0 && row < args.rows, fold_row);
 }
 
 // A cluster of `cluster` CTAs per row. blockIdx.x = row * cluster + rank.
@@ -415,13 +432,19 @@ row_ragged_kernel(RowArgs args, int cluster) {
     if constexpr (kScaled) {
       if (head != kept_head) {
         kept_head = head;
-        if (edge >= 0 && weight) w_edge = weight[edge];
-        if (edge >= 0 && bias) b_edge = bias[edge];
+        // (without weight or bias: 1 and -0, which change nothing)
+        w_edge = edge >= 0 && weight ? weight[edge] : from_compute<T, float>(1.f);
+        b_edge = edge >= 0 && bias ? bias[edge] : from_compute<T, float>(-0.f);
 #pragma unroll
         for (int j = 0; j < K; ++j) {
           if (first + j * THREADS < vectors) {
             const int at = head + (first + j * THREADS) * VEC;
             Vec<T, VEC> scale, shift;
+#pragma unroll
+            for (int e = 0; e < VEC; ++e) {
+              scale.v[e] = from_compute<T, float>(1.f);
+              shift.v[e] = from_compute<T, float>(-0.f);
+            }
             if (weight) scale = load_shifted<T, VEC>(weight, at, width);
             if (bias) shift = load_shifted<T, VEC>(bias, at, width);
             if constexpr (kInRegisters) {
@@ -448,14 +471,11 @@ row_ragged_kernel(RowArgs args, int cluster) {
       }
     };
     const float edge_value = to_compute(x_edge);
-    // f(element value, vector, element) for every element of the vectors this thread holds
-    auto each = [&](auto f) {
+    // sum += f(element value, vector, element) for every element of the vectors this thread holds
+    auto add_each = [&](float& sum, auto f) {
 #pragma unroll
       for (int j = 0; j < K; ++j) {
-        if (first + j * THREADS < vectors) {
-#pragma unroll
-          for (int e = 0; e < VEC; ++e) f(widen(x[j], e), j, e);
-        }
+        if (first + j * THREADS < vectors) add_vector<sizeof(T) == 4, VEC>(sum, [&](int e) { return f(widen(x[j], e), j, e); });
       }
     };
     // result(vector, element) rounded and stored
@@ -481,14 +501,20 @@ row_ragged_kernel(RowArgs args, int cluster) {
 
     if constexpr (OP == kSoftmax) {
       float local = edge >= 0 ? edge_value : -std::numeric_limits<float>::infinity();
-      each([&](float v, int, int) { local = nan_max(local, v); });
+#pragma unroll
+      for (int j = 0; j < K; ++j) {
+        if (first + j * THREADS < vectors) {
+#pragma unroll
+          for (int e = 0; e < VEC; ++e) local = nan_max(local, widen(x[j], e));
+        }
+      }
       const float row_max = fold_row(local, true, 0);
       const float edge_exp = edge >= 0 ? ragged_exp<OutT>(edge_value - row_max) : 0.f;
       float sum = edge_exp;
-      each([&](float v, int j, int e) {
+      add_each(sum, [&](float v, int j, int e) {
         const float value = ragged_exp<OutT>(v - row_max);
-        sum += value;
         if constexpr (sizeof(T) == 4) x[j].v[e] = value;
+        return value;
       });
       const float inverse = 1.f / fold_row(sum, false, 1);
       write([&](int j, int e) { return (sizeof(T) == 4 ? widen(x[j], e) : ragged_exp<OutT>(widen(x[j], e) - row_max)) * inverse; });
@@ -497,28 +523,23 @@ row_ragged_kernel(RowArgs args, int cluster) {
       float mean = 0.f;
       if constexpr (OP == kLayerNorm) {
         float sum = edge >= 0 ? edge_value : 0.f;
-        each([&](float v, int, int) { sum += v; });
+        add_each(sum, [](float v, int, int) { return v; });
         mean = fold_row(sum, false, 0) / static_cast<float>(width);
       }
       float squares = edge >= 0 ? (edge_value - mean) * (edge_value - mean) : 0.f;
-      each([&](float v, int, int) { squares += (v - mean) * (v - mean); });
+      add_each(squares, [&](float v, int, int) { return (v - mean) * (v - mean); });
       const float variance = fold_row(squares, false, 1) / static_cast<float>(width);
       const float rstd = 1.f / sqrtf(variance + static_cast<float>(args.eps));
       if (first == 0) {
         if constexpr (OP == kLayerNorm) store_stat<T>(args.mean, row, mean, args.stat_is_f32);
         store_stat<T>(args.rstd, row, rstd, args.stat_is_f32);
       }
-      auto finish = [&](float v, float scale, float shift) {
-        float value = (v - mean) * rstd;
-        if (weight) value *= scale;
-        if (bias) value += shift;
-        return value;
-      };
+      auto finish = [&](float v, float scale, float shift) { return fmaf((v - mean) * rstd, scale, shift); };
       Vec<T, VEC> scale, shift;
       write([&](int j, int e) {
         if constexpr (kInRegisters) return finish(widen(x[j], e), widen(w[j], e), widen(b[j], e));
-        if (e == 0 && weight) scale = kept[(2 * j) * kThreads];
-        if (e == 0 && bias) shift = kept[(2 * j + 1) * kThreads];
+        if (e == 0) scale = kept[(2 * j) * kThreads];
+        if (e == 0) shift = kept[(2 * j + 1) * kThreads];
         return finish(widen(x[j], e), widen(scale, e), widen(shift, e));
       });
       if (edge >= 0) out_row[edge] = from_compute<OutT, float>(finish(edge_value, to_compute(w_edge), to_compute(b_edge)));

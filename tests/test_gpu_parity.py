@@ -1093,6 +1093,53 @@ def test_reductions_of_short_rows(tq, dtype, rows, width):
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("rows", [8191, 8193, 16385])
+def _relative(got, exact):
+    return ((got.cpu().double() - exact).norm() / exact.norm()).item()
+
+
+@pytest.mark.parametrize("width", [64, 100, 128, 256])
+def test_sums_of_short_f32_rows_lose_no_digits(tq, width):
+    """However few lanes share a row, its f32 sum is as exact as a warp's: 16-byte pieces added in order by 32 lanes, which
+    meet pairwise. 20000 rows, whose rms error two runs of one order share to a per cent or two."""
+    x = torch.randn(20000, width, generator=torch.Generator().manual_seed(width))
+    lanes = torch.nn.functional.pad(x, (0, 512 - width)).view(20000, 4, 32, 4)
+    total = torch.zeros(20000, 32)
+    for piece in range(4):
+        for e in range(4):
+            total = total + lanes[:, piece, :, e]
+    while total.shape[1] > 1:
+        total = total[:, : total.shape[1] // 2] + total[:, total.shape[1] // 2 :]
+    exact = x.double().sum(-1)
+    assert _relative(tq.sum(dev(x), -1), exact) <= 1.03 * _relative(total[:, 0], exact)
+
+
+@pytest.mark.parametrize("rows, width", [(1000, 130), (4000, 50), (20000, 97)])
+def test_f32_column_sums_lose_no_digits_between_vectors(tq, rows, width):
+    """A thread of the ragged columns kernel has more rows than one of the plain kernel; the sums over columns that start between
+    vectors are as exact as those of the same values in whole ones."""
+    g = torch.Generator().manual_seed(width)
+    ragged, plain = [], []
+    for _ in range(20):
+        x = torch.randn(rows, width, generator=g)
+        exact = x.double().sum(0)
+        ragged.append(_relative(tq.sum(_inside(x, 1), 0), exact))
+        plain.append(_relative(tq.sum(dev(torch.nn.functional.pad(x, (0, -width % 4))), 0)[:width], exact))
+    assert sum(ragged) <= 1.1 * sum(plain)
+
+
+@pytest.mark.parametrize("width", [33, 65, 251])
+def test_ragged_f32_layer_norm_is_as_exact_as_whole_vectors(tq, width):
+    """Scaling and shift are one rounding, as where rows are whole vectors: against 64 bits the results of both are equally far off."""
+    whole = (width + 3) // 4 * 4
+    g = torch.Generator().manual_seed(width)
+    errors = []
+    for n in (width, whole):
+        x, w, b = torch.randn(20000, n, generator=g), 1 + torch.randn(n, generator=g) * 0.02, torch.randn(n, generator=g) * 0.02
+        exact = torch.nn.functional.layer_norm(x.double(), [n], w.double(), b.double(), 1e-5)
+        errors.append(_relative(tq.layer_norm(dev(x), [n], dev(w), dev(b), 1e-5), exact))
+    assert errors[0] <= 1.04 * errors[1]
+
+
 @pytest.mark.parametrize("vectors", [1, 7, 8, 9, 16, 17, 32, 33])
 def test_short_rows_of_whole_vectors(tq, dtype, rows, vectors):
     """From 8192 rows on eight lanes share a row of up to 16 vectors, from 16384 on of up to 32; 8193 and 16385 leave sets
