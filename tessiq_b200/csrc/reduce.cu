@@ -343,11 +343,13 @@ reduce_warp_per_slice(const T* __restrict__ in, typename R::Out* __restrict__ ou
   static_assert(LANES >= VEC, "a slice's head and tail are one element per lane");
   const int lane = threadIdx.x % LANES;
   const long long slice = static_cast<long long>(blockIdx.x) * (kBlock / LANES) + threadIdx.x / LANES;
+  if (LANES == 32 && slice >= outer) return;
   typename R::template Local<VEC> local = R::template local_identity<VEC>();
-  if (slice < outer) fold_span<T, R, VEC>(in + slice * reduce, 0, reduce, lane, LANES, local);
+  // (lanes without a slice stay for the shuffles)
+  if (LANES == 32 || slice < outer) fold_span<T, R, VEC>(in + slice * reduce, 0, reduce, lane, LANES, local);
   __syncwarp();
   typename R::Acc acc = warp_reduce<R, LANES>(R::template to_acc<VEC>(local));
-  if (lane == 0 && slice < outer) out[slice] = R::finish(acc, reduce, mean != 0);
+  if (lane == 0 && (LANES == 32 || slice < outer)) out[slice] = R::finish(acc, reduce, mean != 0);
 }
 
 // `split` CTAs per slice, `cluster` of them in one thread-block cluster (cluster divides split).
@@ -465,10 +467,10 @@ reduce_columns(const T* __restrict__ in, typename R::Out* __restrict__ out, long
   typename R::template Local<1> local[VEC], more[kMoreChains ? kMoreChains * VEC : 1];
 #pragma unroll
   for (int e = 0; e < VEC; ++e) local[e] = R::template local_identity<1>();
-
-  if (in_range) {
 #pragma unroll
   for (int i = 0; i < kMoreChains * VEC; ++i) more[i] = local[0];
+
+  if (in_range) {
     const T* base = in + slice * reduce * inner + column;
     constexpr int kBytes = static_cast<int>(sizeof(T)) * VEC;
     constexpr int UNROLL = kUnroll;
@@ -1113,16 +1115,18 @@ tq_status run(const Plan& p, const void* in, void* out, long long outer, long lo
   constexpr int kVec = 16 / sizeof(T);
   switch (p.shape) {
     case Shape::kWarpPerSlice: {
-      // Short slices share a warp. Measured (300000 slices, us with 32 / 16 / 8 lanes): 500 bf16 sum 98.7 / 61.3 / 53.6, argmax
-      // 154.8 / 90.4 / 66.9; 250 f32 sum 78.0 / 51.9 / 50.2; 500 f32 sum 89.6 / 94.3 / 101, argmax 116 / 95 / 102; 80000 of 1000
-      // bf16 sum 28.0 / 28.5 / 31.7, argmax 44.6 / 34.7 / 35.2. Of few slices eight lanes make too few warps: 1000 of 250 f32
-      // 3.1 / 3.2 / 4.0.
+      // Short slices share a warp, of many slices also longer ones; of few, eight or sixteen lanes only make each slice's chain
+      // longer. Measured (us with 32 / 16 / 8 lanes): 300000 slices of 500 bf16 sum 98.7 / 61.3 / 53.6, argmax 154.8 / 90.4 / 66.9; of 250 f32
+      // sum 78.0 / 51.9 / 50.2; of 500 f32 sum 89.6 / 94.3 / 101, argmax 116 / 95 / 102; 40000 of 96 f64 sum 12.3 / 8.0 / 9.4; 1000
+      // slices of 1000 bf16 sum 2.1 / 2.5 / 3.3, argmax 2.7 / 3.2 / 4.4, 12000 6.5 / 6.9 / 6.9 and 8.8 / 8.5 / 7.9; 1000 of
+      // 250 f32 3.1 / 3.2 / 4.0.
       const long long slice_bytes = reduce * static_cast<long long>(sizeof(T));
-      constexpr bool kBusy = sizeof(T) == 2 || std::is_same_v<R, ArgmaxReducer<T>>;
-      const bool many = outer >= 64ll * sm_count(p.device);
-      const int lanes = slice_bytes <= 512 || (slice_bytes <= 1024 && sizeof(T) == 2 && many) ? 8
-                        : slice_bytes <= 1024 || (slice_bytes <= 2048 && kBusy)               ? 16
-                                                                                             : 32;
+      constexpr bool kArgmax = std::is_same_v<R, ArgmaxReducer<T>>, kBusy = sizeof(T) == 2 || kArgmax;
+      const long long per_sm = outer / sm_count(p.device);
+      const int lanes = slice_bytes <= 512                            ? 8
+                        : slice_bytes <= 1024 && per_sm >= 16        ? (sizeof(T) == 2 && per_sm >= 64 ? 8 : 16)
+                        : slice_bytes <= (sizeof(T) == 2 && !kArgmax ? 1536 : 2048) && kBusy && per_sm >= 96 ? 16
+                                                                     : 32;
       const int slices = kBlock / lanes;
       const long long blocks = (outer + slices - 1) / slices;
       TQ_REQUIRE(blocks <= 0x7fffffffLL, TQ_UNSUPPORTED, "%lld slices are more than a grid holds", outer);

@@ -1072,10 +1072,11 @@ def test_transposes_that_fill_no_whole_tile(tq, dtype, rows, cols):
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.float64, torch.bfloat16, torch.float16, torch.int32, torch.int64])
 @pytest.mark.parametrize("rows, width", [(1, 1), (3, 7), (33, 15), (1000, 31), (257, 64), (70, 65), (999, 128), (31, 129), (64, 256), (65, 257),
-                                         (9480, 300), (40, 300), (40, 1001), (13, 1025)])
+                                         (9480, 300), (40, 300), (40, 1001), (13, 1025), (2400, 200), (2400, 500), (14300, 300), (14300, 700)])
 def test_reductions_of_short_rows(tq, dtype, rows, width):
-    """Eight or sixteen lanes a row, or a warp, by bytes, type and number of rows (9480: enough for eight lanes over more than
-    512 bytes): row counts that leave sets of lanes without a row, and rows that start between vectors."""
+    """Eight or sixteen lanes a row, or a warp, by bytes, type and number of rows (of 148 SMs: 16 rows each are enough for sixteen lanes over
+    more than 512 bytes, 64 for eight, 96 for sixteen over more than 1024): row counts that leave sets of lanes
+    without a row, and rows that start between vectors."""
     x = (torch.randn(rows, width, generator=torch.Generator().manual_seed(rows + width)) * 50).to(dtype)
     for shift in (0, 1, 3):
         xd = _inside(x, shift)
@@ -1091,8 +1092,6 @@ def test_reductions_of_short_rows(tq, dtype, rows, width):
         assert ((tq.mean(xd, -1).cpu().double() - exact / width).abs() <= bound * (exact / width).abs() + budget / width).all()
 
 
-@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
-@pytest.mark.parametrize("rows", [8191, 8193, 16385])
 def _relative(got, exact):
     return ((got.cpu().double() - exact).norm() / exact.norm()).item()
 
@@ -1140,6 +1139,8 @@ def test_ragged_f32_layer_norm_is_as_exact_as_whole_vectors(tq, width):
     assert errors[0] <= 1.04 * errors[1]
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("rows", [8191, 8193, 16385])
 @pytest.mark.parametrize("vectors", [1, 7, 8, 9, 16, 17, 32, 33])
 def test_short_rows_of_whole_vectors(tq, dtype, rows, vectors):
     """From 8192 rows on eight lanes share a row of up to 16 vectors, from 16384 on of up to 32; 8193 and 16385 leave sets
