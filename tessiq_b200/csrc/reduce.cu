@@ -1034,7 +1034,19 @@ Plan plan(tq_reduce_op op, tq_dtype dtype, long long outer, long long reduce, lo
     // Rows no whole vector fits go to the ragged form, unless they are so short that most of its lanes would
     // have no column, or the pass is one of statistics (their callers ask for whole vectors).
     const int whole = (op == TQ_ARGMAX ? 4 : 8) < 16 / size ? (op == TQ_ARGMAX ? 4 : 8) : 16 / size;
-    p.ragged = may_be_ragged && vec < whole && (size == 2 || size == 4) && op < kOpSoftmaxStat && inner >= 12 * whole && reduce < (1ll << 31);
+    // ... or they are few and their bytes too: up to so many rows the plain form needs no tickets, and is done while the
+    // ragged one folds (us, plain and ragged: 200 x 709 bf16 sum 3.2 and 4.4, argmax 3.5 and 6.8; 17 x 3001 f32 sum 2.4 and 2.8, argmax
+    // 2.7 and 5.2, 128 x 3001 argmax 4.4 and 6.2; but 300 x 9999 bf16 sum 10.8 and 5.7, 1000 x 50 f32 sum 8.2 and 4.1, argmax 9.3 and
+    // 7.5, 64 x 1000001 f32 sum 100 and 49).
+    const long long rows_without_tickets = size == 2 || op == TQ_ARGMAX ? 288 : 144;
+    const long long elements = outer * reduce * inner;
+    const bool small = reduce < rows_without_tickets && elements * size < (op == TQ_ARGMAX ? 4ll << 20 : 1ll << 20);
+    // ... or argmax of four-byte elements two columns a load (or a row within one tile) over 60 to 300 MB, where the plain
+    // form's waves fill (us, plain and ragged: 40000 x 502 f32 36.6 and 40.5, 160000 x 98 41.8 and 51.8; but 40000 x 370 .8, 10000 x 1002
+    // .78, 2000 x 1250 .39 of the plain form's time, 40000 x 2002 .99, 32768 x 4098 .93).
+    const bool plain_fills = op == TQ_ARGMAX && size == 4 && elements >= 15500000 && elements < 75000000 && (vec >= 2 || inner <= 31 * whole);
+    p.ragged = may_be_ragged && vec < whole && (size == 2 || size == 4) && op < kOpSoftmaxStat && inner >= 12 * whole && reduce < (1ll << 31) && !small &&
+               !plain_fills;
     if (p.ragged) vec = whole;
     p.vec = vec;
     long long groups = (inner + vec - 1) / vec;
@@ -1052,11 +1064,15 @@ Plan plan(tq_reduce_op op, tq_dtype dtype, long long outer, long long reduce, lo
     // One or two waves of CTAs (all of a wave resident at once, equal work each).
     const int waves = (p.ring && !(op == TQ_ARGMAX && size <= 2)) ? 2 : 1;
     long long want = (target_ctas * waves + base_ctas - 1) / base_ctas;
-    // (the ragged form: at least twice the ring's depth of rows a thread; 5003 x 1250 bf16 split finer is all folding)
+    // (the ragged form: at least twice the ring's depth of rows a thread; 5003 x 1250 split finer is all folding, f32 sum 18.2 us against 14.5)
     const long long per_pass = static_cast<long long>(kBlock / lanes) * (p.ragged ? 2 * kRingDepth : kUnroll);
     long long most = reduce / per_pass;
     if (most < 1) most = 1;
     if (want > most) want = most;
+    // Argmax's accumulators leave room for four CTAs an SM, of which clusters of eight fill 24 of 25: whole waves of those. 6 tiles
+    // shared by 200 CTAs each were 150 clusters where 142 run at once: 40256 x 709 f32 49.4 us, now 46.
+    const long long wave = target_ctas * 24 / 25;
+    if (p.ragged && op == TQ_ARGMAX && want * base_ctas > wave) want = want * base_ctas / wave * wave / base_ctas;
     if (want < 1) want = 1;
     // The cluster's reduce-scatter gives every CTA a whole number of threads' accumulators.
     int max_cluster = kMaxCluster;
@@ -1066,7 +1082,8 @@ Plan plan(tq_reduce_op op, tq_dtype dtype, long long outer, long long reduce, lo
       p.cluster = p.split;
     } else {
       if (want > 1024) want = 1024;
-      p.split = static_cast<int>((want + max_cluster - 1) / max_cluster * max_cluster);
+      // (rounded down in the ragged form, whose waves are counted out)
+      p.split = static_cast<int>((p.ragged ? want : want + max_cluster - 1) / max_cluster * max_cluster);
       p.cluster = max_cluster;
     }
     p.tiles = base_ctas;

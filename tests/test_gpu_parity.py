@@ -1029,11 +1029,13 @@ def test_ragged_rows_with_special_values(tq):
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16, torch.int32])
 @pytest.mark.parametrize("shape, dim", [((1003, 205), 0), ((5003, 1250), 0), ((3, 129, 997), 1), ((7, 96), 0), ((700, 249), 0), ((9, 3001), 0),
-                                        ((40000, 131), 0), ((2, 300, 104), 1)])
+                                        ((40000, 131), 0), ((2, 300, 104), 1), ((5, 600001), 0), ((288, 135), 0), ((287, 135), 0),
+                                        ((16000, 1002), 0)])
 def test_columns_of_rows_that_start_between_vectors(tq, dtype, shape, dim):
     """The ragged columns kernel: tiles of 31 vectors at the tile's edges, a first and a last row whose vectors
     would leave the tensor, starts between vectors (with them also widths that are whole vectors), more warps
-    than rows, and splits with and without tickets."""
+    than rows (5 x 600001), and splits with and without tickets; and the plain kernel, which keeps tensors of few rows and bytes (287 rows
+    and fewer for most types) and argmax of four-byte elements over 15.5 to 75 million of them two columns a load."""
     g = torch.Generator().manual_seed(shape[-1])
     x = (torch.randn(*shape, generator=g) * 50).to(dtype)
     for shift in (0, 1, 2, 5):
