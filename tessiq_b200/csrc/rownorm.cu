@@ -758,7 +758,22 @@ tq_status run_ragged(const RowArgs& args, cudaStream_t stream, bool* handled) {
   // Four vectors a thread up to 1024 of them: 20000 x 2003 bf16 LayerNorm / softmax 40 / 34 us with 64 threads
   // against 60 / 44 with 32 that hold eight, 5000 x 8003 40 / 37 with 256 against 44 / 39; but 80000 x 1003 88 / 79
   // with 64 that hold two against 80 / 63 with 32 that hold four.
-  if (in_step) {
+  // The loop kernel, 256 threads a row, stays where it is quicker (us, ragged and loop). Few rows: LayerNorm and RMSNorm
+  // wait for their shifted weights, 64 x 1003 bf16 5.7 and 3.9, 1000 rows 5.4 and 4.8, 1200 rows 6.4 and 6.6; 64 x 250 f32 3.0
+  // and 2.5, 512 rows 3.1 and 3.0; 296 x 2051 f32 6.0 and 4.6, 800 rows 7.0 and 7.0. Many rows that leave a
+  // cluster's threads half empty: 1000 x 8201 f32 softmax 35.0 and 20.5, LayerNorm 41.8 and 23.3, but 148 rows 6.1 and 7.1, 10.6 and 19.1, 300 x
+  // 33001 42.5 and 46.0, and full ones, 300 x 65535, 56 and 149. 16-bit rows into f32, whose expf adds to that: 1600 x 8201 25.7
+  // and 24.3, 3000 rows 51.8 and 41.9.
+  int device = 0;
+  TQ_CUDA(cudaGetDevice(&device));
+  const long long sms = sm_count(device);
+  const bool waits = OP != kSoftmax && vectors > 32 && vectors <= 512 && args.rows < (vectors > 64 && vectors <= 256 ? 7 : 3) * sms;
+  long long room = kBlock * kMaxVectors;       // vectors that a CTA, or the cluster that would take the row, holds
+  while (room < vectors && room < static_cast<long long>(kBlock) * kMaxVectors * kMaxCluster) room *= 2;
+  const bool half_empty = vectors * 4 <= room * 3;
+  const bool long_rows = half_empty && vectors > kBlock * kMaxVectors && args.rows > (vectors <= 2 * kBlock * kMaxVectors ? 2 : 3) * sms;
+  const bool busy = half_empty && sizeof(OutT) > sizeof(T) && vectors > 1024 && args.rows >= 8 * sms;
+  if (in_step && !waits && !long_rows && !busy) {
     if (vectors <= 32) return launch_ragged<T, OutT, VEC, 1, OP, 32>(args, 1, stream);
     if (vectors <= 64) return launch_ragged<T, OutT, VEC, 2, OP, 32>(args, 1, stream);
     if (vectors <= 128) return launch_ragged<T, OutT, VEC, 4, OP, 32>(args, 1, stream);

@@ -973,10 +973,12 @@ def _inside(t, shift):
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("rows, width", [(5, 1), (40, 3), (11, 9), (70, 33), (300, 515), (61, 1003), (4000, 1021), (19, 2051), (13, 4099),
-                                         (9, 8201), (9, 16390), (5, 33001), (3, 131071), (2, 140001)])
+                                         (9, 8201), (9, 16390), (5, 33001), (3, 131071), (2, 140001), (900, 251), (1100, 515), (1100, 1003),
+                                         (900, 2051), (300, 16395), (300, 8201), (1200, 8201)])
 def test_rows_that_start_between_vectors(tq, dtype, rows, width):
     """Every team size of the ragged row kernel, from rows without a whole vector to rows beyond a cluster's
-    registers; 4000 rows: a team takes several. The third shift puts weight and bias off their boundaries too,
+    registers; 4000 rows: a team takes several. LayerNorm and RMSNorm of fewer than 1036 rows of middling width, and more than 296 rows
+    that would leave a cluster half empty, are the loop kernel's. The third shift puts weight and bias off their boundaries too,
     which the loop kernel takes."""
     g = torch.Generator().manual_seed(rows * width)
     x = (torch.randn(rows, width, generator=g) * 2 + 0.5).to(dtype)
