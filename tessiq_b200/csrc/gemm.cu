@@ -3,7 +3,7 @@
 //   C[b] = act(op(A[b]) @ op(B[b]) + bias)      bf16 or f16 operands, f32 accumulation, one rounding
 //
 // Two kernels share the work by shape (choose_tiling): CTA pairs over 256 x 256, 256 x 192 or 256 x 128 tiles
-// (below), and single CTAs over 128 x 128 tiles, several of which may share a tile's K range. In both,
+// (below), and single CTAs over 128 x 128 tiles, several of which may share a tile's K range, or 128 x 256 ones. In both,
 // persistent CTAs walk the tiles and ten warps of a CTA have three jobs:
 //
 //   warp 0, one lane   producer: TMA loads (cp.async.bulk.tensor, 128-byte swizzle) of a 64-wide slice
@@ -22,8 +22,8 @@
 //
 // A product with few rows is a stream of B. 64 x 4096 x 4096 took 35.2 us as 16 tiles of 256 columns on 16 SMs
 // and takes 14.2 as 32 tiles of 128 columns with four CTAs of a cluster on each, which add their partial
-// sums through distributed shared memory (its bytes: 5.4 us; the launch, the first loads and the
-// two cluster barriers are the rest: 768 x 768 with one row takes 6.3).
+// sums through distributed shared memory (kernel times after an L2 flush; in a graph of such launches 12.5. Its bytes: 5.4; the
+// launch, the first loads and the two cluster barriers are the rest: 768 x 768 with one row takes 6.3).
 //
 // Tensor memory holds two f32 accumulators, so the epilogue of tile i
 // runs under the MMAs of tile i+1. Either operand may be K-major (row-major A, nn.Linear weight
