@@ -578,8 +578,8 @@ struct AttentionForm {
 // More queries: 128 keys a step halve the hand-overs of a chain, but only two CTAs share an SM (one for heads above 64)
 // where 64 keys let three (two). 1 x 8 x 4096 causal 68.9 with 64, 54.4 with 128; 64 x 12 x 1024 causal 228.7 and 228.7; 5 ... 9 waves
 // of 200 to 256 tokens 0 - 4 % better with 64; 64 x 6 x 1024 of 128 174.7 and 225. Without a mask, CTAs that fit
-// three an SM but not two are one wave with 64 (384 CTAs over 4096 keys 90.6 and 92.9). Up to 64 keys half of a 128-key step would be empty
-// (64 x 12 x 64 11.4 and 15.5).
+// three an SM but not two are one wave with 64 (384 CTAs over 4096 keys 90.6 and 92.9). Half of a 128-key step may be empty: of the only
+// one (64 x 12 x 64 11.4 and 15.5) or of the last (without a mask 64 x 12 x 700 185.4 and 204).
 AttentionForm choose_attention_form(long long heads, long long q_tokens, long long k_tokens, long long head_dim, bool causal, long long sms) {
   const bool wide = head_dim > kHeadDim;
   if (q_tokens <= kDecodeQueries) {
@@ -599,7 +599,8 @@ AttentionForm choose_attention_form(long long heads, long long q_tokens, long lo
   if (k_tokens <= 64) return {false, 64, false};
   if (wide) return {false, ctas <= sms ? 128 : 64, false};
   const bool thirds = !causal && ctas > 2 * sms && ctas <= 3 * sms;
-  return {false, ctas <= 2 * sms || (k_tokens >= 512 && !thirds) ? 128 : 64, false};
+  const bool half_step = !causal && k_tokens < 1280 && (k_tokens + 63) / 64 % 2 == 1;
+  return {false, ctas <= 2 * sms || (k_tokens >= 512 && !thirds && !half_step) ? 128 : 64, false};
 }
 
 }  // namespace tq

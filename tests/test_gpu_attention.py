@@ -123,7 +123,7 @@ FORMS = [  # batch, heads, queries, keys, width, causal, kernel, keys a step
     (1, 2, 128, 1000, 128, False, "tiles", 128), (1, 3, 333, 333, 96, True, "tiles", 128), (1, 2, 700, 700, 64, True, "tiles", 128),
     (40, 12, 5, 100, 64, False, "tiles", 64), (20, 16, 129, 129, 64, True, "tiles", 64), (50, 6, 200, 200, 64, False, "tiles", 64),
     (13, 12, 64, 300, 128, False, "tiles", 64), (10, 16, 130, 130, 128, True, "tiles", 64), (7, 24, 20, 65, 72, False, "tiles", 64),
-    (30, 12, 130, 600, 64, False, "tiles", 128), (26, 12, 60, 600, 64, False, "tiles", 64),
+    (30, 12, 130, 600, 64, False, "tiles", 128), (30, 12, 130, 700, 64, False, "tiles", 64), (30, 12, 130, 700, 64, True, "tiles", 128), (26, 12, 60, 600, 64, False, "tiles", 64),
     (25, 6, 4, 64, 128, False, "few", 64), (25, 6, 4, 100, 64, False, "few", 64), (25, 6, 3, 77, 32, False, "few", 64),
     (50, 6, 3, 400, 64, False, "few", 64), (50, 6, 2, 515, 96, False, "few", 64), (25, 6, 4, 1000, 128, False, "few", 64),
     (1, 3, 4, 65, 64, False, "few", 128), (1, 3, 3, 100, 40, False, "few", 128), (1, 3, 4, 500, 128, False, "few", 128),
