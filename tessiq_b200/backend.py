@@ -617,7 +617,8 @@ def build_recipe(gm: fx.GraphModule, math_mode: str = "fast") -> Recipe:
             recipe.steps.append(_gemm_epilogue_step(node, gemm_act_at.get(node, "none"), gemm_residual_at.get(node)))
             continue
         if node in passes_through:
-            recipe.steps.append(Step("view", node.name, lambda env, name=passes_through[node].name: env[name], [passes_through[node].name]))
+            recipe.steps.append(Step("view", node.name, lambda env, name=passes_through[node].name: env[name], [passes_through[node].name],
+                                     view=_itself))
             continue
         if node in member_of:
             group = member_of[node]
@@ -662,6 +663,10 @@ def _constant_step(node: fx.Node) -> Step:
     return Step("constant", node.name, run, [])
 
 
+def _itself(value):
+    return value
+
+
 def _gemm_epilogue_step(addmm: fx.Node, activation: str, residual: fx.Node | None) -> Step:
     """act(bias + a @ b) + residual with the activation and the addition in the GEMM's epilogue."""
     bias, a, b = addmm.args[:3]
@@ -685,13 +690,19 @@ def _gemm_epilogue_step(addmm: fx.Node, activation: str, residual: fx.Node | Non
 def _fused_step(node: fx.Node, kernel: FusedKernel, inputs: list[fx.Node]) -> Step:
     dtype = node.meta["val"].dtype
     strided = [read == "strided" for read in kernel.reads]
+    names = [i.name for i in inputs]
 
     def run(env):
-        tensors = [env[i.name] for i in inputs]
-        tensors = [t if (s or t.is_contiguous()) else ops.contiguous(t) for t, s in zip(tensors, strided)]
+        given = [env[name] for name in names]
+        out = ops.fused_again(kernel, given)
+        if out is not None:
+            return out
+        tensors = [t if (s or t.is_contiguous()) else ops.contiguous(t) for t, s in zip(given, strided)]
         shape = broadcast_shape(*[t.shape for t in tensors])   # from the operands, so one recipe serves every size
         out = torch.empty(shape, dtype=dtype, device=tensors[0].device)
         kernel.launch(tensors, out, stream=None)
+        if all(t is g for t, g in zip(tensors, given)):
+            ops.keep_fused(kernel, given, out)
         return out
 
     return Step("fused", node.name, run, [i.name for i in inputs], kernel=kernel)
@@ -730,7 +741,16 @@ def _kernel_step(node: fx.Node) -> Step | None:
         return Step(kind, node.name, run, reads)
 
     if target in VIEWS:
-        return step("view", target if kwargs else _VIEW_METHODS.get(target, target))
+        made = step("view", target if kwargs else _VIEW_METHODS.get(target, target))
+        if len(reads) == 1 and len(args) > 0 and isinstance(args[0], fx.Node):
+            function, rest = (target if kwargs else _VIEW_METHODS.get(target, target)), args[1:]
+
+            def view(value):
+                return function(value, *rest, **kwargs)
+
+            view.picks = target is operator.getitem
+            made.view = view
+        return made
     value = node.meta.get("val")
     first = args[0].meta.get("val") if args and _is_tensor_node(args[0]) else None
     if first is not None and first.dtype not in DTYPE_NAMES:

@@ -1,9 +1,10 @@
-"""Builds libtessiq_b200.so, in tree, for sm_100a.
+"""Builds libtessiq_b200.so, in tree, for sm_100a, and the Python module beside it that launches from it.
 
     python -m tessiq_b200.build [--force] [--verbose]
 
 Each `csrc/*.cu` is compiled to an object with nvcc (in parallel) and the objects are linked into
-`tessiq_b200/libtessiq_b200.so` with the CUDA runtime linked statically. NVRTC (used to instantiate
+`tessiq_b200/libtessiq_b200.so` with the CUDA runtime linked statically; `csrc/launcher.cpp` becomes
+`tessiq_b200/_launcher.so` (torch's headers, the host compiler). NVRTC (used to instantiate
 fused elementwise kernels) is opened at run time, so the library loads on a machine without a GPU
 or a driver. Objects are rebuilt only when a source or header is newer.
 """
@@ -23,6 +24,7 @@ ROOT = PACKAGE.parent
 CSRC = PACKAGE / "csrc"
 OBJECTS = CSRC / "build"
 LIBRARY = PACKAGE / "libtessiq_b200.so"
+LAUNCHER = PACKAGE / "_launcher.so"
 
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
 COMMON = [
@@ -83,7 +85,33 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         result = subprocess.run(command, capture_output=True, text=True)
         if result.returncode != 0:
             raise RuntimeError(f"linking {LIBRARY.name} failed:\n{result.stdout}\n{result.stderr}")
+    build_launcher(force, verbose)
     return LIBRARY
+
+
+def build_launcher(force: bool = False, verbose: bool = False) -> Path:
+    source = CSRC / "launcher.cpp"
+    stamp = max(source.stat().st_mtime, (ROOT / "include" / "tessiq_b200.h").stat().st_mtime, Path(__file__).stat().st_mtime)
+    if not force and LAUNCHER.exists() and LAUNCHER.stat().st_mtime >= stamp:
+        return LAUNCHER
+    import sysconfig
+
+    import torch
+
+    home = Path(torch.__file__).resolve().parent
+    cuda = Path(nvcc()).resolve().parent.parent
+    command = [
+        os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-Wall", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+        *[f"-I{path}" for path in (home / "include", home / "include" / "torch" / "csrc" / "api" / "include", cuda / "include",
+                                   sysconfig.get_paths()["include"], ROOT / "include")],
+        str(source), "-o", str(LAUNCHER), f"-L{home / 'lib'}", "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-ltorch", "-lc10_cuda", "-lc10", "-ldl",
+    ]
+    if verbose:
+        print(" ".join(command), flush=True)
+    result = subprocess.run(command, capture_output=True, text=True)
+    if result.returncode != 0:
+        raise RuntimeError(f"building {LAUNCHER.name} failed:\n{result.stdout}\n{result.stderr}")
+    return LAUNCHER
 
 
 def main() -> None:

@@ -36,6 +36,45 @@ class Step:
     reads: list[str]
     kernel: Any = None
     note: str = ""
+    view: Callable[[Any], Any] | None = None      # a view step: what it makes of the one value it reads
+
+
+class _Views:
+    """A chain of view operators as one step: a view is its sizes, strides and offset within the value the chain starts
+    from, the same for every value of one shape and layout, so the chain is walked for the first such value and is one
+    `as_strided` from then on (of a decoder block's 29 view operators 15 calls are left). A chain that copies is walked each time."""
+
+    def __init__(self, source: str, pick: Callable[[Any], Any] | None, chain: list[Callable[[Any], Any]], escapes: bool):
+        self.source, self.pick, self.chain, self.escapes = source, pick, chain, escapes
+        self._seen: dict = {}
+
+    def __call__(self, env: dict):
+        base = env[self.source]
+        if self.pick is not None:
+            base = self.pick(base)
+        if type(base) is not torch.Tensor and type(base) is not torch.nn.Parameter:
+            return self._walk(base)
+        if not self.chain:
+            return base
+        key = (base.shape, base.stride())
+        found = self._seen.get(key)
+        if found is None:
+            out = self._walk(base)
+            if isinstance(out, torch.Tensor) and out.dtype == base.dtype and out.numel() and out.device == base.device \
+                    and out.untyped_storage().data_ptr() == base.untyped_storage().data_ptr():
+                if len(self._seen) >= 64:
+                    self._seen.clear()
+                offset = out.storage_offset() - base.storage_offset()
+                same = offset == 0 and out.shape == base.shape and out.stride() == base.stride() and not self.escapes
+                self._seen[key] = (same, out.shape, out.stride(), offset)
+            return out
+        same, shape, stride, offset = found
+        return base if same else base.as_strided(shape, stride, base.storage_offset() + offset)
+
+    def _walk(self, value):
+        for view in self.chain:
+            value = view(value)
+        return value
 
 
 @dataclass
@@ -45,19 +84,42 @@ class Recipe:
     outputs: Any = None
     kernels: list[Any] = field(default_factory=list)
     notes: list[str] = field(default_factory=list)   # why a rewrite (fused attention, ...) did not apply
+    _schedule: list[Step] = field(default_factory=list)      # the steps with chains of views made one
     _dead_after: list[list[str]] = field(default_factory=list)
 
     def finish(self) -> None:
-        """Records, for every step, which values no later step reads."""
+        """Makes chains of views one step each and records, for every step, which values no later step reads."""
         kept = {n.name for n in _nodes_in(self.outputs)}
+        self._schedule = self._with_merged_views(kept)
         last: dict[str, int] = {}
-        for i, step in enumerate(self.steps):
+        for i, step in enumerate(self._schedule):
             for name in step.reads:
                 last[name] = i
-        self._dead_after = [[] for _ in self.steps]
+        self._dead_after = [[] for _ in self._schedule]
         for name, i in last.items():
             if name not in kept:
                 self._dead_after[i].append(name)
+
+    def _with_merged_views(self, kept: set[str]) -> list[Step]:
+        views = {step.output: step for step in self.steps if step.view is not None}
+        needed = set(kept)      # values that something other than a view reads
+        for step in self.steps:
+            if step.view is None:
+                needed.update(step.reads)
+        schedule = []
+        for step in self.steps:
+            if step.view is None:
+                schedule.append(step)
+            elif step.output in needed:
+                chain, source = [], step.output
+                while source in views:
+                    chain.append(views[source].view)
+                    source = views[source].reads[0]
+                chain.reverse()
+                # (the first view of a step with several results picks one of them)
+                pick = chain.pop(0) if getattr(chain[0], "picks", False) else None
+                schedule.append(Step("view", step.output, _Views(source, pick, chain, step.output in kept), [source]))
+        return schedule
 
     def counts(self) -> dict[str, int]:
         out: dict[str, int] = {}
@@ -88,7 +150,7 @@ class Recipe:
         if len(args) != len(self.inputs):
             raise ValueError(f"the recipe takes {len(self.inputs)} inputs, not {len(args)}")
         env = dict(zip(self.inputs, args))
-        for step, dead in zip(self.steps, self._dead_after):
+        for step, dead in zip(self._schedule, self._dead_after):
             env[step.output] = step.run(env)
             if keep is not None:
                 keep.append(env[step.output])

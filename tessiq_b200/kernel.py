@@ -14,6 +14,7 @@ Tensors are CUDA tensors; only their pointers, sizes and strides cross into the 
 from __future__ import annotations
 
 import ctypes
+import itertools
 import math
 from functools import lru_cache
 from typing import Sequence
@@ -191,6 +192,9 @@ def layout_for(t: torch.Tensor, out_shape: Sequence[int]) -> _lib.tq_layout:
     return layout
 
 
+_codes = itertools.count(1 << 32)
+
+
 class FusedKernel(Kernel):
     """One fusion group compiled from a program text (see include/tessiq_b200.h).
 
@@ -227,6 +231,7 @@ class FusedKernel(Kernel):
         handle = ctypes.c_void_p()
         check(lib.tq_fused_create(program.encode(), ctypes.byref(handle)))
         self._handle = handle
+        self.code = next(_codes)       # of this kernel's plans in the launcher; never used again for another
         self._pointers = ctypes.c_void_p * max(len(names), 1)
         self._doubles = ctypes.c_double * max(len(self.scalars), 1)
         self._plans: dict = {}
@@ -625,12 +630,18 @@ class GemmKernel(Kernel):
         bias = inputs[2] if self.has_bias else None
         residual = inputs[-1] if self.has_residual else None
         device = _device_of([t for t in (a, b, bias, residual, out) if t is not None])
-        key = _signature(a, b, bias, residual, out)
-        plan = self._plans.get(key) or _keep(self._plans, key, self._plan(inputs, a, b, bias, residual, out))
-        dtype, lda, trans_a, ldb, trans_b, m, n, k, batch, stride_a, stride_b = plan
+        dtype, lda, trans_a, ldb, trans_b, m, n, k, batch, stride_a, stride_b = self.plan(inputs, out)
         check(lib.tq_gemm_bias_act_residual_launch(dtype, self.activation, a.data_ptr(), lda, trans_a, b.data_ptr(), ldb, trans_b,
                                                    _pointer(bias), _pointer(residual), n, m * n, out.data_ptr(), n, m, n, k,
                                                    batch, stride_a, stride_b, m * n, device, _stream(stream, device)))
+
+    def plan(self, inputs, out):
+        """(type, leading dimensions and transpositions of a and b, m, n, k, batch, their batch strides) of a launch."""
+        a, b = inputs[0], inputs[1]
+        bias = inputs[2] if self.has_bias else None
+        residual = inputs[-1] if self.has_residual else None
+        key = _signature(a, b, bias, residual, out)
+        return self._plans.get(key) or _keep(self._plans, key, self._plan(inputs, a, b, bias, residual, out))
 
     def _plan(self, inputs, a, b, bias, residual, out):
         if a.dim() != b.dim() or a.dim() not in (2, 3):
@@ -696,10 +707,14 @@ class AttentionKernel(Kernel):
         self._check_count(inputs)
         q, k, v = inputs
         device = _device_of([q, k, v, out])
-        key = _signature(q, k, v, out)
-        dtype, extents = self._plans.get(key) or _keep(self._plans, key, self._plan(q, k, v, out))
+        dtype, extents = self.plan(q, k, v, out)
         check(lib.tq_attention_launch(dtype, q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), *extents, self.scale, int(self.causal), device,
                                       _stream(stream, device)))
+
+    def plan(self, q, k, v, out):
+        """(type, extents and strides) of a launch."""
+        key = _signature(q, k, v, out)
+        return self._plans.get(key) or _keep(self._plans, key, self._plan(q, k, v, out))
 
     def _plan(self, q, k, v, out):
         if not (q.dtype == k.dtype == v.dtype == out.dtype):

@@ -17,13 +17,11 @@ from typing import Sequence
 
 import torch
 
-from . import _lib
+from . import _launcher
 from .kernel import (DTYPE_NAMES, REDUCE_OPS, AttentionKernel, FusedKernel, GemmKernel, LayerNormKernel, PackKernel, SoftmaxKernel, _device_of,
-                     _keep, _pointer, _stream, broadcast_shape, check_status, classify_read, dtype_code, launch_reduce, launch_transposed,
-                     prefers_transposed, reduce_workspace_bytes, workspace)
-from ._lib import Declined, check, lib
-
-import ctypes
+                     _pointer, _stream, broadcast_shape, check_status, classify_read, dtype_code, launch_reduce, launch_transposed,
+                     prefers_transposed, reduce_workspace_bytes, transposed_workspace_bytes, workspace)
+from ._lib import LIBRARY_PATH, Declined, check, lib
 
 UNARY = {"abs", "neg", "relu", "sigmoid", "sqrt", "tanh", "exp", "expm1", "log", "log1p", "log2", "log10", "rsqrt",
          "reciprocal", "sin", "cos", "tan", "asin", "acos", "atan", "sinh", "cosh", "floor", "ceil", "trunc", "round",
@@ -31,6 +29,7 @@ UNARY = {"abs", "neg", "relu", "sigmoid", "sqrt", "tanh", "exp", "expm1", "log",
 BINARY = {"add", "sub", "mul", "div", "pow", "maximum", "minimum", "gt", "ge", "lt", "le", "eq", "ne", "logical_and",
           "logical_or", "swiglu"}
 COMPARES = {"gt", "ge", "lt", "le", "eq", "ne", "logical_and", "logical_or", "logical_not"}
+_ELEMENTWISE_CODES = {(op, mode): 1000 + 2 * i + j for i, op in enumerate(sorted(UNARY | BINARY | {"where"})) for j, mode in enumerate(("fast", "precise"))}
 
 
 @lru_cache(maxsize=512)
@@ -41,7 +40,18 @@ def _kernel(program: str) -> FusedKernel:
 _pack = PackKernel()
 _softmax_kernel, _layer_norm_kernel = lru_cache(maxsize=64)(SoftmaxKernel), lru_cache(maxsize=64)(LayerNormKernel)
 _gemm_kernel, _attention_kernel = lru_cache(maxsize=64)(GemmKernel), lru_cache(maxsize=64)(AttentionKernel)
-_PLAIN = (torch.Tensor, torch.nn.Parameter)     # a subclass, or a tracer's stand-in, goes the long way every time
+
+# Repeated calls (csrc/launcher.cpp): every entry point asks the launcher first, which answers None for a signature it has no
+# plan for; the long way below it leaves one when a call was a single launch over the operands as they came.
+_launcher.setup(torch.nn.Parameter, workspace, str(LIBRARY_PATH))
+_FUSED, _REDUCE, _PACK, _SOFTMAX, _LAYER_NORM, _TRANSPOSED, _BATCH_NORM, _GEMM, _ATTENTION = range(9)      # launcher.cpp: Family
+_call, _keep_plan = _launcher.call, _launcher.keep
+_CODES = {name: 1 + i for i, name in enumerate(("pack", "softmax", "layer_norm", "native_layer_norm", "batch_norm", "attention", "sum", "mean", "amax",
+                                                "amin", "argmax", "gemm none", "gemm gelu", "gemm gelu_erf", "gemm gelu_tanh"))}
+
+
+def _fused_ints(kernel: FusedKernel, elements: int, divisors) -> tuple:
+    return (kernel._handle.value, elements, *divisors)
 
 
 def fused(program: str, inputs: Sequence[torch.Tensor], out: torch.Tensor, scalars: Sequence[float] = ()) -> torch.Tensor:
@@ -50,18 +60,29 @@ def fused(program: str, inputs: Sequence[torch.Tensor], out: torch.Tensor, scala
     return out
 
 
+def fused_again(kernel: FusedKernel, tensors: Sequence[torch.Tensor]) -> torch.Tensor | None:
+    """What `kernel` makes of operands of a signature that `keep_fused` has seen; None for any other."""
+    return _call(kernel.code, *tensors)
+
+
+def keep_fused(kernel: FusedKernel, tensors: Sequence[torch.Tensor], out: torch.Tensor) -> None:
+    elements, divisors, layouts = kernel.plan(tensors, out)
+    if elements:
+        _keep_plan(False, kernel.code, tuple(tensors), _FUSED, (out,), _fused_ints(kernel, elements, divisors), (), bytes(layouts), kernel)
+
+
 def contiguous(x: torch.Tensor) -> torch.Tensor:
     """A packed copy of any view, by the pack kernel; `x` itself when it already is packed."""
-    if x.is_contiguous():
-        return x
-    out = torch.empty(x.shape, dtype=x.dtype, device=x.device)
-    _pack.launch([x], out, stream=None)
-    return out
+    return x if x.is_contiguous() else clone(x)
 
 
 def clone(x: torch.Tensor) -> torch.Tensor:
+    out = _call(_CODES["pack"], x)
+    if out is not None:
+        return out
     out = torch.empty(x.shape, dtype=x.dtype, device=x.device)
     _pack.launch([x], out, stream=None)
+    _keep_plan(False, _CODES["pack"], (x,), _PACK, (out,), (x.element_size(), x.dim(), *x.shape, *x.stride()), (), b"", None)
     return out
 
 
@@ -131,23 +152,10 @@ def elementwise(op: str, *operands, math_mode: str = "fast", out: torch.Tensor |
     operands must share an element type (mixed types are promoted by torch on its host path in the
     reference, which here is a decline); Python numbers become kernel scalars. `out` writes into an
     existing tensor (an operand itself for the in-place form) under the reference's conditions."""
-    if out is None:
-        key = [op, math_mode]
-        for o in operands:
-            if type(o) in _PLAIN:
-                key += (o.dtype, o.shape, o.stride(), o.get_device())
-            elif isinstance(o, torch.Tensor):
-                key = None
-                break
-            else:
-                key.append(type(o))
-        key = None if key is None else tuple(key)
-        plan = _elementwise_plans.get(key)
-        if plan is not None:
-            kernel, size, stride, dtype, where, device, start = plan
-            result = torch.empty_strided(size, stride, dtype=dtype, device=where)
-            kernel.start([o for o in operands if isinstance(o, torch.Tensor)], result.data_ptr(), *start,
-                         [o for o in operands if not isinstance(o, torch.Tensor)], device, _stream(None, device))
+    code = _ELEMENTWISE_CODES.get((op, math_mode)) if out is None else None
+    if code is not None:
+        result = _launcher.elementwise(code, *operands)
+        if result is not None:
             return result
     tensors = [o for o in operands if isinstance(o, torch.Tensor)]
     if not tensors:
@@ -188,12 +196,10 @@ def elementwise(op: str, *operands, math_mode: str = "fast", out: torch.Tensor |
     lines.append(f"out r {DTYPE_NAMES[out_dtype]}")
     kernel = _kernel("\n".join(lines))
     kernel.launch(inputs, packed, stream=None, scalars=scalars)
-    if out is None and key is not None:
-        _keep(_elementwise_plans, key, (kernel, result.shape, result.stride(), result.dtype, result.device, device, kernel.plan(inputs, packed)))
+    if code is not None:
+        elements, divisors, layouts = kernel.plan(inputs, packed)
+        _keep_plan(True, code, operands, _FUSED, (result,), _fused_ints(kernel, elements, divisors), (), bytes(layouts), kernel)
     return result
-
-
-_elementwise_plans: dict = {}
 
 
 def elementwise_(op: str, target: torch.Tensor, *others, math_mode: str = "fast") -> torch.Tensor:
@@ -212,20 +218,10 @@ def cast(x: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
 
 
 def _reduce(op: str, x: torch.Tensor, dim, keepdim: bool) -> torch.Tensor:
+    result = _call(_CODES[op], x, dim, keepdim)
+    if result is not None:
+        return result
     device = _device_of([x])
-    key = None
-    axes = tuple(dim) if isinstance(dim, (list, tuple)) else (dim,)
-    if type(x) in _PLAIN and all(type(d) is int or d is None for d in axes):
-        key = (op, x.dtype, x.shape, x.stride(), device, axes, dim is None, bool(keepdim))
-        plan = _reduce_plans.get(key)
-        if plan is not None:
-            code, dtype, extents, out_dtype, shape, nbytes = plan
-            out = torch.empty(shape, dtype=out_dtype, device=x.device)
-            stream = _stream(None, device)
-            scratch = workspace(device, stream, nbytes)
-            check(lib.tq_reduce_launch(code, dtype, x.data_ptr(), out.data_ptr(), *extents, _pointer(scratch),
-                                       0 if scratch is None else scratch.numel(), device, stream))
-            return out
     rank = x.dim()
     if rank == 0:
         raise Declined("a reduction of a tensor without axes has no kernel")  # reduction.cpp:110-113
@@ -247,13 +243,12 @@ def _reduce(op: str, x: torch.Tensor, dim, keepdim: bool) -> torch.Tensor:
         extents = (math.prod(kept_shape), math.prod(x.shape[d] for d in dims), 1)
     out = torch.empty(kept_shape, dtype=out_dtype, device=x.device)
     launch_reduce(op, base, out, *extents, device, _stream(None, device))
-    if key is not None and base.data_ptr() == x.data_ptr():      # read where it lies: the extents say all there is to say
-        code, dtype = REDUCE_OPS[op], dtype_code(x.dtype)
-        _keep(_reduce_plans, key, (code, dtype, extents, out_dtype, final_shape, reduce_workspace_bytes(code, dtype, *extents, device)))
-    return out.reshape(final_shape)
-
-
-_reduce_plans: dict = {}
+    result = out.reshape(final_shape)
+    if base.data_ptr() == x.data_ptr():      # read where it lies: the extents say all there is to say
+        number, dtype = REDUCE_OPS[op], dtype_code(x.dtype)
+        _keep_plan(False, _CODES[op], (x, dim, keepdim), _REDUCE, (result,),
+                   (number, dtype, *extents, reduce_workspace_bytes(number, dtype, *extents, device)), (), b"", None)
+    return result
 
 
 def _extents_in_place(x: torch.Tensor, dims: list[int], kept: list[int]):
@@ -322,6 +317,10 @@ def _transposed_base(x: torch.Tensor):
 
 
 def softmax(x: torch.Tensor, dim: int = -1, half_to_float: bool = False) -> torch.Tensor:
+    out = _call(_CODES["softmax"], x, dim, half_to_float)
+    if out is not None:
+        return out
+    operands = (x, dim, half_to_float)
     out_dtype = torch.float32 if half_to_float else x.dtype
     transposed = _transposed_base(x) if (x.dim() and dim % x.dim() == x.dim() - 1 and not half_to_float) else None
     if transposed is not None and not prefers_transposed("softmax", x.dtype, *transposed[1:]):
@@ -333,19 +332,41 @@ def softmax(x: torch.Tensor, dim: int = -1, half_to_float: bool = False) -> torc
         device = _device_of([x])
         try:
             launch_transposed("softmax", base, None, None, out, batch, rows, cols, 0.0, device, _stream(None, device))
+            _keep_transposed("softmax", operands, base, out, batch, rows, cols, 0.0, device)
             return out
         except Declined:
             pass
-    x = contiguous(x)
+    if not x.is_contiguous():
+        return softmax(clone(x), dim, half_to_float)
     out = torch.empty(x.shape, dtype=out_dtype, device=x.device)
     if x.numel():
         _softmax_kernel(dim, half_to_float).launch([x], out, stream=None)
+        along = 0 if x.dim() == 0 else dim % x.dim()
+        extent = x.shape[along] if x.dim() else 1
+        _keep_plan(False, _CODES["softmax"], operands, _SOFTMAX, (out,),
+                   (dtype_code(x.dtype), dtype_code(out_dtype), math.prod(x.shape[:along]), extent, math.prod(x.shape[along + 1 :])), (), b"", None)
     return out
+
+
+def _keep_transposed(kind: str, operands: tuple, base, out, batch: int, rows: int, cols: int, eps: float, device: int) -> None:
+    layer_norm, dtype = kind == "layer_norm", dtype_code(base.dtype)
+    _keep_plan(False, _CODES[kind], operands, _TRANSPOSED, (out,),
+               (int(layer_norm), dtype, batch, rows, cols, transposed_workspace_bytes(layer_norm, dtype, batch, rows, cols, device)), (float(eps),), b"", None)
+
+
+def _keep_layer_norm(name: str, operands: tuple, x, normalized_rank: int, eps: float, outputs: tuple) -> None:
+    width = math.prod(x.shape[x.dim() - normalized_rank :])
+    dtype = dtype_code(x.dtype)
+    _keep_plan(False, _CODES[name], operands, _LAYER_NORM, outputs, (dtype, dtype, x.numel() // max(width, 1), width), (float(eps),), b"", None)
 
 
 def native_layer_norm(x, normalized_shape, weight, bias, eps):
     """(y, mean, rstd) as `aten::native_layer_norm` returns them: statistics shaped [..., 1, …]
     and in the input's type."""
+    found = _call(_CODES["native_layer_norm"], x, weight, bias, normalized_shape, eps)
+    if found is not None:
+        return found
+    operands = (x, weight, bias, normalized_shape, eps)
     normalized_shape = list(normalized_shape)
     k = len(normalized_shape)
     if list(x.shape[x.dim() - k :]) != normalized_shape:
@@ -359,10 +380,16 @@ def native_layer_norm(x, normalized_shape, weight, bias, eps):
     rstd = torch.empty(stat_shape, dtype=x.dtype, device=x.device)
     if x.numel():
         _layer_norm_kernel(k, float(eps)).launch([x, weight, bias], out, stream=None, mean=mean, rstd=rstd)
+        if all(now is given for now, given in zip((x, weight, bias), operands)):
+            _keep_layer_norm("native_layer_norm", operands, x, k, eps, (out, mean, rstd))
     return out, mean, rstd
 
 
 def layer_norm(x, normalized_shape, weight=None, bias=None, eps=1e-5):
+    out = _call(_CODES["layer_norm"], x, weight, bias, normalized_shape, eps)
+    if out is not None:
+        return out
+    operands = (x, weight, bias, normalized_shape, eps)
     transposed = _transposed_base(x) if len(list(normalized_shape)) == 1 else None
     if transposed is not None and all(t is None or (t.dtype == x.dtype and t.numel() == x.shape[-1]) for t in (weight, bias)):
         base, batch, rows, cols = transposed
@@ -371,14 +398,20 @@ def layer_norm(x, normalized_shape, weight=None, bias=None, eps=1e-5):
         try:
             launch_transposed("layer_norm", base, None if weight is None else contiguous(weight), None if bias is None else contiguous(bias),
                               out, batch, rows, cols, eps, device, _stream(None, device))
+            if all(t is None or t.is_contiguous() for t in (weight, bias)):
+                _keep_transposed("layer_norm", operands, base, out, batch, rows, cols, eps, device)
             return out
         except Declined:
             pass
-    x = contiguous(x)
+    if not x.is_contiguous():
+        return layer_norm(clone(x), normalized_shape, weight, bias, eps)
     out = torch.empty_like(x)
     if x.numel():
-        _layer_norm_kernel(len(list(normalized_shape)), float(eps)).launch(
+        k = len(list(normalized_shape))
+        _layer_norm_kernel(k, float(eps)).launch(
             [x, None if weight is None else contiguous(weight), None if bias is None else contiguous(bias)], out, stream=None)
+        if all(t is None or t.is_contiguous() for t in (weight, bias)):
+            _keep_layer_norm("layer_norm", operands, x, k, eps, (out,))
     return out
 
 
@@ -398,6 +431,9 @@ def rms_norm(x, weight, eps):
 
 def batch_norm_eval(x, weight, bias, running_mean, running_var, eps):
     """Eval-mode batch norm of an [N, C, ...] tensor (csrc/tessiq/torch/eager_norm.cpp:136-199)."""
+    out = _call(_CODES["batch_norm"], x, weight, bias, running_mean, running_var, eps)
+    if out is not None:
+        return out
     if x.dim() < 2:
         raise Declined("BatchNorm needs at least [N, C]")
     if running_mean is None or running_var is None:
@@ -412,12 +448,16 @@ def batch_norm_eval(x, weight, bias, running_mean, running_var, eps):
     n, c = x.shape[0], x.shape[1]
     inner = math.prod(x.shape[2:])
     out = torch.empty_like(x)
-    check(lib.tq_batch_norm_eval_launch(dtype_code(x.dtype), dtype_code(param_dtypes.pop()), _pointer(x),
+    param_dtype = dtype_code(param_dtypes.pop())
+    check(lib.tq_batch_norm_eval_launch(dtype_code(x.dtype), param_dtype, _pointer(x),
                                         _pointer(None if weight is None else contiguous(weight)),
                                         _pointer(None if bias is None else contiguous(bias)),
                                         _pointer(contiguous(running_mean)), _pointer(contiguous(running_var)),
                                         _pointer(out), n, c, inner, float(eps), device,
                                         _stream(None, device)))
+    if out.numel() and all(t.is_contiguous() for t in params):
+        _keep_plan(False, _CODES["batch_norm"], (x, weight, bias, running_mean, running_var, eps), _BATCH_NORM, (out,),
+                   (dtype_code(x.dtype), param_dtype, n, c, inner), (float(eps),), b"", None)
     return out
 
 
@@ -438,12 +478,19 @@ def _realigned(t):
 
 
 def _gemm(a, b, bias, activation, residual=None):
+    code = _CODES.get("gemm " + activation, 0)
+    out = _call(code, a, b, bias, residual)
+    if out is not None:
+        return out
     out = torch.empty([*a.shape[:-1], b.shape[-1]], dtype=a.dtype, device=a.device)
     if out.numel() == 0:
         return out
     kernel = _gemm_kernel(activation, has_bias=bias is not None, has_residual=residual is not None)
     try:
-        kernel.launch([t for t in (a, b, bias, residual) if t is not None], out, stream=None)
+        operands = [t for t in (a, b, bias, residual) if t is not None]
+        kernel.launch(operands, out, stream=None)
+        dtype, *extents = kernel.plan(operands, out)
+        _keep_plan(False, code, (a, b, bias, residual), _GEMM, (out,), (dtype, kernel.activation, *extents), (), b"", None)
     except Declined:
         moved = [_realigned(t) for t in (a, b, bias, residual)]
         if all(m is t for m, t in zip(moved, (a, b, bias, residual))):
@@ -495,6 +542,10 @@ def attention(q, k, v, scale=None, causal=False, token_major=True):
     [batch, tokens, heads, 64] buffer, so `.transpose(1, 2).reshape(batch, tokens, heads * 64)` after it
     is free; without, it is a packed [batch, heads, tokens, 64] tensor (free to fold into
     [batch * heads, tokens, 64]). The kernel writes either through its output strides."""
+    operands = (q, k, v, scale, causal, token_major)
+    out = _call(_CODES["attention"], *operands)
+    if out is not None:
+        return out
     batch, heads, tokens, width = q.shape
     scale = 1.0 / math.sqrt(width) if scale is None else scale
     if token_major:
@@ -502,7 +553,11 @@ def attention(q, k, v, scale=None, causal=False, token_major=True):
     else:
         out = torch.empty([batch, heads, tokens, width], dtype=q.dtype, device=q.device)
     if out.numel():
-        _attention_kernel(float(scale), bool(causal)).launch([q, k, v], out, stream=None)
+        kernel = _attention_kernel(float(scale), bool(causal))
+        kernel.launch([q, k, v], out, stream=None)
+        dtype, extents = kernel.plan(q, k, v, out)
+        _keep_plan(False, _CODES["attention"], operands, _ATTENTION, (out,),
+                   (dtype, *extents[:5], *[n for strides in extents[5:] for n in strides], int(bool(causal))), (float(scale),), b"", None)
     return out
 
 
