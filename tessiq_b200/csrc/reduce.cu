@@ -72,6 +72,22 @@ struct SumReducer {
       local += part[0];
     }
   }
+  // Two rows, or four, of neighbouring columns: added to one another first (floating types of 32 and 64 bits).
+  static constexpr bool kPairs = std::is_floating_point_v<T>;
+  template <int V> __device__ static void step_pair(Acc* local, const Vec<T, V>& a, const Vec<T, V>& b) {
+#pragma unroll
+    for (int e = 0; e < V; ++e) local[e] += static_cast<Acc>(to_compute(a.v[e])) + static_cast<Acc>(to_compute(b.v[e]));
+  }
+  template <int V> __device__ static void step_four(Acc* local, const Vec<T, V> (&x)[4]) {
+#pragma unroll
+    for (int e = 0; e < V; ++e)
+      local[e] += (static_cast<Acc>(to_compute(x[0].v[e])) + static_cast<Acc>(to_compute(x[1].v[e]))) +
+                  (static_cast<Acc>(to_compute(x[2].v[e])) + static_cast<Acc>(to_compute(x[3].v[e])));
+  }
+  template <int V> __device__ static void step_single(Acc* local, const Vec<T, V>& a) {
+#pragma unroll
+    for (int e = 0; e < V; ++e) local[e] += static_cast<Acc>(to_compute(a.v[e]));
+  }
   template <int VEC> __device__ static Acc to_acc(Acc local) { return local; }
   __device__ static Out finish(Acc a, long long count, bool mean) {
     if constexpr (!std::is_integral_v<C>) {
@@ -428,29 +444,66 @@ reduce_cta_per_slice(const T* __restrict__ in, typename R::Out* __restrict__ out
 // read beside it are elements of its neighbours, gathered and never used. Only a vector that would begin before
 // the tensor (its first row) or end behind it (its last) is read column by column. Rows of odd length used
 // to be read an element, or four bytes, a lane: 40256 x 709 bf16 44.6 us a reduction where the bytes take 8.8.
+//
+// Sums are brought together in trees and pairs throughout: with a chain of additions in its place the error against 64 bits of an f32 sum or
+// LayerNorm grew by up to a seventh when clusters took over from tickets and a thread's rows became more.
+//
+// What the kernel would divide by comes as shifts and quotients from the host: a small reduction is as long as its chain
+// of instructions, and a dozen divisions were a tenth of it.
+struct ColumnArgs {
+  long long reduce, inner;
+  long long chunk;          // rows of a CTA: reduce / split, rounded up
+  int lanes_shift;          // log2 of the threads along inner
+  int shares_shift;         // log2 of the threads that fold an item of the CTA's tile
+  int split, cluster_shift, clusters;      // CTAs of a column tile, of a cluster (log2), clusters of a tile
+  int mean;
+};
+
+// `count` accumulators (a power of two), `stride` apart, as a tree.
+template <typename R>
+__device__ __forceinline__ typename R::Acc fold_tree(const typename R::Acc* from, int count, int stride) {
+  using Acc = typename R::Acc;
+  if constexpr (rescales<R>::value) {
+    float m = from[0].m;
+    for (int i = 1; i < count; ++i) m = R::larger(m, from[i * stride].m);
+    float s = R::scaled(from[0], m);
+    for (int i = 1; i < count; i += 2) s += i + 1 < count ? R::scaled(from[i * stride], m) + R::scaled(from[(i + 1) * stride], m) : R::scaled(from[i * stride], m);
+    return Acc{m, s};
+  } else {
+    Acc total = from[0];
+    if (count >= 2) total = R::combine(total, from[stride]);
+    if (count >= 4) total = R::combine(total, R::combine(from[2 * stride], from[3 * stride]));
+    for (int i = 4; i < count; i += 4)
+      total = R::combine(total, R::combine(R::combine(from[i * stride], from[(i + 1) * stride]), R::combine(from[(i + 2) * stride], from[(i + 3) * stride])));
+    return total;
+  }
+}
+
 template <typename T, typename R, int VEC, bool RING, bool RAGGED = false>
 __global__ void __launch_bounds__(kBlock, sizeof(typename R::Acc) > 8 ? 4 : 5)
-reduce_columns(const T* __restrict__ in, typename R::Out* __restrict__ out, long long reduce,
-               long long inner, int lanes_x, int split, int cluster, int mean,
+reduce_columns(const T* __restrict__ in, typename R::Out* __restrict__ out, const ColumnArgs args,
                typename R::Acc* __restrict__ partials, unsigned* __restrict__ tickets) {
   using Acc = typename R::Acc;
+  constexpr int kVecShift = VEC == 8 ? 3 : VEC == 4 ? 2 : VEC == 2 ? 1 : 0;
+  static_assert(VEC == 1 << kVecShift);
+  const long long reduce = args.reduce, inner = args.inner;
+  const int lanes_x = 1 << args.lanes_shift, cluster = 1 << args.cluster_shift;
   extern __shared__ __align__(16) unsigned char dynamic_smem[];
   Acc* rows_scratch = reinterpret_cast<Acc*>(dynamic_smem);              // [kBlock * VEC]
   Acc* cluster_scratch = rows_scratch + kBlock * VEC;                    // [lanes_x * VEC]
   __shared__ bool is_last;
 
   if (cluster > 1) cluster_start();
-  const int tx = threadIdx.x % lanes_x;
-  const int ty = threadIdx.x / lanes_x;
-  const int lanes_y = kBlock / lanes_x;
+  const int tx = threadIdx.x & (lanes_x - 1);
+  const int ty = threadIdx.x >> args.lanes_shift;
+  const int lanes_y = kBlock >> args.lanes_shift;
   const long long slice = blockIdx.z;
   const int part = blockIdx.y;
   const int tile_columns = RAGGED ? (lanes_x - 1) * VEC : lanes_x * VEC;
   const long long first_column = static_cast<long long>(blockIdx.x) * tile_columns;
 
-  long long chunk = (reduce + split - 1) / split;
-  const long long begin = static_cast<long long>(part) * chunk;
-  long long end = begin + chunk;
+  const long long begin = static_cast<long long>(part) * args.chunk;
+  long long end = begin + args.chunk;
   if (end > reduce) end = reduce;
 
   int before = 0;
@@ -461,9 +514,9 @@ reduce_columns(const T* __restrict__ in, typename R::Out* __restrict__ out, long
   const long long column = first_column + tx * VEC - before;       // of this thread's vectors
   const bool in_range = column < inner;
 
-  // The ragged form gives a thread more rows than the plain one does. f32 sums take every fourth row into a chain of its own,
-  // so that they lose no digits by it.
-  constexpr int kMoreChains = RAGGED && std::is_same_v<R, SumReducer<float>> ? 3 : 0;
+  // A thread of the ring takes many rows. Sums of 32 and 64 bits take them two at a time into four chains, so that they
+  // lose no digits by it (moments of 32-bit elements into two: their state is larger).
+  constexpr int kMoreChains = !RING ? 0 : std::is_same_v<R, SumReducer<float>> || std::is_same_v<R, SumReducer<double>> ? 3 : std::is_same_v<R, MomentsReducer<float>> ? 1 : 0;
   typename R::template Local<1> local[VEC], more[kMoreChains ? kMoreChains * VEC : 1];
 #pragma unroll
   for (int e = 0; e < VEC; ++e) local[e] = R::template local_identity<1>();
@@ -524,7 +577,10 @@ reduce_columns(const T* __restrict__ in, typename R::Out* __restrict__ out, long
         if (count > 0) {
           const Vec<T, VEC> x = load_stream<T, VEC>(source);
 #pragma unroll
-          for (int e = 0; e < VEC; ++e) R::template seed<1>(local[e], x.v[e]);
+          for (int e = 0; e < VEC; ++e) {
+            R::template seed<1>(local[e], x.v[e]);
+            if constexpr (kMoreChains > 0) more[e] = local[e];
+          }
         }
       }
 #pragma unroll
@@ -532,13 +588,21 @@ reduce_columns(const T* __restrict__ in, typename R::Out* __restrict__ out, long
         if (d < count) copy(d);
         asm volatile("cp.async.commit_group;" ::: "memory");   // one group per row, empty past the end
       }
+      Vec<T, VEC> held;      // the first row of a pair
       for (int i = 0; i < count; i += kRingDepth) {
 #pragma unroll
         for (int d = 0; d < kRingDepth; ++d) {
           if (i + d < count) {
             asm volatile("cp.async.wait_group %0;" ::"n"(kRingDepth - 2) : "memory");   // row i + d has landed
             const Vec<T, VEC> x = ring[d * kBlock];
-            if constexpr (R::kSeeded) {
+            if constexpr (has_pairs<R>::value) {
+              if (d % 2 == 0) {
+                held = x;
+              } else {
+                constexpr int kChains = kMoreChains + 1;
+                R::template step_pair<VEC>(d / 2 % kChains ? more + (d / 2 % kChains - 1) * VEC : local, held, x);
+              }
+            } else if constexpr (R::kSeeded) {
 #pragma unroll
               for (int e = 0; e < VEC; ++e) R::template step_seeded<1>(local[e], x.v[e]);
             } else if constexpr (has_column_step<R>::value) {
@@ -546,13 +610,7 @@ reduce_columns(const T* __restrict__ in, typename R::Out* __restrict__ out, long
               ri += lanes_y;
             } else {
 #pragma unroll
-              for (int e = 0; e < VEC; ++e) {
-                if constexpr (kMoreChains > 0) {
-                  R::template step<1>(d % 4 ? more[(d % 4 - 1) * VEC + e] : local[e], x.v[e], ri);
-                } else {
-                  R::template step<1>(local[e], x.v[e], ri);
-                }
-              }
+              for (int e = 0; e < VEC; ++e) R::template step<1>(local[e], x.v[e], ri);
               ri += lanes_y;
             }
             if (i + d + kRingDepth - 1 < count) copy((d + kRingDepth - 1) % kRingDepth);   // into the slot read one row ago
@@ -561,6 +619,9 @@ reduce_columns(const T* __restrict__ in, typename R::Out* __restrict__ out, long
         }
       }
       asm volatile("cp.async.wait_group 0;" ::: "memory");
+      if constexpr (has_pairs<R>::value) {
+        if (count % 2 != 0) R::template step_single<VEC>(local, held);
+      }
       if constexpr (R::kSeeded) {
 #pragma unroll
         for (int e = 0; e < VEC; ++e) R::template set_count<1>(local[e], count);
@@ -575,6 +636,18 @@ reduce_columns(const T* __restrict__ in, typename R::Out* __restrict__ out, long
         for (int u = 0; u < UNROLL; ++u) {
           const long long ri = r + static_cast<long long>(u) * lanes_y;
           if (ri < end) x[u] = load_stream<T, VEC>(base + ri * inner);
+        }
+        if constexpr (has_pairs<R>::value && !R::kSeeded) {
+          static_assert(UNROLL == 4);
+          if (r + 3ll * lanes_y < end) {
+            if constexpr (std::is_same_v<R, SumReducer<T>>) {
+              R::template step_four<VEC>(local, x);
+            } else {
+              R::template step_pair<VEC>(local, x[0], x[1]);
+              R::template step_pair<VEC>(local, x[2], x[3]);
+            }
+            continue;
+          }
         }
 #pragma unroll
         for (int u = 0; u < UNROLL; ++u) {
@@ -592,45 +665,75 @@ reduce_columns(const T* __restrict__ in, typename R::Out* __restrict__ out, long
     }
   }
 
-  // Across ty, through shared memory, in a fixed order.
+  // Across the rows of the CTA, in a fixed order and by every thread: shuffles bring a warp's rows together (where whole
+  // vectors line up), then a thread folds its share of an item's rows in shared memory.
   Acc acc[VEC];
 #pragma unroll
   for (int e = 0; e < VEC; ++e) {
+    if constexpr (kMoreChains == 1) R::template add_chain<1>(local[e], more[e]);
     acc[e] = R::template to_acc<1>(local[e]);
-    if constexpr (kMoreChains > 0) acc[e] = (acc[e] + more[e]) + (more[VEC + e] + more[2 * VEC + e]);
+    if constexpr (kMoreChains == 3) acc[e] = (acc[e] + more[e]) + (more[VEC + e] + more[2 * VEC + e]);
   }
+  const int items = lanes_x * VEC;                // at most kBlock
+  int rows = lanes_y, row = ty;
+  bool writes = true;
+  if constexpr (!RAGGED) {
+    if (lanes_x < 32) {
+      if constexpr (rescales<R>::value) {
 #pragma unroll
-  for (int e = 0; e < VEC; ++e) {
-    const int item = tx * VEC + e - before;
-    if (!RAGGED || (item >= 0 && item < tile_columns)) rows_scratch[ty * lanes_x * VEC + item] = acc[e];
+        for (int e = 0; e < VEC; ++e) {
+          float m = acc[e].m;
+          for (int offset = lanes_x; offset < 32; offset *= 2) m = R::larger(m, shfl_xor(m, offset));
+          float s = R::scaled(acc[e], m);
+          for (int offset = lanes_x; offset < 32; offset *= 2) s += shfl_xor(s, offset);
+          acc[e] = Acc{m, s};
+        }
+      } else {
+        for (int offset = lanes_x; offset < 32; offset *= 2) {
+#pragma unroll
+          for (int e = 0; e < VEC; ++e) acc[e] = R::combine(acc[e], R::shuffle(acc[e], offset));
+        }
+      }
+      rows = kWarps;
+      row = threadIdx.x / 32;
+      writes = (threadIdx.x & 31) < lanes_x;
+    }
+  }
+  if (writes) {
+#pragma unroll
+    for (int e = 0; e < VEC; ++e) {
+      const int item = tx * VEC + e - before;
+      if (!RAGGED || (item >= 0 && item < tile_columns)) rows_scratch[row * items + item] = acc[e];
+    }
   }
   __syncthreads();
-  const bool holder = ty == 0 && (!RAGGED || tx < lanes_x - 1);
-  if (holder) {
-    if constexpr (RAGGED) {
-#pragma unroll
-      for (int e = 0; e < VEC; ++e) acc[e] = rows_scratch[tx * VEC + e];
-    }
-    for (int y = 1; y < lanes_y; ++y) {
-#pragma unroll
-      for (int e = 0; e < VEC; ++e) {
-        acc[e] = R::combine(acc[e], rows_scratch[(y * lanes_x + tx) * VEC + e]);
-      }
+  const int shares = 1 << args.shares_shift;      // threads an item
+  const int my_item = threadIdx.x & (items - 1), share = threadIdx.x >> (args.lanes_shift + kVecShift);
+  Acc total = R::identity();
+  if (share < shares && (!RAGGED || my_item < tile_columns))
+    total = fold_tree<R>(rows_scratch + share * items + my_item, rows >> args.shares_shift, items << args.shares_shift);
+  if (shares > 1) {
+    __syncthreads();
+    if (share > 0 && share < shares) rows_scratch[share * items + my_item] = total;
+    __syncthreads();
+    if (share == 0 && (!RAGGED || my_item < tile_columns)) {
+      rows_scratch[my_item] = total;
+      total = fold_tree<R>(rows_scratch + my_item, shares, items);
     }
   }
+  const bool holder = share == 0 && (!RAGGED || my_item < tile_columns);
 
   // Across the CTAs of the cluster: a reduce-scatter through distributed shared memory. The
   // tile's `items` accumulators are cut into `cluster` equal slices; every CTA sends slice q of
   // its accumulators to CTA q, one cluster barrier, and CTA q folds what it received in rank
   // order. Each CTA then owns items [rank * slice_items, (rank + 1) * slice_items) of the tile.
-  const int items = lanes_x * VEC;
-  const int slice_items = items / cluster;  // a multiple of VEC: cluster <= lanes_x, both powers of 2
+  const int slice_shift = args.lanes_shift + kVecShift - args.cluster_shift, slice_items = 1 << slice_shift;      // cluster <= items
   unsigned rank = 0;
   typename R::Out* out_row = out + slice * inner;
   const long long tile_column = first_column;
   // what of the tile's items is a column of this tile
   const long long live = inner - tile_column < tile_columns ? inner - tile_column : tile_columns;
-  const int clusters = split / cluster;
+  const int clusters = args.clusters;
   const long long tile = slice * gridDim.x + blockIdx.x;
   Acc* tile_partials = partials + tile * clusters * items;
 
@@ -638,39 +741,25 @@ reduce_columns(const T* __restrict__ in, typename R::Out* __restrict__ out, long
     cg::cluster_group group = cg::this_cluster();
     rank = group.block_rank();
     cluster_started();
-    if (holder) {
-      const int item = tx * VEC;
-      Acc* owner = group.map_shared_rank(cluster_scratch, item / slice_items);
-#pragma unroll
-      for (int e = 0; e < VEC; ++e) owner[rank * slice_items + item % slice_items + e] = acc[e];
-    }
+    if (holder) group.map_shared_rank(cluster_scratch, my_item >> slice_shift)[rank * slice_items + (my_item & (slice_items - 1))] = total;
     group.sync();
     // Thread t < slice_items now finishes item rank * slice_items + t.
     if (threadIdx.x < slice_items) {
-      Acc total = cluster_scratch[threadIdx.x];
-      for (int j = 1; j < cluster; ++j) total = R::combine(total, cluster_scratch[j * slice_items + threadIdx.x]);
+      const Acc total = fold_tree<R>(cluster_scratch + threadIdx.x, cluster, slice_items);
       const int item = rank * slice_items + threadIdx.x;
       if (clusters == 1) {
-        if (item < live) out_row[tile_column + item] = R::finish(total, reduce, mean != 0);
+        if (item < live) out_row[tile_column + item] = R::finish(total, reduce, args.mean != 0);
       } else {
-        tile_partials[(part / cluster) * items + item] = total;
+        tile_partials[(part >> args.cluster_shift) * items + item] = total;
       }
     }
     if (clusters == 1) return;
   } else {
     if (clusters == 1) {
-      if (holder) {
-#pragma unroll
-        for (int e = 0; e < VEC; ++e) {
-          if (tx * VEC + e < live) out_row[tile_column + tx * VEC + e] = R::finish(acc[e], reduce, mean != 0);
-        }
-      }
+      if (holder && my_item < live) out_row[tile_column + my_item] = R::finish(total, reduce, args.mean != 0);
       return;
     }
-    if (holder) {
-#pragma unroll
-      for (int e = 0; e < VEC; ++e) tile_partials[part * items + tx * VEC + e] = acc[e];
-    }
+    if (holder) tile_partials[part * items + my_item] = total;
   }
 
   // Across clusters: every CTA has written its share of its cluster's partial; the last CTA of
@@ -680,7 +769,7 @@ reduce_columns(const T* __restrict__ in, typename R::Out* __restrict__ out, long
   __syncthreads();
   if (threadIdx.x == 0) {
     const unsigned ticket = atomicAdd(&tickets[tile], 1u);
-    is_last = ticket == static_cast<unsigned>(split - 1);
+    is_last = ticket == static_cast<unsigned>(args.split - 1);
   }
   __syncthreads();
   if (!is_last) return;
@@ -699,7 +788,7 @@ reduce_columns(const T* __restrict__ in, typename R::Out* __restrict__ out, long
         if (j + u < clusters) total = R::combine(total, batch[u]);
       }
     }
-    out_row[tile_column + item] = R::finish(total, reduce, mean != 0);
+    out_row[tile_column + item] = R::finish(total, reduce, args.mean != 0);
   }
 }
 
@@ -944,6 +1033,7 @@ struct Plan {
   size_t acc_bytes = 0;
   size_t partial_bytes = 0;   // scratch for partials (0 when one cluster covers a slice)
   size_t ticket_bytes = 0;
+  size_t required = 0;        // scratch a caller has to bring: what the forms with partials need, also where another one runs
   // the streaming columns kernel
   int device = 0;
   int grid = 0;               // CTAs: one per SM
@@ -986,10 +1076,92 @@ bool plan_stream(Plan& p, tq_reduce_op op, tq_dtype dtype, long long outer, long
   return true;
 }
 
+int log2_of(int power) {
+  int shift = 0;
+  while ((1 << (shift + 1)) <= power) ++shift;
+  return shift;
+}
+
+// Expected times, us, of a column reduction over `bytes` by the streaming kernel, and by clusters that meet over tickets (the
+// clearing of the tickets, partials in memory and the last CTA's fold are the fixed part; more for accumulators of 16
+// bytes and where rows start between vectors). Kernel times of [5184 x 1000] f16, [3072 x 4096], [16384 x 1024], [131072 x 128] f32,
+// [40000 x 300], [262144 x 128] bf16 sums by tickets: 12.4, 16.3, 19.9, 23.1, 18.6, 30.9. (With plain loads and all CTAs in one wave of five an
+// SM HBM is reached in the end: 32768 x 4096 f32 86; 16384 x 8192, whose 768 CTAs are more, 108.)
+double stream_time(tq_reduce_op op, int size, long long bytes) { return 8.0 + bytes / 6.0e6 + (op == TQ_ARGMAX && size == 2 ? 6.0 : 0.0); }
+double ticketed_time(const Plan& p, tq_reduce_op op, long long bytes, int sms) {
+  if (!p.ring && p.tiles * p.split <= 5ll * sms) return std::min(9.0 + bytes / 5.2e6, 14.0 + bytes / 7.4e6);
+  return 9.0 + bytes / 5.2e6 + (op == TQ_ARGMAX || op == kOpMoments ? 8.0 : 0.0) + (p.ragged ? 4.0 : 0.0);
+}
+
+// Whether one cluster (or one CTA) takes a tile of columns whole: no partials, no tickets, nothing to clear. The tile's width (lanes) and
+// the cluster are chosen by expected time: the launch and the folds; every CTA's bytes at the 38 KB a us that the
+// cp.async ring gets through one CTA of an SM, 48 for two and more together (30 and 32 where a row's piece is 64 bytes, 16 and 20
+// where it is 32); the reducer's work per row of a thread (argmax, the statistics); HBM, of which pieces of 256 bytes get most
+// (32768 x 4096 f32 sum 85.5 us in 256 bytes by clusters of four, 90 in 512 by eight, 110 in 128 by two); and what CTAs beyond two
+// an SM cost (1 us per further wave of 296: 256 CTAs measured best at every size). us, before and now: 5003 x 1250 bf16 sum 12.4 and
+// 6.0, argmax 16.6 and 9.2; 1000 x 1000 f32 sum 10.3 and 3.8; 5184 x 1000 f16 LayerNorm over the view 40.7 and 13.9; 3072 x 4096
+// f32 sum 17.2 and 11.6, argmax 39 and 12.3; 16384 x 8192 f32 sum 108 and 85; 20000 x 64 bf16 sum 10.3 and 6.1. Tall and narrow
+// tensors of some size have too few tiles for it (131072 x 128 f32 sum 23 by tickets, 28 so), and argmax and statistics over
+// 200 MB and more stay with the streaming kernel (32768 x 4096 argmax from a cold L2 bf16 56.5 and 66, f32 91.9 and 98).
+bool plan_one_cluster(Plan& p, tq_reduce_op op, int size, long long outer, long long reduce, long long inner, int sms, double others) {
+  const long long groups = (inner + p.vec - 1) / p.vec;
+  const long long bytes = outer * reduce * inner * size;
+  const bool statistic = op >= kOpSoftmaxStat, heavy = op == TQ_ARGMAX || op == kOpMoments;       // accumulators of 16 bytes
+  if ((op == TQ_ARGMAX || statistic) && bytes >= (200ll << 20)) return false;
+  if (reduce >= (1ll << 31)) return false;              // the ring counts a thread's rows in 32 bits
+  double best = 0.95 * others;
+  bool found = false;
+  for (int lanes = p.ragged || p.vec > kBlock / 64 ? 32 : 64; lanes >= 2; lanes /= 2) {
+    const int piece = lanes * p.vec * size;
+    if (piece < 32 || (p.ragged && lanes < 4)) break;
+    const long long tiles = p.ragged ? (inner + (lanes - 1) * p.vec - 1) / ((lanes - 1) * p.vec) : (groups + lanes - 1) / lanes;
+    const int rows_at_once = kBlock / lanes;
+    const double one = piece >= 128 ? 38e3 : piece >= 64 ? 30e3 : 16e3;        // bytes a us
+    const double together = piece >= 128 ? 48e3 : piece >= 64 ? 32e3 : 20e3;
+    for (int cluster = 1; cluster <= kMaxCluster; cluster *= 2) {
+      if (cluster > lanes * p.vec || (cluster > 1 && reduce < 2ll * cluster * rows_at_once)) break;
+      const long long ctas = tiles * outer * cluster;
+      const long long rows = (reduce + cluster - 1) / cluster;
+      const double an_sm = static_cast<double>((ctas + sms - 1) / sms);
+      const double cta_bytes = static_cast<double>(rows) * piece;
+      // (up to six rows a thread are two trips of plain loads, which start sooner: 512 x 768 f32 sum 2.8 and 3.1, 1000 x 1000 3.7 and 4.0)
+      const bool few = rows <= 6ll * rows_at_once && size >= 4 && op != TQ_ARGMAX && !statistic && !p.ragged;
+      if (lanes > 32 && !few) break;
+      const double rate = an_sm > 1 ? std::min(together, an_sm * one) : one;
+      const double work = static_cast<double>(rows) / rows_at_once *
+                          (op == TQ_ARGMAX ? 0.1 : op == kOpMoments ? 0.03 * an_sm : op == kOpSoftmaxStat ? (size == 2 ? 0.11 : 0.05) * std::max(an_sm, 1.7) : 0.03);
+      const double moving = std::max({bytes / (piece >= 256 ? 6.2e6 : 5.8e6), an_sm * cta_bytes / rate, work}) * (piece == 256 ? 0.96 : 1.0);
+      const double time = 2.3 + (cluster > 1 ? (heavy ? 1.6 : 0.8) : 0.0) + (heavy ? 0.15 : 0.05) * log2_of(std::max(32 / lanes, 1)) + (few ? 0.0 : 0.4) +
+                          moving + std::max(0.0, static_cast<double>(ctas) / (2.0 * sms) - 1.0);
+      if (time >= best) continue;
+      best = time;
+      found = true;
+      p.lanes_x = lanes;
+      p.split = p.cluster = cluster;
+      p.column_tiles = tiles;
+      p.tiles = tiles * outer;
+      p.ring = !few;
+    }
+  }
+  return found;
+}
+
 int floor_pow2(long long v) {
   int p = 1;
   while (static_cast<long long>(p) * 2 <= v) p *= 2;
   return p;
+}
+
+// Partials and tickets, where a slice or a tile of columns is shared by more than one cluster.
+void add_scratch(Plan& p) {
+  const int clusters = p.split / p.cluster;
+  if (clusters > 1) {
+    const long long items = p.shape == Shape::kColumns ? p.lanes_x * p.vec : 1;
+    p.partial_bytes = static_cast<size_t>(p.tiles) * clusters * items * p.acc_bytes;
+    p.partial_bytes = (p.partial_bytes + 255) / 256 * 256;
+    p.ticket_bytes = (static_cast<size_t>(p.tiles) * sizeof(unsigned) + 255) / 256 * 256;
+  }
+  p.required = p.partial_bytes + p.ticket_bytes;
 }
 
 Plan plan(tq_reduce_op op, tq_dtype dtype, long long outer, long long reduce, long long inner,
@@ -1024,7 +1196,8 @@ Plan plan(tq_reduce_op op, tq_dtype dtype, long long outer, long long reduce, lo
     }
     p.tiles = outer;
   } else {
-    if (plan_stream(p, op, dtype, outer, reduce, inner, device, vec_bytes_limit)) return p;
+    Plan stream = p;
+    const bool may_stream = plan_stream(stream, op, dtype, outer, reduce, inner, device, vec_bytes_limit);
     p.shape = Shape::kColumns;
     int vec = vec_bytes_limit / size;
     if (vec > 8) vec = 8;
@@ -1049,14 +1222,15 @@ Plan plan(tq_reduce_op op, tq_dtype dtype, long long outer, long long reduce, lo
                !plain_fills;
     if (p.ragged) vec = whole;
     p.vec = vec;
-    long long groups = (inner + vec - 1) / vec;
+    const long long groups = (inner + vec - 1) / vec;
+    Plan whole_tiles = p;
     // A warp reads 32 vectors (512 bytes) of one row; the CTA's 8 warps read 8 consecutive rows.
     // Measured on B200 at [32768, 4096]: 4-byte sums and extremes are fastest with plain unrolled
     // loads, 64 lanes along `inner` and one wave of CTAs; 2-byte types and argmax (whose state
     // costs registers) with the cp.async ring and 32 lanes.
     p.ring = (size <= 2 || op == TQ_ARGMAX || op >= kOpSoftmaxStat) && reduce < (1ll << 31);   // the ring counts a thread's rows in 32 bits
     if (p.ragged) p.ring = true;
-    int lanes = p.ring ? 32 : 64;
+    int lanes = p.ring || vec > kBlock / 64 ? 32 : 64;      // an item of the tile a thread, at most
     while (lanes > 1 && lanes / 2 >= groups && !p.ragged) lanes /= 2;
     p.lanes_x = lanes;
     p.column_tiles = p.ragged ? (inner + (lanes - 1) * vec - 1) / ((lanes - 1) * vec) : (groups + lanes - 1) / lanes;
@@ -1087,14 +1261,15 @@ Plan plan(tq_reduce_op op, tq_dtype dtype, long long outer, long long reduce, lo
       p.cluster = max_cluster;
     }
     p.tiles = base_ctas;
+    add_scratch(p);
+    if (may_stream) stream.required = stream.partial_bytes + stream.ticket_bytes;
+    const Plan& other = may_stream ? stream : p;
+    const double others = may_stream ? stream_time(op, size, elements * size) : ticketed_time(p, op, elements * size, sms);
+    if (!plan_one_cluster(whole_tiles, op, size, outer, reduce, inner, sms, others)) return other;
+    whole_tiles.required = other.required;
+    return whole_tiles;
   }
-  const int clusters = p.split / p.cluster;
-  if (clusters > 1) {
-    const long long items = p.shape == Shape::kColumns ? p.lanes_x * p.vec : 1;
-    p.partial_bytes = static_cast<size_t>(p.tiles) * clusters * items * p.acc_bytes;
-    p.partial_bytes = (p.partial_bytes + 255) / 256 * 256;
-    p.ticket_bytes = (static_cast<size_t>(p.tiles) * sizeof(unsigned) + 255) / 256 * 256;
-  }
+  add_scratch(p);
   return p;
 }
 
@@ -1178,9 +1353,18 @@ tq_status run(const Plan& p, const void* in, void* out, long long outer, long lo
           TQ_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        static_cast<int>(smem)));
         }
-        if (tq_status s = launch_clustered(kernel, grid, dim3(1, p.cluster, 1), smem, stream, input,
-                                           output, reduce, inner, p.lanes_x, p.split, p.cluster,
-                                           mean ? 1 : 0, partials, tickets)) {
+        ColumnArgs args = {};
+        args.reduce = reduce;
+        args.inner = inner;
+        args.chunk = (reduce + p.split - 1) / p.split;
+        args.lanes_shift = log2_of(p.lanes_x);
+        const int items = p.lanes_x * vec, rows = p.ragged || p.lanes_x > 32 ? kBlock / p.lanes_x : kWarps;
+        while ((items << (args.shares_shift + 1)) <= kBlock && (2 << args.shares_shift) <= rows) ++args.shares_shift;
+        args.split = p.split;
+        args.cluster_shift = log2_of(p.cluster);
+        args.clusters = p.split / p.cluster;
+        args.mean = mean ? 1 : 0;
+        if (tq_status s = launch_clustered(kernel, grid, dim3(1, p.cluster, 1), smem, stream, input, output, args, partials, tickets)) {
           return s;
         }
         return check_launch("reduce_columns");
@@ -1329,7 +1513,7 @@ size_t slice_stats_workspace_bytes(int kind, tq_dtype dtype, long long outer, lo
   const int op = kind == 0 ? kOpSoftmaxStat : kOpMoments;
   for (int limit = 16; limit >= dtype_size(dtype); limit /= 2) {
     const Plan p = plan(op, dtype, outer, reduce, inner, device, limit);
-    if (p.partial_bytes + p.ticket_bytes > bytes) bytes = p.partial_bytes + p.ticket_bytes;
+    bytes = std::max(bytes, p.required);
   }
   return bytes;
 }
@@ -1339,7 +1523,7 @@ tq_status slice_stats_launch(int kind, tq_dtype dtype, const void* in, void* sta
   const int op = kind == 0 ? kOpSoftmaxStat : kOpMoments;
   const int size = dtype_size(dtype);
   const Plan p = plan(op, dtype, outer, reduce, inner, device, inner == 1 ? 16 : column_vec_bytes(in, inner, size));
-  const size_t need = p.partial_bytes + p.ticket_bytes;
+  const size_t need = p.required;
   TQ_REQUIRE(need == 0 || (workspace != nullptr && workspace_bytes >= need && aligned_to(workspace, 16)), TQ_INVALID_ARGUMENT,
              "the statistics pass needs %zu bytes of 16-byte-aligned scratch and was given %zu", need, workspace_bytes);
   switch (dtype) {
@@ -1364,7 +1548,7 @@ tq_status tq_reduce_workspace_bytes(tq_reduce_op op, tq_dtype dtype, int64_t out
   // which changes its tiling: answer with the largest need over the widths it may pick.
   for (int limit = 16; limit >= tq::dtype_size(dtype); limit /= 2) {
     tq::Plan p = tq::plan(op, dtype, outer, reduce, inner, device, limit);
-    if (p.partial_bytes + p.ticket_bytes > *bytes) *bytes = p.partial_bytes + p.ticket_bytes;
+    *bytes = std::max(*bytes, p.required);
   }
   return TQ_OK;
 }
@@ -1384,7 +1568,7 @@ tq_status tq_reduce_launch(tq_reduce_op op, tq_dtype dtype, const void* in, void
   if (tq_status s = device_scope.status()) return s;
   tq::Plan p = tq::plan(op, dtype, outer, reduce, inner, device,
                         inner == 1 ? 16 : tq::column_vec_bytes(in, inner, size));
-  const size_t need = p.partial_bytes + p.ticket_bytes;
+  const size_t need = p.required;
   TQ_REQUIRE(need == 0 || (workspace != nullptr && workspace_bytes >= need), TQ_INVALID_ARGUMENT,
              "this reduction needs %zu bytes of scratch and was given %zu", need, workspace_bytes);
   TQ_REQUIRE(need == 0 || tq::aligned_to(workspace, 16), TQ_INVALID_ARGUMENT,
@@ -1415,7 +1599,7 @@ tq_status tq_reduce_partial_launch(tq_reduce_op op, tq_dtype dtype, const void* 
   if (tq_status s = device_scope.status()) return s;
   // the plan of the plain reduction over [1, count, 1]: same kernels, same scratch, another finish
   const tq::Plan p = tq::plan(op == TQ_MEAN ? TQ_SUM : op, dtype, 1, count, 1, device, 16);
-  const size_t need = p.partial_bytes + p.ticket_bytes;
+  const size_t need = p.required;
   TQ_REQUIRE(need == 0 || (workspace != nullptr && workspace_bytes >= need && tq::aligned_to(workspace, 16)), TQ_INVALID_ARGUMENT,
              "this reduction needs %zu bytes of 16-byte-aligned scratch (tq_reduce_workspace_bytes) and was given %zu", need, workspace_bytes);
   cudaStream_t cuda_stream = static_cast<cudaStream_t>(stream);
@@ -1447,8 +1631,8 @@ tq_status tq_reduce_launch_static(tq_reduce_op op, tq_dtype dtype, const void* i
   if (tq_status s = device_scope.status()) return s;
   const int limit = inner == 1 ? 16 : tq::column_vec_bytes(in, inner, size);
   tq::Plan p = tq::plan(op, dtype, outer, reduce, inner, device, limit);
-  if (p.partial_bytes + p.ticket_bytes > tq::kStaticScratchBytes) p = tq::plan(op, dtype, outer, reduce, inner, device, limit, false);
-  const size_t need = p.partial_bytes + p.ticket_bytes;
+  if (p.required > tq::kStaticScratchBytes) p = tq::plan(op, dtype, outer, reduce, inner, device, limit, false);
+  const size_t need = p.required;
   TQ_REQUIRE(need <= tq::kStaticScratchBytes, TQ_RESOURCE_EXHAUSTED,
              "this reduction needs %zu bytes of scratch; the built-in scratch of tq_reduce_launch_static holds %zu. "
              "Use tq_reduce_launch with caller-provided scratch for extents this large",

@@ -94,6 +94,10 @@ struct SoftmaxStatReducer {
     const float scale_b = b.m == m ? 1.f : stat_exp2((b.m - m) * kLog2e);
     return Acc{m, a.s * scale_a + b.s * scale_b};
   }
+  // Several at once: all rescaled to the largest maximum, once each, then added up.
+  static constexpr bool kRescales = true;
+  __device__ static float larger(float a, float b) { return ExtremeReducer<float, true>::combine(a, b); }
+  __device__ static float scaled(Acc a, float m) { return a.m == m ? a.s : a.s * stat_exp2((a.m - m) * kLog2e); }
   __device__ static Acc shuffle(Acc a, int offset) { return Acc{shfl_xor(a.m, offset), shfl_xor(a.s, offset)}; }
   template <int VEC> using Local = Acc;
   template <int VEC> __device__ static Acc local_identity() { return identity(); }
@@ -144,6 +148,32 @@ struct SoftmaxStatReducer {
       for (int e = 0; e < V; ++e) step<1>(local[e], x.v[e], 0);
     }
   }
+  // Two rows at a time: their terms are added to one another first. (Results of two-byte elements are rounded far above what that keeps.)
+  static constexpr bool kPairs = sizeof(T) == 4;
+  template <int V> __device__ static void step_pair(Acc* local, const Vec<T, V>& a, const Vec<T, V>& b) {
+    float t[V], u[V];
+    bool near = true;
+#pragma unroll
+    for (int e = 0; e < V; ++e) {
+      t[e] = (to_compute(a.v[e]) - local[e].m) * kLog2e;
+      u[e] = (to_compute(b.v[e]) - local[e].m) * kLog2e;
+      near = near && t[e] <= kSlack && u[e] <= kSlack;
+    }
+    if (near) {
+#pragma unroll
+      for (int e = 0; e < V; ++e) local[e].s += stat_exp2(t[e]) + stat_exp2(u[e]);
+    } else {
+#pragma unroll
+      for (int e = 0; e < V; ++e) {
+        step<1>(local[e], a.v[e], 0);
+        step<1>(local[e], b.v[e], 0);
+      }
+    }
+  }
+  template <int V> __device__ static void step_single(Acc* local, const Vec<T, V>& a) {
+#pragma unroll
+    for (int e = 0; e < V; ++e) step<1>(local[e], a.v[e], 0);
+  }
   template <int VEC> __device__ static Acc to_acc(Acc local) { return local; }
   // A slice whose maximum is +inf is NaN throughout (inf - inf), as the plain three-pass form gives.
   __device__ static Out finish(Acc a, long long, bool) {
@@ -177,7 +207,8 @@ struct MomentsReducer {
     if (b.n == 0.f) return a;
     const float n = a.n + b.n;
     const float delta = b.mean - a.mean;
-    return Acc{n, a.mean + delta * (b.n / n), a.m2 + b.m2 + delta * delta * (a.n * b.n / n), 0.f};
+    const float share = b.n / n;
+    return Acc{n, a.mean + delta * share, a.m2 + b.m2 + delta * delta * (a.n * share), 0.f};
   }
   __device__ static Acc shuffle(Acc a, int offset) {
     return Acc{shfl_xor(a.n, offset), shfl_xor(a.mean, offset), shfl_xor(a.m2, offset), 0.f};
@@ -208,6 +239,24 @@ struct MomentsReducer {
     local.s1 += d;
     local.s2 = fmaf(d, d, local.s2);
   }
+  static constexpr bool kPairs = sizeof(T) == 4;
+  template <int V> __device__ static void step_pair(Local<1>* local, const Vec<T, V>& a, const Vec<T, V>& b) {
+#pragma unroll
+    for (int e = 0; e < V; ++e) {
+      const float d = to_compute(a.v[e]) - local[e].pivot, f = to_compute(b.v[e]) - local[e].pivot;
+      local[e].s1 += d + f;
+      local[e].s2 += fmaf(f, f, d * d);
+    }
+  }
+  // (both with one pivot)
+  template <int VEC> __device__ static void add_chain(Local<VEC>& local, const Local<VEC>& other) {
+    local.s1 += other.s1;
+    local.s2 += other.s2;
+  }
+  template <int V> __device__ static void step_single(Local<1>* local, const Vec<T, V>& a) {
+#pragma unroll
+    for (int e = 0; e < V; ++e) step_seeded<1>(local[e], a.v[e]);
+  }
   template <int VEC> __device__ static void set_count(Local<VEC>& local, int count) { local.n = static_cast<float>(count); }
   template <int VEC> __device__ static Acc to_acc(const Local<VEC>& local) {
     if (local.n == 0.f) return identity();
@@ -217,6 +266,14 @@ struct MomentsReducer {
   }
   __device__ static Out finish(Acc a, long long, bool) { return Out{a.mean, a.m2 / a.n}; }
 };
+
+// Whether a reducer takes two rows at a time (step_pair above).
+template <typename R, typename = void> struct has_pairs : std::false_type {};
+template <typename R> struct has_pairs<R, std::void_t<decltype(R::kPairs)>> : std::bool_constant<R::kPairs> {};
+
+// Whether several accumulators are brought together by one rescaling each (SoftmaxStatReducer::scaled).
+template <typename R, typename = void> struct rescales : std::false_type {};
+template <typename R> struct rescales<R, std::void_t<decltype(R::kRescales)>> : std::bool_constant<R::kRescales> {};
 
 // Whether a reducer steps V neighbouring columns at once (step_columns above).
 template <typename R, typename = void> struct has_column_step : std::false_type {};

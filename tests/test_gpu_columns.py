@@ -1,0 +1,85 @@
+"""Reductions over columns and over transposed views, around the forms one cluster of CTAs takes whole: one CTA and clusters
+of two to eight, row pieces of 32 to 1024 bytes, rows that divide nothing, one row a thread, special values in each part."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def tq():
+    if not torch.cuda.is_available():
+        pytest.fail("the gpu tests need a CUDA device")
+    from tessiq_b200 import ops
+
+    return ops
+
+
+SHAPES = [  # outer, reduce, inner
+    (1, 1, 64), (1, 2, 8), (1, 31, 2048), (1, 64, 2048), (1, 257, 40), (1, 512, 768), (1, 700, 32), (1, 1000, 1000), (1, 1003, 1003), (3, 300, 520),
+    (1, 2049, 333), (1, 5003, 1250), (1, 4096, 768), (1, 20000, 64), (1, 300, 9999), (5, 1111, 96), (1, 3072, 4096), (2, 40, 24), (1, 9000, 8), (1, 40000, 301),
+]
+DTYPES = [torch.float32, torch.bfloat16, torch.float16, torch.float64, torch.int32]
+
+
+def drawn(shape, dtype, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    if dtype == torch.int32:
+        return torch.randint(-1000, 1000, shape, generator=g, device="cuda", dtype=torch.int32)
+    return torch.randn(shape, generator=g, device="cuda", dtype=torch.float64).to(dtype)
+
+
+@pytest.mark.parametrize("dtype", DTYPES, ids=lambda d: str(d)[6:])
+@pytest.mark.parametrize("shape", SHAPES, ids=lambda s: "x".join(map(str, s)))
+def test_columns(tq, shape, dtype):
+    """Sums within the rounding of a tree with chains of up to 60 additions (2^-24 each, 2^-53 for f64) and of the result; the others exact."""
+    outer, reduce, inner = shape
+    for off in (0, 1):       # and a base between vectors
+        x = drawn((outer * reduce * inner + off,), dtype, reduce + inner)[off:].view(shape)
+        wide = x.double()
+        unit = {torch.float32: 2.0**-24, torch.bfloat16: 2.0**-8, torch.float16: 2.0**-11, torch.float64: 2.0**-53, torch.int32: 0.0}[dtype]
+        bound = 60 * (2.0**-53 if dtype == torch.float64 else 2.0**-24) * wide.abs().sum(1) * (dtype != torch.int32)
+        total = wide.sum(1)
+        assert ((tq.sum(x, 1).double() - total).abs() <= bound + unit * total.abs()).all()
+        if dtype != torch.int32:
+            assert ((tq.mean(x, 1).double() - total / reduce).abs() <= bound / reduce + 2 * unit * total.abs() / reduce + 2.0**-24).all()
+        assert torch.equal(tq.amax(x, 1), x.amax(1)) and torch.equal(tq.amin(x, 1), x.amin(1))
+        best = x.max(1, keepdim=True).values
+        first = torch.where(x == best, torch.arange(reduce, device="cuda").view(1, -1, 1), reduce).amin(1)      # the lowest index of the largest value
+        assert torch.equal(tq.argmax(x, 1), first)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16], ids=["f32", "bf16"])
+@pytest.mark.parametrize("shape", [(64, 2048), (512, 768), (700, 32), (1000, 1000), (5184, 1000), (3072, 4096), (16384, 1024), (20000, 64)], ids=str)
+def test_rows_of_a_transposed_view(tq, shape, dtype):
+    x = drawn(shape, dtype, 7)
+    w, b = drawn(shape[:1], dtype, 8), drawn(shape[:1], dtype, 9)
+    wide = x.t().double()
+    exact = torch.softmax(wide, -1)
+    got = tq.softmax(x.t(), -1).double()
+    rel = 2e-6 if dtype == torch.float32 else 2.0**-8 + 2e-6      # f32: ex2, the sum and a product, a few 2^-24 each
+    assert ((got - exact).abs() <= rel * exact).all()
+    exact = torch.nn.functional.layer_norm(wide, [shape[0]], w.double(), b.double(), 1e-5)
+    got = tq.layer_norm(x.t(), [shape[0]], w, b, 1e-5).double()
+    assert ((got - exact).abs() <= rel * exact.abs() + 4e-6 * (1 + exact.abs().max())).all()
+
+
+@pytest.mark.parametrize("shape", [(64, 2048), (512, 768), (3072, 4096), (700, 32)], ids=str)
+def test_special_values_in_columns(tq, shape):
+    rows, cols = shape
+    x = drawn(shape, torch.float32, 11)
+    x[rows - 1, 0] = float("nan")
+    x[rows // 2, 1] = float("inf")
+    x[:, 2] = float("-inf")
+    x[0, 3] = float("-inf")
+    x[:, 4] = torch.finfo(torch.float32).min
+    assert torch.equal(tq.amax(x, 0).isnan(), x.amax(0).isnan()) and torch.equal(tq.amax(x, 0)[1:], x.amax(0)[1:])
+    arg = tq.argmax(x, 0)
+    assert arg[0] == rows - 1 and arg[1] == rows // 2 and arg[2] == 0 and arg[4] == 0
+    sums = tq.sum(x, 0)
+    assert sums[0].isnan() and sums[1] == float("inf") and sums[2] == float("-inf") and sums[3] == float("-inf")
+    soft, exact = tq.softmax(x.t(), -1), torch.softmax(x.t().double(), -1)
+    assert torch.equal(soft.isnan(), exact.isnan())
+    keep = ~exact.isnan().any(1)
+    assert ((soft.double() - exact).abs()[keep] <= 2e-6 * exact[keep]).all()
