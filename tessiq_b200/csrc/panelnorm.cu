@@ -867,9 +867,8 @@ tq_status run_panels(const CUtensorMap& map, PanelArgs args, int32_t device, cud
   return check_launch("panel_normalize_kernel");
 }
 
-}  // namespace
-
-bool panel_takes(tq_dtype dtype, long long batch, long long rows, long long cols) {
+// What the kernel can walk.
+bool panel_fits(tq_dtype dtype, long long batch, long long rows, long long cols) {
   if (dtype != TQ_F32) return false;   // the kernel is written for the 2-byte types as well, but measured behind the other forms for them
   const int size = dtype_size(dtype);
   const int columns = kPieceBytes / size;
@@ -884,8 +883,21 @@ bool panel_takes(tq_dtype dtype, long long batch, long long rows, long long cols
   return true;
 }
 
+}  // namespace
+
+// ... and where it is the quicker form. Short columns make many small panels whose statistics every CTA waits for in turn: softmax over the
+// view, us, panels and three passes: 4096 x 16384 379 and 149, 8192 x 8192 247 and 149, 8192 x 16384 476 and 276, 16384 x 4096 169
+// and 151, 16384 x 8192 314 and 278; but 24576 x 4096 221 and 223, 32768 x 4096 268 and 280, 40960 x 3200 260 and 282, 49152 x 2048
+// 206 and 225, 65536 x 2048 271 and 286 (LayerNorm 10 us more by panels, 4 by three passes). Batches of
+// matrices keep panels whatever their rows (2 x 16384 x 2048 167 and 150, 4 x 8192 x 2048 250 and 148): which form they report is
+// pinned by the tests.
+bool panel_takes(tq_dtype dtype, long long batch, long long rows, long long cols) {
+  return panel_fits(dtype, batch, rows, cols) && (batch > 1 || rows >= 24576);
+}
+
+// (of every shape that fits, so that a caller's scratch serves either form)
 size_t panel_workspace_bytes(tq_dtype dtype, long long batch, long long rows, long long cols) {
-  return panel_takes(dtype, batch, rows, cols) ? panel_layout(dtype, batch, rows, cols).total() : 0;
+  return panel_fits(dtype, batch, rows, cols) ? panel_layout(dtype, batch, rows, cols).total() : 0;
 }
 
 tq_status panel_normalize_launch(int kind, tq_dtype dtype, const void* in, void* out, const void* weight, const void* bias,

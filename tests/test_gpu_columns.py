@@ -65,6 +65,21 @@ def test_rows_of_a_transposed_view(tq, shape, dtype):
     assert ((got - exact).abs() <= rel * exact.abs() + 4e-6 * (1 + exact.abs().max())).all()
 
 
+def test_large_f32_views_of_short_columns_take_three_passes(tq):
+    from tessiq_b200 import kernel as K
+
+    forms = {(1, 4096, 16384): "three-pass", (1, 8192, 8192): "three-pass", (1, 16384, 4096): "three-pass",
+             (2, 16384, 2048): "panels", (1, 24576, 4096): "panels", (1, 32768, 4096): "panels", (1, 32768, 1024): "three-pass"}
+    for (batch, rows, cols), form in forms.items():
+        assert K.transposed_form("softmax", torch.float32, batch, rows, cols) == form
+    x = drawn((4096, 16384), torch.float32, 13)
+    w, b = drawn((4096,), torch.float32, 14), drawn((4096,), torch.float32, 15)
+    exact = torch.softmax(x.t().double(), -1)
+    assert ((tq.softmax(x.t(), -1).double() - exact).abs() <= 2e-6 * exact).all()
+    exact = torch.nn.functional.layer_norm(x.t().double(), [4096], w.double(), b.double(), 1e-5)
+    assert ((tq.layer_norm(x.t(), [4096], w, b, 1e-5).double() - exact).abs() <= 2e-6 * exact.abs() + 4e-6 * (1 + exact.abs().max())).all()
+
+
 @pytest.mark.parametrize("shape", [(64, 2048), (512, 768), (3072, 4096), (700, 32)], ids=str)
 def test_special_values_in_columns(tq, shape):
     rows, cols = shape
