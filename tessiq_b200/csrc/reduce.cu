@@ -1217,6 +1217,7 @@ Plan plan(tq_reduce_op op, tq_dtype dtype, long long outer, long long reduce, lo
     // ... or argmax of four-byte elements two columns a load (or a row within one tile) over 60 to 300 MB, where the plain
     // form's waves fill (us, plain and ragged: 40000 x 502 f32 36.6 and 40.5, 160000 x 98 41.8 and 51.8; but 40000 x 370 .8, 10000 x 1002
     // .78, 2000 x 1250 .39 of the plain form's time, 40000 x 2002 .99, 32768 x 4098 .93).
+    // (Both measured with tickets. The one-cluster form below takes either kind of load as it is chosen here.)
     const bool plain_fills = op == TQ_ARGMAX && size == 4 && elements >= 15500000 && elements < 75000000 && (vec >= 2 || inner <= 31 * whole);
     p.ragged = may_be_ragged && vec < whole && (size == 2 || size == 4) && op < kOpSoftmaxStat && inner >= 12 * whole && reduce < (1ll << 31) && !small &&
                !plain_fills;
