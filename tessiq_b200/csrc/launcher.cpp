@@ -330,6 +330,11 @@ PyObject* keep(PyObject*, PyObject* args) {
   if (!int_list(ints, plan->ints)) return nullptr;
   for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(doubles); ++i) plan->doubles.push_back(PyFloat_AsDouble(PyTuple_GET_ITEM(doubles, i)));
   if (PyErr_Occurred()) return nullptr;
+  // Behind the operands that `launch` reads come numbers, whose values the key holds, unless a number came as a tensor: the long way
+  // read its value, of which the key has nothing.
+  const Py_ssize_t operands_of[] = {kMostOperands, 1, 1, 1, 3, plan->ints.size() > 0 && plan->ints[0] == 0 ? 1 : 3, 5, 4, 3};
+  for (Py_ssize_t i = operands_of[family]; i < PyTuple_GET_SIZE(operands); ++i)
+    if (THPVariable_Check(PyTuple_GET_ITEM(operands, i))) Py_RETURN_FALSE;
   // what `launch` reads of each family
   const size_t least[] = {2, 6, 2, 5, 4, 6, 5, 12, 19};
   const bool has_double = family == kLayerNorm || family == kTransposed || family == kBatchNorm || family == kAttention;

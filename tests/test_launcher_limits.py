@@ -1,0 +1,47 @@
+"""What a plan of the native launcher (csrc/launcher.cpp) does not stand for, and what it leaves behind."""
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def tq():
+    if not torch.cuda.is_available():
+        pytest.fail("the gpu tests need a CUDA device")
+    from tessiq_b200 import ops
+
+    return ops
+
+
+def drawn(shape, seed, dtype=torch.float32):
+    return torch.randn(shape, generator=torch.Generator(device="cuda").manual_seed(seed), device="cuda").to(dtype)
+
+
+def on_device(value):
+    return torch.tensor(value, device="cuda")
+
+
+# ---- numbers that come as tensors: their values are no part of a signature ----------------------
+
+
+@pytest.mark.parametrize("name", ["layer_norm", "layer_norm of a view", "native_layer_norm", "batch_norm", "attention", "softmax", "argmax", "sum"])
+def test_a_number_given_as_a_tensor_is_read_on_every_call(tq, name):
+    x, w = drawn((48, 64), 1), drawn((64,), 2)
+    q = drawn((1, 2, 32, 64), 3, torch.bfloat16)
+    call, values = {
+        "layer_norm": (lambda eps: tq.layer_norm(x, [64], w, w, eps), (1e-5, 3.0)),
+        "layer_norm of a view": (lambda eps: tq.layer_norm(x.t(), [48], None, None, eps), (1e-5, 3.0)),
+        "native_layer_norm": (lambda eps: tq.native_layer_norm(x, [64], w, w, eps)[0], (1e-5, 3.0)),
+        "batch_norm": (lambda eps: tq.batch_norm_eval(x, w, w, w, w.abs(), eps), (1e-5, 3.0)),
+        "attention": (lambda scale: tq.attention(q, q, q, scale, False), (0.125, 1.0)),
+        "softmax": (lambda half_to_float: tq.softmax(x.bfloat16(), -1, half_to_float), (False, True)),
+        "argmax": (lambda dim: tq.argmax(x, dim), (0, 1)),
+        "sum": (lambda keepdim: tq.sum(x, 0, keepdim), (False, True)),
+    }[name]
+    expected = [call(value) for value in values]
+    for _ in range(2):
+        for value, right in zip(values, expected):
+            got = call(on_device(value))
+            assert got.dtype == right.dtype and torch.equal(got, right)
