@@ -20,6 +20,7 @@
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
 #include <c10/cuda/CUDAStream.h>
+#include <c10/util/strides.h>
 
 #include <dlfcn.h>
 
@@ -57,7 +58,7 @@ bool find_entry(void* handle, const char* name, Function& entry) {
 struct Output {
   std::vector<int64_t> sizes, strides;
   at::ScalarType dtype;
-  bool packed;
+  bool packed;      // the strides are those of `empty`
 };
 
 struct Plan {
@@ -346,7 +347,10 @@ PyObject* keep(PyObject*, PyObject* args) {
     if (!THPVariable_Check(o)) Py_RETURN_FALSE;
     const at::Tensor& t = THPVariable_Unpack(o);
     if (!t.is_cuda() || t.get_device() != call.device) Py_RETURN_FALSE;
-    plan->outputs.push_back(Output{t.sizes().vec(), t.strides().vec(), t.scalar_type(), t.is_contiguous()});
+    // (contiguous tensors may have any stride along an axis of one element, and later results have the first one's)
+    Output output{t.sizes().vec(), t.strides().vec(), t.scalar_type(), false};
+    output.packed = c10::IntArrayRef(output.strides) == c10::IntArrayRef(c10::contiguous_strides(t.sizes()));
+    plan->outputs.push_back(std::move(output));
   }
   if (plan->outputs.empty()) Py_RETURN_FALSE;
   if (family == kFused) plan->ints.push_back(1);      // (never without a divisor to point at)

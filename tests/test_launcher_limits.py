@@ -45,3 +45,14 @@ def test_a_number_given_as_a_tensor_is_read_on_every_call(tq, name):
         for value, right in zip(values, expected):
             got = call(on_device(value))
             assert got.dtype == right.dtype and torch.equal(got, right)
+
+# ---- results of later calls -----------------------------------------------------------------------
+
+
+def test_strides_of_later_results_are_those_of_the_first(tq):
+    wide = drawn((8, 16), 5)
+    for x in (wide[:1, :8], wide[:, :1], wide[3:4, 2:3], drawn((6, 4, 5), 6)[:, 2:3], drawn((6, 5), 7).t()):
+        first = tq.elementwise("mul", x, 2.0)
+        for _ in range(2):
+            again = tq.elementwise("mul", x, 2.0)
+            assert again.stride() == first.stride() and torch.equal(again, first)
