@@ -7,6 +7,7 @@
 #include <cstdint>
 #include <cstdio>
 #include <functional>
+#include <mutex>
 #include <string>
 
 #include "tessiq_b200.h"
@@ -64,6 +65,10 @@ class DeviceScope {
 int sm_count(int32_t device);
 
 // Checks the launch that was just queued.
+// Held while a call's operations on `scratch` (ticket words cleared, partials, statistics, the kernel that reads them) go into a
+// stream, so that two host threads that share a stream and its scratch do not mix theirs. Nothing is held for null.
+std::unique_lock<std::mutex> hold_scratch(const void* scratch);
+
 inline tq_status check_launch(const char* what) {
   cudaError_t status = cudaGetLastError();
   if (status != cudaSuccess) {

@@ -1574,6 +1574,7 @@ tq_status tq_reduce_launch(tq_reduce_op op, tq_dtype dtype, const void* in, void
              "this reduction needs %zu bytes of scratch and was given %zu", need, workspace_bytes);
   TQ_REQUIRE(need == 0 || tq::aligned_to(workspace, 16), TQ_INVALID_ARGUMENT,
              "scratch memory must be 16-byte aligned");
+  const auto held = tq::hold_scratch(p.ticket_bytes != 0 ? workspace : nullptr);
   cudaStream_t cuda_stream = static_cast<cudaStream_t>(stream);
   switch (dtype) {
     case TQ_F32: return tq::run_op<float>(op, p, in, out, outer, reduce, inner, workspace, cuda_stream);
@@ -1603,6 +1604,7 @@ tq_status tq_reduce_partial_launch(tq_reduce_op op, tq_dtype dtype, const void* 
   const size_t need = p.required;
   TQ_REQUIRE(need == 0 || (workspace != nullptr && workspace_bytes >= need && tq::aligned_to(workspace, 16)), TQ_INVALID_ARGUMENT,
              "this reduction needs %zu bytes of 16-byte-aligned scratch (tq_reduce_workspace_bytes) and was given %zu", need, workspace_bytes);
+  const auto held = tq::hold_scratch(p.ticket_bytes != 0 ? workspace : nullptr);
   cudaStream_t cuda_stream = static_cast<cudaStream_t>(stream);
 #define TQ_PARTIAL(T)                                                                                                                      \
   switch (op) {                                                                                                                            \
@@ -1642,6 +1644,7 @@ tq_status tq_reduce_launch_static(tq_reduce_op op, tq_dtype dtype, const void* i
   if (need != 0) {
     if (tq_status s = tq::static_scratch_for(device, &scratch)) return s;
   }
+  const auto held = tq::hold_scratch(scratch);
   // Partials are overwritten before they are read and the ticket words are cleared by the launch
   // itself (a memset node on `stream`), so whatever the previous call left behind does not matter.
   cudaStream_t cuda_stream = static_cast<cudaStream_t>(stream);

@@ -948,6 +948,7 @@ tq_status transposed_launch(int kind, tq_dtype dtype, const void* in, const void
   TQ_REQUIRE(workspace != nullptr && workspace_bytes >= need && tq::aligned_to(workspace, 16), TQ_INVALID_ARGUMENT,
              "this call needs %zu bytes of 16-byte-aligned scratch and was given %zu", need, workspace_bytes);
   cudaStream_t cuda_stream = static_cast<cudaStream_t>(stream);
+  const auto held = tq::hold_scratch(workspace);
   unsigned char* scratch = static_cast<unsigned char*>(workspace);
   bool handled = false;
   if (tq_status s = tq::slab_normalize_launch(kind, dtype, in, out, weight, bias, batch, rows, cols, static_cast<float>(eps), cuda_stream, &handled)) return s;

@@ -17,6 +17,12 @@ int g_sm_count[kMaxDevices] = {0};
 int32_t* g_status_word[kMaxDevices] = {nullptr};
 }  // namespace
 
+std::unique_lock<std::mutex> hold_scratch(const void* scratch) {
+  static std::mutex locks[64];      // by address: two blocks may share one, and a call holds one at a time
+  if (scratch == nullptr) return std::unique_lock<std::mutex>();
+  return std::unique_lock<std::mutex>(locks[(reinterpret_cast<uintptr_t>(scratch) >> 9) * 0x9e3779b97f4a7c15ull >> 58]);
+}
+
 void set_error(const char* text) { g_error = text ? text : ""; }
 
 tq_status fail(tq_status code, const char* format, ...) {

@@ -16,6 +16,7 @@ from __future__ import annotations
 import ctypes
 import itertools
 import math
+import threading
 from functools import lru_cache
 from typing import Sequence
 
@@ -323,6 +324,7 @@ def reduction_extents(shape: Sequence[int], first_axis: int, last_axis: int) -> 
 
 _workspaces: dict[tuple[int, int], torch.Tensor] = {}
 _outgrown: dict[tuple[int, int], list[torch.Tensor]] = {}
+_workspaces_lock = threading.Lock()
 
 
 def workspace(device: int, stream: int, nbytes: int) -> torch.Tensor | None:
@@ -331,17 +333,21 @@ def workspace(device: int, stream: int, nbytes: int) -> torch.Tensor | None:
     is replaced by one at least twice its size and KEPT: a launch still in flight on the raw stream,
     a captured CUDA graph or a recorded tq_recipe may hold its address (the library keeps pointers
     as given), and PyTorch's allocator orders reuse only against its own current stream. Doubling
-    bounds what the kept blocks hold to the size of the live one; release_workspaces() frees all."""
+    bounds what the kept blocks hold to the size of the live one; release_workspaces() frees all.
+    Threads that share a stream share its block: the library takes their calls on it one at a time."""
     if nbytes == 0:
         return None
     key = (device, stream)
     block = _workspaces.get(key)
     if block is None or block.numel() < nbytes:
-        if block is not None:
-            _outgrown.setdefault(key, []).append(block)
-        size = max(nbytes, 1 << 20, 2 * block.numel() if block is not None else 0)
-        block = torch.empty(size, dtype=torch.uint8, device=f"cuda:{device}")
-        _workspaces[key] = block
+        with _workspaces_lock:      # two threads that find no block make one
+            block = _workspaces.get(key)
+            if block is None or block.numel() < nbytes:
+                size = max(nbytes, 1 << 20, 2 * block.numel() if block is not None else 0)
+                larger = torch.empty(size, dtype=torch.uint8, device=f"cuda:{device}")
+                if block is not None:
+                    _outgrown.setdefault(key, []).append(block)
+                _workspaces[key] = block = larger
     return block
 
 
