@@ -1348,11 +1348,13 @@ tq_status run(const Plan& p, const void* in, void* out, long long outer, long lo
                  "a reduction with kept axes on both sides and %lld leading slices has no kernel", outer);
       dim3 grid(static_cast<unsigned>(p.column_tiles), p.split, static_cast<unsigned>(outer));
       auto go = [&](auto kernel, int vec) -> tq_status {
-        const size_t smem = (static_cast<size_t>(kBlock) * vec + static_cast<size_t>(p.lanes_x) * vec) * sizeof(Acc) +
-                            static_cast<size_t>(kRingDepth) * kBlock * vec * sizeof(T);
-        if (smem > 40 * 1024) {
-          TQ_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                       static_cast<int>(smem)));
+        const size_t fixed = static_cast<size_t>(kBlock) * vec * sizeof(Acc) + static_cast<size_t>(kRingDepth) * kBlock * vec * sizeof(T);
+        const size_t smem = fixed + static_cast<size_t>(p.lanes_x) * vec * sizeof(Acc);
+        // The kernel's limit is always that of its widest tile, an item a thread: another thread's launch of a narrower one does not lower it
+        // between this setting and this launch.
+        const size_t most = fixed + kBlock * sizeof(Acc);
+        if (most > 40 * 1024) {
+          TQ_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(most)));
         }
         ColumnArgs args = {};
         args.reduce = reduce;

@@ -23,7 +23,6 @@
 #include <cooperative_groups.h>
 
 #include <cstdlib>
-#include <mutex>
 
 #include "common.h"
 
@@ -252,12 +251,10 @@ __global__ void __launch_bounds__(kSlabThreads, 1) slab_normalize_kernel(SlabArg
 template <typename T, int KIND>
 tq_status slab_launch(const SlabArgs& args, long long batch, cudaStream_t stream) {
   constexpr int V = 16 / static_cast<int>(sizeof(T));
-  const size_t smem = static_cast<size_t>(args.rows_per_cta) * 32 + (kSlabWarps * 2 * V + 3 * 2 * V + 2 * V) * sizeof(float) + 128;
-  static std::mutex mutex;
-  {
-    std::lock_guard<std::mutex> lock(mutex);
-    TQ_CUDA(cudaFuncSetAttribute(slab_normalize_kernel<T, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-  }
+  constexpr size_t kRest = (kSlabWarps * 2 * V + 3 * 2 * V + 2 * V) * sizeof(float) + 128;
+  const size_t smem = static_cast<size_t>(args.rows_per_cta) * 32 + kRest;
+  // (always the limit of the longest columns: another thread's launch over shorter ones does not lower it before this one's)
+  TQ_CUDA(cudaFuncSetAttribute(slab_normalize_kernel<T, KIND>, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(kSlabMaxDataBytes + kRest)));
   const long long clusters = (args.cols / (2 * V)) * batch;
   cudaLaunchConfig_t config = {};
   config.gridDim = dim3(static_cast<unsigned>(clusters * kSlabCluster));

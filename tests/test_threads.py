@@ -74,3 +74,28 @@ def test_threads_on_one_stream(own_stream):
                     assert torch.equal(got, right)
 
     run_threads(work, count)
+
+
+@pytest.mark.gpu
+def test_threads_with_tiles_of_different_widths():
+    """One kernel, launched by threads on streams of their own with other amounts of shared memory: no launch is refused for another's."""
+    from tessiq_b200 import kernel as K
+    from tessiq_b200 import ops
+
+    shapes = {"argmax": [(1000, 8192), (3000, 64), (700, 512), (2000, 2048)], "sum": [(1000, 8192), (3000, 64), (700, 512), (2000, 2048)]}
+    data = {shape: torch.randn(shape, generator=torch.Generator(device="cuda").manual_seed(6), device="cuda").bfloat16() for shape in shapes["sum"]}
+    columns = [torch.randn(rows, 16, device="cuda").t() for rows in (8192, 12288, 32768, 49152)]      # slabs of other lengths
+    assert all(K.transposed_form("softmax", torch.float32, 1, c.shape[1], 16) == "slab" for c in columns)
+    expected = {(op, shape): getattr(ops, op)(data[shape], 0) for op in shapes for shape in data}
+    rows = [ops.softmax(c, -1) for c in columns]
+    torch.cuda.synchronize()
+
+    def work(i):
+        shape = shapes["sum"][i]
+        with torch.cuda.stream(torch.cuda.Stream()):
+            for _ in range(300):
+                for op in shapes:
+                    assert torch.equal(getattr(ops, op)(data[shape], 0), expected[op, shape])
+                assert torch.equal(ops.softmax(columns[i], -1), rows[i])
+
+    run_threads(work, 4)
