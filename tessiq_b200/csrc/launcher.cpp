@@ -16,6 +16,7 @@
 #include <torch/csrc/autograd/python_variable.h>
 #include <torch/csrc/Dtype.h>
 #include <torch/csrc/Exceptions.h>
+#include <torch/csrc/utils/object_ptr.h>
 #include <ATen/EmptyTensor.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <c10/core/impl/TorchDispatchModeTLS.h>
@@ -238,6 +239,14 @@ tq_status launch(const Plan& p, const Call& call, const std::vector<at::Tensor>&
   return TQ_INTERNAL;
 }
 
+// A new reference: the scratch tensor a plan's launch needs, or None.
+PyObject* needed(const Plan& plan, const Call& call, void* stream) {
+  const int64_t bytes = plan.family == kReduce || plan.family == kTransposed ? plan.ints[5] : 0;
+  if (bytes <= 0) Py_RETURN_NONE;
+  return PyObject_CallFunction(workspace_function, "iKL", call.device, static_cast<unsigned long long>(reinterpret_cast<uintptr_t>(stream)),
+                               static_cast<long long>(bytes));
+}
+
 PyObject* run(PyObject* const* values, Py_ssize_t count, bool by_type) {
   if (count < 2 || !PyLong_CheckExact(values[0])) Py_RETURN_NONE;
   Call call;
@@ -248,17 +257,10 @@ PyObject* run(PyObject* const* values, Py_ssize_t count, bool by_type) {
   void* const stream = c10::cuda::getCurrentCUDAStream(static_cast<c10::DeviceIndex>(call.device)).stream();
   void* scratch = nullptr;
   size_t scratch_bytes = 0;
-  PyObject* block = nullptr;       // keeps the scratch until the launch has it
-  const int64_t needs = plan->family == kReduce ? plan->ints[5] : plan->family == kTransposed ? plan->ints[5] : 0;
-  if (needs > 0) {
-    block = PyObject_CallFunction(workspace_function, "iKL", call.device, static_cast<unsigned long long>(reinterpret_cast<uintptr_t>(stream)),
-                                  static_cast<long long>(needs));
-    if (block == nullptr) return nullptr;
-    if (!THPVariable_Check(block)) {
-      Py_DECREF(block);
-      Py_RETURN_NONE;
-    }
-    const at::Tensor& t = THPVariable_Unpack(block);
+  THPObjectPtr block(needed(*plan, call, stream));      // keeps the scratch until the launch has it, or an exception (no memory) leaves
+  if (!block) return nullptr;
+  if (THPVariable_Check(block.get())) {
+    const at::Tensor& t = THPVariable_Unpack(block.get());
     scratch = t.mutable_data_ptr();
     scratch_bytes = static_cast<size_t>(t.numel());
   }
@@ -273,7 +275,6 @@ PyObject* run(PyObject* const* values, Py_ssize_t count, bool by_type) {
                              : at::detail::empty_strided_cuda(o.sizes, o.strides, o.dtype, device));
     status = launch(*plan, call, out, scratch, scratch_bytes, stream);
   }
-  Py_XDECREF(block);
   if (status != TQ_OK) Py_RETURN_NONE;
   if (out.size() == 1) return THPVariable_Wrap(std::move(out[0]));
   PyObject* tuple = PyTuple_New(static_cast<Py_ssize_t>(out.size()));

@@ -56,3 +56,31 @@ def test_strides_of_later_results_are_those_of_the_first(tq):
         for _ in range(2):
             again = tq.elementwise("mul", x, 2.0)
             assert again.stride() == first.stride() and torch.equal(again, first)
+
+
+# ---- scratch ---------------------------------------------------------------------------------------
+
+
+def test_a_failed_allocation_leaves_no_reference_to_the_scratch(tq):
+    """The result does not fit: torch's error, the scratch block as it was, and the next call works."""
+    import sys
+
+    from tessiq_b200 import kernel as K
+
+    x = drawn((2048, 4096), 8)
+    expected = tq.softmax(x.t(), -1)
+    assert torch.equal(tq.softmax(x.t(), -1), expected)
+    block = K.workspace(0, torch.cuda.current_stream().cuda_stream, 1)
+    before = sys.getrefcount(block)
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    torch.cuda.set_per_process_memory_fraction(torch.cuda.memory_reserved() / torch.cuda.get_device_properties(0).total_memory)
+    try:
+        for _ in range(3):
+            with pytest.raises(torch.OutOfMemoryError):
+                held = [tq.softmax(x.t(), -1) for _ in range(64)]      # (what the allocator has left over may serve the first ones)
+                del held
+    finally:
+        torch.cuda.set_per_process_memory_fraction(1.0)
+    assert sys.getrefcount(block) == before
+    assert torch.equal(tq.softmax(x.t(), -1), expected)
