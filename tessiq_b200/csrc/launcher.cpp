@@ -5,8 +5,8 @@
 // goes the long way through ops.py, which checks everything, picks the kernel and, once its launch has succeeded,
 // leaves a plan here (`keep`). Later calls of that signature (`call`) find the plan, allocate the result, take
 // torch's current stream and launch: 3 to 4 us where the same steps took 9 to 14 in Python, on kernels of 2 to 5.
-// A plan holds numbers only (and the compiled kernel it names), never an address or a tensor of a call; the table
-// is emptied when it is full. Whatever is not a plain CUDA tensor, runs under a dispatch mode, or fails to launch
+// A plan holds numbers only (and the compiled kernel it names), never an address or a tensor of a call; the table's
+// older half goes when it is full. Whatever is not a plain CUDA tensor, runs under a dispatch mode, or fails to launch
 // is answered with None, and the caller takes the long way, which raises what there is to raise.
 //
 // torch's headers are used for tensors, the caching allocator and streams only; the kernels are reached through the
@@ -28,6 +28,7 @@
 #include <cstring>
 #include <memory>
 #include <unordered_map>
+#include <utility>
 #include <vector>
 
 #include "tessiq_b200.h"
@@ -78,12 +79,18 @@ struct Plan {
   }
 };
 
-constexpr size_t kMostPlans = 2048;
+constexpr size_t kMostPlans = 2048;       // of both generations
 constexpr int kMostOperands = 16;
 
+// Two generations: when the younger one is full the older one goes, and a plan found in the older one joins the younger. So a program of
+// more signatures than the table holds loses those it has not used for kMostPlans / 2 others, and never all at once.
+using PlanMap = std::unordered_multimap<uint64_t, std::shared_ptr<const Plan>>;
+struct Plans {
+  PlanMap young, old;
+};
 // (never destroyed: at exit there may be no interpreter left to give the holders back to)
-std::unordered_multimap<uint64_t, std::shared_ptr<const Plan>>& plans() {
-  static auto* table = new std::unordered_multimap<uint64_t, std::shared_ptr<const Plan>>;
+Plans& plans() {
+  static auto* table = new Plans;
   return *table;
 }
 PyObject* parameter_class = nullptr;     // torch.nn.Parameter
@@ -189,10 +196,30 @@ uint64_t hash_of(const std::vector<int64_t>& key) {
 }
 
 // (a copy that shares ownership: the launch runs without the GIL, and the table may be emptied meanwhile)
+void remember(uint64_t hash, std::shared_ptr<const Plan> plan) {
+  PlanMap gone;      // (what the holders' destructors run finds the table whole)
+  Plans& table = plans();
+  if (table.young.size() >= kMostPlans / 2) {
+    gone = std::exchange(table.old, std::exchange(table.young, PlanMap()));
+  }
+  table.young.emplace(hash, std::move(plan));
+}
+
 std::shared_ptr<const Plan> find(const std::vector<int64_t>& key) {
-  const auto range = plans().equal_range(hash_of(key));
-  for (auto it = range.first; it != range.second; ++it)
-    if (it->second->key == key) return it->second;
+  const uint64_t hash = hash_of(key);
+  Plans& table = plans();
+  for (PlanMap* generation : {&table.young, &table.old}) {
+    const auto range = generation->equal_range(hash);
+    for (auto it = range.first; it != range.second; ++it) {
+      if (it->second->key != key) continue;
+      std::shared_ptr<const Plan> found = it->second;
+      if (generation == &table.old) {
+        table.old.erase(it);
+        remember(hash, found);
+      }
+      return found;
+    }
+  }
   return nullptr;
 }
 
@@ -361,14 +388,9 @@ PyObject* keep(PyObject*, PyObject* args) {
     Py_INCREF(holder);
     plan->holder = holder;
   }
-  if (plans().size() >= kMostPlans) {
-    auto old = std::move(plans());      // (what the holders' destructors run finds the table whole)
-    plans() = {};
-    old.clear();
-  }
   if (find(plan->key) == nullptr) {
-    const uint64_t h = hash_of(plan->key);
-    plans().emplace(h, std::move(plan));
+    const uint64_t hash = hash_of(plan->key);
+    remember(hash, std::move(plan));
   }
   Py_RETURN_TRUE;
   END_HANDLE_TH_ERRORS
@@ -399,7 +421,7 @@ PyObject* setup(PyObject*, PyObject* args) {
   Py_RETURN_NONE;
 }
 
-PyObject* size(PyObject*, PyObject*) { return PyLong_FromSize_t(plans().size()); }
+PyObject* size(PyObject*, PyObject*) { return PyLong_FromSize_t(plans().young.size() + plans().old.size()); }
 
 PyMethodDef methods[] = {
     {"call", reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(call_planned)), METH_FASTCALL, nullptr},

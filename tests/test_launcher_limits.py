@@ -84,3 +84,18 @@ def test_a_failed_allocation_leaves_no_reference_to_the_scratch(tq):
         torch.cuda.set_per_process_memory_fraction(1.0)
     assert sys.getrefcount(block) == before
     assert torch.equal(tq.softmax(x.t(), -1), expected)
+
+
+# ---- the table ------------------------------------------------------------------------------------
+
+
+def test_a_plan_in_use_outlasts_others(tq):
+    from tessiq_b200 import _launcher
+
+    x, hot = torch.arange(5000, device="cuda", dtype=torch.float32), drawn((3, 7), 9)
+    tq.clone(hot)
+    for n in range(1, 4800):
+        tq.clone(x[:n])
+        if n % 100 == 0:
+            assert torch.equal(_launcher.call(tq._CODES["pack"], hot), hot), n
+    assert _launcher.size() <= 2048
