@@ -178,7 +178,8 @@ enum {
                    No counterpart kernel in the reference: aten.argmax runs on its host. */
 };
 
-/* Scratch bytes `tq_reduce_launch` needs for these extents (0 when it needs none). The scratch
+/* Scratch bytes that are enough for `tq_reduce_launch` at these extents whatever the input's alignment (0
+ * when no form needs any). A launch asks for what the form it takes needs, which may be less. The scratch
  * holds per-CTA partials of slices that are split over several CTAs and a ticket counter. */
 tq_status tq_reduce_workspace_bytes(tq_reduce_op op,
                                     tq_dtype dtype,
@@ -218,9 +219,10 @@ tq_status tq_reduce_launch(tq_reduce_op op,
  * the library holds that array until the process exits, whether or not this function is called.
  * It never calls cudaMalloc, cudaFree or any allocating library routine.
  *
- *   - Extents whose scratch need (tq_reduce_workspace_bytes) exceeds TQ_STATIC_SCRATCH_BYTES are
- *     refused with TQ_RESOURCE_EXHAUSTED and a message naming both sizes; nothing is launched.
- *     Reductions that need no scratch at all are never refused for size.
+ *   - A reduction whose kernel needs more scratch than TQ_STATIC_SCRATCH_BYTES is refused with
+ *     TQ_RESOURCE_EXHAUSTED and a message naming both sizes; nothing is launched. Where
+ *     tq_reduce_workspace_bytes answers no more than that, none is refused, and a reduction whose
+ *     kernel needs no scratch is never refused for size.
  *   - The first call on each device looks up the array's device address (one host-side runtime
  *     query, no device work). Make that first call outside of any stream capture.
  *   - All calls on a device share the one array. A call clears the words it needs cleared itself,

@@ -1033,7 +1033,8 @@ struct Plan {
   size_t acc_bytes = 0;
   size_t partial_bytes = 0;   // scratch for partials (0 when one cluster covers a slice)
   size_t ticket_bytes = 0;
-  size_t required = 0;        // scratch a caller has to bring: what the forms with partials need, also where another one runs
+  size_t reported = 0;        // what the workspace query answers: the need of the form with partials, also where another one runs
+  size_t need() const { return partial_bytes + ticket_bytes; }      // what a launch of this plan uses, and asks for
   // the streaming columns kernel
   int device = 0;
   int grid = 0;               // CTAs: one per SM
@@ -1161,7 +1162,7 @@ void add_scratch(Plan& p) {
     p.partial_bytes = (p.partial_bytes + 255) / 256 * 256;
     p.ticket_bytes = (static_cast<size_t>(p.tiles) * sizeof(unsigned) + 255) / 256 * 256;
   }
-  p.required = p.partial_bytes + p.ticket_bytes;
+  p.reported = p.need();
 }
 
 Plan plan(tq_reduce_op op, tq_dtype dtype, long long outer, long long reduce, long long inner,
@@ -1263,11 +1264,11 @@ Plan plan(tq_reduce_op op, tq_dtype dtype, long long outer, long long reduce, lo
     }
     p.tiles = base_ctas;
     add_scratch(p);
-    if (may_stream) stream.required = stream.partial_bytes + stream.ticket_bytes;
+    if (may_stream) stream.reported = stream.need();
     const Plan& other = may_stream ? stream : p;
     const double others = may_stream ? stream_time(op, size, elements * size) : ticketed_time(p, op, elements * size, sms);
     if (!plan_one_cluster(whole_tiles, op, size, outer, reduce, inner, sms, others)) return other;
-    whole_tiles.required = other.required;
+    whole_tiles.reported = other.reported;
     return whole_tiles;
   }
   add_scratch(p);
@@ -1516,7 +1517,7 @@ size_t slice_stats_workspace_bytes(int kind, tq_dtype dtype, long long outer, lo
   const int op = kind == 0 ? kOpSoftmaxStat : kOpMoments;
   for (int limit = 16; limit >= dtype_size(dtype); limit /= 2) {
     const Plan p = plan(op, dtype, outer, reduce, inner, device, limit);
-    bytes = std::max(bytes, p.required);
+    bytes = std::max(bytes, p.reported);
   }
   return bytes;
 }
@@ -1526,7 +1527,7 @@ tq_status slice_stats_launch(int kind, tq_dtype dtype, const void* in, void* sta
   const int op = kind == 0 ? kOpSoftmaxStat : kOpMoments;
   const int size = dtype_size(dtype);
   const Plan p = plan(op, dtype, outer, reduce, inner, device, inner == 1 ? 16 : column_vec_bytes(in, inner, size));
-  const size_t need = p.required;
+  const size_t need = p.need();
   TQ_REQUIRE(need == 0 || (workspace != nullptr && workspace_bytes >= need && aligned_to(workspace, 16)), TQ_INVALID_ARGUMENT,
              "the statistics pass needs %zu bytes of 16-byte-aligned scratch and was given %zu", need, workspace_bytes);
   switch (dtype) {
@@ -1548,10 +1549,11 @@ tq_status tq_reduce_workspace_bytes(tq_reduce_op op, tq_dtype dtype, int64_t out
   *bytes = 0;
   if (outer == 0 || inner == 0) return TQ_OK;
   // The input's alignment is unknown here and decides the vector width of the columns kernel,
-  // which changes its tiling: answer with the largest need over the widths it may pick.
+  // which changes its tiling: answer with the largest need over the widths it may pick. (An answer that does not change
+  // with the rule that picks between the forms: where one cluster takes a tile of columns whole, a launch needs none of it.)
   for (int limit = 16; limit >= tq::dtype_size(dtype); limit /= 2) {
     tq::Plan p = tq::plan(op, dtype, outer, reduce, inner, device, limit);
-    *bytes = std::max(*bytes, p.required);
+    *bytes = std::max(*bytes, p.reported);
   }
   return TQ_OK;
 }
@@ -1571,7 +1573,7 @@ tq_status tq_reduce_launch(tq_reduce_op op, tq_dtype dtype, const void* in, void
   if (tq_status s = device_scope.status()) return s;
   tq::Plan p = tq::plan(op, dtype, outer, reduce, inner, device,
                         inner == 1 ? 16 : tq::column_vec_bytes(in, inner, size));
-  const size_t need = p.required;
+  const size_t need = p.need();
   TQ_REQUIRE(need == 0 || (workspace != nullptr && workspace_bytes >= need), TQ_INVALID_ARGUMENT,
              "this reduction needs %zu bytes of scratch and was given %zu", need, workspace_bytes);
   TQ_REQUIRE(need == 0 || tq::aligned_to(workspace, 16), TQ_INVALID_ARGUMENT,
@@ -1603,7 +1605,7 @@ tq_status tq_reduce_partial_launch(tq_reduce_op op, tq_dtype dtype, const void* 
   if (tq_status s = device_scope.status()) return s;
   // the plan of the plain reduction over [1, count, 1]: same kernels, same scratch, another finish
   const tq::Plan p = tq::plan(op == TQ_MEAN ? TQ_SUM : op, dtype, 1, count, 1, device, 16);
-  const size_t need = p.required;
+  const size_t need = p.need();
   TQ_REQUIRE(need == 0 || (workspace != nullptr && workspace_bytes >= need && tq::aligned_to(workspace, 16)), TQ_INVALID_ARGUMENT,
              "this reduction needs %zu bytes of 16-byte-aligned scratch (tq_reduce_workspace_bytes) and was given %zu", need, workspace_bytes);
   const auto held = tq::hold_scratch(p.ticket_bytes != 0 ? workspace : nullptr);
@@ -1636,8 +1638,8 @@ tq_status tq_reduce_launch_static(tq_reduce_op op, tq_dtype dtype, const void* i
   if (tq_status s = device_scope.status()) return s;
   const int limit = inner == 1 ? 16 : tq::column_vec_bytes(in, inner, size);
   tq::Plan p = tq::plan(op, dtype, outer, reduce, inner, device, limit);
-  if (p.required > tq::kStaticScratchBytes) p = tq::plan(op, dtype, outer, reduce, inner, device, limit, false);
-  const size_t need = p.required;
+  if (p.need() > tq::kStaticScratchBytes) p = tq::plan(op, dtype, outer, reduce, inner, device, limit, false);
+  const size_t need = p.need();
   TQ_REQUIRE(need <= tq::kStaticScratchBytes, TQ_RESOURCE_EXHAUSTED,
              "this reduction needs %zu bytes of scratch; the built-in scratch of tq_reduce_launch_static holds %zu. "
              "Use tq_reduce_launch with caller-provided scratch for extents this large",
