@@ -1110,6 +1110,7 @@ bool plan_one_cluster(Plan& p, tq_reduce_op op, int size, long long outer, long 
   const bool statistic = op >= kOpSoftmaxStat, heavy = op == TQ_ARGMAX || op == kOpMoments;       // accumulators of 16 bytes
   if ((op == TQ_ARGMAX || statistic) && bytes >= (200ll << 20)) return false;
   if (reduce >= (1ll << 31)) return false;              // the ring counts a thread's rows in 32 bits
+  if (outer > 65535) return false;                      // planes of a grid; the streaming kernel has no such limit
   double best = 0.95 * others;
   bool found = false;
   for (int lanes = p.ragged || p.vec > kBlock / 64 ? 32 : 64; lanes >= 2; lanes /= 2) {
