@@ -479,8 +479,11 @@ __device__ __forceinline__ typename R::Acc fold_tree(const typename R::Acc* from
   }
 }
 
+// Five CTAs an SM, four where the state needs the registers: accumulators of 16 bytes, and f64 sums by plain loads, whose four rows in flight
+// and their sum did not fit 48 registers any more (us with five and four: 3158 x 464 of 32 slices 108 and 57.5, 62403 x 1415 293 and
+// 196, 50 x 16168 of 32 49.5 and 37.4; f64 extremes over 32768 x 2048, in more CTAs than run at once by fours, 115 and 129).
 template <typename T, typename R, int VEC, bool RING, bool RAGGED = false>
-__global__ void __launch_bounds__(kBlock, sizeof(typename R::Acc) > 8 ? 4 : 5)
+__global__ void __launch_bounds__(kBlock, sizeof(typename R::Acc) > 8 || (std::is_same_v<R, SumReducer<double>> && !RING) ? 4 : 5)
 reduce_columns(const T* __restrict__ in, typename R::Out* __restrict__ out, const ColumnArgs args,
                typename R::Acc* __restrict__ partials, unsigned* __restrict__ tickets) {
   using Acc = typename R::Acc;
