@@ -18,6 +18,7 @@
 #include <cooperative_groups.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstdlib>
 #include <limits>
 #include <mutex>
@@ -1086,15 +1087,30 @@ int log2_of(int power) {
   return shift;
 }
 
-// Expected times, us, of a column reduction over `bytes` by the streaming kernel, and by clusters that meet over tickets (the
-// clearing of the tickets, partials in memory and the last CTA's fold are the fixed part; more for accumulators of 16
-// bytes and where rows start between vectors). Kernel times of [5184 x 1000] f16, [3072 x 4096], [16384 x 1024], [131072 x 128] f32,
-// [40000 x 300], [262144 x 128] bf16 sums by tickets: 12.4, 16.3, 19.9, 23.1, 18.6, 30.9. (With plain loads and all CTAs in one wave of five an
-// SM HBM is reached in the end: 32768 x 4096 f32 86; 16384 x 8192, whose 768 CTAs are more, 108.)
+// Expected times, us, of a column reduction over `bytes` by the streaming kernel, and in the shape that the reduction's split gives it: fits to
+// measured times, no bounds (part of a tensor is in L2 when a program calls, so that their rates may pass that of HBM).
+//
+// By clusters that meet over tickets the clearing of the tickets, partials in memory and the last CTA's fold are the fixed part; more for
+// accumulators of 16 bytes and where rows start between vectors. Kernel times of [5184 x 1000] f16, [3072 x 4096], [16384 x 1024],
+// [131072 x 128] f32, [40000 x 300], [262144 x 128] bf16 sums by tickets: 12.4, 16.3, 19.9, 23.1, 18.6, 30.9. (With plain loads and all CTAs
+// in one wave of five an SM HBM is reached in the end: 32768 x 4096 f32 86; 16384 x 8192, whose 768 CTAs are more, 108.) f64 takes longer
+// (us, so and by one-cluster tiles: 32768 x 2048 sum 113 and 86, extreme 115 and 86; sum 7977 x 424 of 32 slices 190 and 148, 62403 x 1415 196 and
+// 123, 6749 x 5879 95 and 62); only of a few rows plain loads are as quick (35 x 69685 of two slices 13.4 and 18.8).
+//
+// Where one cluster covers a tile by itself there are no tickets to pay for, and from some size on that tells: plain loads of 16 bytes run near
+// HBM's rate, less a third of what a last wave leaves idle (us of the split and of one-cluster tiles: 1060 x 44716 f32 30 and 36, 3897 x 29600
+// 70 and 77, 2 x 6431 x 11176 90 and 103, 237 x 30096 of two slices 12.2 and 14; i32 sums, added up in 64 bits, 1494 x 17040 of two 40 and 39).
 double stream_time(tq_reduce_op op, int size, long long bytes) { return 8.0 + bytes / 6.0e6 + (op == TQ_ARGMAX && size == 2 ? 6.0 : 0.0); }
-double ticketed_time(const Plan& p, tq_reduce_op op, long long bytes, int sms) {
-  if (!p.ring && p.tiles * p.split <= 5ll * sms) return std::min(9.0 + bytes / 5.2e6, 14.0 + bytes / 7.4e6);
-  return 9.0 + bytes / 5.2e6 + (op == TQ_ARGMAX || op == kOpMoments ? 8.0 : 0.0) + (p.ragged ? 4.0 : 0.0);
+double split_time(const Plan& p, tq_reduce_op op, tq_dtype dtype, long long reduce, long long bytes, int sms) {
+  const bool light = op != TQ_ARGMAX && op < kOpSoftmaxStat, tickets = p.split > p.cluster;
+  const bool whole_loads = p.vec * dtype_size(dtype) == 16;
+  if (light && dtype == TQ_F64 && (tickets || (bytes >= 30000000 && reduce >= 80))) return 9.0 + bytes / (whole_loads ? 3.5e6 : 2.5e6);
+  const double ticketed = !p.ring && p.tiles * p.split <= 5ll * sms
+                              ? std::min(9.0 + bytes / 5.2e6, 14.0 + bytes / 7.4e6)
+                              : 9.0 + bytes / 5.2e6 + (light || op == kOpSoftmaxStat ? 0.0 : 8.0) + (p.ragged ? 4.0 : 0.0);
+  if (!light || tickets || p.ring || !whole_loads || dtype_size(dtype) != 4 || (op == TQ_SUM && dtype == TQ_I32) || bytes < 120000000) return ticketed;
+  const double waves = static_cast<double>(p.tiles) * p.split / (5.0 * sms);
+  return std::min(ticketed, 3.0 + bytes / 7.0e6 * (waves > 1.0 ? 1.0 + 0.35 * (std::ceil(waves) - waves) / waves : 1.0));
 }
 
 // Whether one cluster (or one CTA) takes a tile of columns whole: no partials, no tickets, nothing to clear. The tile's width (lanes) and
@@ -1270,7 +1286,7 @@ Plan plan(tq_reduce_op op, tq_dtype dtype, long long outer, long long reduce, lo
     add_scratch(p);
     if (may_stream) stream.reported = stream.need();
     const Plan& other = may_stream ? stream : p;
-    const double others = may_stream ? stream_time(op, size, elements * size) : ticketed_time(p, op, elements * size, sms);
+    const double others = may_stream ? stream_time(op, size, elements * size) : split_time(p, op, dtype, reduce, elements * size, sms);
     if (!plan_one_cluster(whole_tiles, op, size, outer, reduce, inner, sms, others)) return other;
     whole_tiles.reported = other.reported;
     return whole_tiles;
