@@ -636,10 +636,11 @@ class GemmKernel(Kernel):
         bias = inputs[2] if self.has_bias else None
         residual = inputs[-1] if self.has_residual else None
         device = _device_of([t for t in (a, b, bias, residual, out) if t is not None])
-        dtype, lda, trans_a, ldb, trans_b, m, n, k, batch, stride_a, stride_b = self.plan(inputs, out)
+        dtype, lda, trans_a, ldb, trans_b, m, n, k, batch, stride_a, stride_b = plan = self.plan(inputs, out)
         check(lib.tq_gemm_bias_act_residual_launch(dtype, self.activation, a.data_ptr(), lda, trans_a, b.data_ptr(), ldb, trans_b,
                                                    _pointer(bias), _pointer(residual), n, m * n, out.data_ptr(), n, m, n, k,
                                                    batch, stride_a, stride_b, m * n, device, _stream(stream, device)))
+        return plan
 
     def plan(self, inputs, out):
         """(type, leading dimensions and transpositions of a and b, m, n, k, batch, their batch strides) of a launch."""
@@ -713,9 +714,10 @@ class AttentionKernel(Kernel):
         self._check_count(inputs)
         q, k, v = inputs
         device = _device_of([q, k, v, out])
-        dtype, extents = self.plan(q, k, v, out)
+        dtype, extents = plan = self.plan(q, k, v, out)
         check(lib.tq_attention_launch(dtype, q.data_ptr(), k.data_ptr(), v.data_ptr(), out.data_ptr(), *extents, self.scale, int(self.causal), device,
                                       _stream(stream, device)))
+        return plan
 
     def plan(self, q, k, v, out):
         """(type, extents and strides) of a launch."""

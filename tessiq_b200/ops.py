@@ -488,8 +488,7 @@ def _gemm(a, b, bias, activation, residual=None):
     kernel = _gemm_kernel(activation, has_bias=bias is not None, has_residual=residual is not None)
     try:
         operands = [t for t in (a, b, bias, residual) if t is not None]
-        kernel.launch(operands, out, stream=None)
-        dtype, *extents = kernel.plan(operands, out)
+        dtype, *extents = kernel.launch(operands, out, stream=None)
         _keep_plan(False, code, (a, b, bias, residual), _GEMM, (out,), (dtype, kernel.activation, *extents), (), b"", None)
     except Declined:
         moved = [_realigned(t) for t in (a, b, bias, residual)]
@@ -554,8 +553,7 @@ def attention(q, k, v, scale=None, causal=False, token_major=True):
         out = torch.empty([batch, heads, tokens, width], dtype=q.dtype, device=q.device)
     if out.numel():
         kernel = _attention_kernel(float(scale), bool(causal))
-        kernel.launch([q, k, v], out, stream=None)
-        dtype, extents = kernel.plan(q, k, v, out)
+        dtype, extents = kernel.launch([q, k, v], out, stream=None)
         _keep_plan(False, _CODES["attention"], operands, _ATTENTION, (out,),
                    (dtype, *extents[:5], *[n for strides in extents[5:] for n in strides], int(bool(causal))), (float(scale),), b"", None)
     return out
