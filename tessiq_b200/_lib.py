@@ -141,6 +141,15 @@ def _load() -> ctypes.CDLL:
 lib = _load()
 
 
+def load_launcher():
+    """The module `_launcher` (csrc/launcher.cpp)."""
+    try:
+        from . import _launcher
+    except ImportError as reason:
+        raise ImportError(f"{LIBRARY_PATH.parent / '_launcher.so'} is missing or does not load ({reason}): build it with `python -m tessiq_b200.build`") from reason
+    return _launcher
+
+
 def last_error() -> str:
     return lib.tq_last_error().decode("utf-8", "replace")
 

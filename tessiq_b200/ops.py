@@ -17,11 +17,10 @@ from typing import Sequence
 
 import torch
 
-from . import _launcher
 from .kernel import (DTYPE_NAMES, REDUCE_OPS, AttentionKernel, FusedKernel, GemmKernel, LayerNormKernel, PackKernel, SoftmaxKernel, _device_of,
                      _pointer, _stream, broadcast_shape, check_status, classify_read, dtype_code, launch_reduce, launch_transposed,
                      prefers_transposed, reduce_workspace_bytes, transposed_workspace_bytes, workspace)
-from ._lib import LIBRARY_PATH, Declined, check, lib
+from ._lib import LIBRARY_PATH, Declined, check, lib, load_launcher
 
 UNARY = {"abs", "neg", "relu", "sigmoid", "sqrt", "tanh", "exp", "expm1", "log", "log1p", "log2", "log10", "rsqrt",
          "reciprocal", "sin", "cos", "tan", "asin", "acos", "atan", "sinh", "cosh", "floor", "ceil", "trunc", "round",
@@ -43,6 +42,7 @@ _gemm_kernel, _attention_kernel = lru_cache(maxsize=64)(GemmKernel), lru_cache(m
 
 # Repeated calls (csrc/launcher.cpp): every entry point asks the launcher first, which answers None for a signature it has no
 # plan for; the long way below it leaves one when a call was a single launch over the operands as they came.
+_launcher = load_launcher()
 _launcher.setup(torch.nn.Parameter, workspace, str(LIBRARY_PATH))
 _FUSED, _REDUCE, _PACK, _SOFTMAX, _LAYER_NORM, _TRANSPOSED, _BATCH_NORM, _GEMM, _ATTENTION = range(9)      # launcher.cpp: Family
 _call, _keep_plan = _launcher.call, _launcher.keep
