@@ -8,6 +8,7 @@ raises for the same `ErrorCode` (csrc/bindings/module.cpp:75-92).
 from __future__ import annotations
 
 import ctypes
+import sys
 from ctypes import POINTER, c_char_p, c_double, c_int32, c_int64, c_size_t, c_void_p
 from pathlib import Path
 
@@ -142,11 +143,18 @@ lib = _load()
 
 
 def load_launcher():
-    """The module `_launcher` (csrc/launcher.cpp)."""
+    """The module `_launcher` (csrc/launcher.cpp), which was built against the headers of one torch for one Python."""
+    import torch
+
+    rebuild = "build it with `python -m tessiq_b200.build`"
     try:
         from . import _launcher
     except ImportError as reason:
-        raise ImportError(f"{LIBRARY_PATH.parent / '_launcher.so'} is missing or does not load ({reason}): build it with `python -m tessiq_b200.build`") from reason
+        raise ImportError(f"{LIBRARY_PATH.parent / '_launcher.so'} is missing or does not load ({reason}): {rebuild}") from reason
+    built_for = getattr(_launcher, "BUILT_FOR", "another torch")
+    running = f"torch {torch.__version__}, Python {sys.version_info.major}.{sys.version_info.minor}"
+    if built_for != running:
+        raise ImportError(f"{_launcher.__file__} was built for {built_for}, and this is {running}: {rebuild}")
     return _launcher
 
 

@@ -89,28 +89,38 @@ def build(force: bool = False, verbose: bool = False) -> Path:
     return LIBRARY
 
 
+def launcher_is_current(built_for: str) -> bool:
+    """Whether the module is newer than its sources and was built for this torch and Python."""
+    sources = (CSRC / "launcher.cpp", ROOT / "include" / "tessiq_b200.h", Path(__file__))
+    noted = OBJECTS / "launcher.built_for"
+    return (LAUNCHER.exists() and LAUNCHER.stat().st_mtime >= max(s.stat().st_mtime for s in sources)
+            and noted.exists() and noted.read_text() == built_for)
+
+
 def build_launcher(force: bool = False, verbose: bool = False) -> Path:
-    source = CSRC / "launcher.cpp"
-    stamp = max(source.stat().st_mtime, (ROOT / "include" / "tessiq_b200.h").stat().st_mtime, Path(__file__).stat().st_mtime)
-    if not force and LAUNCHER.exists() and LAUNCHER.stat().st_mtime >= stamp:
-        return LAUNCHER
     import sysconfig
 
     import torch
 
+    built_for = f"torch {torch.__version__}, Python {sys.version_info.major}.{sys.version_info.minor}"
+    if not force and launcher_is_current(built_for):
+        return LAUNCHER
+    OBJECTS.mkdir(parents=True, exist_ok=True)
     home = Path(torch.__file__).resolve().parent
     cuda = Path(nvcc()).resolve().parent.parent
     command = [
         os.environ.get("CXX", "g++"), "-O2", "-std=c++17", "-fPIC", "-shared", "-Wall", f"-D_GLIBCXX_USE_CXX11_ABI={int(torch._C._GLIBCXX_USE_CXX11_ABI)}",
+        f'-DTQ_BUILT_FOR="{built_for}"',
         *[f"-I{path}" for path in (home / "include", home / "include" / "torch" / "csrc" / "api" / "include", cuda / "include",
                                    sysconfig.get_paths()["include"], ROOT / "include")],
-        str(source), "-o", str(LAUNCHER), f"-L{home / 'lib'}", "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-ltorch", "-lc10_cuda", "-lc10", "-ldl",
+        str(CSRC / "launcher.cpp"), "-o", str(LAUNCHER), f"-L{home / 'lib'}", "-ltorch_python", "-ltorch_cuda", "-ltorch_cpu", "-ltorch", "-lc10_cuda", "-lc10", "-ldl",
     ]
     if verbose:
         print(" ".join(command), flush=True)
     result = subprocess.run(command, capture_output=True, text=True)
     if result.returncode != 0:
         raise RuntimeError(f"building {LAUNCHER.name} failed:\n{result.stdout}\n{result.stderr}")
+    (OBJECTS / "launcher.built_for").write_text(built_for)
     return LAUNCHER
 
 

@@ -435,4 +435,12 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_launcher", nullptr, -1, methods, 
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__launcher() { return PyModule_Create(&module); }
+PyMODINIT_FUNC PyInit__launcher() {
+  PyObject* const made = PyModule_Create(&module);
+  // the torch and the Python whose headers these are, for the importer to compare
+  if (made != nullptr && PyModule_AddStringConstant(made, "BUILT_FOR", TQ_BUILT_FOR) != 0) {
+    Py_DECREF(made);
+    return nullptr;
+  }
+  return made;
+}

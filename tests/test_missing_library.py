@@ -1,4 +1,4 @@
-"""What an import says when a built file is missing."""
+"""What an import says when a built file is missing or is another torch's."""
 
 import os
 import shutil
@@ -7,6 +7,7 @@ import sys
 from pathlib import Path
 
 import pytest
+import torch
 
 PACKAGE = Path(__file__).resolve().parent.parent / "tessiq_b200"
 
@@ -28,3 +29,28 @@ def message_of_import(tmp_path, with_library):
 def test_a_missing_file_is_named_with_the_command_that_builds_it(tmp_path, with_library, missing):
     message = message_of_import(tmp_path, with_library)
     assert f"{missing} is missing" in message and "python -m tessiq_b200.build" in message
+
+
+def test_the_launcher_is_loaded_into_its_own_torch_only(monkeypatch):
+    from tessiq_b200 import _lib
+
+    assert _lib.load_launcher().BUILT_FOR.startswith(f"torch {torch.__version__}")
+    monkeypatch.setattr(torch, "__version__", "2.99.0+cu999")
+    with pytest.raises(ImportError, match="built for torch .*python -m tessiq_b200.build"):
+        _lib.load_launcher()
+
+
+def test_the_launcher_is_built_again_for_another_torch(monkeypatch, tmp_path):
+    from tessiq_b200 import build
+
+    running = f"torch {torch.__version__}, Python {sys.version_info.major}.{sys.version_info.minor}"
+    monkeypatch.setattr(build, "LAUNCHER", tmp_path / "_launcher.so")
+    monkeypatch.setattr(build, "OBJECTS", tmp_path)
+    assert not build.launcher_is_current(running)
+    build.LAUNCHER.touch()      # newer than every source
+    assert not build.launcher_is_current(running)
+    (tmp_path / "launcher.built_for").write_text(running)
+    assert build.launcher_is_current(running)
+    assert not build.launcher_is_current(running.replace("torch ", "torch 2.99."))
+    os.utime(build.LAUNCHER, (0, 0))
+    assert not build.launcher_is_current(running)
