@@ -99,3 +99,69 @@ def test_a_plan_in_use_outlasts_others(tq):
         if n % 100 == 0:
             assert torch.equal(_launcher.call(tq._CODES["pack"], hot), hot), n
     assert _launcher.size() <= 2048
+
+
+# ---- what takes the long way ------------------------------------------------------------------------
+
+
+class Tagged(torch.Tensor):
+    pass
+
+
+def planned(tq, x):
+    from tessiq_b200 import _launcher
+
+    return _launcher.call(tq._CODES["softmax"], x, -1, False)
+
+
+def test_only_plain_tensors_have_plans(tq):
+    from torch.utils._python_dispatch import TorchDispatchMode
+
+    class Watching(TorchDispatchMode):
+        def __torch_dispatch__(self, function, types, args=(), kwargs=None):
+            return function(*args, **(kwargs or {}))
+
+    x = drawn((9, 33), 10)
+    expected = tq.softmax(x, -1)
+    assert torch.equal(planned(tq, x), expected)
+    assert torch.equal(planned(tq, torch.nn.Parameter(x)), expected)
+    assert planned(tq, x.as_subclass(Tagged)) is None and torch.equal(tq.softmax(x.as_subclass(Tagged), -1).as_subclass(torch.Tensor), expected)
+    assert planned(tq, x.cpu()) is None and planned(tq, x.to("meta")) is None
+    with Watching():
+        assert planned(tq, x) is None and torch.equal(tq.softmax(x, -1), expected)
+    seen = []
+
+    def inside(row):
+        seen.append(planned(tq, row))
+        return row.sum()
+
+    torch.func.vmap(inside)(x.expand(2, 9, 33).contiguous())
+    torch.func.grad(inside)(x)
+    torch.func.functionalize(inside)(x)
+    assert seen == [None, None, None]
+
+
+def test_inference_mode_and_gradients(tq):
+    x = drawn((9, 35), 11)
+    with torch.inference_mode():
+        results = [tq.softmax(x, -1) for _ in range(3)]
+        assert all(r.is_inference() for r in results)
+    leaf = x.clone().requires_grad_()
+    for _ in range(3):
+        plain, of_leaf = tq.softmax(x, -1), tq.softmax(leaf, -1)
+        assert not plain.is_inference() and torch.equal(plain, results[0])
+        assert not of_leaf.requires_grad and torch.equal(of_leaf, plain)
+
+
+def test_another_alignment_of_a_shape_is_another_signature(tq):
+    for dtype in (torch.float32, torch.bfloat16):
+        data = drawn((40 * 64 + 8,), 12, dtype)
+        for _ in range(2):
+            for start in (0, 1, 2, 4, 0, 3):
+                x = data[start : start + 40 * 64].view(40, 64)
+                exact = x.double()
+                assert torch.equal(tq.clone(x), x) and torch.equal(tq.elementwise("mul", x, 2.0), x * 2)
+                rel = 2.0**-8 if dtype == torch.bfloat16 else 1e-6
+                for dim in (0, 1):
+                    assert ((tq.sum(x, dim).double() - exact.sum(dim)).abs() <= rel * exact.abs().sum(dim)).all()
+                    assert torch.equal(tq.amax(x, dim), x.amax(dim))
