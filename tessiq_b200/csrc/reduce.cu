@@ -1147,7 +1147,7 @@ bool plan_one_cluster(Plan& p, tq_reduce_op op, int size, long long outer, long 
       const double cta_bytes = static_cast<double>(rows) * piece;
       // (up to six rows a thread are two trips of plain loads, which start sooner: 512 x 768 f32 sum 2.8 and 3.1, 1000 x 1000 3.7 and 4.0)
       const bool few = rows <= 6ll * rows_at_once && size >= 4 && op != TQ_ARGMAX && !statistic && !p.ragged;
-      if (lanes > 32 && !few) break;
+      if (lanes > 32 && !few) break;      // (larger clusters of 64 lanes could be few again, and were the expected best of none of 700 shapes of 20 to 200 rows)
       const double rate = an_sm > 1 ? std::min(together, an_sm * one) : one;
       const double work = static_cast<double>(rows) / rows_at_once *
                           (op == TQ_ARGMAX ? 0.1 : op == kOpMoments ? 0.03 * an_sm : op == kOpSoftmaxStat ? (size == 2 ? 0.11 : 0.05) * std::max(an_sm, 1.7) : 0.03);
@@ -1238,7 +1238,10 @@ Plan plan(tq_reduce_op op, tq_dtype dtype, long long outer, long long reduce, lo
     // ... or argmax of four-byte elements two columns a load (or a row within one tile) over 60 to 300 MB, where the plain
     // form's waves fill (us, plain and ragged: 40000 x 502 f32 36.6 and 40.5, 160000 x 98 41.8 and 51.8; but 40000 x 370 .8, 10000 x 1002
     // .78, 2000 x 1250 .39 of the plain form's time, 40000 x 2002 .99, 32768 x 4098 .93).
-    // (Both measured with tickets. The one-cluster form below takes either kind of load as it is chosen here.)
+    // (Both measured where the split had tickets; few rows need none by either kind of load now. The one-cluster form below takes the kind
+    // that is chosen here and has not been measured with the other: 200 x 709 bf16 sum 3.2, argmax 3.4, 40000 x 502 f32 argmax 20.1,
+    // 160000 x 98 35.8. Plain loads of one two-byte column, which no ring carries, are slower there than its estimate says: 20000 x 65
+    // bf16 sum 15.0 for 8.6, with tickets 18.7.)
     const bool plain_fills = op == TQ_ARGMAX && size == 4 && elements >= 15500000 && elements < 75000000 && (vec >= 2 || inner <= 31 * whole);
     p.ragged = may_be_ragged && vec < whole && (size == 2 || size == 4) && op < kOpSoftmaxStat && inner >= 12 * whole && reduce < (1ll << 31) && !small &&
                !plain_fills;
