@@ -787,9 +787,18 @@ def _kernel_step(node: fx.Node) -> Step | None:
     return None
 
 
+def _view(value, *size):
+    """`value.view(size)`, of a packed copy where the value's strides do not allow it: the graph was traced with the strides that torch's
+    elementwise operators give (their operand's), and a fused kernel's result is packed."""
+    try:
+        return value.view(*size)
+    except RuntimeError:
+        return (ops.contiguous(value) if value.is_cuda and value.element_size() <= 8 else value.contiguous()).view(*size)
+
+
 # The tensor methods behind the commonest view operators: the same views at half the cost of a call through
 # the operator registry, of which a decoder block makes thirty.
-_VIEW_METHODS = {aten.view.default: torch.Tensor.view, aten.reshape.default: torch.Tensor.reshape, aten.permute.default: torch.Tensor.permute,
+_VIEW_METHODS = {aten.view.default: _view, aten._unsafe_view.default: _view, aten.reshape.default: torch.Tensor.reshape, aten.permute.default: torch.Tensor.permute,
                  aten.transpose.int: torch.Tensor.transpose, aten.t.default: torch.Tensor.t, aten.unsqueeze.default: torch.Tensor.unsqueeze}
 
 
