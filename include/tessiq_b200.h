@@ -193,8 +193,9 @@ tq_status tq_reduce_workspace_bytes(tq_reduce_op op,
  * (csrc/tessiq/codegen/reduction.h:69-117). Output type: the input's, except TQ_ARGMAX -> int64
  * and TQ_SUM of int32 -> int64 (torch's promotion, eager_reduction.cpp:77-89). f16/bf16 are
  * accumulated in f32. `workspace` must hold `tq_reduce_workspace_bytes` bytes of device memory
- * that no other launch in flight uses; it may be null when that size is 0. reduce == 0, or a
- * mean over an integer type, is TQ_UNSUPPORTED (reduction.cpp:110-113,148-152). */
+ * that no other launch in flight uses, except earlier ones of the same stream, whichever host thread
+ * they came from; it may be null when that size is 0. reduce == 0, or a mean over an integer type,
+ * is TQ_UNSUPPORTED (reduction.cpp:110-113,148-152). */
 tq_status tq_reduce_launch(tq_reduce_op op,
                            tq_dtype dtype,
                            const void* in,

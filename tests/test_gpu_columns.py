@@ -134,3 +134,11 @@ def test_f32_column_sums_lose_no_digits_to_long_chains(tq):
         rows = rows[0::2] + rows[1::2]
     assert units(rows[0]) > 0.7      # one chain a thread, and a tree
     assert units(tq.sum(x, 0)) <= 0.7
+
+
+@pytest.mark.parametrize("dtype, rows, cols", [(torch.float64, 79, 48000), (torch.float64, 80, 48000), (torch.float64, 80, 46800), (torch.float64, 2000, 77),
+                                               (torch.float32, 300, 100000), (torch.float32, 300, 99968), (torch.int32, 300, 100004)], ids=str)
+def test_both_sides_of_where_the_form_changes(tq, dtype, rows, cols):
+    """f64 of 80 rows and 30 MB or less, 120 MB of four-byte elements: whole numbers, whose sums are exact in any order, with ties."""
+    x = torch.randint(-9, 10, (rows, cols), generator=torch.Generator(device="cuda").manual_seed(rows), device="cuda").to(dtype)
+    assert torch.equal(tq.sum(x, 0), x.sum(0)) and torch.equal(tq.amax(x, 0), x.amax(0)) and torch.equal(tq.amin(x, 0), x.amin(0))
